@@ -19,7 +19,7 @@ CSRC = PKG / "csrc"
 OBJ = PKG / "_build"
 LIB = PKG / "lib" / "libnusif_gb300.so"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-SOURCES = ["runtime.cpp", "parameter.cpp", "discretization.cu", "solver.cu", "multigrid.cu",
+SOURCES = ["runtime.cpp", "parameter.cpp", "discretization.cu", "solver.cu", "rb_sweep.cu", "multigrid.cu",
            "solver_static.cu", "output.cu", "batch.cu", "unet.cu", "unet_tc.cu", "guess.cu"]
 
 

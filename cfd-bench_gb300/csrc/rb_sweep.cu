@@ -1,0 +1,675 @@
+// Red-black SOR, iterations 2 and on, as whole-iteration sweeps on the change
+// of p (src/solver-rb.c:50-151 semantics; the first iteration runs on p
+// itself, k_sor_pass in solver.cu).
+//
+// The scheme is linear: with P the pressure after the first iteration (whose
+// ghosts then equal the cells beside them) and p = P + d, an iteration relaxes
+// d against r0 = rhs - A P, formed once in FP64, and the residual is the
+// same. d and r0 are kept as pairs of FP32 numbers (df32.cuh; plain doubles
+// with arith fp64), so an update needs no split of binary64 operands and no
+// FP64 instruction, and its rounding scales with |d|, not |p|: the error of
+// the solve against 64 bits was measured no larger than with the residual
+// split from p in every use. At the end p = P + d in binary64. The factors
+// are folded into the constants: an update is c + D with
+//   D = -factor r = f_x (w + e) + f_y (s + n) + f_z (b + t) - omega c - factor r0,
+// and the sum of r^2 is that of D^2 over factor^2.
+//
+// Layout: d and r0 with the colours apart, [colour][k][j][t], t the pair
+// (2t, 2t+1) of a row, so a thread's loads and stores are contiguous over the
+// warp whatever colour it works on. Indices are 0-based here; the first
+// colour ((i + j + k) odd, 1-based) has an even 0-based sum.
+//
+// One kernel is one iteration, exact: it reads d, writes the other copy, so
+// no block reads what another writes. A thread owns one pair of columns and
+// marches over A.kb planes: at plane k it relaxes the pair's first-colour
+// cell of plane k and then, in the same column, the second-colour cell of
+// plane k - 1, whose neighbours are all new by then. z-neighbours and one
+// x-neighbour are in its registers; the other x- and both y-neighbours come
+// from half planes (one colour) in shared memory: eight 8-byte accesses for
+// two updates and one barrier per plane. The tile's rows are surrounded by
+// one row (and pair, where x is tiled) that only relaxes the first colour,
+// again by its owner: blocks are independent.
+//
+// Walls: the stale ghost of the reference is the wall cell's old value. d has
+// a ghost row and plane on each side; they hold the wall's cells with the
+// colours exchanged, which puts a wall cell's old value where each of its
+// neighbours looks, and so does the missing second column of an odd row's
+// last pair. In x the wall is a select.
+//
+// The stop test costs no tail: block sums of D^2 go to part_out, and every
+// block of the next iteration's kernel folds them, in one order, while its
+// first planes load, then decides alike (k_rb_fold first where there are
+// many). R_m, the carried residual after m iterations, is kept in res[m & 1]:
+// kernel n reads R_(n-2) and iteration n - 1's sums, block 0 stores R_(n-1).
+// Sums stay pairs of FP32 numbers to the end: an FP64 instruction costs a
+// warp 16 cycles of GB300's FP64 pipe, and a block-wide FP64 reduction more
+// than a plane.
+//
+// What bounds it: at 128^3 instruction issue (about 215 thread instructions per
+// cell, ring included; k_sor_pass in two launches about 520), at 64^3 half
+// issue, half the launch and its first loads (about 3 us). An iteration, two
+// launches of k_sor_pass -> one sweep: 128^3 43.6 -> 17.1 us, 64^3 16.7 -> 5.6,
+// 200 x 40 x 40 18 -> 7.4, and the error against 64 bits 1.5e-14 -> 0.97e-14,
+// 1.1e-14 -> 1.2e-15, 6.5e-13 -> 8.8e-14. One cooperative kernel for all
+// iterations, its blocks exchanging sums through L2, took 2 us more per
+// iteration than launches (two device-wide fences); letting the next kernel's
+// blocks in early took 1 us more (they double up on the idle SMs).
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+#include "df32.cuh"
+#include "nusif_internal.h"
+#include "reduce.cuh"
+#include "solver_internal.h"
+
+namespace nusif {
+namespace {
+
+constexpr int kMaxThreads = 640;
+
+template <typename V>
+struct Consts {
+  V fx, fy, fz, momega, mfactor;
+};
+
+Consts<df::f2> consts(const SorArgs &A, df::f2)
+{
+  const double f = A.factor;
+  return { df::from_double_rn(f * A.idx2), df::from_double_rn(f * A.idy2),
+           df::from_double_rn(f * A.idz2), df::from_double_rn(-f * A.diag),
+           df::from_double_rn(-f) };
+}
+Consts<double> consts(const SorArgs &A, double)
+{
+  const double f = A.factor;
+  return { f * A.idx2, f * A.idy2, f * A.idz2, -f * A.diag, -f };
+}
+
+// the change D of a cell c with the neighbours w, e, s, n, b, t; r = -factor
+// r0. CUBE: one spacing on all axes, one product instead of three.
+template <bool CUBE>
+__device__ __forceinline__ df::f2 change(const Consts<df::f2> &C, df::f2 c, df::f2 w, df::f2 e,
+    df::f2 s, df::f2 n, df::f2 b, df::f2 t, df::f2 r)
+{
+  using namespace df;
+  f2 v = fma_u(C.momega, c, r);
+  if (CUBE) {
+    v = fma_u(add_u(add_u(add_u(w, e), add_u(s, n)), add_u(b, t)), C.fx, v);
+  } else {
+    v = fma_u(add_u(w, e), C.fx, v);
+    v = fma_u(add_u(s, n), C.fy, v);
+    v = fma_u(add_u(b, t), C.fz, v);
+  }
+  return renorm(v.hi, v.lo);
+}
+template <bool CUBE>
+__device__ __forceinline__ double change(const Consts<double> &C, double c, double w, double e,
+    double s, double n, double b, double t, double r)
+{
+  double v = ::fma(C.momega, c, r);
+  v = ::fma(w + e, C.fx, v);
+  v = ::fma(s + n, C.fy, v);
+  return ::fma(b + t, C.fz, v);
+}
+__device__ __forceinline__ df::f2 moved(df::f2 c, df::f2 D) { return df::add(c, D); }
+__device__ __forceinline__ double moved(double c, double D) { return c + D; }
+__device__ __forceinline__ void add_square(df::f2 &acc, df::f2 D)
+{
+  acc = df::add_u(acc, df::mul_u(D, D));
+}
+__device__ __forceinline__ void add_square(double &acc, double D) { acc = ::fma(D, D, acc); }
+__device__ __forceinline__ df::f2 as_pair(df::f2 a) { return df::renorm(a.hi, a.lo); }
+__device__ __forceinline__ df::f2 as_pair(double a) { return df::split(a); }
+__device__ __forceinline__ df::f2 to_cell(double x, df::f2) { return df::split(x); }
+__device__ __forceinline__ double to_cell(double x, double) { return x; }
+__device__ __forceinline__ double plus(double p, df::f2 d)
+{
+  return (p + df::widen(d.hi)) + df::widen(d.lo);
+}
+__device__ __forceinline__ double plus(double p, double d) { return p + d; }
+
+struct SweepArgs {
+  int nx, ny, nz, np;  // np: pairs per row
+  int pitch;           // cells of one colour's plane: np * (ny + 2)
+  int half;            // cells of one colour's array: pitch * (nz + 4), planes -2 .. nz + 1
+  int own, halo;       // pairs a block owns per row; 1 where x is tiled
+  int rows;            // rows a block owns
+  int kb;              // planes a block owns
+  // offset of pair T of row j (-1 .. ny) of plane k (-2 .. nz + 1)
+  __host__ __device__ __forceinline__ int at(int T, int j, int k) const
+  {
+    return (k + 2) * pitch + (j + 1) * np + T;
+  }
+};
+
+__device__ __forceinline__ df::f2 warp_total(df::f2 v)
+{
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    v = df::add(v, df::f2{ __shfl_xor_sync(0xffffffffu, v.hi, o),
+                           __shfl_xor_sync(0xffffffffu, v.lo, o) });
+  return v;
+}
+
+// one warp's sum of a list of pairs, in a fixed order
+__device__ __forceinline__ df::f2 fold_pairs(const df::f2 *part, int np, int lane)
+{
+  constexpr int kAtOnce = 5;  // loads in flight
+  const float2 *list = reinterpret_cast<const float2 *>(part);
+  df::f2 v{ 0.0f, 0.0f };
+  for (int q0 = lane; q0 < np; q0 += 32 * kAtOnce) {
+    float2 x[kAtOnce];
+#pragma unroll
+    for (int u = 0; u < kAtOnce; u++) x[u] = __ldcg(list + min(q0 + 32 * u, np - 1));
+#pragma unroll
+    for (int u = 0; u < kAtOnce; u++)
+      if (q0 + 32 * u < np) v = df::add(v, df::f2{ x[u].x, x[u].y });
+  }
+  return warp_total(v);
+}
+
+__device__ __forceinline__ bool is_done(const RbState *st)
+{
+  return *reinterpret_cast<const volatile int *>(&st->s.done) != 0;
+}
+
+// the carried residual after an iteration whose D^2 sum to `sum`
+__device__ __forceinline__ double carried(const RbState *st, double before, df::f2 sum)
+{
+  return (before + df::to_double(sum) * st->inv_factor2) * st->inv_ncell;
+}
+
+// a pair's cell in one column: the new first-colour value two planes below
+// the one it is relaxed in next, and the old second-colour value one below
+template <typename V>
+struct Window {
+  V nf, o;
+};
+// what a step reads from memory: first colour of plane k, second of k + 1, and
+// r of the first colour of k and of the second of k - 1; the ring rows' outer
+// neighbour
+template <typename V>
+struct Ahead {
+  V f, s, rf, rs, e;
+};
+
+// iteration n, with the np sums of the previous one in part_in (np 0: that one
+// ran on p itself)
+template <typename V, bool CUBE>
+__global__ void __launch_bounds__(kMaxThreads) k_rb_sweep(SweepArgs A, Consts<V> C,
+    const V *d, V *dout, const V *r0, RbState *st, const df::f2 *part_in, df::f2 *part_out, int n,
+    int np)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ df::f2 sm[kMaxThreads / 32];
+  __shared__ int go_on;
+  const int pw = A.own + 2 * A.halo, nrow = A.rows + 2;
+  const int plane_n = pw * nrow, plane_o = pw * (nrow + 2);
+  // old second colour of plane k (rows j0 - 2 .. j0 + rows + 1), new first
+  // colour of plane k (one row less on each side), two planes each
+  V *const olds = reinterpret_cast<V *>(smem_raw);
+  V *const news = olds + 2 * plane_o;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const bool live = tid < plane_n;
+  const int row = min(tid / pw, nrow - 1), t = tid - (tid / pw) * pw;
+  const int T = (int)blockIdx.x * A.own + t - A.halo;  // the pair
+  const int j = (int)blockIdx.y * A.rows + row - 1;
+  const int k0 = blockIdx.z * A.kb, k1 = min(k0 + A.kb, A.nz) - 1;
+  const int nx = A.nx, ny = A.ny, nz = A.nz, pitch = A.pitch, half = A.half;
+  const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+  const bool cell_in = live && T >= 0 && T < A.np && j >= 0 && j < ny;
+  const bool own = cell_in && t >= A.halo && t < A.halo + A.own && row >= 1 && row <= A.rows;
+  const bool lower = row == 0, upper = row == nrow - 1, ring = live && (lower || upper);
+  // loads stay in the array: pairs in the row, rows up to the ghost rows
+  const int Tc = min(max(T, 0), A.np - 1);
+  const int base = A.at(Tc, min(j, ny), k0 - 1);  // plane k0 - 1
+  const int base_e = A.at(Tc, min(max(lower ? j - 1 : j + 1, -1), ny), k0 - 1) + half;
+
+  // step q = k - (k0 - 1); window X is the column relaxed in even steps
+  const int colx = (j + k0 - 1) & 1;
+  const auto wall = [&](int col) { return col == 0 ? T == 0 : 2 * T + 1 >= nx - 1; };
+  const bool wall_x = wall(colx), wall_y = wall(1 - colx);
+  const bool lone = 2 * T + 1 >= nx;  // odd nx: the last pair has no second column
+  const bool valid_x = cell_in && !(lone && colx == 1), valid_y = cell_in && !(lone && colx == 0);
+  // shared-memory offsets: own cell, and the x-neighbour outside the pair
+  const int so = (row + 1) * pw + t, sf = row * pw + t;
+  const int dl = t > 0 ? -1 : 0, dr = t < pw - 1 ? 1 : 0;
+  const int ax = colx ? dr : dl, ay = colx ? dl : dr;
+  const int s_ring = lower ? t : (nrow + 1) * pw + t;
+
+  // everything read from here on is the previous kernel's work; all of it is
+  // asked for at once
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const bool over = is_done(st);
+  int o = base;  // plane k's offset
+  Window<V> X, Y;
+  Ahead<V> a0, a1;  // of even and odd steps
+  X.o = d[base + half - pitch];
+  Y.o = d[base + half];
+  a0.f = d[base];
+  a0.s = d[base + half + pitch];
+  a0.rf = r0[base];
+  a1.f = d[base + pitch];
+  a1.s = d[base + half + 2 * pitch];
+  a1.rf = r0[base + pitch];
+  a1.rs = r0[base + half];
+  a0.rs = a1.rs;
+  a0.e = a1.e = a0.f;
+  if (ring) {
+    a0.e = d[base_e];
+    a1.e = d[base_e + pitch];
+  }
+  X.nf = Y.nf = X.o;  // not used before they are set
+  if (tid < 32) {
+    // the previous iteration's residual, and whether this one runs
+    const double before = __ldcg(&st->res[n & 1]), first = __ldcg(&st->s.res);
+    const double epssq = __ldcg(&st->s.epssq);
+    const int itermax = __ldcg(&st->s.itermax);
+    bool go = true;
+    if (np > 0) {
+      const df::f2 sum = fold_pairs(part_in, np, lane);
+      if (lane == 0) {
+        const double res = carried(st, before, sum);
+        go = res >= epssq && n - 1 < itermax;
+        if (bid == 0 && !over) {
+          st->res[(n - 1) & 1] = res;
+          if (!go) {
+            st->s.res = res;
+            st->s.it = n - 1;
+            st->s.done = 1;
+          }
+        }
+      }
+    } else if (bid == 0 && lane == 0) {
+      st->res[(n - 1) & 1] = first;
+    }
+    if (lane == 0) go_on = go && !over;
+  }
+  __syncthreads();
+  if (!go_on) return;
+
+  V acc{};
+  // P: the window relaxed in this step, Q: the other one
+  const auto step = [&](int k, Window<V> &P, Window<V> &Q, Ahead<V> &a, int buf, bool wallP,
+                        bool validP, int adj) {
+    V *const so_k = olds + buf * plane_o + so, *const nf_k = news + buf * plane_n + sf;
+    const V *const nf_m = news + (buf ^ 1) * plane_n + sf;
+    if (live) so_k[0] = Q.o;
+    if (ring) olds[buf * plane_o + s_ring] = a.e;
+    const V fc = a.f, sup = a.s, rf = a.rf, rs = a.rs;
+    if (k + 2 <= k1 + 1) {
+      a.f = d[o + 2 * pitch];
+      a.s = d[o + 3 * pitch + half];
+      a.rf = r0[o + 2 * pitch];
+      a.rs = r0[o + pitch + half];
+      if (ring) a.e = d[base_e + (o - base) + 2 * pitch];
+    }
+    __syncthreads();
+    // first colour of plane k
+    V nw = fc;
+    {
+      V x1 = so_k[adj];
+      if (wallP) x1 = fc;
+      const V D = change<CUBE>(C, fc, x1, Q.o, so_k[-pw], so_k[pw], P.o, sup, rf);
+      if (validP && k >= 0 && k < nz) {
+        nw = moved(fc, D);
+        if (own && k >= k0 && k <= k1) add_square(acc, D);
+      }
+    }
+    if (live) nf_k[0] = nw;
+    // second colour of plane k - 1, in the same column
+    if (own && k > k0) {
+      V x1 = nf_m[adj];
+      if (wallP) x1 = P.o;
+      V fv = Q.nf, m = P.o;
+      const V D = change<CUBE>(C, P.o, x1, Q.nf, nf_m[-pw], nf_m[pw], P.nf, nw, rs);
+      if (validP) {
+        m = moved(P.o, D);
+        add_square(acc, D);
+      }
+      if (lone) {  // the missing column's entry holds its neighbour's value
+        if (validP) fv = m;
+        else m = fv;
+      }
+      V *const w = dout + (o - pitch);
+      w[0] = fv;
+      w[half] = m;
+      if (j == 0) {
+        w[half - A.np] = fv;
+        w[-A.np] = m;
+      }
+      if (j == ny - 1) {
+        w[half + A.np] = fv;
+        w[A.np] = m;
+      }
+      if (k == 1) {
+        w[half - pitch] = fv;
+        w[-pitch] = m;
+      }
+      if (k == nz) {
+        w[half + pitch] = fv;
+        w[pitch] = m;
+      }
+    }
+    o += pitch;
+    P.nf = nw;
+    P.o = sup;
+  };
+  for (int k = k0 - 1; k <= k1 + 1; k += 2) {
+    step(k, X, Y, a0, 0, wall_x, valid_x, ax);
+    if (k + 1 <= k1 + 1) step(k + 1, Y, X, a1, 1, wall_y, valid_y, ay);
+  }
+  const df::f2 ws = warp_total(as_pair(acc));
+  if (lane == 0) sm[tid >> 5] = ws;
+  __syncthreads();
+  if (tid < 32) {
+    const int nw = blockDim.x >> 5;
+    const df::f2 sum = warp_total(lane < nw ? sm[lane] : df::f2{ 0.0f, 0.0f });
+    if (lane == 0) part_out[bid] = sum;
+  }
+}
+
+// after the first iteration: r = -factor (rhs - A P) in FP64, d = 0 with its
+// ghosts (one thread per entry of a colour's array)
+template <typename V>
+__global__ void __launch_bounds__(256) k_rb_open(SweepArgs A, SorArgs S, const double *__restrict__ p,
+    const double *__restrict__ rhs, V *__restrict__ d, V *__restrict__ r0, const RbState *st)
+{
+  if (is_done(st)) return;
+  const int q = blockIdx.x * 256 + threadIdx.x;
+  if (q >= A.half) return;
+  d[q] = d[q + A.half] = V();
+  const int T = q % A.np, jk = q / A.np, j = jk % (A.ny + 2) - 1, k = jk / (A.ny + 2) - 2;
+  if (j < 0 || j >= A.ny || k < 0 || k >= A.nz) return;
+  const int sj = S.g.sj, sk = S.g.sk;
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    const int i = 2 * T + e;
+    double r = 0.0;
+    if (i < A.nx) {
+      const int c = (k + 1) * sk + (j + 1) * sj + i + 1;
+      const double lap = (p[c - 1] + p[c + 1]) * S.idx2 + (p[c - sj] + p[c + sj]) * S.idy2 +
+                         (p[c - sk] + p[c + sk]) * S.idz2 - S.diag * p[c];
+      r = rhs[c] - lap;
+    }
+    r0[((i + j + k) & 1) * A.half + q] = to_cell(-S.factor * r, V());
+  }
+}
+
+// p = P + d on the cells and the six ghost faces, once the solve is over
+// (direct: the iterations that ran on p itself)
+template <typename V>
+__global__ void __launch_bounds__(256) k_rb_close(SweepArgs A, Dims g, double *__restrict__ p,
+    const V *__restrict__ d0, const V *__restrict__ d1, const RbState *st, int direct)
+{
+  if (!is_done(st) || st->s.it <= direct) return;
+  const V *d = (st->s.it & 1) ? d1 : d0;
+  const int q = blockIdx.x * 256 + threadIdx.x;
+  if (q >= A.np * A.ny * A.nz) return;
+  const int T = q % A.np, jk = q / A.np, j = jk % A.ny, k = jk / A.ny;
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    const int i = 2 * T + e;
+    if (i >= A.nx) continue;
+    double *c = p + ((k + 1) * g.sk + (j + 1) * g.sj + i + 1);
+    const double v = plus(*c, d[((i + j + k) & 1) * A.half + A.at(T, j, k)]);
+    *c = v;
+    if (i == 0) c[-1] = v;
+    if (i == A.nx - 1) c[1] = v;
+    if (j == 0) c[-g.sj] = v;
+    if (j == A.ny - 1) c[g.sj] = v;
+    if (k == 0) c[-g.sk] = v;
+    if (k == A.nz - 1) c[g.sk] = v;
+  }
+}
+
+// a long list of block sums folded once instead of by every block of the next sweep
+__global__ void __launch_bounds__(1024) k_rb_fold(const RbState *st, const df::f2 *part, int np,
+    df::f2 *out)
+{
+  if (is_done(st)) return;
+  __shared__ df::f2 sm[32];
+  const int t = threadIdx.x;
+  df::f2 v{ 0.0f, 0.0f };
+  for (int q = t; q < np; q += 1024) {
+    const float2 x = __ldcg(reinterpret_cast<const float2 *>(part) + q);
+    v = df::add(v, df::f2{ x.x, x.y });
+  }
+  v = warp_total(v);
+  if ((t & 31) == 0) sm[t >> 5] = v;
+  __syncthreads();
+  if (t >= 32) return;
+  v = warp_total(sm[t]);
+  if (t == 0) *out = v;
+}
+
+// after a chunk of sweeps that ended with iteration n: its residual, and
+// whether the solve is over (one warp)
+__global__ void k_rb_finish(RbState *st, const df::f2 *part, int n, int np)
+{
+  if (is_done(st)) return;
+  const df::f2 s = fold_pairs(part, np, threadIdx.x);
+  if (threadIdx.x == 0) {
+    const double res = carried(st, st->res[(n - 1) & 1], s);
+    st->s.res = res;
+    st->s.it = n;
+    st->s.done = !(res >= st->s.epssq && n < st->s.itermax);
+  }
+}
+
+constexpr int kFoldMax = 1024;   // block sums that each block of the next sweep folds itself
+
+int up(int a, int b) { return (a + b - 1) / b; }
+
+int sm_count()
+{
+  int dev = 0, n = 152;
+  if (cudaGetDevice(&dev) == cudaSuccess)
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n;
+}
+
+// Tile and depth of a sweep. Rows of at most kPairs pairs are whole (no ring
+// in x); longer ones are cut evenly. Rows and planes per block: the least time
+// of the busiest SM, steps x (0.20 us + 0.035 us for each warp it holds), as
+// measured at 64^3, 128^3 and 200 x 40 x 40 over 4-10 rows and 2-32 planes
+// (the 0.20 us are the two dependent updates of a step, the rest their issue;
+// a launch adds about 3 us whatever the shape).
+SweepArgs sweep_shape(int nx, int ny, int nz)
+{
+  constexpr int kPairs = 64;
+  SweepArgs a;
+  a.nx = nx;
+  a.ny = ny;
+  a.nz = nz;
+  a.np = up(nx, 2);
+  a.pitch = a.np * (ny + 2);
+  a.half = a.pitch * (nz + 4);
+  const int gx = a.np <= kPairs ? 1 : up(a.np, kPairs - 2);
+  a.own = up(a.np, gx);
+  a.halo = gx > 1 ? 1 : 0;
+  const int pw = a.own + 2 * a.halo, sms = sm_count();
+  double best = 1e300;
+  a.rows = 1;
+  a.kb = nz;
+  for (int rows = 1; rows <= 40; rows++) {
+    const int threads = up(pw * (rows + 2), 32) * 32;
+    if (threads > kMaxThreads) break;
+    for (int kb = 1; kb <= nz && kb <= 64; kb++) {
+      const int64_t blocks = (int64_t)gx * up(ny, rows) * up(nz, kb);
+      const double warps = (double)((blocks + sms - 1) / sms) * (threads / 32);
+      const double cost = (kb + 3) * (0.20 + 0.035 * warps);
+      if (cost < best) {
+        best = cost;
+        a.rows = rows;
+        a.kb = kb;
+      }
+    }
+  }
+  return a;
+}
+
+}  // namespace
+
+// what a solver keeps for its sweeps: the shape, and the device memory (two
+// copies of d, and r0; null where the grid is beyond their 32-bit offsets or
+// the memory is not to be had: then every iteration runs on p)
+struct RbPlan {
+  SweepArgs a;
+  dim3 grid;
+  int threads = 0, blocks = 0;
+  size_t smem = 0;
+  bool cube = false;  // one spacing on all axes
+  void *cells = nullptr;
+};
+
+namespace {
+
+// programmatic launch: the next sweep's blocks come in while the last of this
+// one's leave (and without it each launch took a multiple of 2.05 us)
+template <typename V>
+bool launch_sweep(const RbPlan &P, const Consts<V> &C, const V *d, V *dout, const V *r0,
+    RbState *st, const df::f2 *part_in, df::f2 *part_out, int n, int np)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = P.grid;
+  cfg.blockDim = dim3(P.threads);
+  cfg.dynamicSmemBytes = P.smem;
+  cfg.stream = stream();
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, P.cube ? k_rb_sweep<V, true> : k_rb_sweep<V, false>, P.a, C, d, dout, r0,
+      st, part_in, part_out, n, np);
+  return launched("k_rb_sweep");
+}
+
+template <typename V>
+double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, const double *rhs)
+{
+  const Dims &g = A.g;
+  const RbPlan &P = *ss->rb_plan;
+  const SweepArgs &a = P.a;
+  const bool sweeps = P.cells != nullptr;
+  const int nb = sweeps ? P.blocks : 0, nb1 = 2 * sor_blocks(A);
+  const bool folded = nb > kFoldMax;
+  // the first iteration's sums, then the sweeps' two lists and one value for each
+  if (!reduce_scratch_alloc(ss->red, nb1 > 2 * nb + 2 ? nb1 : 2 * nb + 2)) return NAN;
+  df::f2 *const lists = reinterpret_cast<df::f2 *>(ss->red.partials);
+  df::f2 *const part[2] = { lists, lists + nb };
+  df::f2 *const sum[2] = { lists + 2 * nb, lists + 2 * nb + 1 };
+  V *const cells = reinterpret_cast<V *>(P.cells);
+  V *const d[2] = { cells, cells + 2 * (size_t)a.half };
+  V *const r0 = d[1] + 2 * (size_t)a.half;
+  const Consts<V> C = consts(A, V());
+  cudaStream_t q = stream();
+  RbState *st = ss->d_rb, *h = ss->h_rb;
+  memset(h, 0, sizeof(*h));
+  h->s.res = 1.0;
+  h->s.epssq = s->eps * s->eps;
+  h->s.itermax = s->itermax;
+  h->s.ncell = (double)(g.imax * g.jmax * g.kmax);
+  h->inv_ncell = 1.0 / h->s.ncell;
+  h->inv_factor2 = 1.0 / (A.factor * A.factor);
+  h->s.done = !((h->s.res >= h->s.epssq) && (0 < h->s.itermax));
+  if (h->s.done) return h->s.res;
+  if (!cuda_ok(cudaMemcpyAsync(st, h, sizeof(RbState), cudaMemcpyHostToDevice, q),
+          "solve state upload"))
+    return NAN;
+  // the first iteration runs on p, and a second one where the last solve took
+  // no more: opening and closing the sweeps costs about one iteration on p
+  const auto on_p = [&](int count) {
+    for (int c = 0; c < count; c++)
+      if (!launch_rb_iteration(A, p, rhs, &st->s, ss->red, !ss->ext.arith_fp64)) return false;
+    return true;
+  };
+  const int direct = ss->last_iterations == 2 && s->itermax >= 2 ? 2 : 1;
+  if (!on_p(direct)) return NAN;
+  int n = direct;
+  // queue iterations in chunks; the first chunk matches the previous solve's count
+  int chunk = ss->last_iterations > 0 ? ss->last_iterations - direct : 16;
+  while (!h->s.done) {
+    if (!sweeps) {
+      const int count = chunk < s->itermax - n ? chunk : s->itermax - n;
+      if (!on_p(count)) return NAN;
+      n += count;
+    } else if (chunk > 0 && n < s->itermax) {
+      if (n == direct) {
+        k_rb_open<V><<<(unsigned)up(a.half, 256), 256, 0, q>>>(a, A, p, rhs, d[n & 1], r0, st);
+        if (!launched("k_rb_open")) return NAN;
+      }
+      for (int c = 0; c < chunk && n < s->itermax; c++) {
+        n++;
+        const int in = (n - 1) & 1, out = n & 1;
+        const bool first = n == direct + 1;
+        if (folded && !first) {
+          k_rb_fold<<<1, 1024, 0, q>>>(st, part[in], nb, sum[in]);
+          if (!launched("k_rb_fold")) return NAN;
+        }
+        if (!launch_sweep<V>(P, C, d[in], d[out], r0, st, folded ? sum[in] : part[in], part[out], n,
+                first ? 0 : folded ? 1 : nb))
+          return NAN;
+      }
+      k_rb_finish<<<1, 32, 0, q>>>(st, part[n & 1], n, nb);
+      if (!launched("k_rb_finish")) return NAN;
+      k_rb_close<V><<<(unsigned)up(a.np * a.ny * a.nz, 256), 256, 0, q>>>(a, g, p, d[0], d[1], st,
+          direct);
+      if (!launched("k_rb_close")) return NAN;
+    }
+    if (!cuda_ok(cudaMemcpyAsync(h, st, sizeof(RbState), cudaMemcpyDeviceToHost, q),
+            "solve state download"))
+      return NAN;
+    if (!cuda_ok(cudaStreamSynchronize(q), "solve sync")) return NAN;
+    chunk = ss->last_iterations > 64 ? ss->last_iterations / 8 : 8;
+  }
+  return h->s.res;
+}
+
+}  // namespace
+
+// shape and device memory of the sweeps on a grid
+bool rb_sweep_alloc(SolverState *ss, const Dims &g, bool cube)
+{
+  if (ss->rb_plan && ss->rb_plan->a.nx == g.imax && ss->rb_plan->a.ny == g.jmax &&
+      ss->rb_plan->a.nz == g.kmax && ss->rb_plan->cube == cube)
+    return true;
+  rb_sweep_free(ss);
+  RbPlan *P = ss->rb_plan = new RbPlan();
+  SweepArgs &a = P->a = sweep_shape(g.imax, g.jmax, g.kmax);
+  const int pw = a.own + 2 * a.halo;
+  P->threads = up(pw * (a.rows + 2), 32) * 32;
+  P->grid = dim3(up(a.np, a.own), up(a.ny, a.rows), up(a.nz, a.kb));
+  P->blocks = (int)(P->grid.x * P->grid.y * P->grid.z);
+  P->cube = cube;
+  P->smem = 2 * (size_t)pw * (a.rows + 2 + a.rows + 4) * 8;
+  const int64_t half = (int64_t)a.np * (a.ny + 2) * (a.nz + 4);
+  if (2 * half < ((int64_t)1 << 31) &&
+      cudaMalloc(&P->cells, 3 * 2 * (size_t)half * 8) != cudaSuccess) {
+    cudaGetLastError();
+    P->cells = nullptr;
+  }
+  return cuda_ok(cudaMalloc(&ss->d_rb, sizeof(RbState)), "cudaMalloc(rb state)") &&
+         cuda_ok(cudaMallocHost(&ss->h_rb, sizeof(RbState)), "cudaMallocHost(rb state)");
+}
+
+void rb_sweep_free(SolverState *ss)
+{
+  if (ss->d_rb) cudaFree(ss->d_rb);
+  if (ss->h_rb) cudaFreeHost(ss->h_rb);
+  ss->d_rb = ss->h_rb = nullptr;
+  if (!ss->rb_plan) return;
+  if (ss->rb_plan->cells) cudaFree(ss->rb_plan->cells);
+  delete ss->rb_plan;
+  ss->rb_plan = nullptr;
+}
+
+double rb_sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, const double *rhs)
+{
+  return ss->ext.arith_fp64 ? sweep_solve<double>(s, ss, A, p, rhs)
+                            : sweep_solve<df::f2>(s, ss, A, p, rhs);
+}
+
+}  // namespace nusif

@@ -366,36 +366,11 @@ static double solve_rb(Solver *s, SolverState *ss, double *p, const double *rhs)
   const Grid *gr = s->grid;
   const Dims g = make_dims(gr->imax, gr->jmax, gr->kmax);
   const SorArgs A = make_sor_args(g, gr->dx, gr->dy, gr->dz, s->omega);
-  const int nb = sor_blocks(A);
-  if (!reduce_scratch_alloc(ss->red, 2 * nb)) return NAN;
-  SolveState *h = ss->h_state;
-  h->res = 1.0;
-  h->it = 0;
-  h->epssq = s->eps * s->eps;
-  h->itermax = s->itermax;
-  h->ncell = (double)(gr->imax * gr->jmax * gr->kmax);
-  h->done = !((h->res >= h->epssq) && (h->it < h->itermax));
-  if (!cuda_ok(cudaMemcpyAsync(ss->d_state, h, sizeof(SolveState), cudaMemcpyHostToDevice,
-                   stream()),
-          "solve state upload"))
-    return NAN;
-  // queue iterations in chunks; the first chunk matches the previous solve's count
-  int chunk = ss->last_iterations > 0 ? ss->last_iterations : 16;
-  if (chunk > s->itermax) chunk = s->itermax;
-  while (!h->done) {
-    for (int q = 0; q < chunk; q++)
-      if (!launch_rb_iteration(A, p, rhs, ss->d_state, ss->red, !ss->ext.arith_fp64))
-        return NAN;
-    if (!cuda_ok(cudaMemcpyAsync(h, ss->d_state, sizeof(SolveState), cudaMemcpyDeviceToHost,
-                     stream()),
-            "solve state download"))
-      return NAN;
-    if (!cuda_ok(cudaStreamSynchronize(stream()), "solve sync")) return NAN;
-    chunk = ss->last_iterations > 64 ? ss->last_iterations / 8 : 8;
-  }
-  ss->last_iterations = h->it;
-  if (verbose()) printf("Solver took %d iterations to reach %f\n", h->it, sqrt(h->res));
-  return h->res;
+  if (!rb_sweep_alloc(ss, g, A.idx2 == A.idy2 && A.idy2 == A.idz2)) return NAN;
+  const double res = rb_sweep_solve(s, ss, A, p, rhs);
+  ss->last_iterations = ss->h_rb->s.it;  // 0 where the loop condition failed at once
+  if (verbose()) printf("Solver took %d iterations to reach %f\n", ss->last_iterations, sqrt(res));
+  return res;
 }
 
 // solve for kind mg-ref: the observable part of src/solver-mg.c:299-402
@@ -482,6 +457,10 @@ void initSolver(Solver *s, Discretization *d, Parameter *p)
   memset(ss->h_state, 0, sizeof(SolveState));
   if (kind == SOLVER_MG || kind == SOLVER_MG_MIXED) {
     if (!mg_setup(s, d, ss)) return;
+  } else if (kind == SOLVER_RB) {
+    const Grid &gr = d->grid;
+    if (!rb_sweep_alloc(ss, make_dims(gr.imax, gr.jmax, gr.kmax), gr.dx == gr.dy && gr.dy == gr.dz))
+      return;
   } else if (kind == SOLVER_MG_REF) {
     if (verbose()) printf("Using Multigrid solver with %d levels\n", s->levels);
   }
@@ -533,6 +512,7 @@ void nusifFreeSolver(Solver *s)
   guess_free(ss->guess);
   ss->guess = nullptr;
   mg_free(s, ss);
+  rb_sweep_free(ss);
   if (ss->d_state) cudaFree(ss->d_state);
   if (ss->h_state) cudaFreeHost(ss->h_state);
   reduce_scratch_free(ss->red);

@@ -18,6 +18,13 @@ struct SolveState {
   int pad;
 };
 
+// The same for a red-black solve by whole-iteration sweeps (rb_sweep.cu).
+struct RbState {
+  SolveState s;
+  double res[2];  // carried residual after m iterations, at m & 1
+  double inv_ncell, inv_factor2;
+};
+
 struct SorArgs {
   Dims g;
   double idx2, idy2, idz2, diag, factor;
@@ -37,6 +44,12 @@ bool launch_sor_sweep(const SorArgs &A, double *p, const double *rhs, bool ghost
 bool launch_residual_ref(const SorArgs &A, const double *p, const double *rhs, SolveState *st,
     ReduceScratch &red);
 bool launch_pressure_ghosts(const Dims &g, double *p);
+// red-black solve by whole-iteration sweeps (rb_sweep.cu)
+struct SolverState;
+// cube: one spacing on all axes
+bool rb_sweep_alloc(SolverState *ss, const Dims &g, bool cube);
+void rb_sweep_free(SolverState *ss);
+double rb_sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, const double *rhs);
 
 struct MgHierarchy;  // multigrid.cu
 
@@ -46,6 +59,9 @@ struct SolverState {
   SolveState *d_state = nullptr;
   SolveState *h_state = nullptr;  // pinned
   ReduceScratch red;
+  RbState *d_rb = nullptr;   // rb: device state of the sweeps
+  RbState *h_rb = nullptr;   // pinned
+  struct RbPlan *rb_plan = nullptr;  // rb: the sweeps' shape and device memory
   int last_iterations = 0;
   MgHierarchy *mg = nullptr;
   struct GuessState *guess = nullptr;  // learned warm start (guess.cu)
