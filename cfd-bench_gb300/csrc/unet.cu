@@ -24,9 +24,8 @@
 //    first optionally at half resolution (nearest upsampling and the concat
 //    of the decoder are never materialised). The same kernel computes input
 //    gradients with tap-flipped, transposed weights.
-//  - k_wgrad_mma: weight gradients as a GEMM over cells (M = cout, N = cin,
-//    K = cells) on the tensor cores, one block per (chunk of cells, tap),
-//    per-chunk partials folded in a fixed order (deterministic).
+//  - k_wgrad (unet_wgrad.cu): weight gradients of every layer as GEMMs over
+//    the cells on the tensor cores.
 //  - plain FP32 kernels for the 2-channel input layer and the 1-channel output
 //    layer, pooling, masks, the loss and Adam.
 #include <cuda_bf16.h>
@@ -39,6 +38,7 @@
 #include "nusif_internal.h"
 #include "unet_internal.h"
 #include "unet_tc.h"
+#include "unet_wgrad.h"
 
 namespace nusif {
 namespace {
@@ -64,13 +64,6 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t *>(&v);
-}
-
-__device__ __forceinline__ uint32_t pack_raw(bf16 lo, bf16 hi)
-{
-  const uint32_t a = *reinterpret_cast<const unsigned short *>(&lo);
-  const uint32_t b = *reinterpret_cast<const unsigned short *>(&hi);
-  return a | (b << 16);
 }
 
 // D += A(16x16, row) * B(16x8, col), BF16 inputs, FP32 accumulators
@@ -195,151 +188,6 @@ __global__ void __launch_bounds__(128) k_conv_mma(ConvArgs a)
   }
 }
 
-// ------------------------------------------------------------------ tensor-core weight gradient
-
-struct WgradArgs {
-  ConvSrc s0, s1;  // the layer's input, as in the forward pass
-  const bf16 *g;   // masked output gradient [cells][COUT]
-  Vol v;
-  int64_t chunk;   // cells per block (multiple of 64)
-  float *partial;  // [chunks][27][COUT][CIN]
-};
-
-// dW[tap][co][ci] = sum over cells of G[cell][co] * X[cell + off(tap)][ci]:
-// A = G^T (co x cells), B = shifted X (cells x ci); 64-cell tiles staged in
-// shared memory, fragments assembled from 16-bit shared loads.
-template <int COUT, int CIN>
-__global__ void __launch_bounds__(128) k_wgrad_mma(WgradArgs a)
-{
-  constexpr int kT = 64;
-  constexpr int MT = COUT / 16, NT = CIN / 8, TILES = MT * NT, TPW = (TILES + 3) / 4;
-  constexpr int GP = COUT + 2, XP = CIN + 2;  // padded rows (16-bit elements)
-  __shared__ bf16 gs[kT][GP];
-  __shared__ bf16 xs[kT][XP];
-  const int tap = blockIdx.y;
-  const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int64_t ncell = a.v.cells();
-  const int64_t c_begin = blockIdx.x * a.chunk;
-  const int64_t c_end = min(c_begin + a.chunk, ncell);
-  const int hZ = a.v.Z >> 1, hY = a.v.Y >> 1, hX = a.v.X >> 1;
-  float acc[TPW][4];
-#pragma unroll
-  for (int q = 0; q < TPW; q++) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.0f;
-  for (int64_t c0 = c_begin; c0 < c_end; c0 += kT) {
-    // stage G rows and the tap-shifted input rows of 64 cells
-    for (int e = threadIdx.x; e < kT * (COUT / 2); e += blockDim.x) {
-      const int r = e / (COUT / 2), k = 2 * (e % (COUT / 2));
-      const int64_t c = c0 + r;
-      uint32_t v = 0;
-      if (c < c_end) v = ld_pair(a.g + c * COUT + k);
-      *reinterpret_cast<uint32_t *>(&gs[r][k]) = v;
-    }
-    for (int e = threadIdx.x; e < kT * (CIN / 2); e += blockDim.x) {
-      const int r = e / (CIN / 2), k = 2 * (e % (CIN / 2));
-      const int64_t c = c0 + r;
-      uint32_t v = 0;
-      if (c < c_end) {
-        int b, z, y, x;
-        decompose(a.v, c, b, z, y, x);
-        z += dz;
-        y += dy;
-        x += dx;
-        if (z >= 0 && z < a.v.Z && y >= 0 && y < a.v.Y && x >= 0 && x < a.v.X) {
-          if (k < a.s0.c) {
-            const int64_t n = a.s0.up ? (((int64_t)b * hZ + (z >> 1)) * hY + (y >> 1)) * hX + (x >> 1)
-                                      : (((int64_t)b * a.v.Z + z) * a.v.Y + y) * a.v.X + x;
-            v = ld_pair(a.s0.p + n * a.s0.c + k);
-          } else {
-            const int64_t n = (((int64_t)b * a.v.Z + z) * a.v.Y + y) * a.v.X + x;
-            v = ld_pair(a.s1.p + n * a.s1.c + (k - a.s0.c));
-          }
-        }
-      }
-      *reinterpret_cast<uint32_t *>(&xs[r][k]) = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int ks = 0; ks < kT; ks += 16) {
-#pragma unroll
-      for (int q = 0; q < TPW; q++) {
-        const int tile = warp + 4 * q;
-        if (tile >= TILES) break;
-        const int m0 = (tile / NT) * 16, n0 = (tile % NT) * 8;
-        const int k0 = ks + 2 * t;
-        uint32_t A[4];
-        A[0] = pack_raw(gs[k0][m0 + g], gs[k0 + 1][m0 + g]);
-        A[1] = pack_raw(gs[k0][m0 + g + 8], gs[k0 + 1][m0 + g + 8]);
-        A[2] = pack_raw(gs[k0 + 8][m0 + g], gs[k0 + 9][m0 + g]);
-        A[3] = pack_raw(gs[k0 + 8][m0 + g + 8], gs[k0 + 9][m0 + g + 8]);
-        const uint32_t b0 = pack_raw(xs[k0][n0 + g], xs[k0 + 1][n0 + g]);
-        const uint32_t b1 = pack_raw(xs[k0 + 8][n0 + g], xs[k0 + 9][n0 + g]);
-        mma_bf16(acc[q], A, b0, b1);
-      }
-    }
-    __syncthreads();
-  }
-  float *out = a.partial + ((int64_t)blockIdx.x * 27 + tap) * COUT * CIN;
-#pragma unroll
-  for (int q = 0; q < TPW; q++) {
-    const int tile = warp + 4 * q;
-    if (tile >= TILES) break;
-    const int m0 = (tile / NT) * 16, n0 = (tile % NT) * 8;
-    out[(m0 + g) * CIN + n0 + 2 * t] = acc[q][0];
-    out[(m0 + g) * CIN + n0 + 2 * t + 1] = acc[q][1];
-    out[(m0 + g + 8) * CIN + n0 + 2 * t] = acc[q][2];
-    out[(m0 + g + 8) * CIN + n0 + 2 * t + 1] = acc[q][3];
-  }
-}
-
-// dst[i] = sum over chunks of partial[chunk][i] (fixed order)
-__global__ void k_fold_chunks(const float *__restrict__ partial, int chunks, int n,
-    float *__restrict__ dst)
-{
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float s = 0.0f;
-  for (int c = 0; c < chunks; c++) s += partial[(int64_t)c * n + i];
-  dst[i] = s;
-}
-
-// per-channel sums of a [cells][C] BF16 gradient: block partials (fixed order)
-template <int C>
-__global__ void __launch_bounds__(256) k_channel_sum(const bf16 *__restrict__ g, int64_t ncell,
-    int64_t chunk, float *__restrict__ partial)
-{
-  constexpr int R = 256 / C;  // cells in flight per block step
-  __shared__ float sm[256];
-  const int ch = threadIdx.x % C, row = threadIdx.x / C;
-  const int64_t c_begin = blockIdx.x * chunk, c_end = min(c_begin + chunk, ncell);
-  float s = 0.0f;
-  for (int64_t c = c_begin + row; c < c_end; c += R) s += __bfloat162float(g[c * C + ch]);
-  sm[threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.x < C) {
-    float tot = 0.0f;
-    for (int r = 0; r < R; r++) tot += sm[r * C + threadIdx.x];
-    partial[(int64_t)blockIdx.x * C + threadIdx.x] = tot;
-  }
-}
-
-// same for an FP32 [cells] gradient (the output layer's bias)
-__global__ void __launch_bounds__(256) k_scalar_sum(const float *__restrict__ g, int64_t ncell,
-    int64_t chunk, float *__restrict__ partial)
-{
-  __shared__ float sm[256];
-  const int64_t c_begin = blockIdx.x * chunk, c_end = min(c_begin + chunk, ncell);
-  float s = 0.0f;
-  for (int64_t c = c_begin + threadIdx.x; c < c_end; c += 256) s += g[c];
-  sm[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sm[threadIdx.x] += sm[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partial[blockIdx.x] = sm[0];
-}
-
 // ------------------------------------------------------------------ plain layers
 
 // e0a: 2 -> 16, ReLU (FP32 arithmetic on BF16 values)
@@ -418,59 +266,11 @@ __global__ void __launch_bounds__(256) k_conv_last_dgrad(const float *__restrict
     *reinterpret_cast<float2 *>(dx + c * 16 + i) = make_float2(acc[i], acc[i + 1]);
 }
 
-// weight gradients of the plain layers, one block per (chunk, tap):
-// partial[chunk][tap][co][ci] = sum over the chunk of G[c][co] * X[c + off][ci]
-template <int CO, int CI, bool G_BF16>
-__global__ void __launch_bounds__(256) k_wgrad_plain(const void *g_, const bf16 *__restrict__ x,
-    Vol v, int64_t chunk, float *__restrict__ partial)
-{
-  constexpr int N = CO * CI;
-  __shared__ float sm[256];
-  const int tap = blockIdx.y;
-  const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-  const int64_t ncell = v.cells();
-  const int64_t c_begin = blockIdx.x * chunk, c_end = min(c_begin + chunk, ncell);
-  float acc[N];
-#pragma unroll
-  for (int i = 0; i < N; i++) acc[i] = 0.0f;
-  for (int64_t c = c_begin + threadIdx.x; c < c_end; c += 256) {
-    int b, z, y, xx;
-    decompose(v, c, b, z, y, xx);
-    z += dz;
-    y += dy;
-    xx += dx;
-    if (z < 0 || z >= v.Z || y < 0 || y >= v.Y || xx < 0 || xx >= v.X) continue;
-    const int64_t n = (((int64_t)b * v.Z + z) * v.Y + y) * v.X + xx;
-    float gv[CO], xv[CI];
-#pragma unroll
-    for (int o = 0; o < CO; o++)
-      gv[o] = G_BF16 ? __bfloat162float(static_cast<const bf16 *>(g_)[c * CO + o])
-                     : static_cast<const float *>(g_)[c * CO + o];
-#pragma unroll
-    for (int i = 0; i < CI; i++) xv[i] = __bfloat162float(x[n * CI + i]);
-#pragma unroll
-    for (int o = 0; o < CO; o++)
-#pragma unroll
-      for (int i = 0; i < CI; i++) acc[o * CI + i] += gv[o] * xv[i];
-  }
-  float *out = partial + ((int64_t)blockIdx.x * 27 + tap) * N;
-  for (int i = 0; i < N; i++) {
-    sm[threadIdx.x] = acc[i];
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-      if (threadIdx.x < w) sm[threadIdx.x] += sm[threadIdx.x + w];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) out[i] = sm[0];
-    __syncthreads();
-  }
-}
-
 // ------------------------------------------------------------------ elementwise
 
-// the 2-channel FP32 input as BF16, once as [cells][2] (the first layer's
-// weight gradient) and once zero-padded to [cells][16] (the tensor-core
-// first layer: K must be a multiple of 16)
+// the 2-channel FP32 input as BF16, once as [cells][2] (the plain first
+// layer) and once zero-padded to [cells][16] (the tensor-core first layer and
+// its weight gradient: channels in groups of 16)
 __global__ void k_input_bf16(const float *__restrict__ x, int64_t n, bf16 *__restrict__ x2,
     bf16 *__restrict__ x16)
 {
@@ -611,11 +411,19 @@ __global__ void __launch_bounds__(256) k_mse(const float *__restrict__ out,
   if (threadIdx.x == 0) partial[blockIdx.x] = sm[0];
 }
 
-__global__ void k_fold_loss(const double *__restrict__ partial, int nb, int64_t n, float *loss)
+__global__ void __launch_bounds__(256) k_fold_loss(const double *__restrict__ partial, int nb,
+    int64_t n, float *loss)
 {
+  __shared__ double sm[256];
   double s = 0.0;
-  for (int i = 0; i < nb; i++) s += partial[i];
-  *loss = (float)(s / (double)n);
+  for (int i = threadIdx.x; i < nb; i += 256) s += partial[i];
+  sm[threadIdx.x] = s;
+  __syncthreads();
+  for (int w = 128; w > 0; w >>= 1) {
+    if (threadIdx.x < w) sm[threadIdx.x] += sm[threadIdx.x + w];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *loss = (float)(sm[0] / (double)n);
 }
 
 __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m,
@@ -741,14 +549,6 @@ bool ensure_partial(UNetState *u, int64_t n)
   return true;
 }
 
-// cells per block of the weight-gradient kernels: at most 256 chunks
-int64_t wgrad_chunk(int64_t ncell)
-{
-  int64_t c = (ncell + 255) / 256;
-  c = (c + 63) / 64 * 64;
-  return c < 64 ? 64 : c;
-}
-
 template <int COUT, bool OUT_BF16>
 bool conv_mma(const ConvSrc &s0, const ConvSrc &s1, const Vol &v, const bf16 *w, const float *bias,
     int relu, void *out)
@@ -813,52 +613,15 @@ bool dgrad(UNetState *u, int l, const Vol &v, float *dx)
   return false;
 }
 
-template <int COUT, int CIN>
-bool wgrad_launch(const WgradArgs &a, int chunks)
-{
-  k_wgrad_mma<COUT, CIN><<<dim3(chunks, 27), 128, 0, stream()>>>(a);
-  return launched("k_wgrad_mma");
-}
-
-// weight and bias gradients of a tensor-core layer from G and its input
-bool wgrad(UNetState *u, int l, const ConvSrc &s0, const ConvSrc &s1, const Vol &v)
+// weight and bias gradients of a layer from G (or, for the output layer, the
+// FP32 gradient g32 itself) and its input
+bool wgrad(UNetState *u, int l, const ConvSrc &s0, const ConvSrc &s1, const Vol &v,
+    const float *g32 = nullptr)
 {
   const int co = kDesc[l].cout, ci = kDesc[l].cin;
-  const int64_t n = v.cells(), chunk = wgrad_chunk(n);
-  const int chunks = (int)((n + chunk - 1) / chunk);
-  if (!ensure_partial(u, (int64_t)chunks * 27 * co * ci)) return false;
-  WgradArgs a;
-  a.s0 = s0;
-  a.s1 = s1;
-  a.g = u->G;
-  a.v = v;
-  a.chunk = chunk;
-  a.partial = u->partial;
-  bool ok = false;
-  if (co == 16 && ci == 16) ok = wgrad_launch<16, 16>(a, chunks);
-  else if (co == 32 && ci == 16) ok = wgrad_launch<32, 16>(a, chunks);
-  else if (co == 32 && ci == 32) ok = wgrad_launch<32, 32>(a, chunks);
-  else if (co == 64 && ci == 32) ok = wgrad_launch<64, 32>(a, chunks);
-  else if (co == 32 && ci == 96) ok = wgrad_launch<32, 96>(a, chunks);
-  else if (co == 16 && ci == 48) ok = wgrad_launch<16, 48>(a, chunks);
-  else fail(NUSIF_ERR_STATE, "unet: no weight-gradient kernel for %dx%d", co, ci);
-  if (!ok) return false;
-  const int nw = 27 * co * ci;
-  k_fold_chunks<<<(nw + 255) / 256, 256, 0, stream()>>>(u->partial, chunks, nw, u->grad + u->w_off[l]);
-  if (!launched("k_fold_chunks")) return false;
-  // bias: per-channel sums of G (partials after the weight partials are folded)
-  const int64_t bchunk = (n + 1023) / 1024 * 4 < 256 ? 256 : (n + 1023) / 1024 * 4;
-  const int bblocks = (int)((n + bchunk - 1) / bchunk);
-  if (!ensure_partial(u, (int64_t)bblocks * co)) return false;
-  switch (co) {
-  case 16: k_channel_sum<16><<<bblocks, 256, 0, stream()>>>(u->G, n, bchunk, u->partial); break;
-  case 32: k_channel_sum<32><<<bblocks, 256, 0, stream()>>>(u->G, n, bchunk, u->partial); break;
-  case 64: k_channel_sum<64><<<bblocks, 256, 0, stream()>>>(u->G, n, bchunk, u->partial); break;
-  default: fail(NUSIF_ERR_STATE, "unet: no bias-gradient kernel for %d channels", co); return false;
-  }
-  if (!launched("k_channel_sum")) return false;
-  k_fold_chunks<<<1, 64, 0, stream()>>>(u->partial, bblocks, co, u->grad + u->b_off[l]);
-  return launched("k_fold_chunks");
+  return ensure_partial(u, wgrad_scratch(co, ci, v.B, v.Z, v.Y, v.X)) &&
+         wgrad_conv({ s0.p, s0.c, s0.up }, { s1.p, s1.c, s1.up }, u->G, g32, co, ci, v.B, v.Z, v.Y,
+             v.X, u->partial, u->grad + u->w_off[l], u->grad + u->b_off[l]);
 }
 
 bool mask(const float *dy, const bf16 *y, int64_t n, bf16 *g)
@@ -933,51 +696,6 @@ bool unet_forward(UNetState *u)
   return launched("k_conv_last");
 }
 
-namespace {
-
-// plain-layer weight gradients: out layer (dout FP32 x d0b) and e0a (G x input)
-bool wgrad_out(UNetState *u, const Vol &v)
-{
-  const int64_t n = v.cells(), chunk = wgrad_chunk(n);
-  const int chunks = (int)((n + chunk - 1) / chunk);
-  if (!ensure_partial(u, (int64_t)chunks * 27 * 16)) return false;
-  k_wgrad_plain<1, 16, false><<<dim3(chunks, 27), 256, 0, stream()>>>(u->dout, u->d0b, v, chunk,
-      u->partial);
-  if (!launched("k_wgrad_plain")) return false;
-  k_fold_chunks<<<(27 * 16 + 255) / 256, 256, 0, stream()>>>(u->partial, chunks, 27 * 16,
-      u->grad + u->w_off[L_OUT]);
-  if (!launched("k_fold_chunks")) return false;
-  const int64_t bchunk = 4096;
-  const int bblocks = (int)((n + bchunk - 1) / bchunk);
-  if (!ensure_partial(u, bblocks)) return false;
-  k_scalar_sum<<<bblocks, 256, 0, stream()>>>(u->dout, n, bchunk, u->partial);
-  if (!launched("k_scalar_sum")) return false;
-  k_fold_chunks<<<1, 32, 0, stream()>>>(u->partial, bblocks, 1, u->grad + u->b_off[L_OUT]);
-  return launched("k_fold_chunks");
-}
-
-bool wgrad_first(UNetState *u, const Vol &v)
-{
-  const int64_t n = v.cells(), chunk = wgrad_chunk(n);
-  const int chunks = (int)((n + chunk - 1) / chunk);
-  if (!ensure_partial(u, (int64_t)chunks * 27 * 32)) return false;
-  k_wgrad_plain<16, 2, true><<<dim3(chunks, 27), 256, 0, stream()>>>(u->G, u->x, v, chunk,
-      u->partial);
-  if (!launched("k_wgrad_plain")) return false;
-  k_fold_chunks<<<(27 * 32 + 255) / 256, 256, 0, stream()>>>(u->partial, chunks, 27 * 32,
-      u->grad + u->w_off[L_E0A]);
-  if (!launched("k_fold_chunks")) return false;
-  const int64_t bchunk = (n + 1023) / 1024 * 4 < 256 ? 256 : (n + 1023) / 1024 * 4;
-  const int bblocks = (int)((n + bchunk - 1) / bchunk);
-  if (!ensure_partial(u, (int64_t)bblocks * 16)) return false;
-  k_channel_sum<16><<<bblocks, 256, 0, stream()>>>(u->G, n, bchunk, u->partial);
-  if (!launched("k_channel_sum")) return false;
-  k_fold_chunks<<<1, 64, 0, stream()>>>(u->partial, bblocks, 16, u->grad + u->b_off[L_E0A]);
-  return launched("k_fold_chunks");
-}
-
-}  // namespace
-
 // loss against `target` and the gradient of every parameter into u->grad
 bool unet_backward(UNetState *u, const float *target)
 {
@@ -988,10 +706,10 @@ bool unet_backward(UNetState *u, const float *target)
   const int lblocks = (int)((n0 + lchunk - 1) / lchunk);
   k_mse<<<lblocks, 256, 0, stream()>>>(u->out, target, n0, lchunk, u->dout, u->loss_partial);
   if (!launched("k_mse")) return false;
-  k_fold_loss<<<1, 1, 0, stream()>>>(u->loss_partial, lblocks, n0, u->loss);
+  k_fold_loss<<<1, 256, 0, stream()>>>(u->loss_partial, lblocks, n0, u->loss);
   if (!launched("k_fold_loss")) return false;
   // out
-  if (!wgrad_out(u, v0)) return false;
+  if (!wgrad(u, L_OUT, { u->d0b, 16, 0 }, none, v0, u->dout)) return false;
   k_conv_last_dgrad<<<(unsigned)((n0 + 255) / 256), 256, 0, stream()>>>(u->dout, v0, u->wb[L_OUT],
       u->F2);
   if (!launched("k_conv_last_dgrad")) return false;
@@ -1027,7 +745,7 @@ bool unet_backward(UNetState *u, const float *target)
   if (!wgrad(u, L_E0B, { u->e0a, 16, 0 }, none, v0) || !dgrad(u, L_E0B, v0, u->F1)) return false;
   // e0a (no input gradient)
   if (!mask(u->F1, u->e0a, 16 * n0, u->G)) return false;
-  return wgrad_first(u, v0);
+  return wgrad(u, L_E0A, { u->x16, 16, 0 }, none, v0);
 }
 
 bool unet_set_input(UNetState *u, const float *x, const Vol &v)
