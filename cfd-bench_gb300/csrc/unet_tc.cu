@@ -470,6 +470,338 @@ __global__ void __launch_bounds__(kThreads, conv_min_blocks(NCH)) k_conv_tc(cons
   }
 }
 
+// ------------------------------------------------------------------ marching form
+//
+// The layers of up to 48 channels on either side (every full-resolution layer,
+// forward and input gradient). k_conv_tc loads a tile's neighbourhood nine
+// times, in boxes of 32- to 128-byte rows, and that many short rows, not the
+// products, set its pace (about 5000 cycles a tile of a 16 -> 16 layer). Here
+// a block owns a column of 8 x 16 cells and marches over the planes. A plane
+// (10 x 18 cells around the column) is fetched once, by 16-byte cp.async, and
+// used once: its products go to the three output planes it belongs to, as one
+// tcgen05.mma per (dy, dx) and 16 channels with N = 3 x channels out, the
+// weights of the three dz side by side. That also reads A from shared memory a
+// third as often, which is what bounds a product of so few columns (128 rows of
+// 32 bytes each time).
+//
+// The operand needs no copy per tap: a cell's 8-channel group is 16 bytes, eight
+// cells along x are one 8 x 16-byte core matrix of the unswizzled K-major
+// layout, the next eight rows of the operand are the next y, and a tap is an
+// offset of the start address by whole cells. All weights stay in shared memory.
+//
+// Accumulators of the output planes are groups of N columns in a ring in tensor
+// memory, so the window of three slides by N columns a plane (two products where
+// it wraps). A group starts from zeros, which the epilogue stores after it has
+// drained it. Every output is summed in the order of k_conv_tc (dz, dy, dx, then
+// channels), so the results are the same bits.
+constexpr int kColX = 8, kColY = 16;                // cells of a column
+constexpr int kInX = kColX + 2, kInY = kColY + 2;   // and of the plane it reads
+constexpr int kRowB = kInX * 16;                    // bytes of a y-row of one 8-channel group
+constexpr int kGroupB = kInY * kRowB;               // bytes of one 8-channel group of a plane
+constexpr int kSlotsC = 4;                          // planes in shared memory
+constexpr int kMaxGroups = 8;
+constexpr int kColThreads = 256;  // warp 0 products, 1-3 loads, 4-7 epilogue
+constexpr int kLoaders = 96;
+
+struct ColParams {
+  const __nv_bfloat16 *s0, *s1;  // sources of C0 and C1 channels
+  const __nv_bfloat16 *w;        // [27][N][C0 + C1]
+  int C0, C1;
+  int X, Y, Z, B;
+  int tx, ty;      // columns per row and per plane
+  int zl, zt;      // planes of a march, marches per column
+  int items;
+  int tmem_cols, groups;
+  const float *bias;
+  int relu, out_bf16, out_ch;
+  void *out;
+  int *err;
+};
+
+struct March {
+  int x0, y0, b, z0, z1;
+};
+
+__device__ __forceinline__ March march_of(const ColParams &P, int t)
+{
+  March m;
+  m.x0 = (t % P.tx) * kColX;
+  int r = t / P.tx;
+  m.y0 = (r % P.ty) * kColY;
+  r /= P.ty;
+  m.z0 = (r % P.zt) * P.zl;
+  m.z1 = min(m.z0 + P.zl, P.Z) - 1;
+  m.b = r / P.zt;
+  return m;
+}
+
+// unswizzled K-major descriptor: lead = bytes between the two 8-element halves
+// of K, stride = bytes between groups of 8 rows
+__device__ __forceinline__ uint64_t smem_desc_plain(uint32_t addr, uint32_t lead, uint32_t stride)
+{
+  uint64_t d = (uint64_t)((addr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)((lead >> 4) & 0x3FFFu) << 16;
+  d |= (uint64_t)((stride >> 4) & 0x3FFFu) << 32;
+  d |= 1ull << 46;
+  return d;
+}
+
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr)
+{
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr),
+      "r"(0u)
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+__device__ __forceinline__ void fence_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// NCH output and CIN input channels, 16, 32 or 48 each
+template <int NCH, int CIN>
+struct Col {
+  static constexpr int kHalves = CIN / 8;                   // 8-channel groups
+  static constexpr uint32_t kSlotB = kHalves * kGroupB;
+  static constexpr uint32_t kTapB = kHalves * 3 * NCH * 16;  // weights of one (dy, dx)
+  static constexpr uint32_t kWeightB = 9 * kTapB;
+  static constexpr size_t kSmem = kBarBytes + 128 + kWeightB + kSlotsC * kSlotB;
+};
+
+template <int NCH, int CIN>
+__global__ void __launch_bounds__(kColThreads) k_conv_col(const ColParams P)
+{
+  using L = Col<NCH, CIN>;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
+  uint64_t *full = bars, *empty = bars + kSlotsC, *acc_full = bars + 2 * kSlotsC,
+           *acc_empty = acc_full + kMaxGroups;
+  static_assert((2 * kSlotsC + 2 * kMaxGroups) * 8 + 8 <= kBarBytes, "barriers overlap the flags");
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + kBarBytes - 8);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + kBarBytes - 4);
+  const uint32_t weights = smem_u32(smem) + kBarBytes, planes = weights + L::kWeightB;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (tid == 0) {
+    for (int s = 0; s < kSlotsC; s++) {
+      mbar_init(smem_u32(full + s), kLoaders);
+      mbar_init(smem_u32(empty + s), 1);
+    }
+    for (int g = 0; g < kMaxGroups; g++) {
+      mbar_init(smem_u32(acc_full + g), 1);
+      mbar_init(smem_u32(acc_empty + g), 128);
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tmem_slot)),
+                 "r"(P.tmem_cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  // weights: per (dy, dx) and 8 channels, rows dz = +1, 0, -1 of N channels: the
+  // row blocks of output planes p - 1, p, p + 1 for an input plane p
+  for (int i = tid; i < 27 * NCH * L::kHalves; i += kColThreads) {
+    const int h = i % L::kHalves, r = i / L::kHalves, n = r % NCH, tap = r / NCH;
+    const int dz = tap / 9 - 1, dydx = tap % 9;
+    const uint4 v = *reinterpret_cast<const uint4 *>(P.w + ((size_t)tap * NCH + n) * CIN + 8 * h);
+    const uint32_t at = (uint32_t)(dydx * (int)L::kTapB + (h * 3 * NCH + (1 - dz) * NCH + n) * 16);
+    *reinterpret_cast<uint4 *>(smem + kBarBytes + at) = v;
+  }
+  fence_proxy();
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = *tmem_slot;
+  if (warp >= 4) {  // every group starts from zeros
+    for (int c = 0; c < P.groups * NCH; c += 16)
+      tmem_zero16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)c);
+    tmem_wait_st();
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+
+  if (warp >= 1 && warp <= 3) {
+    // ---------------- loads: one plane a slot ----------------
+    const int t0 = tid - 32;
+    int slot = 0, prev = -1;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; ok && t < P.items; t += gridDim.x) {
+      const March m = march_of(P, t);
+      const int p1 = min(m.z1 + 1, P.Z - 1);
+      for (int p = max(m.z0 - 1, 0); p <= p1; p++) {
+        if (!mbar_wait(smem_u32(empty + slot), phase ^ 1u, abort_flag, P.err)) {
+          ok = false;
+          break;
+        }
+        const int64_t row0 = ((int64_t)m.b * P.Z + p) * P.Y;
+        const uint32_t dst0 = planes + (uint32_t)slot * L::kSlotB;
+        for (int i = t0; i < kInY * kInX * L::kHalves; i += kLoaders) {
+          const int h = i % L::kHalves, c = i / L::kHalves, cx = c % kInX, cy = c / kInX;
+          const int x = m.x0 - 1 + cx, y = m.y0 - 1 + cy;
+          const bool in = x >= 0 && x < P.X && y >= 0 && y < P.Y;
+          const bool second = 8 * h >= P.C0;
+          const int cs = second ? P.C1 : P.C0, ch = second ? 8 * h - P.C0 : 8 * h;
+          const __nv_bfloat16 *src =
+              (second ? P.s1 : P.s0) + (in ? ((row0 + y) * P.X + x) * cs + ch : 0);
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                           dst0 + (uint32_t)(h * kGroupB + cy * kRowB + cx * 16)),
+                       "l"(src), "r"(in ? 16 : 0)
+                       : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (prev >= 0) {  // the plane before this one is in
+          asm volatile("cp.async.wait_group 1;" ::: "memory");
+          fence_proxy();
+          mbar_arrive(smem_u32(full + prev));
+        }
+        prev = slot;
+        if (++slot == kSlotsC) {
+          slot = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (prev >= 0) {
+      fence_proxy();
+      mbar_arrive(smem_u32(full + prev));
+    }
+  } else if (warp == 0 && lane == 0) {
+    // ---------------- products ----------------
+    int slot = 0;
+    uint32_t phase = 0;
+    int seq = 0;  // output planes opened so far; plane number q of them uses group q % groups
+    bool ok = true, issued = false;
+    const uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTileM >> 4) << 24);
+    for (int t = blockIdx.x; ok && t < P.items; t += gridDim.x) {
+      const March m = march_of(P, t);
+      const int q0 = seq;  // the number of output plane z0
+      const int p1 = min(m.z1 + 1, P.Z - 1);
+      for (int p = max(m.z0 - 1, 0); p <= p1; p++) {
+        const int za = max(p - 1, m.z0), zb = min(p + 1, m.z1);  // output planes of this one
+        while (ok && seq <= q0 + zb - m.z0) {  // groups entering the window are drained and zero
+          const int g = seq % P.groups;
+          ok = mbar_wait(smem_u32(acc_empty + g), ((uint32_t)(seq / P.groups) & 1u) ^ 1u, abort_flag,
+              P.err);
+          seq++;
+        }
+        if (!ok || !mbar_wait(smem_u32(full + slot), phase, abort_flag, P.err)) {
+          ok = false;
+          break;
+        }
+        fence_after();
+        const int ga = (q0 + za - m.z0) % P.groups, cnt = zb - za + 1;
+        const int n1 = min(cnt, P.groups - ga), n2 = cnt - n1;  // groups up to the ring's end, and after
+        const uint32_t d1 = tmem + (uint32_t)(ga * NCH);
+        const uint32_t i1 = idesc0 | ((uint32_t)(n1 * NCH >> 3) << 17);
+        const uint32_t i2 = idesc0 | ((uint32_t)(n2 * NCH >> 3) << 17);
+        const uint64_t a0 =
+            smem_desc_plain(planes + (uint32_t)slot * L::kSlotB, kGroupB, kRowB);
+        const uint64_t b0 = smem_desc_plain(
+            weights + (uint32_t)((za - (p - 1)) * NCH * 16), 3 * NCH * 16, 128);
+        for (int dy = 0; dy < 3; dy++)
+          for (int dx = 0; dx < 3; dx++) {
+#pragma unroll
+            for (int j = 0; j < CIN / 16; j++) {
+              const uint64_t a = a0 + (uint64_t)((j * 2 * kGroupB + dy * kRowB + dx * 16) >> 4);
+              const uint64_t b =
+                  b0 + (uint64_t)(((dy * 3 + dx) * (int)L::kTapB + j * 2 * 3 * NCH * 16) >> 4);
+              mma_f16(d1, a, b, i1, 1u);
+              if (n2 > 0) mma_f16(tmem, a, b + (uint64_t)(n1 * NCH), i2, 1u);
+            }
+          }
+        issued = true;
+        mma_commit(smem_u32(empty + slot));
+        if (p - 1 >= m.z0) mma_commit(smem_u32(acc_full + (q0 + p - 1 - m.z0) % P.groups));
+        if (p == p1 && p1 == m.z1) mma_commit(smem_u32(acc_full + (q0 + p - m.z0) % P.groups));
+        if (++slot == kSlotsC) {
+          slot = 0;
+          phase ^= 1u;
+        }
+      }
+    }
+    if (!ok && issued) {
+      // wait for every product already issued, on a barrier that nothing else completes now
+      mma_commit(smem_u32(empty + slot));
+      mbar_drain(smem_u32(empty + slot), phase);
+    }
+  } else if (warp >= 4) {
+    // ---------------- epilogue: tensor memory -> bias, ReLU -> global ----------------
+    const int q = warp & 3, row = 32 * q + lane;  // accumulator row: 8 y + x in the column
+    int seq = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; ok && t < P.items; t += gridDim.x) {
+      const March m = march_of(P, t);
+      const int x = m.x0 + (row & 7), y = m.y0 + (row >> 3);
+      const bool in = x < P.X && y < P.Y;
+      for (int z = m.z0; z <= m.z1; z++, seq++) {
+        const int g = seq % P.groups;
+        const bool ready = mbar_wait(smem_u32(acc_full + g), (uint32_t)(seq / P.groups) & 1u,
+            abort_flag, P.err);
+        if (!__all_sync(0xffffffffu, ready)) {
+          ok = false;
+          break;
+        }
+        fence_after();
+        const uint32_t addr = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(g * NCH);
+        float v[NCH];
+#pragma unroll
+        for (int c = 0; c < NCH; c += 16) {
+          float part[16];
+          tmem_ld16(addr + (uint32_t)c, part);
+#pragma unroll
+          for (int e = 0; e < 16; e++) v[c + e] = part[e];
+        }
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < NCH; c += 16) tmem_zero16(addr + (uint32_t)c);
+        tmem_wait_st();
+        fence_before();
+        mbar_arrive(smem_u32(acc_empty + g));
+        if (!in) continue;
+        const int64_t cell = (((int64_t)m.b * P.Z + z) * P.Y + y) * P.X + x;
+        if (P.out_ch == 1) {  // one channel (the output layer, its weights padded to 16 rows)
+          const float r = v[0] + (P.bias ? __ldg(P.bias) : 0.0f);
+          static_cast<float *>(P.out)[cell] = P.relu ? fmaxf(r, 0.0f) : r;
+          continue;
+        }
+#pragma unroll
+        for (int c = 0; c < NCH; c++) {
+          const float r = v[c] + (P.bias ? __ldg(P.bias + c) : 0.0f);
+          v[c] = P.relu ? fmaxf(r, 0.0f) : r;
+        }
+        if (P.out_bf16) {
+          uint4 *o = reinterpret_cast<uint4 *>(static_cast<__nv_bfloat16 *>(P.out) + cell * NCH);
+#pragma unroll
+          for (int c = 0; c < NCH; c += 8)
+            o[c / 8] = make_uint4(pack2(v[c], v[c + 1]), pack2(v[c + 2], v[c + 3]),
+                pack2(v[c + 4], v[c + 5]), pack2(v[c + 6], v[c + 7]));
+        } else {
+          float4 *o = reinterpret_cast<float4 *>(static_cast<float *>(P.out) + cell * NCH);
+#pragma unroll
+          for (int c = 0; c < NCH; c += 4)
+            o[c / 4] = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+        }
+      }
+    }
+  }
+  fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    __syncwarp();
+    fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(P.tmem_cols)
+                 : "memory");
+  }
+}
+
 // ------------------------------------------------------------------ host side
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
@@ -632,6 +964,65 @@ bool launch_tc(const CUtensorMap &a0, const CUtensorMap &a1, const CUtensorMap &
   return launched("k_conv_tc");
 }
 
+template <int NCH, int CIN>
+bool launch_col(ColParams P)
+{
+  using L = Col<NCH, CIN>;
+  P.tmem_cols = NCH == 16 ? 128 : 256;
+  P.groups = P.tmem_cols / NCH < kMaxGroups ? P.tmem_cols / NCH : kMaxGroups;
+  static bool attr_set[64] = {};
+  int dev = 0;
+  if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice")) return false;
+  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+    if (!cuda_ok(cudaFuncSetAttribute(k_conv_col<NCH, CIN>,
+                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kSmem),
+            "k_conv_col shared memory"))
+      return false;
+    attr_set[dev] = true;
+  }
+  // a persistent grid: no more blocks than can be resident at once, by shared
+  // memory (1 KB reserved per block), registers and tensor memory
+  static int regs = 0;
+  if (regs == 0) {
+    cudaFuncAttributes fa{};
+    if (!cuda_ok(cudaFuncGetAttributes(&fa, k_conv_col<NCH, CIN>), "k_conv_col attributes"))
+      return false;
+    regs = ((fa.numRegs + 7) / 8) * 8 * kColThreads;
+  }
+  int per_sm = (int)((228 * 1024) / (L::kSmem + 1024));
+  if (per_sm > 65536 / regs) per_sm = 65536 / regs;
+  if (per_sm > 512 / P.tmem_cols) per_sm = 512 / P.tmem_cols;
+  if (per_sm < 1) per_sm = 1;
+  const int wave = sm_count_tc() * per_sm;
+  // planes of a march: the least (marches of the busiest block) x (planes + 2
+  // read around them)
+  const int64_t columns = (int64_t)P.B * P.tx * P.ty;
+  int64_t best = -1;
+  for (int zl = 1; zl <= P.Z; zl++) {
+    const int64_t n = columns * ((P.Z + zl - 1) / zl);
+    const int64_t cost = ((n + wave - 1) / wave) * (zl + 2);
+    if (best < 0 || cost < best) {
+      best = cost;
+      P.zl = zl;
+    }
+  }
+  P.zt = (P.Z + P.zl - 1) / P.zl;
+  P.items = (int)(columns * P.zt);
+  const int grid = P.items < wave ? P.items : wave;
+  k_conv_col<NCH, CIN><<<grid, kColThreads, L::kSmem, stream()>>>(P);
+  return launched("k_conv_col");
+}
+
+template <int NCH>
+bool launch_col_cin(const ColParams &P)
+{
+  switch (P.C0 + P.C1) {
+  case 16: return launch_col<NCH, 16>(P);
+  case 32: return launch_col<NCH, 32>(P);
+  default: return launch_col<NCH, 48>(P);
+  }
+}
+
 }  // namespace
 
 bool tc_conv_supported(int X, int Y, int Z, int B, int N, int C0, int C1)
@@ -669,6 +1060,31 @@ bool tc_conv(const void *s0, int C0, const void *s1, int C1, int B, int Z, int Y
   }
   P.out = out;
   P.err = err;
+  if (N <= 48 && C0 + C1 <= 48) {
+    ColParams c{};
+    c.s0 = static_cast<const __nv_bfloat16 *>(s0);
+    c.s1 = static_cast<const __nv_bfloat16 *>(s1);
+    c.w = static_cast<const __nv_bfloat16 *>(w);
+    c.C0 = C0;
+    c.C1 = C1;
+    c.X = X;
+    c.Y = Y;
+    c.Z = Z;
+    c.B = B;
+    c.tx = (X + kColX - 1) / kColX;
+    c.ty = (Y + kColY - 1) / kColY;
+    c.bias = bias;
+    c.relu = relu;
+    c.out_bf16 = P.out_bf16;
+    c.out_ch = P.out_ch;
+    c.out = out;
+    c.err = err;
+    switch (N) {
+    case 16: return launch_col_cin<16>(c);
+    case 32: return launch_col_cin<32>(c);
+    default: return launch_col_cin<48>(c);
+    }
+  }
   CUtensorMap a0, a1, w0, w1;
   if (!map_volume(&a0, s0, C0, X, Y, Z * B)) return false;
   if (!map_weights(&w0, w, C0 + C1, N, C0)) return false;
