@@ -250,12 +250,8 @@ __device__ __forceinline__ Tile tile_of(const TcParams &P, int t)
   return r;
 }
 
-// resident blocks per SM the compiler keeps registers for: eight of the
-// 16-channel layers (the full-resolution ones, bound by per-block latency)
-constexpr int conv_min_blocks(int nch) { return nch == 16 ? 8 : 1; }
-
 template <int NCH>  // output channels, a multiple of 16
-__global__ void __launch_bounds__(kThreads, conv_min_blocks(NCH)) k_conv_tc(const __grid_constant__ CUtensorMap tm_a0,
+__global__ void __launch_bounds__(kThreads) k_conv_tc(const __grid_constant__ CUtensorMap tm_a0,
     const __grid_constant__ CUtensorMap tm_a1, const __grid_constant__ CUtensorMap tm_w0,
     const __grid_constant__ CUtensorMap tm_w1, const TcParams P)
 {
@@ -910,11 +906,8 @@ bool launch_tc(const CUtensorMap &a0, const CUtensorMap &a1, const CUtensorMap &
   P.tx_bytes = tx;
   const size_t stage_bytes = P.stage_bytes;
   // two stages: the fewer the stages, the more blocks an SM holds, and more
-  // blocks measured faster than deeper pipelines (the 128^3 forward pass:
-  // 1.77 ms with 2 stages and six blocks of 16 -> 16 layers per SM (1.73 ms
-  // with eight, their registers capped for it), 1.81 ms
-  // with 4, 2.36 ms with 8, 2.43 ms with 16 stages and two blocks per SM);
-  // NUSIF_TC_STAGES overrides the count
+  // blocks measured faster than deeper pipelines; NUSIF_TC_STAGES overrides the
+  // count
   int stages = 2;
   if (const char *e = getenv("NUSIF_TC_STAGES")) {
     const int s = atoi(e);
@@ -1013,14 +1006,15 @@ bool launch_col(ColParams P)
   return launched("k_conv_col");
 }
 
-template <int NCH>
-bool launch_col_cin(const ColParams &P)
+// the layers of the marching form, as 100 N + channels in: at most 48 channels
+// on either side (the weights of all taps and four planes fit shared memory
+// several blocks at a time)
+bool col_layer(int N, int C)
 {
-  switch (P.C0 + P.C1) {
-  case 16: return launch_col<NCH, 16>(P);
-  case 32: return launch_col<NCH, 32>(P);
-  default: return launch_col<NCH, 48>(P);
+  switch (100 * N + C) {
+  case 1616: case 1632: case 1648: case 3216: case 3232: case 4816: return true;
   }
+  return false;
 }
 
 }  // namespace
@@ -1030,7 +1024,7 @@ bool tc_conv_supported(int X, int Y, int Z, int B, int N, int C0, int C1)
   if (X <= 0 || Y <= 0 || Z <= 0 || B <= 0) return false;
   auto ok_c = [](int c) { return c == 16 || c == 32 || c == 64; };
   if (!ok_c(C0) || (C1 != 0 && !ok_c(C1))) return false;
-  if (N != 16 && N != 32 && N != 48 && N != 64 && N != 96) return false;
+  if (!col_layer(N, C0 + C1) && N != 32 && N != 64 && N != 96) return false;
   if (X % kTileX || Y % kTileY) return false;
   return encode_fn() != nullptr;
 }
@@ -1060,7 +1054,7 @@ bool tc_conv(const void *s0, int C0, const void *s1, int C1, int B, int Z, int Y
   }
   P.out = out;
   P.err = err;
-  if (N <= 48 && C0 + C1 <= 48) {
+  if (col_layer(N, C0 + C1)) {
     ColParams c{};
     c.s0 = static_cast<const __nv_bfloat16 *>(s0);
     c.s1 = static_cast<const __nv_bfloat16 *>(s1);
@@ -1079,10 +1073,13 @@ bool tc_conv(const void *s0, int C0, const void *s1, int C1, int B, int Z, int Y
     c.out_ch = P.out_ch;
     c.out = out;
     c.err = err;
-    switch (N) {
-    case 16: return launch_col_cin<16>(c);
-    case 32: return launch_col_cin<32>(c);
-    default: return launch_col_cin<48>(c);
+    switch (100 * N + C0 + C1) {
+    case 1616: return launch_col<16, 16>(c);
+    case 1632: return launch_col<16, 32>(c);
+    case 1648: return launch_col<16, 48>(c);
+    case 3216: return launch_col<32, 16>(c);
+    case 3232: return launch_col<32, 32>(c);
+    default: return launch_col<48, 16>(c);
     }
   }
   CUtensorMap a0, a1, w0, w1;
@@ -1096,9 +1093,7 @@ bool tc_conv(const void *s0, int C0, const void *s1, int C1, int B, int Z, int Y
     w1 = w0;
   }
   switch (N) {
-  case 16: return launch_tc<16>(a0, a1, w0, w1, P);
   case 32: return launch_tc<32>(a0, a1, w0, w1, P);
-  case 48: return launch_tc<48>(a0, a1, w0, w1, P);
   case 64: return launch_tc<64>(a0, a1, w0, w1, P);
   case 96: return launch_tc<96>(a0, a1, w0, w1, P);
   }

@@ -91,8 +91,13 @@ struct Layout {
 };
 
 // G32: G is one FP32 channel, stored as the three BF16 channels whose sum it
-// is (24 bits), the other rows of the tile zero
-template <int TM, int TN, bool G32>
+// is (24 bits), the other rows of the tile zero.
+// ROWS: the tensor core's own FP32 accumulation truncates, so a long chain of
+// products drifts (2e-5 of a gradient over two million cells). The first and
+// the last layer, whose gradients were plain FP32 sums before, keep a chain to
+// one row and add the rows with rounding (2e-7); at 16 x 16 channels that costs
+// 155 -> 220 us on two million cells.
+template <int TM, int TN, bool G32, bool ROWS>
 __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
 {
   using L = Layout<TM, TN>;
@@ -122,19 +127,54 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
   const uint32_t b_off = (uint32_t)((mr + (mat & 1) * 8) * L::kXp + (mat >> 1) * 16);
   const int dz = warp / 3, dy = warp % 3 - 1;
 
-  float acc[3][MT][NT][4], bias[MT][4];
+  float acc[3][MT][NT][4], bias[MT][4], bias_sum[MT][2];
+  float sum[ROWS ? 3 : 1][ROWS ? MT : 1][ROWS ? NT : 1][4];
+  const auto clear = [&] {
 #pragma unroll
-  for (int t = 0; t < 3; t++)
+    for (int t = 0; t < 3; t++)
+#pragma unroll
+      for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) acc[t][m][n][e] = 0.0f;
 #pragma unroll
     for (int m = 0; m < MT; m++)
 #pragma unroll
-      for (int n = 0; n < NT; n++)
+      for (int e = 0; e < 4; e++) bias[m][e] = 0.0f;
+  };
+  // ROWS: the row's products join the sums
+  const auto gather = [&] {
+    if constexpr (ROWS) {
 #pragma unroll
-        for (int e = 0; e < 4; e++) acc[t][m][n][e] = 0.0f;
+      for (int t = 0; t < 3; t++)
 #pragma unroll
-  for (int m = 0; m < MT; m++)
+        for (int m = 0; m < MT; m++)
 #pragma unroll
-    for (int e = 0; e < 4; e++) bias[m][e] = 0.0f;
+          for (int n = 0; n < NT; n++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) sum[t][m][n][e] += acc[t][m][n][e];
+#pragma unroll
+      for (int m = 0; m < MT; m++) {
+        bias_sum[m][0] += bias[m][0];
+        bias_sum[m][1] += bias[m][2];
+      }
+      clear();
+    }
+  };
+  clear();
+  if constexpr (ROWS) {
+#pragma unroll
+    for (int t = 0; t < 3; t++)
+#pragma unroll
+      for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) sum[t][m][n][e] = 0.0f;
+  }
+#pragma unroll
+  for (int m = 0; m < MT; m++) bias_sum[m][0] = bias_sum[m][1] = 0.0f;
   if (G32) {  // the rows that stay zero
     for (int i = tid; i < 2 * L::kGrow / 16; i += kThreads)
       reinterpret_cast<uint4 *>(gs)[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -229,7 +269,18 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
             }
           }
       }
+      gather();
     }
+  }
+  if constexpr (ROWS) {
+#pragma unroll
+    for (int t = 0; t < 3; t++)
+#pragma unroll
+      for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+          for (int e = 0; e < 4; e++) acc[t][m][n][e] = sum[t][m][n][e];
   }
   float *const out =
       A.partial + ((int64_t)part * gridDim.x + blockIdx.x) * (27 * TM * TN + TM);
@@ -250,8 +301,8 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
   if (warp == 4 && (lane & 3) == 0) {
 #pragma unroll
     for (int m = 0; m < MT; m++) {
-      out[27 * TM * TN + 16 * m + g] = bias[m][0];
-      out[27 * TM * TN + 16 * m + g + 8] = bias[m][2];
+      out[27 * TM * TN + 16 * m + g] = ROWS ? bias_sum[m][0] : bias[m][0];
+      out[27 * TM * TN + 16 * m + g + 8] = ROWS ? bias_sum[m][1] : bias[m][2];
     }
   }
 }
@@ -324,7 +375,7 @@ Plan plan(int co, int ci, int B, int Z, int Y, int X)
   return p;
 }
 
-template <int TM, int TN, bool G32>
+template <int TM, int TN, bool G32, bool ROWS>
 bool launch(const Plan &p, const Args &a)
 {
   constexpr int bytes = Layout<TM, TN>::kSmem;
@@ -332,13 +383,13 @@ bool launch(const Plan &p, const Args &a)
   int dev = 0;
   if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice")) return false;
   if (dev >= 0 && dev < 64 && !set[dev]) {
-    if (!cuda_ok(cudaFuncSetAttribute(k_wgrad<TM, TN, G32>,
+    if (!cuda_ok(cudaFuncSetAttribute(k_wgrad<TM, TN, G32, ROWS>,
                      cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
             "k_wgrad shared memory"))
       return false;
     set[dev] = true;
   }
-  k_wgrad<TM, TN, G32><<<dim3(p.blocks, p.parts), kThreads, bytes, stream()>>>(a);
+  k_wgrad<TM, TN, G32, ROWS><<<dim3(p.blocks, p.parts), kThreads, bytes, stream()>>>(a);
   return launched("k_wgrad");
 }
 
@@ -372,11 +423,12 @@ bool wgrad_conv(const WgradSrc &s0, const WgradSrc &s1, const void *g, const flo
   a.parts_n = p.parts_n;
   a.partial = scratch;
   bool ok = false;
-  if (g32) ok = launch<16, 16, true>(p, a);
-  else if (p.tm == 16 && p.tn == 16) ok = launch<16, 16, false>(p, a);
-  else if (p.tm == 16 && p.tn == 48) ok = launch<16, 48, false>(p, a);
-  else if (p.tm == 32 && p.tn == 16) ok = launch<32, 16, false>(p, a);
-  else ok = launch<32, 32, false>(p, a);
+  if (g32) ok = launch<16, 16, true, true>(p, a);
+  else if (ci < 16) ok = launch<16, 16, false, true>(p, a);
+  else if (p.tm == 16 && p.tn == 16) ok = launch<16, 16, false, false>(p, a);
+  else if (p.tm == 16 && p.tn == 48) ok = launch<16, 48, false, false>(p, a);
+  else if (p.tm == 32 && p.tn == 16) ok = launch<32, 16, false, false>(p, a);
+  else ok = launch<32, 32, false, false>(p, a);
   if (!ok) return false;
   const int n = 27 * co * ci + co;
   k_wgrad_fold<<<(n + 31) / 32, 256, 0, stream()>>>(scratch, p.blocks, p.tm, p.tn, p.parts_n, co, ci,
