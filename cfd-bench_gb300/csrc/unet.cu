@@ -33,6 +33,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include "nusif_internal.h"
@@ -240,30 +241,58 @@ __global__ void __launch_bounds__(256) k_conv_last(const bf16 *__restrict__ x, V
   y[c] = acc;
 }
 
-// input gradient of the output layer: dX[c][i] = sum_tap dout[c - off] W[tap][i]
-__global__ void __launch_bounds__(256) k_conv_last_dgrad(const float *__restrict__ dout, Vol v,
-    const bf16 *__restrict__ w, float *__restrict__ dx)
+// masked input gradient of the output layer: G[c][i] = (sum over taps of
+// dout[c - off] W[tap][i]) where y > 0, in BF16; four cells of a row per
+// thread, so a tap's weights are read once for four
+__global__ void __launch_bounds__(128) k_conv_last_dgrad(const float *__restrict__ dout, Vol v,
+    const bf16 *__restrict__ w, const bf16 *__restrict__ y, bf16 *__restrict__ g)
 {
-  __shared__ float ws[27 * 16];
+  __shared__ __align__(16) float ws[27 * 16];
   for (int i = threadIdx.x; i < 27 * 16; i += blockDim.x) ws[i] = __bfloat162float(w[i]);
   __syncthreads();
-  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c >= v.cells()) return;
-  int b, z, yy, xx;
-  decompose(v, c, b, z, yy, xx);
-  float acc[16];
+  const int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (4 * q >= v.cells()) return;
+  int b, z, yy, x0;
+  decompose(v, 4 * q, b, z, yy, x0);  // x is a multiple of 4
+  float acc[4][16];
 #pragma unroll
-  for (int i = 0; i < 16; i++) acc[i] = 0.0f;
-  for (int tap = 0; tap < 27; tap++) {
-    const int nz = z - (tap / 9 - 1), ny = yy - ((tap / 3) % 3 - 1), nx = xx - (tap % 3 - 1);
-    if (nz < 0 || nz >= v.Z || ny < 0 || ny >= v.Y || nx < 0 || nx >= v.X) continue;
-    const float d = dout[(((int64_t)b * v.Z + nz) * v.Y + ny) * v.X + nx];
+  for (int c = 0; c < 4; c++)
 #pragma unroll
-    for (int i = 0; i < 16; i++) acc[i] += d * ws[tap * 16 + i];
+    for (int i = 0; i < 16; i++) acc[c][i] = 0.0f;
+  for (int zy = 0; zy < 9; zy++) {
+    const int nz = z - (zy / 3 - 1), ny = yy - (zy % 3 - 1);
+    if (nz < 0 || nz >= v.Z || ny < 0 || ny >= v.Y) continue;
+    const float *row = dout + (((int64_t)b * v.Z + nz) * v.Y + ny) * v.X + x0;
+    const float4 m = *reinterpret_cast<const float4 *>(row);
+    const float d[6] = { x0 > 0 ? row[-1] : 0.0f, m.x, m.y, m.z, m.w,
+                         x0 + 4 < v.X ? row[4] : 0.0f };
+#pragma unroll
+    for (int dx = 0; dx < 3; dx++) {  // tap dx - 1 reads the cell at x - (dx - 1)
+      const float *wt = ws + (3 * zy + dx) * 16;
+#pragma unroll
+      for (int i = 0; i < 16; i++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) acc[c][i] += d[c + 2 - dx] * wt[i];
+    }
   }
 #pragma unroll
-  for (int i = 0; i < 16; i += 2)
-    *reinterpret_cast<float2 *>(dx + c * 16 + i) = make_float2(acc[i], acc[i + 1]);
+  for (int c = 0; c < 4; c++) {
+    const uint4 *k = reinterpret_cast<const uint4 *>(y + (4 * q + c) * 16);
+    uint4 *o = reinterpret_cast<uint4 *>(g + (4 * q + c) * 16);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      float t[8], m[8];
+      const uint4 yv = k[h];
+      const uint32_t u[4] = { yv.x, yv.y, yv.z, yv.w };
+#pragma unroll
+      for (int e = 0; e < 8; e++) {
+        m[e] = __uint_as_float(e & 1 ? u[e / 2] & 0xffff0000u : u[e / 2] << 16);
+        t[e] = m[e] > 0.0f ? acc[c][8 * h + e] : 0.0f;
+      }
+      o[h] = make_uint4(pack_bf16(t[0], t[1]), pack_bf16(t[2], t[3]), pack_bf16(t[4], t[5]),
+          pack_bf16(t[6], t[7]));
+    }
+  }
 }
 
 // ------------------------------------------------------------------ elementwise
@@ -313,78 +342,156 @@ __global__ void k_upsample(const bf16 *__restrict__ c, Vol fv, int C, bf16 *__re
   }
 }
 
-// G = bf16(dY * (Y > 0))
+// One thread per 8 channels of a cell in the kernels below: threads run over
+// the 8-channel groups of a row of cells, blocks over rows and planes (no
+// division of a flat index). groups: of a row.
+struct RowIndex {
+  int g, y;  // group in the row, row
+  int64_t zb, zstep;
+};
+
+__device__ __forceinline__ RowIndex row_index()
+{
+  return { (int)(blockIdx.x * blockDim.x + threadIdx.x), (int)blockIdx.y, (int64_t)blockIdx.z,
+    (int64_t)gridDim.z };
+}
+
+__device__ __forceinline__ void unpack8(uint4 w, float (&f)[8])
+{
+  const uint32_t u[4] = { w.x, w.y, w.z, w.w };
+#pragma unroll
+  for (int e = 0; e < 8; e++)  // BF16 is the upper half of a float
+    f[e] = __uint_as_float(e & 1 ? u[e / 2] & 0xffff0000u : u[e / 2] << 16);
+}
+
+__device__ __forceinline__ uint4 pack8(const float (&f)[8])
+{
+  return make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]),
+      pack_bf16(f[6], f[7]));
+}
+
+__device__ __forceinline__ void load8(const float *p, float (&f)[8])
+{
+  const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
+  f[0] = a.x;
+  f[1] = a.y;
+  f[2] = a.z;
+  f[3] = a.w;
+  f[4] = b.x;
+  f[5] = b.y;
+  f[6] = b.z;
+  f[7] = b.w;
+}
+
+// bf16(d * (Y > 0)) of 8 channels
+__device__ __forceinline__ uint4 masked8(const float (&d)[8], uint4 y)
+{
+  float m[8], r[8];
+  unpack8(y, m);
+#pragma unroll
+  for (int e = 0; e < 8; e++) r[e] = m[e] > 0.0f ? d[e] : 0.0f;
+  return pack8(r);
+}
+
+// G = bf16(dY * (Y > 0)), n groups of 8
 __global__ void k_relu_mask(const float *__restrict__ dy, const bf16 *__restrict__ y, int64_t n,
     bf16 *__restrict__ g)
 {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    g[i] = __float2bfloat16_rn(__bfloat162float(y[i]) > 0.0f ? dy[i] : 0.0f);
+       i += (int64_t)gridDim.x * blockDim.x) {
+    float d[8];
+    load8(dy + 8 * i, d);
+    reinterpret_cast<uint4 *>(g)[i] = masked8(d, reinterpret_cast<const uint4 *>(y)[i]);
+  }
 }
 
-// 2x2x2 mean of a [fine cells][C] BF16 volume; one thread per (coarse cell, channel)
-__global__ void k_pool(const bf16 *__restrict__ f, Vol fv, int C, bf16 *__restrict__ o)
+// 2x2x2 mean of a [fine cells][C] BF16 volume (grid over the coarse volume)
+__global__ void k_pool(const bf16 *__restrict__ f, Vol cv, int C, bf16 *__restrict__ o)
 {
-  const Vol cv = { fv.B, fv.Z / 2, fv.Y / 2, fv.X / 2 };
-  const int64_t n = cv.cells() * C;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int ch = (int)(i % C);
-    int b, z, y, x;
-    decompose(cv, i / C, b, z, y, x);
-    float s = 0.0f;
+  const int g8 = C / 8;
+  const RowIndex r = row_index();
+  if (r.g >= cv.X * g8) return;
+  const int x = r.g / g8, grp = r.g - x * g8;
+  for (int64_t zb = r.zb; zb < (int64_t)cv.B * cv.Z; zb += r.zstep) {
+    float s[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) s[e] = 0.0f;
+#pragma unroll
     for (int q = 0; q < 8; q++) {
-      const int64_t fc = (((int64_t)b * fv.Z + 2 * z + (q >> 2)) * fv.Y + 2 * y + ((q >> 1) & 1)) * fv.X +
-                         2 * x + (q & 1);
-      s += __bfloat162float(f[fc * C + ch]);
+      const int64_t fc =
+          ((2 * zb + (q >> 2)) * (2 * cv.Y) + 2 * r.y + ((q >> 1) & 1)) * (2 * cv.X) + 2 * x + (q & 1);
+      float v[8];
+      unpack8(reinterpret_cast<const uint4 *>(f)[fc * g8 + grp], v);
+#pragma unroll
+      for (int e = 0; e < 8; e++) s[e] += v[e];
     }
-    o[i] = __float2bfloat16_rn(s * 0.125f);
+#pragma unroll
+    for (int e = 0; e < 8; e++) s[e] *= 0.125f;
+    reinterpret_cast<uint4 *>(o)[((zb * cv.Y + r.y) * cv.X + x) * g8 + grp] = pack8(s);
   }
 }
 
-// fine gradient += coarse gradient / 8 (adjoint of the mean pool)
-__global__ void k_pool_back_add(const float *__restrict__ gc, Vol fv, int C, float *__restrict__ gf)
+// the masked gradient of a layer whose output went to the next layer's skip
+// (gf, fine) and to the mean pool (gc, coarse: a child's share is an eighth)
+__global__ void k_pool_back_mask(const float *__restrict__ gf, const float *__restrict__ gc, Vol fv,
+    int C, const bf16 *__restrict__ y, bf16 *__restrict__ g)
 {
-  const int64_t n = fv.cells() * C;
-  const Vol cv = { fv.B, fv.Z / 2, fv.Y / 2, fv.X / 2 };
+  const int g8 = C / 8;
+  const RowIndex r = row_index();
+  if (r.g >= fv.X * g8) return;
+  const int x = r.g / g8, grp = r.g - x * g8;
+  for (int64_t zb = r.zb; zb < (int64_t)fv.B * fv.Z; zb += r.zstep) {  // Z is even: (b, z / 2) is zb / 2
+    const int64_t i = ((zb * fv.Y + r.y) * fv.X + x) * g8 + grp;
+    const int64_t c = (((zb >> 1) * (fv.Y / 2) + (r.y >> 1)) * (fv.X / 2) + (x >> 1)) * g8 + grp;
+    float a[8], b[8];
+    load8(gf + 8 * i, a);
+    load8(gc + 8 * c, b);
+#pragma unroll
+    for (int e = 0; e < 8; e++) a[e] += 0.125f * b[e];
+    reinterpret_cast<uint4 *>(g)[i] = masked8(a, reinterpret_cast<const uint4 *>(y)[i]);
+  }
+}
+
+// the masked gradient of a layer whose output was upsampled: the sum over a
+// coarse cell's 8 children of the first Cu channels of a fine gradient of
+// `stride` channels (grid over the coarse volume)
+__global__ void k_up_back_mask(const float *__restrict__ d, int stride, Vol cv, int Cu,
+    const bf16 *__restrict__ y, bf16 *__restrict__ g)
+{
+  const int g8 = Cu / 8;
+  const RowIndex r = row_index();
+  if (r.g >= cv.X * g8) return;
+  const int x = r.g / g8, grp = r.g - x * g8;
+  for (int64_t zb = r.zb; zb < (int64_t)cv.B * cv.Z; zb += r.zstep) {
+    float s[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) s[e] = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const int64_t fc =
+          ((2 * zb + (q >> 2)) * (2 * cv.Y) + 2 * r.y + ((q >> 1) & 1)) * (2 * cv.X) + 2 * x + (q & 1);
+      float v[8];
+      load8(d + fc * stride + 8 * grp, v);
+#pragma unroll
+      for (int e = 0; e < 8; e++) s[e] += v[e];
+    }
+    const int64_t i = ((zb * cv.Y + r.y) * cv.X + x) * g8 + grp;
+    reinterpret_cast<uint4 *>(g)[i] = masked8(s, reinterpret_cast<const uint4 *>(y)[i]);
+  }
+}
+
+// the last Cs channels of a gradient of Cu + Cs channels, n groups of 8
+__global__ void k_skip_part(const float *__restrict__ dcat, int64_t n, int Cu, int Cs,
+    float *__restrict__ dskip)
+{
+  const int g8 = Cs / 8;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const int ch = (int)(i % C);
-    int b, z, y, x;
-    decompose(fv, i / C, b, z, y, x);
-    const int64_t cc = (((int64_t)b * cv.Z + z / 2) * cv.Y + y / 2) * cv.X + x / 2;
-    gf[i] += 0.125f * gc[cc * C + ch];
-  }
-}
-
-// split the gradient of a concat [up(coarse) Cu, skip Cs] at fine resolution:
-// skip part copied out, upsampled part summed over the 8 children (adjoint of
-// nearest upsampling)
-__global__ void k_split_concat(const float *__restrict__ dcat, Vol fv, int Cu, int Cs,
-    float *__restrict__ dskip, float *__restrict__ dcoarse)
-{
-  const int C = Cu + Cs;
-  const int64_t nskip = fv.cells() * Cs;
-  const Vol cv = { fv.B, fv.Z / 2, fv.Y / 2, fv.X / 2 };
-  const int64_t nup = cv.cells() * Cu;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nskip + nup;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    if (i < nskip) {
-      const int64_t c = i / Cs;
-      dskip[i] = dcat[c * C + Cu + (i % Cs)];
-    } else {
-      const int64_t k = i - nskip;
-      const int ch = (int)(k % Cu);
-      int b, z, y, x;
-      decompose(cv, k / Cu, b, z, y, x);
-      float s = 0.0f;
-      for (int q = 0; q < 8; q++) {
-        const int64_t fc = (((int64_t)b * fv.Z + 2 * z + (q >> 2)) * fv.Y + 2 * y + ((q >> 1) & 1)) *
-                               fv.X + 2 * x + (q & 1);
-        s += dcat[fc * C + ch];
-      }
-      dcoarse[k] = s;
-    }
+    const int64_t c = i / g8;
+    const float4 *s =
+        reinterpret_cast<const float4 *>(dcat + c * (Cu + Cs) + Cu + 8 * (i - c * g8));
+    reinterpret_cast<float4 *>(dskip)[2 * i] = s[0];
+    reinterpret_cast<float4 *>(dskip)[2 * i + 1] = s[1];
   }
 }
 
@@ -477,11 +584,12 @@ struct UNetState {
   int64_t cap0 = 0;  // level-0 cells the workspace holds
   bf16 *x = nullptr, *e0a = nullptr, *e0b = nullptr, *p0 = nullptr, *e1a = nullptr,
        *e1b = nullptr, *p1 = nullptr, *e2a = nullptr, *d1a = nullptr, *d1b = nullptr,
-       *d0a = nullptr, *d0b = nullptr, *G = nullptr;
+       *d0a = nullptr, *d0b = nullptr, *G = nullptr,
+       *G2 = nullptr;  // masked output gradient of the current layer, and of the next
   float *out = nullptr, *dout = nullptr, *F1 = nullptr, *F2 = nullptr, *Fe0b = nullptr,
         *Fe1b = nullptr, *partial = nullptr;
   int64_t partial_cap = 0;
-  bf16 *up1 = nullptr, *up0 = nullptr;  // materialised up(e2a) [n1][64], up(d1b) [n0][32]
+  bf16 *up1 = nullptr;                  // materialised up(e2a) [n1][64]
   bf16 *x16 = nullptr;                  // input zero-padded to 16 channels
   bf16 *w_first16 = nullptr, *w_last16 = nullptr;  // e0a and out weights padded to [27][16][16]
   int *err = nullptr;                   // device: a tensor-core kernel's wait timed out
@@ -526,10 +634,10 @@ bool ensure_workspace(UNetState *u, const Vol &v)
             dalloc(u, &u->p0, 16 * n1) && dalloc(u, &u->e1a, 32 * n1) && dalloc(u, &u->e1b, 32 * n1) &&
             dalloc(u, &u->p1, 32 * n2) && dalloc(u, &u->e2a, 64 * n2) && dalloc(u, &u->d1a, 32 * n1) &&
             dalloc(u, &u->d1b, 32 * n1) && dalloc(u, &u->d0a, 16 * n0) && dalloc(u, &u->d0b, 16 * n0) &&
-            dalloc(u, &u->G, 16 * n0) && dalloc(u, &u->out, n0) && dalloc(u, &u->dout, n0) &&
+            dalloc(u, &u->G, 16 * n0) && dalloc(u, &u->G2, 16 * n0) && dalloc(u, &u->out, n0) && dalloc(u, &u->dout, n0) &&
             dalloc(u, &u->F1, 48 * n0) && dalloc(u, &u->F2, 16 * n0) && dalloc(u, &u->Fe0b, 16 * n0) &&
             dalloc(u, &u->Fe1b, 32 * n1) && dalloc(u, &u->loss_partial, 1024) &&
-            dalloc(u, &u->up1, 64 * n1) && dalloc(u, &u->up0, 32 * n0) &&
+            dalloc(u, &u->up1, 64 * n1) &&
             dalloc(u, &u->x16, 16 * n0);
   if (!ok) return false;
   u->cap0 = n0;
@@ -577,14 +685,16 @@ bool fwd(UNetState *u, int l, const ConvSrc &s0, const ConvSrc &s1, const Vol &v
   const float *bias = u->master + u->b_off[l];
   if (tc_ok(u, v, kDesc[l].cout, s0.c, s1.c)) {
     const bf16 *a0 = s0.p;
-    if (s0.up) {  // the decoder's upsampled source, materialised at full resolution
-      bf16 *dst = s0.c == 64 ? u->up1 : u->up0;
-      k_upsample<<<blocks_for(v.cells() * (s0.c / 8)), 256, 0, stream()>>>(s0.p, v, s0.c, dst);
+    int up = s0.up;
+    if (up && !tc_conv_marches(kDesc[l].cout, s0.c + s1.c)) {
+      // the decoder's upsampled source, materialised at full resolution
+      k_upsample<<<blocks_for(v.cells() * (s0.c / 8)), 256, 0, stream()>>>(s0.p, v, s0.c, u->up1);
       if (!launched("k_upsample")) return false;
-      a0 = dst;
+      a0 = u->up1;
+      up = 0;
     }
-    return tc_conv(a0, s0.c, s1.p, s1.c, v.B, v.Z, v.Y, v.X, u->wb[l], kDesc[l].cout, bias, 1, true,
-        out, u->err);
+    return tc_conv(a0, s0.c, s1.p, s1.c, v.B, v.Z, v.Y, v.X, u->wb[l], kDesc[l].cout, bias, 1,
+        TC_BF16, out, u->err, up);
   }
   switch (kDesc[l].cout) {
   case 16: return conv_mma<16, true>(s0, s1, v, u->wb[l], bias, 1, out);
@@ -602,7 +712,7 @@ bool dgrad(UNetState *u, int l, const Vol &v, float *dx)
   const ConvSrc none = { nullptr, 0, 0 };
   if (tc_ok(u, v, kDesc[l].cin, kDesc[l].cout, 0))
     return tc_conv(u->G, kDesc[l].cout, nullptr, 0, v.B, v.Z, v.Y, v.X, u->wt[l], kDesc[l].cin,
-        nullptr, 0, false, dx, u->err);
+        nullptr, 0, TC_F32, dx, u->err);
   switch (kDesc[l].cin) {
   case 16: return conv_mma<16, false>(g, none, v, u->wt[l], nullptr, 0, dx);
   case 32: return conv_mma<32, false>(g, none, v, u->wt[l], nullptr, 0, dx);
@@ -624,23 +734,66 @@ bool wgrad(UNetState *u, int l, const ConvSrc &s0, const ConvSrc &s1, const Vol 
              v.X, u->partial, u->grad + u->w_off[l], u->grad + u->b_off[l]);
 }
 
+// the grid of the row-indexed kernels: 8-channel groups of a row, rows, planes
+dim3 row_grid(const Vol &v, int C)
+{
+  const int64_t planes = (int64_t)v.B * v.Z;
+  return dim3((v.X * (C / 8) + 127) / 128, v.Y, (unsigned)(planes < 65535 ? planes : 65535));
+}
+
+// n values, a multiple of 8
 bool mask(const float *dy, const bf16 *y, int64_t n, bf16 *g)
 {
-  k_relu_mask<<<blocks_for(n), 256, 0, stream()>>>(dy, y, n, g);
+  k_relu_mask<<<blocks_for(n / 8), 256, 0, stream()>>>(dy, y, n / 8, g);
   return launched("k_relu_mask");
 }
 
-bool pool_back(const float *gc, const Vol &fv, int C, float *gf)
+bool pool(const bf16 *f, const Vol &cv, int C, bf16 *o)
 {
-  k_pool_back_add<<<blocks_for(fv.cells() * C), 256, 0, stream()>>>(gc, fv, C, gf);
-  return launched("k_pool_back_add");
+  k_pool<<<row_grid(cv, C), 128, 0, stream()>>>(f, cv, C, o);
+  return launched("k_pool");
 }
 
-bool split(const float *dcat, const Vol &fv, int Cu, int Cs, float *dskip, float *dcoarse)
+bool pool_back_mask(const float *gf, const float *gc, const Vol &fv, int C, const bf16 *y, bf16 *g)
 {
-  const int64_t n = fv.cells() * Cs + fv.cells() / 8 * Cu;
-  k_split_concat<<<blocks_for(n), 256, 0, stream()>>>(dcat, fv, Cu, Cs, dskip, dcoarse);
-  return launched("k_split_concat");
+  k_pool_back_mask<<<row_grid(fv, C), 128, 0, stream()>>>(gf, gc, fv, C, y, g);
+  return launched("k_pool_back_mask");
+}
+
+// a layer's input gradient, masked by its input y (the layer before's output):
+// u->G becomes that layer's masked output gradient
+bool dgrad_mask(UNetState *u, int l, const Vol &v, const bf16 *y)
+{
+  const int n = kDesc[l].cin, c = kDesc[l].cout;
+  if (tc_ok(u, v, n, c, 0) && tc_conv_marches(n, c)) {
+    if (!tc_conv(u->G, c, nullptr, 0, v.B, v.Z, v.Y, v.X, u->wt[l], n, nullptr, 0, TC_MASKED, u->G2,
+            u->err, 0, y))
+      return false;
+    std::swap(u->G, u->G2);
+    return true;
+  }
+  return dgrad(u, l, v, u->F1) && mask(u->F1, y, n * v.cells(), u->G);
+}
+
+// the gradient of a concat [up(coarse) Cu, skip Cs]: the skip part to dskip,
+// the upsampled part masked by the coarse layer's output y to u->G
+bool dgrad_concat(UNetState *u, int l, const Vol &v, int Cu, int Cs, const bf16 *y, float *dskip)
+{
+  const int n = kDesc[l].cin, c = kDesc[l].cout;
+  const Vol cv = { v.B, v.Z / 2, v.Y / 2, v.X / 2 };
+  const bool split = Cu == 32 && Cs == 16 && tc_ok(u, v, n, c, 0) && tc_conv_marches(n, c);
+  if (split) {
+    if (!tc_conv(u->G, c, nullptr, 0, v.B, v.Z, v.Y, v.X, u->wt[l], n, nullptr, 0, TC_SPLIT, u->F1,
+            u->err, 0, nullptr, dskip))
+      return false;
+  } else {
+    const int64_t groups = v.cells() * (Cs / 8);
+    if (!dgrad(u, l, v, u->F1)) return false;
+    k_skip_part<<<blocks_for(groups), 256, 0, stream()>>>(u->F1, groups, Cu, Cs, dskip);
+    if (!launched("k_skip_part")) return false;
+  }
+  k_up_back_mask<<<row_grid(cv, Cu), 128, 0, stream()>>>(u->F1, split ? Cu : n, cv, Cu, y, u->G);
+  return launched("k_up_back_mask");
 }
 
 Vol half(const Vol &v) { return { v.B, v.Z / 2, v.Y / 2, v.X / 2 }; }
@@ -669,7 +822,7 @@ bool unet_forward(UNetState *u)
   const ConvSrc none = { nullptr, 0, 0 };
   if (tc_ok(u, v0, 16, 16, 0)) {
     if (!tc_conv(u->x16, 16, nullptr, 0, v0.B, v0.Z, v0.Y, v0.X, u->w_first16, 16,
-            u->master + u->b_off[L_E0A], 1, true, u->e0a, u->err))
+            u->master + u->b_off[L_E0A], 1, TC_BF16, u->e0a, u->err))
       return false;
   } else {
     k_conv_first<<<(unsigned)((n0 + 255) / 256), 256, 0, stream()>>>(u->x, v0, u->wb[L_E0A],
@@ -677,12 +830,10 @@ bool unet_forward(UNetState *u)
     if (!launched("k_conv_first")) return false;
   }
   if (!fwd(u, L_E0B, { u->e0a, 16, 0 }, none, v0, u->e0b)) return false;
-  k_pool<<<blocks_for(v1.cells() * 16), 256, 0, stream()>>>(u->e0b, v0, 16, u->p0);
-  if (!launched("k_pool")) return false;
+  if (!pool(u->e0b, v1, 16, u->p0)) return false;
   if (!fwd(u, L_E1A, { u->p0, 16, 0 }, none, v1, u->e1a)) return false;
   if (!fwd(u, L_E1B, { u->e1a, 32, 0 }, none, v1, u->e1b)) return false;
-  k_pool<<<blocks_for(v2.cells() * 32), 256, 0, stream()>>>(u->e1b, v1, 32, u->p1);
-  if (!launched("k_pool")) return false;
+  if (!pool(u->e1b, v2, 32, u->p1)) return false;
   if (!fwd(u, L_E2A, { u->p1, 32, 0 }, none, v2, u->e2a)) return false;
   if (!fwd(u, L_D1A, { u->e2a, 64, 1 }, { u->e1b, 32, 0 }, v1, u->d1a)) return false;
   if (!fwd(u, L_D1B, { u->d1a, 32, 0 }, none, v1, u->d1b)) return false;
@@ -690,7 +841,7 @@ bool unet_forward(UNetState *u)
   if (!fwd(u, L_D0B, { u->d0a, 16, 0 }, none, v0, u->d0b)) return false;
   if (tc_ok(u, v0, 16, 16, 0))
     return tc_conv(u->d0b, 16, nullptr, 0, v0.B, v0.Z, v0.Y, v0.X, u->w_last16, 16,
-        u->master + u->b_off[L_OUT], 0, false, u->out, u->err, 1);
+        u->master + u->b_off[L_OUT], 0, TC_ONE, u->out, u->err);
   k_conv_last<<<(unsigned)((n0 + 255) / 256), 256, 0, stream()>>>(u->d0b, v0, u->wb[L_OUT],
       u->master + u->b_off[L_OUT], u->out);
   return launched("k_conv_last");
@@ -700,7 +851,7 @@ bool unet_forward(UNetState *u)
 bool unet_backward(UNetState *u, const float *target)
 {
   const Vol v0 = u->vol, v1 = half(v0), v2 = half(v1);
-  const int64_t n0 = v0.cells(), n1 = v1.cells(), n2 = v2.cells();
+  const int64_t n0 = v0.cells();
   const ConvSrc none = { nullptr, 0, 0 };
   const int64_t lchunk = (n0 + 1023) / 1024 < 256 ? 256 : (n0 + 1023) / 1024;
   const int lblocks = (int)((n0 + lchunk - 1) / lchunk);
@@ -710,41 +861,34 @@ bool unet_backward(UNetState *u, const float *target)
   if (!launched("k_fold_loss")) return false;
   // out
   if (!wgrad(u, L_OUT, { u->d0b, 16, 0 }, none, v0, u->dout)) return false;
-  k_conv_last_dgrad<<<(unsigned)((n0 + 255) / 256), 256, 0, stream()>>>(u->dout, v0, u->wb[L_OUT],
-      u->F2);
+  k_conv_last_dgrad<<<(unsigned)((n0 / 4 + 127) / 128), 128, 0, stream()>>>(u->dout, v0,
+      u->wb[L_OUT], u->d0b, u->G);
   if (!launched("k_conv_last_dgrad")) return false;
   // d0b
-  if (!mask(u->F2, u->d0b, 16 * n0, u->G)) return false;
-  if (!wgrad(u, L_D0B, { u->d0a, 16, 0 }, none, v0) || !dgrad(u, L_D0B, v0, u->F1)) return false;
+  if (!wgrad(u, L_D0B, { u->d0a, 16, 0 }, none, v0) || !dgrad_mask(u, L_D0B, v0, u->d0a)) return false;
   // d0a (input concat [up(d1b) 32, e0b 16])
-  if (!mask(u->F1, u->d0a, 16 * n0, u->G)) return false;
-  if (!wgrad(u, L_D0A, { u->d1b, 32, 1 }, { u->e0b, 16, 0 }, v0) || !dgrad(u, L_D0A, v0, u->F1))
+  if (!wgrad(u, L_D0A, { u->d1b, 32, 1 }, { u->e0b, 16, 0 }, v0) ||
+      !dgrad_concat(u, L_D0A, v0, 32, 16, u->d1b, u->Fe0b))
     return false;
-  if (!split(u->F1, v0, 32, 16, u->Fe0b, u->F2)) return false;
   // d1b
-  if (!mask(u->F2, u->d1b, 32 * n1, u->G)) return false;
-  if (!wgrad(u, L_D1B, { u->d1a, 32, 0 }, none, v1) || !dgrad(u, L_D1B, v1, u->F1)) return false;
+  if (!wgrad(u, L_D1B, { u->d1a, 32, 0 }, none, v1) || !dgrad_mask(u, L_D1B, v1, u->d1a)) return false;
   // d1a (input concat [up(e2a) 64, e1b 32])
-  if (!mask(u->F1, u->d1a, 32 * n1, u->G)) return false;
-  if (!wgrad(u, L_D1A, { u->e2a, 64, 1 }, { u->e1b, 32, 0 }, v1) || !dgrad(u, L_D1A, v1, u->F2))
+  if (!wgrad(u, L_D1A, { u->e2a, 64, 1 }, { u->e1b, 32, 0 }, v1) ||
+      !dgrad_concat(u, L_D1A, v1, 64, 32, u->e2a, u->Fe1b))
     return false;
-  if (!split(u->F2, v1, 64, 32, u->Fe1b, u->F1)) return false;
-  // e2a
-  if (!mask(u->F1, u->e2a, 64 * n2, u->G)) return false;
-  if (!wgrad(u, L_E2A, { u->p1, 32, 0 }, none, v2) || !dgrad(u, L_E2A, v2, u->F2)) return false;
-  if (!pool_back(u->F2, v1, 32, u->Fe1b)) return false;
+  // e2a, whose input is the pooled e1b
+  if (!wgrad(u, L_E2A, { u->p1, 32, 0 }, none, v2) || !dgrad(u, L_E2A, v2, u->F2) ||
+      !pool_back_mask(u->Fe1b, u->F2, v1, 32, u->e1b, u->G))
+    return false;
   // e1b
-  if (!mask(u->Fe1b, u->e1b, 32 * n1, u->G)) return false;
-  if (!wgrad(u, L_E1B, { u->e1a, 32, 0 }, none, v1) || !dgrad(u, L_E1B, v1, u->F1)) return false;
-  // e1a
-  if (!mask(u->F1, u->e1a, 32 * n1, u->G)) return false;
-  if (!wgrad(u, L_E1A, { u->p0, 16, 0 }, none, v1) || !dgrad(u, L_E1A, v1, u->F2)) return false;
-  if (!pool_back(u->F2, v0, 16, u->Fe0b)) return false;
+  if (!wgrad(u, L_E1B, { u->e1a, 32, 0 }, none, v1) || !dgrad_mask(u, L_E1B, v1, u->e1a)) return false;
+  // e1a, whose input is the pooled e0b
+  if (!wgrad(u, L_E1A, { u->p0, 16, 0 }, none, v1) || !dgrad(u, L_E1A, v1, u->F2) ||
+      !pool_back_mask(u->Fe0b, u->F2, v0, 16, u->e0b, u->G))
+    return false;
   // e0b
-  if (!mask(u->Fe0b, u->e0b, 16 * n0, u->G)) return false;
-  if (!wgrad(u, L_E0B, { u->e0a, 16, 0 }, none, v0) || !dgrad(u, L_E0B, v0, u->F1)) return false;
+  if (!wgrad(u, L_E0B, { u->e0a, 16, 0 }, none, v0) || !dgrad_mask(u, L_E0B, v0, u->e0a)) return false;
   // e0a (no input gradient)
-  if (!mask(u->F1, u->e0a, 16 * n0, u->G)) return false;
   return wgrad(u, L_E0A, { u->x16, 16, 0 }, none, v0);
 }
 

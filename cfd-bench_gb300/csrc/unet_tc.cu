@@ -66,8 +66,7 @@ struct TcParams {
   const float *bias;     // [N] or nullptr
   int relu;
   int out_bf16;
-  int out_ch;            // leading channels stored per cell (N, or 1 for a padded 1-channel layer)
-  void *out;             // [cells][out_ch]
+  void *out;             // [cells][N]
   int *err;
 };
 
@@ -427,18 +426,12 @@ __global__ void __launch_bounds__(kThreads) k_conv_tc(const __grid_constant__ CU
       const Tile tl = tile_of(P, t);
       const int64_t cell =
           ((int64_t)tl.zb * P.Y + tl.y0 + (row & 7)) * P.X + tl.x0 + (row >> 3);
-      if (P.out_ch == 1) {  // one channel (the output layer, its weights padded to 16 rows)
-        const float x = v[0] + (P.bias ? __ldg(P.bias) : 0.0f);
-        static_cast<float *>(P.out)[cell] = P.relu ? fmaxf(x, 0.0f) : x;
-      } else {
 #pragma unroll
-        for (int c = 0; c < NCH; c++) {
-          const float x = v[c] + (P.bias ? __ldg(P.bias + c) : 0.0f);
-          v[c] = P.relu ? fmaxf(x, 0.0f) : x;
-        }
+      for (int c = 0; c < NCH; c++) {
+        const float x = v[c] + (P.bias ? __ldg(P.bias + c) : 0.0f);
+        v[c] = P.relu ? fmaxf(x, 0.0f) : x;
       }
-      if (P.out_ch == 1) {
-      } else if (P.out_bf16) {
+      if (P.out_bf16) {
         uint4 *o = reinterpret_cast<uint4 *>(static_cast<__nv_bfloat16 *>(P.out) + cell * NCH);
 #pragma unroll
         for (int c = 0; c < NCH; c += 8)
@@ -502,15 +495,16 @@ constexpr int kLoaders = 96;
 struct ColParams {
   const __nv_bfloat16 *s0, *s1;  // sources of C0 and C1 channels
   const __nv_bfloat16 *w;        // [27][N][C0 + C1]
-  int C0, C1;
+  int C0, C1, up0;               // up0: source 0 at half resolution, read by nearest upsampling
   int X, Y, Z, B;
   int tx, ty;      // columns per row and per plane
   int zl, zt;      // planes of a march, marches per column
   int items;
   int tmem_cols, groups;
   const float *bias;
-  int relu, out_bf16, out_ch;
-  void *out;
+  int relu, kind;  // TcOut
+  void *out, *out2;
+  const __nv_bfloat16 *mask;
   int *err;
 };
 
@@ -623,6 +617,9 @@ __global__ void __launch_bounds__(kColThreads) k_conv_col(const ColParams P)
 
   if (warp >= 1 && warp <= 3) {
     // ---------------- loads: one plane a slot ----------------
+    // this thread's chunks (a cell's 8 channels) of a plane: where they go, and
+    // per march where they come from (offset in the plane, -1: outside)
+    constexpr int kPer = (kInY * kInX * L::kHalves + kLoaders - 1) / kLoaders;
     const int t0 = tid - 32;
     int slot = 0, prev = -1;
     uint32_t phase = 0;
@@ -630,21 +627,36 @@ __global__ void __launch_bounds__(kColThreads) k_conv_col(const ColParams P)
     for (int t = blockIdx.x; ok && t < P.items; t += gridDim.x) {
       const March m = march_of(P, t);
       const int p1 = min(m.z1 + 1, P.Z - 1);
+      int from[kPer];
+#pragma unroll
+      for (int q = 0; q < kPer; q++) {
+        const int i = t0 + q * kLoaders;
+        const int h = i % L::kHalves, c = i / L::kHalves, cx = c % kInX, cy = c / kInX;
+        const int x = m.x0 - 1 + cx, y = m.y0 - 1 + cy;
+        const bool in = x >= 0 && x < P.X && y >= 0 && y < P.Y;
+        const bool second = 8 * h >= P.C0;
+        const int up = second ? 0 : P.up0;
+        const int cell = (y >> up) * (P.X >> up) + (x >> up);
+        from[q] = !in ? -1 : second ? cell * P.C1 + 8 * h - P.C0 : cell * P.C0 + 8 * h;
+      }
       for (int p = max(m.z0 - 1, 0); p <= p1; p++) {
         if (!mbar_wait(smem_u32(empty + slot), phase ^ 1u, abort_flag, P.err)) {
           ok = false;
           break;
         }
-        const int64_t row0 = ((int64_t)m.b * P.Z + p) * P.Y;
+        const int64_t zb = (int64_t)m.b * P.Z + p;
+        const __nv_bfloat16 *const b0 =
+            P.s0 + (P.up0 ? ((int64_t)m.b * (P.Z >> 1) + (p >> 1)) * (P.Y >> 1) * (P.X >> 1)
+                          : zb * P.Y * P.X) * P.C0;
+        const __nv_bfloat16 *const b1 = P.s1 + zb * P.Y * P.X * P.C1;
         const uint32_t dst0 = planes + (uint32_t)slot * L::kSlotB;
-        for (int i = t0; i < kInY * kInX * L::kHalves; i += kLoaders) {
+#pragma unroll
+        for (int q = 0; q < kPer; q++) {
+          const int i = t0 + q * kLoaders;
           const int h = i % L::kHalves, c = i / L::kHalves, cx = c % kInX, cy = c / kInX;
-          const int x = m.x0 - 1 + cx, y = m.y0 - 1 + cy;
-          const bool in = x >= 0 && x < P.X && y >= 0 && y < P.Y;
-          const bool second = 8 * h >= P.C0;
-          const int cs = second ? P.C1 : P.C0, ch = second ? 8 * h - P.C0 : 8 * h;
-          const __nv_bfloat16 *src =
-              (second ? P.s1 : P.s0) + (in ? ((row0 + y) * P.X + x) * cs + ch : 0);
+          if (q + 1 == kPer && i >= kInY * kInX * L::kHalves) continue;
+          const bool in = from[q] >= 0;
+          const __nv_bfloat16 *src = (8 * h >= P.C0 ? b1 : b0) + (in ? from[q] : 0);
           asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
                            dst0 + (uint32_t)(h * kGroupB + cy * kRowB + cx * 16)),
                        "l"(src), "r"(in ? 16 : 0)
@@ -762,27 +774,45 @@ __global__ void __launch_bounds__(kColThreads) k_conv_col(const ColParams P)
         mbar_arrive(smem_u32(acc_empty + g));
         if (!in) continue;
         const int64_t cell = (((int64_t)m.b * P.Z + z) * P.Y + y) * P.X + x;
-        if (P.out_ch == 1) {  // one channel (the output layer, its weights padded to 16 rows)
+        if (P.kind == TC_ONE) {  // the output layer, its weights padded to 16 rows
           const float r = v[0] + (P.bias ? __ldg(P.bias) : 0.0f);
           static_cast<float *>(P.out)[cell] = P.relu ? fmaxf(r, 0.0f) : r;
           continue;
         }
+        if (P.bias) {
 #pragma unroll
-        for (int c = 0; c < NCH; c++) {
-          const float r = v[c] + (P.bias ? __ldg(P.bias + c) : 0.0f);
-          v[c] = P.relu ? fmaxf(r, 0.0f) : r;
+          for (int c = 0; c < NCH; c++) v[c] += __ldg(P.bias + c);
         }
-        if (P.out_bf16) {
+        if (P.relu) {
+#pragma unroll
+          for (int c = 0; c < NCH; c++) v[c] = fmaxf(v[c], 0.0f);
+        }
+        if (P.kind == TC_MASKED) {
+          const uint4 *k = reinterpret_cast<const uint4 *>(P.mask + cell * NCH);
+#pragma unroll
+          for (int c = 0; c < NCH; c += 8) {
+            const uint4 w = __ldg(k + c / 8);
+            const uint32_t u[4] = { w.x, w.y, w.z, w.w };
+#pragma unroll
+            for (int e = 0; e < 8; e++) {  // as floats: BF16 is the upper half
+              const float f = __uint_as_float(e & 1 ? u[e / 2] & 0xffff0000u : u[e / 2] << 16);
+              v[c + e] = f > 0.0f ? v[c + e] : 0.0f;
+            }
+          }
+        }
+        if (P.kind == TC_BF16 || P.kind == TC_MASKED) {
           uint4 *o = reinterpret_cast<uint4 *>(static_cast<__nv_bfloat16 *>(P.out) + cell * NCH);
 #pragma unroll
           for (int c = 0; c < NCH; c += 8)
             o[c / 8] = make_uint4(pack2(v[c], v[c + 1]), pack2(v[c + 2], v[c + 3]),
                 pack2(v[c + 4], v[c + 5]), pack2(v[c + 6], v[c + 7]));
         } else {
-          float4 *o = reinterpret_cast<float4 *>(static_cast<float *>(P.out) + cell * NCH);
+          const bool split = P.kind == TC_SPLIT;
+          float4 *o = reinterpret_cast<float4 *>(static_cast<float *>(P.out) + cell * (split ? 32 : NCH));
+          float4 *o2 = reinterpret_cast<float4 *>(static_cast<float *>(P.out2) + cell * 16) - 8;
 #pragma unroll
           for (int c = 0; c < NCH; c += 4)
-            o[c / 4] = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+            (split && c >= 32 ? o2 : o)[c / 4] = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
         }
       }
     }
@@ -1029,10 +1059,46 @@ bool tc_conv_supported(int X, int Y, int Z, int B, int N, int C0, int C1)
   return encode_fn() != nullptr;
 }
 
+bool tc_conv_marches(int N, int C) { return col_layer(N, C); }
+
 bool tc_conv(const void *s0, int C0, const void *s1, int C1, int B, int Z, int Y, int X,
-    const void *w, int N, const float *bias, int relu, bool out_bf16, void *out, int *err,
-    int out_ch)
+    const void *w, int N, const float *bias, int relu, TcOut kind, void *out, int *err, int up0,
+    const void *mask, void *out2)
 {
+  if (col_layer(N, C0 + C1)) {
+    ColParams c{};
+    c.s0 = static_cast<const __nv_bfloat16 *>(s0);
+    c.s1 = static_cast<const __nv_bfloat16 *>(s1);
+    c.w = static_cast<const __nv_bfloat16 *>(w);
+    c.C0 = C0;
+    c.C1 = C1;
+    c.up0 = up0;
+    c.X = X;
+    c.Y = Y;
+    c.Z = Z;
+    c.B = B;
+    c.tx = (X + kColX - 1) / kColX;
+    c.ty = (Y + kColY - 1) / kColY;
+    c.bias = bias;
+    c.relu = relu;
+    c.kind = (int)kind;
+    c.out = out;
+    c.out2 = out2;
+    c.mask = static_cast<const __nv_bfloat16 *>(mask);
+    c.err = err;
+    switch (100 * N + C0 + C1) {
+    case 1616: return launch_col<16, 16>(c);
+    case 1632: return launch_col<16, 32>(c);
+    case 1648: return launch_col<16, 48>(c);
+    case 3216: return launch_col<32, 16>(c);
+    case 3232: return launch_col<32, 32>(c);
+    default: return launch_col<48, 16>(c);
+    }
+  }
+  if (up0 || (kind != TC_BF16 && kind != TC_F32)) {
+    fail(NUSIF_ERR_ARG, "unet: a form of convolution that %d -> %d channels has not", C0 + C1, N);
+    return false;
+  }
   TcParams P{};
   P.N = N;
   P.C0 = C0;
@@ -1046,42 +1112,9 @@ bool tc_conv(const void *s0, int C0, const void *s1, int C1, int B, int Z, int Y
   P.ntiles = (int)((int64_t)B * Z * P.ty * P.tx);
   P.bias = bias;
   P.relu = relu;
-  P.out_bf16 = out_bf16 ? 1 : 0;
-  P.out_ch = out_ch > 0 ? out_ch : N;
-  if (P.out_ch != N && !(P.out_ch == 1 && !out_bf16)) {
-    fail(NUSIF_ERR_ARG, "unet: a convolution stores all its channels or one FP32 channel");
-    return false;
-  }
+  P.out_bf16 = kind == TC_BF16 ? 1 : 0;
   P.out = out;
   P.err = err;
-  if (col_layer(N, C0 + C1)) {
-    ColParams c{};
-    c.s0 = static_cast<const __nv_bfloat16 *>(s0);
-    c.s1 = static_cast<const __nv_bfloat16 *>(s1);
-    c.w = static_cast<const __nv_bfloat16 *>(w);
-    c.C0 = C0;
-    c.C1 = C1;
-    c.X = X;
-    c.Y = Y;
-    c.Z = Z;
-    c.B = B;
-    c.tx = (X + kColX - 1) / kColX;
-    c.ty = (Y + kColY - 1) / kColY;
-    c.bias = bias;
-    c.relu = relu;
-    c.out_bf16 = P.out_bf16;
-    c.out_ch = P.out_ch;
-    c.out = out;
-    c.err = err;
-    switch (100 * N + C0 + C1) {
-    case 1616: return launch_col<16, 16>(c);
-    case 1632: return launch_col<16, 32>(c);
-    case 1648: return launch_col<16, 48>(c);
-    case 3216: return launch_col<32, 16>(c);
-    case 3232: return launch_col<32, 32>(c);
-    default: return launch_col<48, 16>(c);
-    }
-  }
   CUtensorMap a0, a1, w0, w1;
   if (!map_volume(&a0, s0, C0, X, Y, Z * B)) return false;
   if (!map_weights(&w0, w, C0 + C1, N, C0)) return false;
