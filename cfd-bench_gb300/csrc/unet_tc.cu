@@ -48,7 +48,7 @@ constexpr int kBoxX = kTileX + 2;       // loaded columns: the tile and one on e
 constexpr int kThreads = 192;  // warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 epilogue
 constexpr int kMaxStages = 16;
 constexpr uint32_t kBarBytes = 512;  // barrier and flag region at the start of shared memory
-constexpr uint64_t kWaitNs = 1000000000ull;  // bound of every mbarrier wait
+constexpr long long kWaitClocks = 2000000000ll;  // bound of every mbarrier wait: about a second
 
 struct TcParams {
   int N;                 // output channels (MMA N)
@@ -73,13 +73,6 @@ struct TcParams {
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
 {
   return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ uint64_t now_ns()
-{
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
 }
 
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
@@ -118,12 +111,13 @@ __device__ __forceinline__ bool mbar_try_sleep(uint32_t bar, uint32_t parity, ui
 __device__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *err)
 {
   if (mbar_try(bar, parity)) return true;
-  const uint64_t t0 = now_ns();
+  long long t0 = 0;
   for (uint32_t round = 1;; round++) {
     if (mbar_try_sleep(bar, parity, 20000u)) return true;
     if ((round & 7u) == 0) {
       if (*abort_flag) return false;
-      if (now_ns() - t0 > kWaitNs) {
+      if (t0 == 0) t0 = clock64();
+      if (clock64() - t0 > kWaitClocks) {
         *abort_flag = 1;
         atomicExch(err, 1);
         return false;
@@ -135,8 +129,8 @@ __device__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_fla
 // bounded wait used while draining after an abort (does not re-raise it)
 __device__ void mbar_drain(uint32_t bar, uint32_t parity)
 {
-  const uint64_t t0 = now_ns();
-  while (!mbar_try(bar, parity) && now_ns() - t0 < kWaitNs) {
+  const long long t0 = clock64();
+  while (!mbar_try(bar, parity) && clock64() - t0 < kWaitClocks) {
   }
 }
 
@@ -500,7 +494,6 @@ struct ColParams {
   int tx, ty;      // columns per row and per plane
   int zl, zt;      // planes of a march, marches per column
   int items;
-  int tmem_cols, groups;
   const float *bias;
   int relu, kind;  // TcOut
   void *out, *out2;
@@ -556,6 +549,8 @@ struct Col {
   static constexpr uint32_t kSlotB = kHalves * kGroupB;
   static constexpr uint32_t kTapB = kHalves * 3 * NCH * 16;  // weights of one (dy, dx)
   static constexpr uint32_t kWeightB = 9 * kTapB;
+  static constexpr int kCols = NCH == 16 ? 128 : 256;  // tensor-memory columns of a block
+  static constexpr int kGroups = kCols / NCH < kMaxGroups ? kCols / NCH : kMaxGroups;
   static constexpr size_t kSmem = kBarBytes + 128 + kWeightB + kSlotsC * kSlotB;
 };
 
@@ -588,7 +583,7 @@ __global__ void __launch_bounds__(kColThreads) k_conv_col(const ColParams P)
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
-                 "r"(P.tmem_cols)
+                 "r"(L::kCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -607,7 +602,7 @@ __global__ void __launch_bounds__(kColThreads) k_conv_col(const ColParams P)
   fence_after();
   const uint32_t tmem = *tmem_slot;
   if (warp >= 4) {  // every group starts from zeros
-    for (int c = 0; c < P.groups * NCH; c += 16)
+    for (int c = 0; c < L::kGroups * NCH; c += 16)
       tmem_zero16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)c);
     tmem_wait_st();
   }
@@ -682,52 +677,74 @@ __global__ void __launch_bounds__(kColThreads) k_conv_col(const ColParams P)
     }
   } else if (warp == 0 && lane == 0) {
     // ---------------- products ----------------
+    // One thread's instructions are the pace of a block here, so rings are
+    // counted, not divided, and every descriptor is a constant away from two.
+    constexpr int G = L::kGroups;
     int slot = 0;
     uint32_t phase = 0;
-    int seq = 0;  // output planes opened so far; plane number q of them uses group q % groups
+    int fresh = 0;            // group of the next output plane to open
+    uint32_t fresh_phase = 1; // parity its drained barrier is waited for
+    int done = 0;             // group of the next output plane to finish
     bool ok = true, issued = false;
     const uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTileM >> 4) << 24);
     for (int t = blockIdx.x; ok && t < P.items; t += gridDim.x) {
       const March m = march_of(P, t);
-      const int q0 = seq;  // the number of output plane z0
       const int p1 = min(m.z1 + 1, P.Z - 1);
+      int ga = fresh;     // group of the lowest output plane in the window
+      int opened = m.z0;  // the next output plane to open
       for (int p = max(m.z0 - 1, 0); p <= p1; p++) {
         const int za = max(p - 1, m.z0), zb = min(p + 1, m.z1);  // output planes of this one
-        while (ok && seq <= q0 + zb - m.z0) {  // groups entering the window are drained and zero
-          const int g = seq % P.groups;
-          ok = mbar_wait(smem_u32(acc_empty + g), ((uint32_t)(seq / P.groups) & 1u) ^ 1u, abort_flag,
-              P.err);
-          seq++;
+        if (p - 1 > m.z0) ga = ga + 1 == G ? 0 : ga + 1;
+        while (ok && opened <= zb) {  // groups entering the window are drained and zero
+          ok = mbar_wait(smem_u32(acc_empty + fresh), fresh_phase, abort_flag, P.err);
+          opened++;
+          if (++fresh == G) {
+            fresh = 0;
+            fresh_phase ^= 1u;
+          }
         }
         if (!ok || !mbar_wait(smem_u32(full + slot), phase, abort_flag, P.err)) {
           ok = false;
           break;
         }
         fence_after();
-        const int ga = (q0 + za - m.z0) % P.groups, cnt = zb - za + 1;
-        const int n1 = min(cnt, P.groups - ga), n2 = cnt - n1;  // groups up to the ring's end, and after
+        const int cnt = zb - za + 1;
+        const int n1 = min(cnt, G - ga), n2 = cnt - n1;  // groups up to the ring's end, and after
         const uint32_t d1 = tmem + (uint32_t)(ga * NCH);
         const uint32_t i1 = idesc0 | ((uint32_t)(n1 * NCH >> 3) << 17);
-        const uint32_t i2 = idesc0 | ((uint32_t)(n2 * NCH >> 3) << 17);
         const uint64_t a0 =
             smem_desc_plain(planes + (uint32_t)slot * L::kSlotB, kGroupB, kRowB);
         const uint64_t b0 = smem_desc_plain(
             weights + (uint32_t)((za - (p - 1)) * NCH * 16), 3 * NCH * 16, 128);
-        for (int dy = 0; dy < 3; dy++)
-          for (int dx = 0; dx < 3; dx++) {
+        const auto a_at = [](int q, int j) {
+          return (uint64_t)((j * 2 * kGroupB + q / 3 * kRowB + q % 3 * 16) >> 4);
+        };
+        const auto b_at = [](int q, int j) {
+          return (uint64_t)((q * (int)L::kTapB + j * 2 * 3 * NCH * 16) >> 4);
+        };
+        if (n2 == 0) {
+#pragma unroll
+          for (int q = 0; q < 9; q++)
+#pragma unroll
+            for (int j = 0; j < CIN / 16; j++)
+              mma_f16(d1, a0 + a_at(q, j), b0 + b_at(q, j), i1, 1u);
+        } else {
+          const uint32_t i2 = idesc0 | ((uint32_t)(n2 * NCH >> 3) << 17);
+          const uint64_t b2 = b0 + (uint64_t)(n1 * NCH);
+#pragma unroll
+          for (int q = 0; q < 9; q++)
 #pragma unroll
             for (int j = 0; j < CIN / 16; j++) {
-              const uint64_t a = a0 + (uint64_t)((j * 2 * kGroupB + dy * kRowB + dx * 16) >> 4);
-              const uint64_t b =
-                  b0 + (uint64_t)(((dy * 3 + dx) * (int)L::kTapB + j * 2 * 3 * NCH * 16) >> 4);
-              mma_f16(d1, a, b, i1, 1u);
-              if (n2 > 0) mma_f16(tmem, a, b + (uint64_t)(n1 * NCH), i2, 1u);
+              mma_f16(d1, a0 + a_at(q, j), b0 + b_at(q, j), i1, 1u);
+              mma_f16(tmem, a0 + a_at(q, j), b2 + b_at(q, j), i2, 1u);
             }
-          }
+        }
         issued = true;
         mma_commit(smem_u32(empty + slot));
-        if (p - 1 >= m.z0) mma_commit(smem_u32(acc_full + (q0 + p - 1 - m.z0) % P.groups));
-        if (p == p1 && p1 == m.z1) mma_commit(smem_u32(acc_full + (q0 + p - m.z0) % P.groups));
+        for (int z = max(p - 1, m.z0); z <= (p == p1 ? m.z1 : p - 1); z++) {
+          mma_commit(smem_u32(acc_full + done));
+          if (++done == G) done = 0;
+        }
         if (++slot == kSlotsC) {
           slot = 0;
           phase ^= 1u;
@@ -742,16 +759,19 @@ __global__ void __launch_bounds__(kColThreads) k_conv_col(const ColParams P)
   } else if (warp >= 4) {
     // ---------------- epilogue: tensor memory -> bias, ReLU -> global ----------------
     const int q = warp & 3, row = 32 * q + lane;  // accumulator row: 8 y + x in the column
-    int seq = 0;
+    int g = L::kGroups - 1;
+    uint32_t phase = 1;
     bool ok = true;
     for (int t = blockIdx.x; ok && t < P.items; t += gridDim.x) {
       const March m = march_of(P, t);
       const int x = m.x0 + (row & 7), y = m.y0 + (row >> 3);
       const bool in = x < P.X && y < P.Y;
-      for (int z = m.z0; z <= m.z1; z++, seq++) {
-        const int g = seq % P.groups;
-        const bool ready = mbar_wait(smem_u32(acc_full + g), (uint32_t)(seq / P.groups) & 1u,
-            abort_flag, P.err);
+      for (int z = m.z0; z <= m.z1; z++) {
+        if (++g == L::kGroups) {
+          g = 0;
+          phase ^= 1u;
+        }
+        const bool ready = mbar_wait(smem_u32(acc_full + g), phase, abort_flag, P.err);
         if (!__all_sync(0xffffffffu, ready)) {
           ok = false;
           break;
@@ -823,7 +843,7 @@ __global__ void __launch_bounds__(kColThreads) k_conv_col(const ColParams P)
     __syncwarp();
     fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"(P.tmem_cols)
+                 "r"(L::kCols)
                  : "memory");
   }
 }
@@ -991,8 +1011,6 @@ template <int NCH, int CIN>
 bool launch_col(ColParams P)
 {
   using L = Col<NCH, CIN>;
-  P.tmem_cols = NCH == 16 ? 128 : 256;
-  P.groups = P.tmem_cols / NCH < kMaxGroups ? P.tmem_cols / NCH : kMaxGroups;
   static bool attr_set[64] = {};
   int dev = 0;
   if (!cuda_ok(cudaGetDevice(&dev), "cudaGetDevice")) return false;
@@ -1014,7 +1032,7 @@ bool launch_col(ColParams P)
   }
   int per_sm = (int)((228 * 1024) / (L::kSmem + 1024));
   if (per_sm > 65536 / regs) per_sm = 65536 / regs;
-  if (per_sm > 512 / P.tmem_cols) per_sm = 512 / P.tmem_cols;
+  if (per_sm > 512 / L::kCols) per_sm = 512 / L::kCols;
   if (per_sm < 1) per_sm = 1;
   const int wave = sm_count_tc() * per_sm;
   // planes of a march: the least (marches of the busiest block) x (planes + 2
