@@ -1408,38 +1408,64 @@ __global__ void __launch_bounds__(kNT) k_mg_prolong_x2(View<T> f, const T *xc, i
 }
 
 // Coarsest level: `sweeps` red-black Gauss-Seidel sweeps from zero by one
-// block, the level held in shared memory (compact layout).
-template <typename T>
-__global__ void __launch_bounds__(512) k_mg_coarse(View<T> v, int sweeps, const MgState *st)
+// block, x in shared memory (compact layout). A thread keeps R cells of each
+// colour for all sweeps: their values, right-hand sides and the shared-memory
+// offsets of their neighbours (their own at a wall), two to a register. One
+// block's issue bounds it: 64 sweeps of 15 x 9 x 21 cells 92 -> 21 us (with
+// the cells found by division in every pass before).
+template <typename T, int R>
+__global__ void __launch_bounds__(1024) k_mg_coarse(View<T> v, int sweeps, const MgState *st)
 {
   if (mg_done(st)) return;
   extern __shared__ unsigned char smem_raw[];
-  T *xs = reinterpret_cast<T *>(smem_raw);
-  T *bs = xs + (int64_t)v.nx * v.ny * v.nz;
-  const int n = v.nx * v.ny * v.nz;
-  for (int q = threadIdx.x; q < n; q += blockDim.x) {
-    xs[q] = 0;
-    bs[q] = v.b[q];
+  const int nx = v.nx, ny = v.ny, nz = v.nz, np = (nx + 1) / 2;  // pairs of cells per row
+  const auto at = [&](unsigned o) -> T & { return *reinterpret_cast<T *>(smem_raw + o); };
+  unsigned own[2][R], xo[2][R], yo[2][R], zo[2][R];
+  T x[2][R], b[2][R];
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const int t = threadIdx.x + r * blockDim.x;
+    const int p = t % np, jk = t / np, j = jk % ny, k = jk / ny;
+#pragma unroll
+    for (int c = 0; c < 2; c++) {  // first colour: (i + j + k) even
+      const int i = 2 * p + ((j + k + c) & 1);
+      const bool in = k < nz && i < nx;
+      const int q = i + nx * (j + ny * k);
+      const auto off = [&](int cell) { return (unsigned)(cell * (int)sizeof(T)); };
+      own[c][r] = in ? off(q) : 0xffffffffu;
+      if (!in) continue;
+      xo[c][r] = off(i > 0 ? q - 1 : q) | off(i < nx - 1 ? q + 1 : q) << 16;
+      yo[c][r] = off(j > 0 ? q - nx : q) | off(j < ny - 1 ? q + nx : q) << 16;
+      zo[c][r] = off(k > 0 ? q - nx * ny : q) | off(k < nz - 1 ? q + nx * ny : q) << 16;
+      b[c][r] = v.b[q];
+      x[c][r] = (T)0;
+      at(own[c][r]) = (T)0;
+    }
   }
   __syncthreads();
-  View<T> s = v;
-  s.x = xs;
-  s.sy = v.nx;
-  s.sz = v.nx * v.ny;
-  s.off = 0;
   for (int it = 0; it < sweeps; it++) {
-    for (int colour = 1; colour >= 0; colour--) {
-      for (int q = threadIdx.x; q < n; q += blockDim.x) {
-        const int i = q % v.nx, j = (q / v.nx) % v.ny, k = q / (v.nx * v.ny);
-        if (((i + j + k + 3) & 1) != colour) continue;
-        const T xc = xs[q];
-        const T r = bs[q] - lap_at(s, xs, i, j, k, q, xc);
-        xs[q] = xc - r * s.inv_diag;
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        if (own[c][r] == 0xffffffffu) continue;
+        const T xc = x[c][r];
+        const T sx = at(xo[c][r] & 0xffffu) + at(xo[c][r] >> 16);
+        const T sy = at(yo[c][r] & 0xffffu) + at(yo[c][r] >> 16);
+        const T sz = at(zo[c][r] & 0xffffu) + at(zo[c][r] >> 16);
+        const T lap = sx * v.ex + sy * v.ey + sz * v.ez - v.diag * xc;
+        const T res = b[c][r] - lap;
+        x[c][r] = xc - res * v.inv_diag;
+        at(own[c][r]) = x[c][r];
       }
       __syncthreads();
     }
   }
-  for (int q = threadIdx.x; q < n; q += blockDim.x) v.x[q] = xs[q];
+#pragma unroll
+  for (int r = 0; r < R; r++)
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+      if (own[c][r] != 0xffffffffu) v.x[own[c][r] / sizeof(T)] = x[c][r];
 }
 
 // Coarsest level, exact: x = Minv * b with Minv the inverse of the coarsest
@@ -2044,9 +2070,17 @@ bool coarse_solve(const View<T> &v, int nsweeps, const MgState *st, const T *min
         st);
     return launched("k_mg_direct");
   }
-  const size_t bytes = 2 * n * sizeof(T);
-  if (bytes <= 48 * 1024) {
-    k_mg_coarse<T><<<1, 512, bytes, stream()>>>(v, nsweeps, st);
+  const size_t bytes = n * sizeof(T);
+  if (bytes <= 24 * 1024) {  // at most 6144 cells: three of each colour per thread
+    const int items = (v.nx + 1) / 2 * v.ny * v.nz;
+    const int r = (items + 1023) / 1024;
+    const int threads = ((items + r - 1) / r + 31) / 32 * 32;
+    switch (r) {
+    case 1: k_mg_coarse<T, 1><<<1, threads, bytes, stream()>>>(v, nsweeps, st); break;
+    case 2: k_mg_coarse<T, 2><<<1, threads, bytes, stream()>>>(v, nsweeps, st); break;
+    case 3: k_mg_coarse<T, 3><<<1, threads, bytes, stream()>>>(v, nsweeps, st); break;
+    default: k_mg_coarse<T, 6><<<1, threads, bytes, stream()>>>(v, nsweeps, st); break;
+    }
     return launched("k_mg_coarse");
   }
   // larger coarsest grids: sweeps in global memory
