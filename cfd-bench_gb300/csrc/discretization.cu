@@ -47,18 +47,74 @@ __global__ void k_fill(double *a, int64_t n, double value)
     a[q] = value;
 }
 
+// The block's largest keys (fp_bits.cuh) of three fields, in every thread of
+// warp 0. Keys stay 32-bit pairs on the integer pipe: a block-wide FP64 maximum
+// would cost microseconds at GB300's FP64 rate.
+struct Key3 {
+  unsigned h[3], l[3];
+};
+
+__device__ __forceinline__ void warp_key_max3(Key3 &k)
+{
+#pragma unroll
+  for (int f = 0; f < 3; f++) warp_key_max(k.h[f], k.l[f]);
+}
+
+__device__ __forceinline__ void block_key_max3(Key3 &k, Key3 (&sm)[kBlock / 32])
+{
+  const int t = flat_tid();
+  warp_key_max3(k);
+  __syncthreads();
+  if ((t & 31) == 0) sm[t >> 5] = k;
+  __syncthreads();
+  if (t >= 32) return;
+  k = sm[t < kBlock / 32 ? t : 0];
+  warp_key_max3(k);
+}
+
+__device__ __forceinline__ unsigned long long key_word(const Key3 &k, int f)
+{
+  return ((unsigned long long)k.h[f] << 32) | k.l[f];
+}
+
+__device__ __forceinline__ void key_word_max(Key3 &k, int f, unsigned long long w)
+{
+  key_max(k.h[f], k.l[f], (unsigned)(w >> 32), (unsigned)w);
+}
+
+// publishes a block's keys; the last block returns true with the grid's keys
+// in warp 0 (partials: 3 words per block)
+__device__ __forceinline__ bool grid_key_max3(Key3 &k, Key3 (&sm)[kBlock / 32],
+    unsigned long long *partials, unsigned *ticket)
+{
+  __shared__ bool last;
+  block_key_max3(k, sm);
+  if (threadIdx.x == 0) {
+    for (int f = 0; f < 3; f++) partials[3 * blockIdx.x + f] = key_word(k, f);
+    last = ticket_is_last(ticket);
+  }
+  __syncthreads();
+  if (!last) return false;
+  for (int q = threadIdx.x; q < (int)gridDim.x; q += kBlock)
+#pragma unroll
+    for (int f = 0; f < 3; f++) key_word_max(k, f, __ldcg(partials + 3 * q + f));
+  return true;
+}
+
 // ---- max |u|, |v|, |w| over the padded arrays (discretization.c:391-401) ----
-// Seeded with DBL_MIN like the reference. Threads compare |x| as bit patterns
-// on the integer pipe (abs_max_key: non-negative doubles order like their
-// bits, NaN skipped as the reference's `>` test skips it), so the FP64 pipe
-// stays free; block maxima go to partials as doubles and the last block
-// folds them.
+// Seeded with DBL_MIN like the reference. |x| is compared as bit patterns
+// (abs_max_key: non-negative doubles order like their bits, NaN skipped as the
+// reference's `>` test skips it); the last block folds the blocks' keys.
 __global__ void __launch_bounds__(kBlock) k_max3(const double *__restrict__ u,
     const double *__restrict__ v, const double *__restrict__ w, int64_t n,
-    double *__restrict__ partials, unsigned *ticket, double *__restrict__ out3)
+    unsigned long long *__restrict__ partials, unsigned *ticket, double *__restrict__ out3)
 {
-  // running maxima as bit-pattern pairs (high, low), seeded with DBL_MIN
-  unsigned uh = 0x00100000u, ul = 0u, vh = 0x00100000u, vl = 0u, wh = 0x00100000u, wl = 0u;
+  Key3 k;  // seeded with DBL_MIN
+#pragma unroll
+  for (int f = 0; f < 3; f++) {
+    k.h[f] = 0x00100000u;
+    k.l[f] = 0u;
+  }
   const int64_t stride = (int64_t)gridDim.x * kBlock;
   // pairs of doubles (cudaMalloc bases are 256-byte aligned)
   const int64_t npair = n / 2;
@@ -67,55 +123,115 @@ __global__ void __launch_bounds__(kBlock) k_max3(const double *__restrict__ u,
   const double2 *w2 = reinterpret_cast<const double2 *>(w);
   for (int64_t q = blockIdx.x * (int64_t)kBlock + threadIdx.x; q < npair; q += stride) {
     double2 a = __ldg(u2 + q), b = __ldg(v2 + q), c = __ldg(w2 + q);
-    abs_max_key(uh, ul, a.x);
-    abs_max_key(uh, ul, a.y);
-    abs_max_key(vh, vl, b.x);
-    abs_max_key(vh, vl, b.y);
-    abs_max_key(wh, wl, c.x);
-    abs_max_key(wh, wl, c.y);
+    abs_max_key(k.h[0], k.l[0], a.x);
+    abs_max_key(k.h[0], k.l[0], a.y);
+    abs_max_key(k.h[1], k.l[1], b.x);
+    abs_max_key(k.h[1], k.l[1], b.y);
+    abs_max_key(k.h[2], k.l[2], c.x);
+    abs_max_key(k.h[2], k.l[2], c.y);
   }
   if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
-    abs_max_key(uh, ul, u[n - 1]);
-    abs_max_key(vh, vl, v[n - 1]);
-    abs_max_key(wh, wl, w[n - 1]);
+    abs_max_key(k.h[0], k.l[0], u[n - 1]);
+    abs_max_key(k.h[1], k.l[1], v[n - 1]);
+    abs_max_key(k.h[2], k.l[2], w[n - 1]);
   }
-  double mu = __hiloint2double((int)uh, (int)ul), mv = __hiloint2double((int)vh, (int)vl),
-         mw = __hiloint2double((int)wh, (int)wl);
-  __shared__ double sm[3][kBlock / 32];
-  mu = block_reduce_max<kBlock>(mu, sm[0]);
-  mv = block_reduce_max<kBlock>(mv, sm[1]);
-  mw = block_reduce_max<kBlock>(mw, sm[2]);
-  __shared__ bool last;
+  __shared__ Key3 sm[kBlock / 32];
+  if (!grid_key_max3(k, sm, partials, ticket)) return;
+  block_key_max3(k, sm);
   if (threadIdx.x == 0) {
-    partials[3 * blockIdx.x + 0] = mu;
-    partials[3 * blockIdx.x + 1] = mv;
-    partials[3 * blockIdx.x + 2] = mw;
-    last = ticket_is_last(ticket);
-  }
-  __syncthreads();
-  if (!last) return;
-  double a = DBL_MIN, b = DBL_MIN, c = DBL_MIN;
-  for (int q = threadIdx.x; q < (int)gridDim.x; q += kBlock) {
-    a = fmax(a, ld_cg(partials + 3 * q + 0));
-    b = fmax(b, ld_cg(partials + 3 * q + 1));
-    c = fmax(c, ld_cg(partials + 3 * q + 2));
-  }
-  a = block_reduce_max<kBlock>(a, sm[0]);
-  b = block_reduce_max<kBlock>(b, sm[1]);
-  c = block_reduce_max<kBlock>(c, sm[2]);
-  if (threadIdx.x == 0) {
-    out3[0] = a;
-    out3[1] = b;
-    out3[2] = c;
+    for (int f = 0; f < 3; f++) out3[f] = __hiloint2double((int)k.h[f], (int)k.l[f]);
     *ticket = 0;
   }
 }
 
-// ---- velocity boundary conditions, one face per launch (discretization.c:119-332) ----
+// ---- velocity boundary conditions (discretization.c:119-332) ----
 // The normal component lives on the wall face (index 0 or n), the tangential
 // components have a ghost cell (0 or n+1) mirrored from the first interior
-// cell. Faces run in the reference order (top, bottom, left, right, front,
-// back) as separate launches: later faces read edge values earlier ones wrote.
+// cell. The reference applies the faces in the order top, bottom, left,
+// right, front, back, and a later face reads what an earlier one wrote. In one
+// launch that order is kept by value:
+//  - only three sets of cells that any face reads are written, the normal
+//    components on the high walls: v at jmax (top), u at imax (right), w at
+//    kmax (back);
+//  - a face later in the order than the writer takes the value the writer
+//    gives (it knows it: zero, or the cell before the wall);
+//  - a face earlier in the order needs the old value, so the writer's thread,
+//    which reads it before it overwrites it, stores that face's ghost too.
+// Grids with an axis of one cell (where the cell before the wall is itself a
+// wall) take k_face, one launch per face: 20 us of launches at 256^3 against 6.
+struct Faces {
+  Dims g;
+  int bc[6];  // top, bottom, left, right, front, back
+};
+
+__device__ __forceinline__ bool face_active(int bc) { return bc == NOSLIP || bc == SLIP || bc == OUTFLOW; }
+__device__ __forceinline__ double face_mirror(int bc, double in) { return bc == NOSLIP ? -in : in; }
+
+__global__ void k_faces(Faces A, double *__restrict__ u, double *__restrict__ v,
+    double *__restrict__ w)
+{
+  enum { TOP, BOTTOM, LEFT, RIGHT, FRONT, BACK };
+  const Dims &g = A.g;
+  const int face = blockIdx.z, bc = A.bc[face];
+  if (!face_active(bc)) return;
+  const int ni = g.imax, nj = g.jmax, nk = g.kmax;
+  const int a = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  const int b = blockIdx.y * blockDim.y + threadIdx.y + 1;
+  // the value v at (i, jmax, k) has after the top face, u at (imax, j, k) after the right one
+  const auto top_v = [&](int64_t c) {  // c: the cell at jmax
+    return !face_active(A.bc[TOP]) ? v[c] : A.bc[TOP] == OUTFLOW ? v[c - g.sj] : 0.0;
+  };
+  const auto right_u = [&](int64_t c) {  // c: the cell at imax
+    return !face_active(A.bc[RIGHT]) ? u[c] : A.bc[RIGHT] == OUTFLOW ? u[c - 1] : 0.0;
+  };
+  if (face <= BOTTOM) {
+    const int i = a, k = b;
+    if (i > ni || k > nk) return;
+    const int64_t row = (int64_t)k * g.sk + i;
+    const int64_t in = row + (int64_t)(face == TOP ? nj : 1) * g.sj;
+    const int64_t ghost = row + (int64_t)(face == TOP ? nj + 1 : 0) * g.sj;
+    if (face == TOP) v[in] = bc == OUTFLOW ? v[in - g.sj] : 0.0;
+    else v[ghost] = bc == OUTFLOW ? v[in] : 0.0;
+    if (!(i == ni && face_active(A.bc[RIGHT]))) u[ghost] = face_mirror(bc, u[in]);
+    if (!(k == nk && face_active(A.bc[BACK]))) w[ghost] = face_mirror(bc, w[in]);
+  } else if (face <= RIGHT) {
+    const int j = a, k = b;
+    if (j > nj || k > nk) return;
+    const int64_t row = (int64_t)k * g.sk + (int64_t)j * g.sj;
+    const int64_t in = row + (face == RIGHT ? ni : 1);
+    const int64_t ghost = row + (face == RIGHT ? ni + 1 : 0);
+    if (face == RIGHT) {
+      const double old = u[in];  // what the top and bottom faces mirror
+      if (j == nj && face_active(A.bc[TOP])) u[in + g.sj] = face_mirror(A.bc[TOP], old);
+      if (j == 1 && face_active(A.bc[BOTTOM])) u[in - g.sj] = face_mirror(A.bc[BOTTOM], old);
+      u[in] = bc == OUTFLOW ? u[in - 1] : 0.0;
+    } else {
+      u[ghost] = bc == OUTFLOW ? u[in] : 0.0;
+    }
+    v[ghost] = face_mirror(bc, j == nj ? top_v(in) : v[in]);
+    if (!(k == nk && face_active(A.bc[BACK]))) w[ghost] = face_mirror(bc, w[in]);
+  } else {
+    const int i = a, j = b;
+    if (i > ni || j > nj) return;
+    const int64_t row = (int64_t)j * g.sj + i;
+    const int64_t in = row + (int64_t)(face == BACK ? nk : 1) * g.sk;
+    const int64_t ghost = row + (int64_t)(face == BACK ? nk + 1 : 0) * g.sk;
+    if (face == BACK) {
+      const double old = w[in];  // what the four side faces mirror
+      if (j == nj && face_active(A.bc[TOP])) w[in + g.sj] = face_mirror(A.bc[TOP], old);
+      if (j == 1 && face_active(A.bc[BOTTOM])) w[in - g.sj] = face_mirror(A.bc[BOTTOM], old);
+      if (i == 1 && face_active(A.bc[LEFT])) w[in - 1] = face_mirror(A.bc[LEFT], old);
+      if (i == ni && face_active(A.bc[RIGHT])) w[in + 1] = face_mirror(A.bc[RIGHT], old);
+      w[in] = bc == OUTFLOW ? w[in - g.sk] : 0.0;
+    } else {
+      w[ghost] = bc == OUTFLOW ? w[in] : 0.0;
+    }
+    u[ghost] = face_mirror(bc, i == ni ? right_u(in) : u[in]);
+    v[ghost] = face_mirror(bc, j == nj ? top_v(in) : v[in]);
+  }
+}
+
+// one face
 struct FaceArgs {
   Dims g;
   int axis, high, bc;
@@ -559,12 +675,17 @@ __global__ void __launch_bounds__(kBlock) k_adapt(Dims g, double fx_arg, double 
 // over the whole arrays, as k_max3. The last block zeroes the slots.
 __global__ void __launch_bounds__(kBlock) k_shell_max3(Dims g, const double *__restrict__ u,
     const double *__restrict__ v, const double *__restrict__ w, unsigned long long *amax_slots,
-    double *__restrict__ partials, unsigned *ticket, double *__restrict__ out3)
+    unsigned long long *__restrict__ partials, unsigned *ticket, double *__restrict__ out3)
 {
   // 32-bit indices: the padded size is below 2^31 (checked at init)
   const int P = g.imax + 2, PQ = g.sk;
   const int n1 = 2 * PQ, n2 = g.kmax * 2 * P, n3 = g.kmax * g.jmax * 2;
-  unsigned uh = 0u, ul = 0u, vh = 0u, vl = 0u, wh = 0u, wl = 0u;
+  Key3 m;  // seeded with DBL_MIN
+#pragma unroll
+  for (int f = 0; f < 3; f++) {
+    m.h[f] = 0x00100000u;
+    m.l[f] = 0u;
+  }
   for (int q = blockIdx.x * kBlock + threadIdx.x; q < n1 + n2 + n3; q += gridDim.x * kBlock) {
     int c;
     if (q < n1) {
@@ -578,44 +699,22 @@ __global__ void __launch_bounds__(kBlock) k_shell_max3(Dims g, const double *__r
       const int k = 1 + r / (2 * g.jmax), rr = r - (k - 1) * (2 * g.jmax);
       c = k * PQ + (1 + (rr >> 1)) * g.sj + ((rr & 1) ? g.imax + 1 : 0);
     }
-    abs_max_key(uh, ul, u[c]);
-    abs_max_key(vh, vl, v[c]);
-    abs_max_key(wh, wl, w[c]);
+    abs_max_key(m.h[0], m.l[0], u[c]);
+    abs_max_key(m.h[1], m.l[1], v[c]);
+    abs_max_key(m.h[2], m.l[2], w[c]);
   }
-  __shared__ double sm[3][kBlock / 32];
-  double mu = block_reduce_max<kBlock>(__hiloint2double((int)uh, (int)ul), sm[0]);
-  double mv = block_reduce_max<kBlock>(__hiloint2double((int)vh, (int)vl), sm[1]);
-  double mw = block_reduce_max<kBlock>(__hiloint2double((int)wh, (int)wl), sm[2]);
-  __shared__ bool last;
+  __shared__ Key3 sm[kBlock / 32];
+  if (!grid_key_max3(m, sm, partials, ticket)) return;
+  for (int q = threadIdx.x; q < 3 * kAmaxSlots; q += kBlock) {
+    const unsigned long long x = amax_slots[q];
+    amax_slots[q] = 0ull;
+#pragma unroll
+    for (int f = 0; f < 3; f++)
+      if (q % 3 == f) key_word_max(m, f, x);
+  }
+  block_key_max3(m, sm);
   if (threadIdx.x == 0) {
-    partials[3 * blockIdx.x + 0] = mu;
-    partials[3 * blockIdx.x + 1] = mv;
-    partials[3 * blockIdx.x + 2] = mw;
-    last = ticket_is_last(ticket);
-  }
-  __syncthreads();
-  if (!last) return;
-  double a = DBL_MIN, b = DBL_MIN, c = DBL_MIN;
-  for (int q = threadIdx.x; q < (int)gridDim.x; q += kBlock) {
-    a = fmax(a, ld_cg(partials + 3 * q + 0));
-    b = fmax(b, ld_cg(partials + 3 * q + 1));
-    c = fmax(c, ld_cg(partials + 3 * q + 2));
-  }
-  for (int q = threadIdx.x; q < kAmaxSlots; q += kBlock) {
-    a = fmax(a, __longlong_as_double((long long)amax_slots[3 * q + 0]));
-    b = fmax(b, __longlong_as_double((long long)amax_slots[3 * q + 1]));
-    c = fmax(c, __longlong_as_double((long long)amax_slots[3 * q + 2]));
-    amax_slots[3 * q + 0] = 0ull;
-    amax_slots[3 * q + 1] = 0ull;
-    amax_slots[3 * q + 2] = 0ull;
-  }
-  a = block_reduce_max<kBlock>(a, sm[0]);
-  b = block_reduce_max<kBlock>(b, sm[1]);
-  c = block_reduce_max<kBlock>(c, sm[2]);
-  if (threadIdx.x == 0) {
-    out3[0] = a;
-    out3[1] = b;
-    out3[2] = c;
+    for (int f = 0; f < 3; f++) out3[f] = __hiloint2double((int)m.h[f], (int)m.l[f]);
     *ticket = 0;
   }
 }
@@ -681,9 +780,13 @@ const dim3 kCellBlock(64, 2, 2);
 bool launch_max3(const Dims &g, const double *u, const double *v, const double *w,
     ReduceScratch &red, double *d_out3)
 {
-  int blocks = 4 * sm_count();
+  // four blocks per SM, fewer where that leaves a thread without a pair: the
+  // last block folds them all
+  const int64_t most = (g.padded / 2 + kBlock - 1) / kBlock;
+  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(4 * sm_count(), most));
   if (!reduce_scratch_alloc(red, 3 * blocks)) return false;
-  k_max3<<<blocks, kBlock, 0, stream()>>>(u, v, w, g.padded, red.partials, red.ticket, d_out3);
+  k_max3<<<blocks, kBlock, 0, stream()>>>(u, v, w, g.padded,
+      reinterpret_cast<unsigned long long *>(red.partials), red.ticket, d_out3);
   return launched("k_max3");
 }
 
@@ -697,6 +800,14 @@ bool launch_bc(const Dims &g, const int bc[6], int problem, double lid, double i
   (void)lid;
   (void)inflow;
   const int n[3] = { g.imax, g.jmax, g.kmax };
+  if (n[0] >= 2 && n[1] >= 2 && n[2] >= 2) {
+    Faces A;
+    A.g = g;
+    for (int f = 0; f < 6; f++) A.bc[f] = bc[order[f][2]];
+    const int ma = std::max(n[0], n[1]), mb = std::max(n[1], n[2]);
+    k_faces<<<dim3((ma + 31) / 32, (mb + 7) / 8, 6), dim3(32, 8), 0, stream()>>>(A, u, v, w);
+    return launched("k_faces");
+  }
   for (int f = 0; f < 6; f++) {
     FaceArgs fa{ g, order[f][0], order[f][1], bc[order[f][2]] };
     if (fa.bc != NOSLIP && fa.bc != SLIP && fa.bc != OUTFLOW) continue;  // periodic: no-op
@@ -805,7 +916,8 @@ bool launch_rhs(const Dims &g, double dt, double dx, double dy, double dz, const
 
 bool launch_interior_sum(const Dims &g, const double *p, ReduceScratch &red, double *d_out)
 {
-  int blocks = 4 * sm_count();
+  const int64_t most = ((int64_t)g.imax * g.jmax * g.kmax + kBlock - 1) / kBlock;
+  const int blocks = (int)std::min<int64_t>(4 * sm_count(), most);
   if (!reduce_scratch_alloc(red, 3 * blocks)) return false;
   k_interior_sum<<<blocks, kBlock, 0, stream()>>>(g, p, red.partials, red.ticket, d_out);
   return launched("k_interior_sum");
@@ -838,8 +950,8 @@ bool launch_shell_max3(const Dims &g, const double *u, const double *v, const do
   int blocks = (int)std::min<int64_t>(4 * sm_count(), (shell + kBlock - 1) / kBlock);
   if (blocks < 1) blocks = 1;
   if (!reduce_scratch_alloc(red, 3 * blocks)) return false;
-  k_shell_max3<<<blocks, kBlock, 0, stream()>>>(g, u, v, w, amax_slots, red.partials, red.ticket,
-      d_out3);
+  k_shell_max3<<<blocks, kBlock, 0, stream()>>>(g, u, v, w, amax_slots,
+      reinterpret_cast<unsigned long long *>(red.partials), red.ticket, d_out3);
   return launched("k_shell_max3");
 }
 
