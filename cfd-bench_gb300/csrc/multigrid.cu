@@ -185,6 +185,15 @@ __device__ __forceinline__ T lap_at(const View<T> &v, const T *x, int i, int j, 
   return sx * v.ex + sy * v.ey + sz * v.ez - v.diag * xc;
 }
 
+// The FP32 seven-point operator with its roundings written out: which of two
+// products a compiler fuses into their sum depends on the code around them (a
+// change there moved a solve by 7e-8).
+__device__ __forceinline__ float lap_f32(float sx, float sy, float sz, float ex, float ey, float ez,
+    float dg, float xc)
+{
+  return __fmaf_rn(-dg, xc, __fmaf_rn(sz, ez, __fmaf_rn(sx, ex, __fmul_rn(sy, ey))));
+}
+
 // One colour of a red-black Gauss-Seidel sweep. ZERO: the sweep starts from
 // x = 0 (the centre is not read; in the odd pass neither are neighbours).
 // A thread owns the cell pair (2t, 2t+1) of a row and relaxes the one of the
@@ -392,12 +401,14 @@ __global__ void __launch_bounds__(kNT) k_mg_restrict_x2(View<T> f, T *bc, int cn
 // A fine plane is held as 4 rows x 4 columns (rows 2J-1 .. 2J+2, columns
 // 2I-1 .. 2I+2; a neighbour beyond a wall is the cell itself, so the clamped
 // index gives it): each row comes as one 8-byte load and its outer columns
-// from the neighbouring lanes, and the planes shared by consecutive fine
-// planes stay in registers. Same arithmetic and summation order as
+// from the neighbouring lanes. Loads run one fine plane ahead of the
+// arithmetic, and only what a later plane needs stays (of the plane below, the
+// four cells themselves; no corners). Same arithmetic and summation order as
 // k_mg_restrict_x2<float>, with 12 vector loads per coarse cell instead of 64
-// scalar ones.
+// scalar ones. Bound by memory latency: with each plane loaded where it was
+// used 55 us at 256^3, so 33.
 template <int FOLD>
-__global__ void __launch_bounds__(kNT) k_mg_restrict_f32(View<float> f, float *bc, int cnx,
+__global__ void __launch_bounds__(kNT, 3) k_mg_restrict_f32(View<float> f, float *bc, int cnx,
     int cny, int cnz, int kcz, float inv_count, MgState *st, double *partials, unsigned *ticket)
 {
   constexpr bool ACCUM = FOLD != FOLD_NONE;
@@ -407,70 +418,111 @@ __global__ void __launch_bounds__(kNT) k_mg_restrict_f32(View<float> f, float *b
   const bool in = I < cnx && J < cny;
   const int i0 = 2 * min(I, cnx - 1), j0 = 2 * min(J, cny - 1);  // loads stay in bounds
   const bool has_l = i0 > 0, has_r = i0 + 2 < f.nx;
-  int64_t roff[4];
+  int roff[4];  // 32-bit offsets: a level has fewer than 2^31 cells
 #pragma unroll
-  for (int r = 0; r < 4; r++) roff[r] = (int64_t)min(max(j0 - 1 + r, 0), f.ny - 1) * f.sy + i0;
+  for (int r = 0; r < 4; r++) roff[r] = f.off + min(max(j0 - 1 + r, 0), f.ny - 1) * f.sy + i0;
   const float *__restrict__ x = f.x;
   const float *__restrict__ b = f.b;
   const float ex = f.ex, ey = f.ey, ez = f.ez, dg = f.diag;
-  auto load_plane = [&](float(&v)[4][4], int k) {
-    const int64_t ko = f.off + (int64_t)min(max(k, 0), f.nz - 1) * f.sz;
+  // what lies outside the warp's 64 columns, for its outer lanes
+  const bool edge = (lane == 0 && has_l) || (lane == 31 && has_r);
+  const int eoff = lane == 0 ? -1 : 2;
+  struct Raw {
+    float2 a[4];
+    float e[4];
+  };
+  struct Plane {
+    float v[4][4];
+  };
+  const auto load = [&](Raw &q, int k) {
+    const int ko = min(max(k, 0), f.nz - 1) * f.sz;
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const float2 a = *reinterpret_cast<const float2 *>(x + ko + roff[r]);
-      float lv = __shfl_up_sync(0xffffffffu, a.y, 1);
-      float rv = __shfl_down_sync(0xffffffffu, a.x, 1);
-      if (lane == 0 && has_l) lv = x[ko + roff[r] - 1];
-      if (lane == 31 && has_r) rv = x[ko + roff[r] + 2];
-      v[r][0] = has_l ? lv : a.x;
-      v[r][1] = a.x;
-      v[r][2] = a.y;
-      v[r][3] = has_r ? rv : a.y;
+    for (int r = 0; r < 4; r++) q.a[r] = *reinterpret_cast<const float2 *>(x + ko + roff[r]);
+#pragma unroll
+    for (int r = 1; r < 3; r++) {  // the outer rows need no outer columns
+      q.e[r] = 0.0f;
+      if (edge) q.e[r] = x[ko + roff[r] + eoff];
     }
   };
-  auto resid = [&](const float(&vm)[4][4], const float(&vc)[4][4], const float(&vp)[4][4],
-                   int kf, float &sum, float &sq) {
-    const int64_t kb = f.off + (int64_t)kf * f.sz;
+  const auto expand = [&](Plane &p, const Raw &q) {
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      p.v[r][1] = q.a[r].x;
+      p.v[r][2] = q.a[r].y;
+    }
+#pragma unroll
+    for (int r = 1; r < 3; r++) {
+      float lv = __shfl_up_sync(0xffffffffu, q.a[r].y, 1);
+      float rv = __shfl_down_sync(0xffffffffu, q.a[r].x, 1);
+      if (lane == 0) lv = q.e[r];
+      if (lane == 31) rv = q.e[r];
+      p.v[r][0] = has_l ? lv : q.a[r].x;
+      p.v[r][3] = has_r ? rv : q.a[r].y;
+    }
+  };
+  struct Rhs {
+    float2 a[2];
+  };
+  const auto load_b = [&](Rhs &q, int k) {
+    const int ko = min(k, f.nz - 1) * f.sz;
+#pragma unroll
+    for (int d = 0; d < 2; d++) q.a[d] = *reinterpret_cast<const float2 *>(b + ko + roff[1 + d]);
+  };
+  // residual of one fine plane (vm: its cells one plane below)
+  const auto resid = [&](const float (&vm)[4], const Plane &vc, const Plane &vp, const Rhs &bb,
+                         float &sum, float &sq) {
 #pragma unroll
     for (int dj = 0; dj < 2; dj++) {
-      const float2 bb = *reinterpret_cast<const float2 *>(b + kb + roff[1 + dj]);
 #pragma unroll
       for (int di = 0; di < 2; di++) {
         const int rj = 1 + dj, ci = 1 + di;
-        const float xc = vc[rj][ci];
-        const float sx = vc[rj][ci - 1] + vc[rj][ci + 1];
-        const float sy = vc[rj - 1][ci] + vc[rj + 1][ci];
-        const float sz = vm[rj][ci] + vp[rj][ci];
-        const float lap = sx * ex + sy * ey + sz * ez - dg * xc;
-        const float r = (di ? bb.y : bb.x) - lap;
+        const float xc = vc.v[rj][ci];
+        const float sx = vc.v[rj][ci - 1] + vc.v[rj][ci + 1];
+        const float sy = vc.v[rj - 1][ci] + vc.v[rj + 1][ci];
+        const float sz = vm[2 * dj + di] + vp.v[rj][ci];
+        const float lap = lap_f32(sx, sy, sz, ex, ey, ez, dg, xc);
+        const float r = (di ? bb.a[dj].y : bb.a[dj].x) - lap;
         sum += r;
         if (ACCUM) sq += r * r;
       }
     }
   };
+  const auto keep = [](float (&vm)[4], const Plane &p) {
+    vm[0] = p.v[1][1];
+    vm[1] = p.v[1][2];
+    vm[2] = p.v[2][1];
+    vm[3] = p.v[2][2];
+  };
   double acc = 0.0;
   const int K0 = blockIdx.z * kcz, K1 = min(K0 + kcz, cnz);
   if (K0 < K1) {
-    float p0[4][4], p1[4][4], p2[4][4], p3[4][4];
-    load_plane(p0, 2 * K0 - 1);
-    load_plane(p1, 2 * K0);
+    Raw q;
+    Rhs r0, r1;
+    Plane A, B;
+    float vm[4];
+    load(q, 2 * K0 - 1);
+    expand(A, q);
+    keep(vm, A);
+    load(q, 2 * K0);
+    load_b(r0, 2 * K0);
+    expand(A, q);
+    load(q, 2 * K0 + 1);
     for (int K = K0; K < K1; K++) {
       float sum = 0.0f, sq = 0.0f;
-      load_plane(p2, 2 * K + 1);
-      resid(p0, p1, p2, 2 * K, sum, sq);
-      load_plane(p3, 2 * K + 2);
-      resid(p1, p2, p3, 2 * K + 1, sum, sq);
+      expand(B, q);
+      load(q, 2 * K + 2);
+      load_b(r1, 2 * K + 1);
+      resid(vm, A, B, r0, sum, sq);
+      keep(vm, A);
+      expand(A, q);
+      load(q, 2 * K + 3);
+      load_b(r0, 2 * K + 2);
+      resid(vm, B, A, r1, sum, sq);
+      keep(vm, B);
       if (in) {
         bc[((int64_t)K * cny + J) * cnx + I] = sum * inv_count;
         if (ACCUM) acc += to_f64(sq);
       }
-#pragma unroll
-      for (int r = 0; r < 4; r++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-          p0[r][c] = p2[r][c];
-          p1[r][c] = p3[r][c];
-        }
     }
   }
   if (!ACCUM) return;
@@ -856,11 +908,12 @@ __global__ void __launch_bounds__(kNT) k_rb_zero_sweep(View<float> v, float *__r
 // x_f += trilinear interpolation of x_c on FP32 levels halved on every axis
 // with fine rows of a multiple of four cells (16-byte aligned): one thread per
 // four consecutive fine cells of a row walks a chunk of coarse planes K and
-// updates fine planes 2K and 2K+1. The x-interpolated values of the two
-// coarse rows it needs are kept for coarse planes K-1, K, K+1, so each coarse
-// plane is read once per thread, as one 8-byte load per row with the outer
-// columns from the neighbouring lanes. Same interpolation order as
-// k_mg_prolong_x4 (x, then y, then z).
+// updates fine planes 2K and 2K+1. The y-interpolated values are kept for
+// coarse planes K-1, K, K+1, so each coarse plane is read once per thread, as
+// one 8-byte load per row with the outer columns from the neighbouring lanes,
+// one plane ahead; the fine cells of a plane pair are asked for before the
+// coarse plane is interpolated. Same interpolation order as k_mg_prolong_x4 (x,
+// then y, then z).
 __global__ void __launch_bounds__(kNT) k_mg_prolong_f32(View<float> f, const float *__restrict__ xc,
     int cnx, int cny, int cnz, int kcz, const MgState *st)
 {
@@ -876,20 +929,34 @@ __global__ void __launch_bounds__(kNT) k_mg_prolong_f32(View<float> f, const flo
   const int Py = j >> 1;
   const int ny_ = (j & 1) ? Py + 1 : Py - 1;
   const int Qy = (ny_ < 0 || ny_ >= cny) ? Py : ny_;
-  const int64_t sy = cnx, sz = (int64_t)cnx * cny;
+  const int sz = cnx * cny;  // 32-bit offsets: a level has fewer than 2^31 cells
+  const int base[2] = { Py * cnx + X0, Qy * cnx + X0 };
   const float w = 0.25f;
+  const bool edge = (lane == 0 && has_m) || (lane == 31 && has_p);
+  const int eoff = lane == 0 ? -1 : 2;
+  struct Raw {
+    float2 a[2];
+    float e[2];
+  };
+  const auto load = [&](Raw &q, int K) {
+    const int ko = min(max(K, 0), cnz - 1) * sz;
+#pragma unroll
+    for (int dy = 0; dy < 2; dy++) {
+      q.a[dy] = *reinterpret_cast<const float2 *>(xc + ko + base[dy]);
+      q.e[dy] = 0.0f;
+      if (edge) q.e[dy] = xc[ko + base[dy] + eoff];
+    }
+  };
   // y-interpolated values of the four fine cells for one coarse plane
-  auto plane = [&](float(&y)[4], int K) {
-    const int Kc = min(max(K, 0), cnz - 1);
+  const auto plane = [&](float(&y)[4], const Raw &q) {
     float o[2][4];
 #pragma unroll
     for (int dy = 0; dy < 2; dy++) {
-      const int64_t base = (int64_t)Kc * sz + (int64_t)(dy ? Qy : Py) * sy;
-      const float2 a = *reinterpret_cast<const float2 *>(xc + base + X0);
+      const float2 a = q.a[dy];
       float am = __shfl_up_sync(0xffffffffu, a.y, 1);
       float ap = __shfl_down_sync(0xffffffffu, a.x, 1);
-      if (lane == 0 && has_m) am = xc[base + X0 - 1];
-      if (lane == 31 && has_p) ap = xc[base + X1 + 1];
+      if (lane == 0) am = q.e[dy];
+      if (lane == 31) ap = q.e[dy];
       if (!has_m) am = a.x;
       if (!has_p) ap = a.y;
       o[dy][0] = a.x + w * (am - a.x);
@@ -903,31 +970,33 @@ __global__ void __launch_bounds__(kNT) k_mg_prolong_f32(View<float> f, const flo
   const int K0 = blockIdx.z * kcz, K1 = min(K0 + kcz, cnz);
   if (K0 >= K1) return;
   float ym[4], y0[4], yp[4];
-  plane(ym, K0 - 1);
-  plane(y0, K0);
+  Raw raw;
+  load(raw, K0 - 1);
+  plane(ym, raw);
+  load(raw, K0);
+  plane(y0, raw);
+  load(raw, K0 + 1);
   float *__restrict__ row = f.x + f.off + (int64_t)j * f.sy + 4 * Q;
   for (int K = K0; K < K1; K++) {
-    plane(yp, K + 1);
+    float4 *const px0 = reinterpret_cast<float4 *>(row + (int64_t)(2 * K) * f.sz);
+    float4 *const px1 = reinterpret_cast<float4 *>(row + (int64_t)(2 * K + 1) * f.sz);
+    const float4 v0 = *px0, v1 = *px1;
+    plane(yp, raw);
+    load(raw, K + 2);
     // fine plane 2K: coarse planes K and K - 1 (K itself at the low wall)
     // fine plane 2K + 1: coarse planes K and K + 1 (K itself at the high wall)
     const bool lo = K > 0, hi = K < cnz - 1;
+    float add[2][4];
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      float add[4];
+    for (int h = 0; h < 2; h++)
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         const float yq = h ? (hi ? yp[q] : y0[q]) : (lo ? ym[q] : y0[q]);
-        add[q] = y0[q] + w * (yq - y0[q]);
+        add[h][q] = y0[q] + w * (yq - y0[q]);
       }
-      if (in) {
-        float4 *px = reinterpret_cast<float4 *>(row + (int64_t)(2 * K + h) * f.sz);
-        float4 v = *px;
-        v.x += add[0];
-        v.y += add[1];
-        v.z += add[2];
-        v.w += add[3];
-        *px = v;
-      }
+    if (in) {
+      *px0 = make_float4(v0.x + add[0][0], v0.y + add[0][1], v0.z + add[0][2], v0.w + add[0][3]);
+      *px1 = make_float4(v1.x + add[1][0], v1.y + add[1][1], v1.z + add[1][2], v1.w + add[1][3]);
     }
 #pragma unroll
     for (int q = 0; q < 4; q++) {
@@ -1997,9 +2066,21 @@ bool restrict_to(const View<T> &f, T *bc, const MgLevelDesc &C, const double *sh
   if constexpr (sizeof(T) == sizeof(float)) {
     if (!shift && C.r[0] == 2 && C.r[1] == 2 && C.r[2] == 2 && f.off % 2 == 0 && f.sy % 2 == 0 &&
         f.sz % 2 == 0 && (int64_t)gx * gy <= cap) {
-      int gz = (int)std::min<int64_t>(C.n[2], cap / ((int64_t)gx * gy));
-      const int kcz = (C.n[2] + gz - 1) / gz;
-      gz = (C.n[2] + kcz - 1) / kcz;
+      // planes per block: the least (waves of three resident blocks per SM) x
+      // (fine planes read, two of them around the chunk)
+      int kcz = C.n[2];
+      int64_t best = INT64_MAX;
+      for (int c = 1; c <= C.n[2]; c++) {
+        const int64_t blocks = (int64_t)gx * gy * ((C.n[2] + c - 1) / c);
+        if (blocks > cap) continue;
+        const int64_t wave = 3 * (int64_t)sm_count_mg();
+        const int64_t cost = ((blocks + wave - 1) / wave) * (2 * c + 2);
+        if (cost < best) {
+          best = cost;
+          kcz = c;
+        }
+      }
+      const int gz = (C.n[2] + kcz - 1) / kcz;
       k_mg_restrict_f32<FOLD><<<dim3(gx, gy, gz), dim3(32, 8), 0, stream()>>>(f, bc, C.n[0],
           C.n[1], C.n[2], kcz, inv, st, red.partials, red.ticket);
       return launched("k_mg_restrict_f32");
