@@ -223,6 +223,96 @@ __global__ void __launch_bounds__(kNT) k_mg_smooth(View<T> v, int colour, const 
   }
 }
 
+// The FP64 pass (`mg`), bound by the FP64 pipe: x_new = (1 - w) x + f_x s_x +
+// f_y s_y + f_z s_z - i (b - shift), with the relaxation w, i = w / diag and
+// f = i e formed on the host: eight FP64 instructions per cell (seven without
+// over-relaxation) where x - i (b - shift - A x) takes ten, and no coarser: both
+// round at the size of x. The next plane's values are asked for before this
+// plane's arithmetic (nothing an update reads is written by its own pass, but
+// its own cell). One colour at 128^3: 25 -> 20 us.
+struct Smooth64 {
+  double fx, fy, fz, keep, inv;  // keep: 1 - w
+  int relaxed;                   // keep is not 0 (a test of a double is an FP64 instruction)
+};
+
+__host__ __device__ __forceinline__ Smooth64 smooth64(const View<double> &v)
+{
+  const double w = v.inv_diag * v.diag;  // the relaxation, up to a rounding
+  return { v.inv_diag * v.ex, v.inv_diag * v.ey, v.inv_diag * v.ez,
+           1.0 - w, v.inv_diag, fabs(w - 1.0) >= 1e-15 };
+}
+
+// the new value from b's term r = i shift - i b and the neighbours' sums
+__device__ __forceinline__ double smooth64_cell(const Smooth64 &C, double r, double sx, double sy,
+    double sz, double xc)
+{
+  r = fma(C.fx, sx, r);
+  r = fma(C.fy, sy, r);
+  r = fma(C.fz, sz, r);
+  return C.relaxed ? fma(C.keep, xc, r) : r;
+}
+
+// b - shift - A x, the operator's terms joined one by one: an FP64 instruction
+// less than forming A x first (rhs: b - shift)
+__device__ __forceinline__ double resid64(const View<double> &v, double rhs, double sx, double sy,
+    double sz, double xc)
+{
+  return fma(-v.ez, sz, fma(-v.ey, sy, fma(-v.ex, sx, fma(v.diag, xc, rhs))));
+}
+
+// the neighbours' sums of a cell, a missing one the cell itself
+template <typename T>
+__device__ __forceinline__ void neighbour_sums(const View<T> &v, const T *x, int i, int j, int k,
+    int64_t c, T xc, T &sx, T &sy, T &sz)
+{
+  sx = (i > 0 ? x[c - 1] : xc) + (i < v.nx - 1 ? x[c + 1] : xc);
+  sy = (j > 0 ? x[c - v.sy] : xc) + (j < v.ny - 1 ? x[c + v.sy] : xc);
+  sz = (k > 0 ? x[c - v.sz] : xc) + (k < v.nz - 1 ? x[c + v.sz] : xc);
+}
+
+template <bool ZERO>
+__global__ void __launch_bounds__(kNT) k_mg_smooth_f64(View<double> v, Smooth64 C, int colour,
+    const double *shift, int kb, const MgState *st)
+{
+  if (mg_done(st)) return;
+  const int t = blockIdx.x * kBX + threadIdx.x;
+  const int j = blockIdx.y * kBY + threadIdx.y;
+  const int k0 = blockIdx.z * kb, k1 = min(k0 + kb, v.nz);
+  if (j >= v.ny || k0 >= k1) return;
+  const double c0 = shift ? C.inv * *shift : 0.0;
+  const bool no_x = ZERO && colour == 1;  // from x = 0: the neighbours are 0 too
+  const auto cell = [&](int k) { return 2 * t + (((j + k + 1) & 1) == colour ? 0 : 1); };
+  struct Stencil {
+    double b, c, w, e, s, n, d, u;
+  };
+  const auto load = [&](int k, Stencil &q) {
+    const int i = cell(k);
+    if (i >= v.nx) return;
+    const int c = v.off + k * v.sz + j * v.sy + i;  // 32-bit: the padded size is below 2^31
+    q.b = v.b[c];
+    if (no_x) return;
+    q.c = ZERO ? 0.0 : v.x[c];
+    q.w = i > 0 ? v.x[c - 1] : q.c;
+    q.e = i < v.nx - 1 ? v.x[c + 1] : q.c;
+    q.s = j > 0 ? v.x[c - v.sy] : q.c;
+    q.n = j < v.ny - 1 ? v.x[c + v.sy] : q.c;
+    q.d = k > 0 ? v.x[c - v.sz] : q.c;
+    q.u = k < v.nz - 1 ? v.x[c + v.sz] : q.c;
+  };
+  Stencil cur{}, nxt{};
+  load(k0, cur);
+  for (int k = k0; k < k1; k++) {
+    if (k + 1 < k1) load(k + 1, nxt);
+    const int i = cell(k);
+    if (i < v.nx) {
+      double r = fma(-C.inv, cur.b, c0);
+      if (!no_x) r = smooth64_cell(C, r, cur.w + cur.e, cur.s + cur.n, cur.d + cur.u, cur.c);
+      v.x[v.off + k * v.sz + j * v.sy + i] = r;
+    }
+    cur = nxt;
+  }
+}
+
 // The FP32 pass on levels with an even row length (every coarsened level and
 // even fine grids): the pair (2t, 2t+1) is read as one 8-byte vector in the
 // row and in the four neighbouring rows, the far x-neighbour comes from the
@@ -343,7 +433,7 @@ __global__ void __launch_bounds__(kNT) k_mg_restrict_x2(View<T> f, T *bc, int cn
   constexpr bool ACCUM = FOLD != FOLD_NONE;
   if (mg_done(st)) return;
   const T sh = shift ? (T)(*shift) : (T)0;
-  const int I = blockIdx.x * 32 + threadIdx.x, J = blockIdx.y * 8 + threadIdx.y;
+  const int I = blockIdx.x * 32 + threadIdx.x, J = blockIdx.y * blockDim.y + threadIdx.y;
   double acc = 0.0;
   if (I < cnx && J < cny) {
     for (int K = blockIdx.z; K < cnz; K += gridDim.z) {
@@ -354,7 +444,15 @@ __global__ void __launch_bounds__(kNT) k_mg_restrict_x2(View<T> f, T *bc, int cn
           for (int di = 0; di < 2; di++) {
             const int i = 2 * I + di, j = J * ry + dj, k = K * rz + dk;
             const int64_t c = f.off + (int64_t)k * f.sz + (int64_t)j * f.sy + i;
-            const T r = (f.b[c] - sh) - lap_at(f, f.x, i, j, k, c, f.x[c]);
+            T r;
+            if constexpr (sizeof(T) == sizeof(double)) {
+              T sx, sy, sz;
+              const T xc = f.x[c];
+              neighbour_sums(f, f.x, i, j, k, c, xc, sx, sy, sz);
+              r = resid64(f, f.b[c] - sh, sx, sy, sz, xc);
+            } else {
+              r = (f.b[c] - sh) - lap_at(f, f.x, i, j, k, c, f.x[c]);
+            }
             sum += r;
             // FP32 levels: a coarse cell's (at most 8) squares summed in FP32,
             // then one FP64 add (the FP64 pipe would bound this kernel)
@@ -1006,6 +1104,70 @@ __global__ void __launch_bounds__(kNT) k_mg_prolong_f32(View<float> f, const flo
   }
 }
 
+// The same for FP64 levels halved on every axis: one thread per coarse column
+// X and fine row walks a chunk of coarse planes and updates the two fine cells
+// of each of two fine planes. Six FP64 instructions per fine cell against
+// fifteen where every fine plane interpolates both coarse planes anew, on the
+// pipe that bounds it: 128^3 62 -> 29 us. Same interpolation order.
+__global__ void __launch_bounds__(kNT) k_mg_prolong_f64(View<double> f,
+    const double *__restrict__ xc, int cnx, int cny, int cnz, int kcz, const MgState *st)
+{
+  if (mg_done(st)) return;
+  const int X = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int K0 = blockIdx.z * kcz, K1 = min(K0 + kcz, cnz);
+  if (X >= cnx || j >= f.ny || K0 >= K1) return;
+  const int Xm = X > 0 ? X - 1 : X, Xp = X < cnx - 1 ? X + 1 : X;
+  const int Py = j >> 1;
+  const int ny_ = (j & 1) ? Py + 1 : Py - 1;
+  const int Qy = (ny_ < 0 || ny_ >= cny) ? Py : ny_;
+  const int sz = cnx * cny, b0 = Py * cnx, b1 = Qy * cnx;
+  struct Raw {
+    double m[2], c[2], p[2];
+  };
+  const auto load = [&](Raw &q, int K) {
+    const double *const z = xc + min(max(K, 0), cnz - 1) * sz;
+    q.m[0] = z[b0 + Xm];
+    q.c[0] = z[b0 + X];
+    q.p[0] = z[b0 + Xp];
+    q.m[1] = z[b1 + Xm];
+    q.c[1] = z[b1 + X];
+    q.p[1] = z[b1 + Xp];
+  };
+  // the two fine cells' x- and y-interpolated values of a coarse plane
+  const auto plane = [&](double(&y)[2], const Raw &q) {
+    const double l0 = q.c[0] + 0.25 * (q.m[0] - q.c[0]), l1 = q.c[1] + 0.25 * (q.m[1] - q.c[1]);
+    const double h0 = q.c[0] + 0.25 * (q.p[0] - q.c[0]), h1 = q.c[1] + 0.25 * (q.p[1] - q.c[1]);
+    y[0] = l0 + 0.25 * (l1 - l0);
+    y[1] = h0 + 0.25 * (h1 - h0);
+  };
+  double ym[2], y0[2], yp[2];
+  Raw raw;
+  load(raw, K0 - 1);
+  plane(ym, raw);
+  load(raw, K0);
+  plane(y0, raw);
+  load(raw, K0 + 1);
+  double *__restrict__ row = f.x + f.off + (int64_t)j * f.sy + 2 * X;
+  for (int K = K0; K < K1; K++) {
+    double *const r0 = row + (int64_t)(2 * K) * f.sz, *const r1 = r0 + f.sz;
+    const double a0 = r0[0], a1 = r0[1], c0 = r1[0], c1 = r1[1];
+    plane(yp, raw);
+    load(raw, K + 2);
+    const bool lo = K > 0, hi = K < cnz - 1;
+    const double m0 = lo ? ym[0] : y0[0], m1 = lo ? ym[1] : y0[1];
+    const double p0 = hi ? yp[0] : y0[0], p1 = hi ? yp[1] : y0[1];
+    r0[0] = a0 + (y0[0] + 0.25 * (m0 - y0[0]));
+    r0[1] = a1 + (y0[1] + 0.25 * (m1 - y0[1]));
+    r1[0] = c0 + (y0[0] + 0.25 * (p0 - y0[0]));
+    r1[1] = c1 + (y0[1] + 0.25 * (p1 - y0[1]));
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      ym[q] = y0[q];
+      y0[q] = yp[q];
+    }
+  }
+}
+
 // One whole red-black Gauss-Seidel sweep in one kernel, exact: reads x_old,
 // writes x_new (ping-pong), so no block ever reads a value another block
 // writes. A block owns a 64 x 8 tile of (i, j) columns and a chunk of planes;
@@ -1619,7 +1781,16 @@ __device__ void tail_smooth(const View<T> &v, int count, bool zero_first)
       for (int q = threadIdx.x; q < n; q += blockDim.x) {
         const int i = q % v.nx, j = (q / v.nx) % v.ny, k = q / (v.nx * v.ny);
         if (((i + j + k + 1) & 1) != colour) continue;
-        if (z && colour == 1) {
+        if constexpr (sizeof(T) == sizeof(double)) {
+          const Smooth64 C = smooth64(v);
+          T r = fma(-C.inv, v.b[q], 0.0), sx, sy, sz;
+          if (!(z && colour == 1)) {
+            const T xc = z ? (T)0 : v.x[q];
+            neighbour_sums(v, v.x, i, j, k, q, xc, sx, sy, sz);
+            r = smooth64_cell(C, r, sx, sy, sz, xc);
+          }
+          v.x[q] = r;
+        } else if (z && colour == 1) {
           v.x[q] = -v.b[q] * v.inv_diag;
         } else {
           const T xc = z ? (T)0 : v.x[q];
@@ -1653,7 +1824,13 @@ __global__ void __launch_bounds__(1024) k_mg_tail(TailArgs<T> a)
           for (int di = 0; di < rx; di++) {
             const int i = I * rx + di, j = J * ry + dj, k = K * rz + dk;
             const int c = (k * v.ny + j) * v.nx + i;
-            sum += v.b[c] - lap_at(v, v.x, i, j, k, c, v.x[c]);
+            if constexpr (sizeof(T) == sizeof(double)) {
+              T sx, sy, sz;
+              neighbour_sums(v, v.x, i, j, k, c, v.x[c], sx, sy, sz);
+              sum += resid64(v, v.b[c], sx, sy, sz, v.x[c]);
+            } else {
+              sum += v.b[c] - lap_at(v, v.x, i, j, k, c, v.x[c]);
+            }
           }
       C.b[q] = sum * inv;
     }
@@ -1975,8 +2152,14 @@ bool smooth_pass(const View<T> &v, int colour, const double *shift, const MgStat
       return launched("k_mg_smooth_f2");
     }
   }
-  k_mg_smooth<T, ZERO><<<grid, dim3(kBX, kBY), 0, stream()>>>(v, colour, shift, kb, st);
-  return launched("k_mg_smooth");
+  if constexpr (sizeof(T) == sizeof(double)) {
+    const Smooth64 C = smooth64(v);
+    k_mg_smooth_f64<ZERO><<<grid, dim3(kBX, kBY), 0, stream()>>>(v, C, colour, shift, kb, st);
+    return launched("k_mg_smooth_f64");
+  } else {
+    k_mg_smooth<T, ZERO><<<grid, dim3(kBX, kBY), 0, stream()>>>(v, colour, shift, kb, st);
+    return launched("k_mg_smooth");
+  }
 }
 
 // `count` sweeps (odd colour, then even); the first from zero when zero_first
@@ -2049,6 +2232,17 @@ bool mx_residual(MgHierarchy *H, const View<double> &v0, MgState *st, int count_
   return launched("k_mx_residual");
 }
 
+// rows of 32 threads per block: eight, fewer where a level has too few blocks
+// for two per SM (an FP64 instruction of a warp takes 16 cycles of its SM, so
+// eight warps on a few SMs are slower than one on each: FP64, from 32^3 to 16^3
+// and back 7.0 + 4.7 -> 5.5 + 3.3 us)
+int rows_per_block(int gx, int ny, int gz)
+{
+  int rows = 8;
+  while (rows > 1 && (int64_t)gx * ((ny + rows - 1) / rows) * gz < 2 * sm_count_mg()) rows >>= 1;
+  return rows;
+}
+
 template <typename T, int FOLD>
 bool restrict_to(const View<T> &f, T *bc, const MgLevelDesc &C, const double *shift, MgState *st,
     ReduceScratch &red)
@@ -2089,7 +2283,9 @@ bool restrict_to(const View<T> &f, T *bc, const MgLevelDesc &C, const double *sh
   if (C.r[0] == 2 && (int64_t)gx * gy <= cap) {
     int gz = C.n[2];
     while (gz > 1 && (int64_t)gx * gy * gz > cap) gz = (gz + 1) / 2;
-    k_mg_restrict_x2<T, FOLD><<<dim3(gx, gy, gz), dim3(32, 8), 0, stream()>>>(f, bc, C.n[0],
+    const int rows = FOLD == FOLD_NONE ? rows_per_block(gx, C.n[1], gz) : 8;
+    const dim3 grid(gx, (C.n[1] + rows - 1) / rows, gz);
+    k_mg_restrict_x2<T, FOLD><<<grid, dim3(32, rows), 0, stream()>>>(f, bc, C.n[0],
         C.n[1], C.n[2], C.r[1], C.r[2], inv, shift, st, red.partials, red.ticket);
     return launched("k_mg_restrict_x2");
   }
@@ -2112,6 +2308,31 @@ bool prolong_to(const View<T> &f, const T *xc, const MgLevelDesc &C, const MgSta
       k_mg_prolong_f32<<<dim3(gx, gy, gz), dim3(32, 8), 0, stream()>>>(f, xc, C.n[0], C.n[1],
           C.n[2], kcz, st);
       return launched("k_mg_prolong_f32");
+    }
+  }
+  if constexpr (sizeof(T) == sizeof(double)) {
+    if (C.r[0] == 2 && C.r[1] == 2 && C.r[2] == 2) {
+      // planes per block: the least (blocks of the busiest SM) x (planes
+      // interpolated, two of them around the chunk, and planes updated), with
+      // three blocks for two SMs at least where the level has them
+      const int gx = (C.n[0] + 31) / 32, gy = (f.ny + 7) / 8, sms = sm_count_mg();
+      int kcz = 1;
+      int64_t best = INT64_MAX;
+      for (int c = 1; c <= C.n[2]; c++) {
+        const int64_t blocks = (int64_t)gx * gy * ((C.n[2] + c - 1) / c);
+        if (c > 1 && 2 * blocks < 3 * sms) break;
+        const int64_t cost = ((blocks + sms - 1) / sms) * (2 * c + 2);
+        if (cost <= best) {
+          best = cost;
+          kcz = c;
+        }
+      }
+      const int gz = (C.n[2] + kcz - 1) / kcz;
+      const int rows = rows_per_block(gx, f.ny, gz);
+      const dim3 grid(gx, (f.ny + rows - 1) / rows, gz);
+      k_mg_prolong_f64<<<grid, dim3(32, rows), 0, stream()>>>(f, xc, C.n[0], C.n[1], C.n[2], kcz,
+          st);
+      return launched("k_mg_prolong_f64");
     }
   }
   if (C.r[0] == 2 && f.nx % 4 == 0) {
