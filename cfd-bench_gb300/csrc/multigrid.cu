@@ -116,6 +116,7 @@ struct MgHierarchy {
   cudaStream_t cap[3] = {};  // capture streams: graph, outer body, inner body
   bool use_graph = true;     // mg_graph: the host-driven solve runs as one graph
   int tail_l0 = 0;           // first level of the one-kernel coarse tail (0: none)
+  int bottom_l0 = 0;         // first level of k_mg_bottom (0: none)
   int kc[kMaxLevels] = {};   // planes per block of each level's one-kernel sweep (0: by rule)
   // FP32 sweeps skipped inside a V-cycle copy x along (odd pre- or post-sweep counts)
   int keep_on_skip = 0;
@@ -1895,6 +1896,325 @@ __global__ void __launch_bounds__(1024) k_mg_tail(TailArgs<T> a)
   }
 }
 
+// The coarse end of an FP32 V-cycle as one cluster of eight blocks: the levels
+// of at most kBottomCells cells, where a launch per sweep and transfer costs
+// more than the work (2-3 us each against 0.2-0.4 us). Every block keeps all
+// these levels in shared memory and walks down them on its own (the same
+// arithmetic in each, so no block waits for another); only the coarsest solve is
+// split: a block multiplies its eighth of the inverse's rows, copied to shared
+// memory while the levels above are smoothed, and sends its values to block 0,
+// which goes up alone. Same operations, roundings and order as the per-level
+// kernels. What is left is latency: a barrier and a chain of shared-memory
+// loads per colour. A level's cells are kept by colour, a pair (2t, 2t+1) of a
+// row in one slot of each (first[p] the cell with (i + j + k) even, second[p]
+// the other), so that neighbouring threads read neighbouring words, and a
+// thread keeps its pairs' values and right-hand sides in registers. Per V(2,2)
+// cycle from 32 x 8 x 8 cells (coarsest 8^3) 32.6 us as sixteen launches, 12.3
+// here. A level of 16384 cells would take 10 us on one SM against 14 as
+// launches spread over the chip: not worth its shared memory.
+constexpr int kBottomCells = 4096, kBottomBlocks = 8, kBottomThreads = 1024;
+constexpr int kBottomDirect = 512;  // cells of the coarsest level at most
+constexpr int kBottomPairs = kBottomCells / 2 / kBottomThreads;  // per thread
+
+struct BottomLevel {
+  int nx, ny, nz;
+  int ry, rz;           // coarsening from the level above (x is always halved)
+  unsigned mrow, mpl;   // 2^32 / (pairs of a row, of a plane), rounded up
+  float ex, ey, ez, diag, inv_diag;
+  int x;                // the level's first-colour values in shared memory, then the others
+  int b;                // its right-hand side, cell by cell
+};
+
+struct BottomArgs {
+  int count;  // levels, the last one the coarsest
+  int pre, post;
+  int rows;         // the inverse's rows per block
+  int res, m, lvl;  // shared memory: residuals, the block's rows, the level table
+  BottomLevel lv[kMaxLevels];
+  const float *minv, *b;
+  float *x;
+  const MgState *st;
+};
+
+// pair p of a level: cells (2t, j, k) and (2t + 1, j, k); valid while p times
+// the divisor stays below 2^32
+__device__ __forceinline__ void bottom_pair(const BottomLevel &L, int p, int &t, int &j, int &k)
+{
+  const int row = L.nx >> 1, plane = row * L.ny;
+  k = L.mpl ? (int)__umulhi((unsigned)p, L.mpl) : p;
+  const int q = p - k * plane;
+  j = L.mrow ? (int)__umulhi((unsigned)q, L.mrow) : q;
+  t = q - j * row;
+}
+
+// `count` red-black sweeps of a level (zero: from x = 0), then, unless `res` is
+// negative, its residual cell by cell. One copy of the code for both ways of
+// the cycle: most of it runs once per launch, from a cold instruction cache.
+__device__ __noinline__ void bottom_sweeps(float *smem, int lvl, int l, int count, bool zero,
+    int res)
+{
+  const BottomLevel L = reinterpret_cast<const BottomLevel *>(smem + lvl)[l];
+  const int row = L.nx >> 1, plane = row * L.ny, pairs = plane * L.nz;
+  float *const x = smem + L.x;
+  int par[kBottomPairs], wall[kBottomPairs];
+  float v[kBottomPairs][2], b[kBottomPairs][2];  // by colour
+#pragma unroll
+  for (int r = 0; r < kBottomPairs; r++) {
+    const int p = threadIdx.x + r * kBottomThreads;
+    if (p >= pairs) break;
+    int t, j, k;
+    bottom_pair(L, p, t, j, k);
+    par[r] = (j + k) & 1;  // the pair's first-colour cell is its left (0) or right one
+    wall[r] = (t > 0) | (t < row - 1) << 1 | (j > 0) << 2 | (j < L.ny - 1) << 3 | (k > 0) << 4 |
+              (k < L.nz - 1) << 5;  // the neighbours there are
+    const float2 q = *reinterpret_cast<const float2 *>(smem + L.b + 2 * p);
+    b[r][0] = par[r] ? q.y : q.x;
+    b[r][1] = par[r] ? q.x : q.y;
+    v[r][0] = v[r][1] = 0.0f;
+    if (!zero) {
+      v[r][0] = x[p];
+      v[r][1] = x[pairs + p];
+    } else if (count == 0) {
+      x[p] = x[pairs + p] = 0.0f;
+    } else {
+      x[pairs + p] = 0.0f;
+    }
+  }
+  __syncthreads();
+  // the operator at a pair's cell of colour h (a neighbour beyond a wall is the
+  // cell itself); the neighbours are of the other colour
+  const auto lap = [&](int r, int h) {
+    const int p = threadIdx.x + r * kBottomThreads, w = wall[r];
+    const float *const o = x + (h ? 0 : pairs) + p;
+    const float c = v[r][h], in = v[r][1 - h];  // the neighbour inside the pair
+    const bool left = par[r] == h;              // the cell is the pair's left one
+    float out = c;
+    if (w & (left ? 1 : 2)) out = o[left ? -1 : 1];
+    const float s = w & 4 ? o[-row] : c, n = w & 8 ? o[row] : c;
+    const float d = w & 16 ? o[-plane] : c, u = w & 32 ? o[plane] : c;
+    return lap_f32(in + out, s + n, d + u, L.ex, L.ey, L.ez, L.diag, c);
+  };
+#pragma unroll 1
+  for (int q = 0; q < count; q++) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+#pragma unroll
+      for (int r = 0; r < kBottomPairs; r++) {
+        const int p = threadIdx.x + r * kBottomThreads;
+        if (p >= pairs) break;
+        v[r][h] = __fmaf_rn(-(b[r][h] - lap(r, h)), L.inv_diag, v[r][h]);
+        x[(h ? pairs : 0) + p] = v[r][h];
+      }
+      __syncthreads();
+    }
+  }
+  if (res < 0) return;
+#pragma unroll
+  for (int r = 0; r < kBottomPairs; r++) {
+    const int p = threadIdx.x + r * kBottomThreads;
+    if (p >= pairs) break;
+    const float r0 = b[r][0] - lap(r, 0), r1 = b[r][1] - lap(r, 1);
+    *reinterpret_cast<float2 *>(smem + res + 2 * p) =
+        par[r] ? make_float2(r1, r0) : make_float2(r0, r1);
+  }
+  __syncthreads();
+}
+
+// the inverse's rows of this block, as one asynchronous copy per 16 KB
+__device__ __forceinline__ void bottom_copy(float *dst, const float *src, unsigned bytes,
+    unsigned bar)
+{
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes)
+               : "memory");
+  const unsigned to = (unsigned)__cvta_generic_to_shared(dst);
+  for (unsigned at = 0; at < bytes; at += 16384)
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+        ::"r"(to + at), "l"(reinterpret_cast<const char *>(src) + at),
+        "r"(min(16384u, bytes - at)), "r"(bar)
+        : "memory");
+}
+
+// waits for the copy, about 10 ms at most
+__device__ __forceinline__ bool bottom_wait(unsigned bar)
+{
+  const long long t0 = clock64();
+  for (;;) {
+    int done;
+    asm volatile(
+        "{ .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n"
+        " selp.s32 %0, 1, 0, p; }\n"
+        : "=r"(done)
+        : "r"(bar)
+        : "memory");
+    if (done) return true;
+    if (clock64() - t0 > 20000000) return false;
+  }
+}
+
+__global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const __grid_constant__ BottomArgs a)
+{
+  extern __shared__ __align__(16) float bottom_smem[];
+  __shared__ __align__(8) unsigned long long arrived;
+  float *const smem = bottom_smem;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool done = mg_done(a.st);  // the same for all blocks: only earlier kernels write it
+  const int m = a.count, nc = a.lv[m - 1].nx * a.lv[m - 1].ny * a.lv[m - 1].nz;
+  const int row0 = blockIdx.x * a.rows, nrows = max(0, min(a.rows, nc - row0));
+  {
+    const int n = a.lv[0].nx * a.lv[0].ny * a.lv[0].nz;
+    float2 q[kBottomPairs];
+#pragma unroll
+    for (int r = 0; r < kBottomPairs; r++) {
+      const int p = tid + r * kBottomThreads;
+      if (2 * p < n) q[r] = reinterpret_cast<const float2 *>(a.b)[p];
+    }
+    if (done) return;
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");  // this block has started
+    if (tid == 0) {
+      const unsigned bar = (unsigned)__cvta_generic_to_shared(&arrived);
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+      bottom_copy(smem + a.m, a.minv + (int64_t)row0 * nc, 4u * nrows * nc, bar);
+    }
+    const int words = m * (int)(sizeof(BottomLevel) / 4);
+    if (tid < words)
+      reinterpret_cast<int *>(smem + a.lvl)[tid] = reinterpret_cast<const int *>(a.lv)[tid];
+#pragma unroll
+    for (int r = 0; r < kBottomPairs; r++) {
+      const int p = tid + r * kBottomThreads;
+      if (2 * p < n) reinterpret_cast<float2 *>(smem + a.lv[0].b)[p] = q[r];
+    }
+    __syncthreads();
+  }
+#pragma unroll 1
+  for (int l = 0; l < m - 1; l++) {
+    bottom_sweeps(smem, a.lvl, l, a.pre, true, a.res);
+    const BottomLevel &C = reinterpret_cast<const BottomLevel *>(smem + a.lvl)[l + 1];
+    const BottomLevel &L = reinterpret_cast<const BottomLevel *>(smem + a.lvl)[l];
+    const int n = C.nx * C.ny * C.nz, ry = C.ry, rz = C.rz, row = L.nx, plane = L.nx * L.ny;
+    const float inv = ry * rz == 4 ? 0.125f : ry * rz == 2 ? 0.25f : 0.5f;
+#pragma unroll 1
+    for (int q = tid; q < n; q += kBottomThreads) {
+      int t, J, K;
+      bottom_pair(C, q >> 1, t, J, K);
+      const float *const f = smem + a.res + K * rz * plane + J * ry * row + 2 * (2 * t + (q & 1));
+      float sum = 0.0f;
+#pragma unroll
+      for (int dk = 0; dk < 2; dk++)
+#pragma unroll
+        for (int dj = 0; dj < 2; dj++) {
+          if (dk >= rz || dj >= ry) continue;
+          const float2 g = *reinterpret_cast<const float2 *>(f + dk * plane + dj * row);
+          sum += g.x;
+          sum += g.y;
+        }
+      smem[C.b + q] = sum * inv;
+    }
+    __syncthreads();
+  }
+  // coarsest level, kept cell by cell: a warp per row of the inverse
+  const bool copied = bottom_wait((unsigned)__cvta_generic_to_shared(&arrived));
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");  // block 0 has started
+  {
+    const BottomLevel &C = reinterpret_cast<const BottomLevel *>(smem + a.lvl)[m - 1];
+    const float *const b = smem + C.b;
+    const unsigned xs = (unsigned)__cvta_generic_to_shared(smem + C.x);
+    unsigned x0;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(x0) : "r"(xs));
+    float bl[kBottomDirect / 32];
+#pragma unroll
+    for (int q = 0; q < kBottomDirect / 32; q++)
+      if (lane + 32 * q < nc) bl[q] = b[lane + 32 * q];
+#pragma unroll 1
+    for (int r = warp; r < nrows; r += kBottomThreads / 32) {
+      const float *const mrow =
+          (copied ? smem + a.m + r * nc : a.minv + (int64_t)(row0 + r) * nc) + lane;
+      float acc = 0.0f;
+#pragma unroll
+      for (int q = 0; q < kBottomDirect / 32; q++)
+        if (lane + 32 * q < nc) acc = __fmaf_rn(mrow[32 * q], bl[q], acc);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane == 0)
+        asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(x0 + 4 * (row0 + r)), "f"(acc)
+                     : "memory");
+    }
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  if (blockIdx.x != 0) return;
+#pragma unroll 1
+  for (int l = m - 2; l >= 0; l--) {
+    const BottomLevel &L = reinterpret_cast<const BottomLevel *>(smem + a.lvl)[l];
+    const BottomLevel &C = reinterpret_cast<const BottomLevel *>(smem + a.lvl)[l + 1];
+    const int plane = (L.nx >> 1) * L.ny, pairs = plane * L.nz;
+    const int crow = C.nx >> 1, cplane = crow * C.ny, cpairs = cplane * C.nz;
+    const bool flat = l + 1 == m - 1;
+    float *const x = smem + L.x;
+    const float *const xc = smem + C.x;
+#pragma unroll 1
+    for (int p = tid; p < pairs; p += kBottomThreads) {
+      int X, j, k;
+      bottom_pair(L, p, X, j, k);
+      int Py = j, Qy = j, Pz = k, Qz = k;
+      float wy = 0.0f, wz = 0.0f;
+      if (C.ry == 2) {
+        Py = j >> 1;
+        const int nb = (j & 1) ? Py + 1 : Py - 1;
+        Qy = (nb < 0 || nb >= C.ny) ? Py : nb;
+        wy = 0.25f;
+      }
+      if (C.rz == 2) {
+        Pz = k >> 1;
+        const int nb = (k & 1) ? Pz + 1 : Pz - 1;
+        Qz = (nb < 0 || nb >= C.nz) ? Pz : nb;
+        wz = 0.25f;
+      }
+      const int Xm = X > 0 ? X - 1 : X, Xp = X < C.nx - 1 ? X + 1 : X;
+      float o[2][2][2];  // per fine cell, per (z, y) line
+#pragma unroll
+      for (int dz = 0; dz < 2; dz++)
+#pragma unroll
+        for (int dy = 0; dy < 2; dy++) {
+          if ((dz && C.rz == 1) || (dy && C.ry == 1)) {  // the same line again
+            o[0][dz][dy] = o[0][dz && C.rz == 2][dy && C.ry == 2];
+            o[1][dz][dy] = o[1][dz && C.rz == 2][dy && C.ry == 2];
+            continue;
+          }
+          const int Y = dy ? Qy : Py, Z = dz ? Qz : Pz;
+          const auto at = [&](int I) {
+            const int pair = Z * cplane + Y * crow + (I >> 1);
+            return xc[flat ? 2 * pair + (I & 1) : pair + ((I + Y + Z) & 1 ? cpairs : 0)];
+          };
+          const float am = at(Xm), a0 = at(X), ap = at(Xp);
+          o[0][dz][dy] = __fmaf_rn(0.25f, am - a0, a0);
+          o[1][dz][dy] = __fmaf_rn(0.25f, ap - a0, a0);
+        }
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const float y0 = __fmaf_rn(wy, o[q][0][1] - o[q][0][0], o[q][0][0]);
+        const float y1 = __fmaf_rn(wy, o[q][1][1] - o[q][1][0], o[q][1][0]);
+        x[p + ((q + j + k) & 1 ? pairs : 0)] += __fmaf_rn(wz, y1 - y0, y0);
+      }
+    }
+    // each thread goes on with the pairs it has just written; the sweeps begin
+    // with a barrier
+    bottom_sweeps(smem, a.lvl, l, a.post, false, -1);
+  }
+  {
+    const BottomLevel &L = reinterpret_cast<const BottomLevel *>(smem + a.lvl)[0];
+    const int pairs = (L.nx >> 1) * L.ny * L.nz;
+    for (int p = tid; p < pairs; p += kBottomThreads) {
+      int t, j, k;
+      bottom_pair(L, p, t, j, k);
+      const float e = smem[L.x + p], o = smem[L.x + pairs + p];
+      reinterpret_cast<float2 *>(a.x)[p] = (j + k) & 1 ? make_float2(o, e) : make_float2(e, o);
+    }
+  }
+}
+
 // the solve state for a right-hand side whose ||b - shift||^2 is nb2
 __device__ void open_solve(MgState *st, double nb2)
 {
@@ -2608,6 +2928,92 @@ bool tail_vcycle(MgHierarchy *H, int l, T **xs, T **bs, bool zero)
   return launched("k_mg_tail");
 }
 
+// The levels that k_mg_bottom takes: from the first of at most kBottomCells
+// cells below the top, where at least one lies above an exactly solved
+// coarsest level and each can be walked as the per-level kernels would (x
+// halved between all of them, rows of a multiple of four cells, as
+// k_rbgs_sweep, k_mg_restrict_x2 and k_mg_prolong_x4 want them). 0: none.
+int bottom_level(const MgHierarchy *H)
+{
+  const MgLevelDesc &Lc = H->lv[H->nl - 1];
+  const int nc = Lc.n[0] * Lc.n[1] * Lc.n[2];
+  if (!H->minv32 || nc % 4 != 0 || nc > kBottomDirect) return 0;
+  int l0 = 0;
+  for (int l = H->nl - 2; l >= 1; l--) {
+    const MgLevelDesc &L = H->lv[l];
+    if ((int64_t)L.n[0] * L.n[1] * L.n[2] > kBottomCells || L.n[0] % 4 != 0 ||
+        H->lv[l + 1].r[0] != 2)
+      break;
+    l0 = l;
+  }
+  return l0;
+}
+
+// levels l .. nl-1 from zero in one cluster (k_mg_bottom)
+bool bottom_vcycle(MgHierarchy *H, int l)
+{
+  BottomArgs a;
+  a.count = H->nl - l;
+  int at = 0;
+  for (int q = 0; q < a.count; q++) {
+    const MgLevelDesc &L = H->lv[l + q];
+    BottomLevel &t = a.lv[q];
+    const View<float> v = compact_view<float>(L, nullptr, nullptr);
+    t.nx = v.nx;
+    t.ny = v.ny;
+    t.nz = v.nz;
+    t.ry = L.r[1];
+    t.rz = L.r[2];
+    const auto magic = [](int d) { return d > 1 ? (unsigned)(((1ull << 32) + d - 1) / d) : 0u; };
+    t.mrow = magic(v.nx / 2);
+    t.mpl = magic(v.nx / 2 * v.ny);
+    t.ex = v.ex;
+    t.ey = v.ey;
+    t.ez = v.ez;
+    t.diag = v.diag;
+    t.inv_diag = v.inv_diag;
+    const int n = (v.nx * v.ny * v.nz + 3) / 4 * 4;
+    t.x = at;
+    t.b = at + n;
+    at += 2 * n;
+  }
+  a.res = at;
+  at += (a.lv[0].nx * a.lv[0].ny * a.lv[0].nz + 3) / 4 * 4;
+  a.lvl = at;
+  at += (a.count * (int)sizeof(BottomLevel) / 4 + 3) / 4 * 4;
+  const MgLevelDesc &Lc = H->lv[H->nl - 1];
+  const int nc = Lc.n[0] * Lc.n[1] * Lc.n[2];
+  a.pre = H->pre;
+  a.post = H->post;
+  a.rows = (nc + kBottomBlocks - 1) / kBottomBlocks;
+  a.m = at;
+  a.minv = H->minv32;
+  a.b = H->b32[l];
+  a.x = H->x32[l];
+  a.st = H->d_state;
+  const size_t bytes = sizeof(float) * ((size_t)at + (size_t)a.rows * nc);
+  static_assert(sizeof(float) * (5 * kBottomCells + kBottomDirect / kBottomBlocks * kBottomDirect) + kMaxLevels * sizeof(BottomLevel) <=
+                    226 * 1024,
+      "shared memory");
+  if (!cuda_ok(cudaFuncSetAttribute(k_mg_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                   (int)bytes),
+          "k_mg_bottom shared memory"))
+    return false;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kBottomBlocks);
+  cfg.blockDim = dim3(kBottomThreads);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.stream = stream();
+  cudaLaunchAttribute at0[1];
+  at0[0].id = cudaLaunchAttributeClusterDimension;
+  at0[0].val.clusterDim.x = kBottomBlocks;
+  at0[0].val.clusterDim.y = at0[0].val.clusterDim.z = 1;
+  cfg.attrs = at0;
+  cfg.numAttrs = 1;
+  if (!cuda_ok(cudaLaunchKernelEx(&cfg, k_mg_bottom, a), "k_mg_bottom")) return false;
+  return launched("k_mg_bottom");
+}
+
 template <typename T>
 bool vcycle(MgHierarchy *H, int l, T **xs, T **bs, bool zero, bool inner_test)
 {
@@ -2616,6 +3022,9 @@ bool vcycle(MgHierarchy *H, int l, T **xs, T **bs, bool zero, bool inner_test)
   const size_t n = (size_t)L.n[0] * L.n[1] * L.n[2];
   MgState *st = H->d_state;
   if (H->tail_l0 > 0 && l == H->tail_l0) return tail_vcycle<T>(H, l, xs, bs, zero);
+  if constexpr (sizeof(T) == sizeof(float)) {
+    if (H->bottom_l0 > 0 && l == H->bottom_l0) return bottom_vcycle(H, l);
+  }
   if (l == H->nl - 1) {
     const T *minv = nullptr;
     if constexpr (sizeof(T) == sizeof(double))
@@ -2829,7 +3238,7 @@ bool mg_setup(Solver *s, Discretization *d, SolverState *ss)
   // residual still decides convergence
   for (int l = 0; l < H->nl; l++) H->lv[l].relax = x.mg_omega;
   // the coarse tail: from the first level below the finest with at most
-  // mg_tail cells (0: off), when it leaves at least two levels to it
+  // mg_tail cells (0: none), when it leaves at least two levels to it
   H->tail_l0 = 0;
   for (int l = 1; x.mg_tail > 0 && l < H->nl - 1; l++) {
     if ((int64_t)H->lv[l].n[0] * H->lv[l].n[1] * H->lv[l].n[2] <= x.mg_tail) {
@@ -2883,6 +3292,7 @@ bool mg_setup(Solver *s, Discretization *d, SolverState *ss)
         return false;
     }
   }
+  if (x.mg_tail == 0) H->bottom_l0 = bottom_level(H);
   const int64_t n0 = (int64_t)d->grid.imax * d->grid.jmax * d->grid.kmax;
   const int red_blocks = std::max(flat_blocks(n0),
       mx_df_blocks(d->grid.imax, d->grid.jmax, d->grid.kmax));

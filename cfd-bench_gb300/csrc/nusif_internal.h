@@ -46,7 +46,7 @@ struct Extras {
   int mg_guess = 0;          // initial guess: 0 previous p, 1 linear, 2 quadratic, 3 cubic
                              // extrapolation in time
   int mg_graph = 1;          // 1: each solve is one CUDA graph launch (while-loops on the device)
-  int mg_tail = 0;           // levels of at most this many cells run as one kernel (0: off)
+  int mg_tail = 0;           // levels of at most this many cells run as one kernel (0: k_mg_bottom's)
   int mg_chunk = 0;          // planes per block of the FP32 one-kernel sweep (0: autotuned)
   int host_fields = 0;       // 1: fields in managed memory (host-readable pointers)
   int mg_guess_probe = 1;    // key mg_probe: learned guess every P-th step after 2 rejections

@@ -468,3 +468,26 @@ def test_integer_pipe_conversions_match_hardware(nusif_lib):
     nan = torch.isnan(want)
     assert torch.equal(torch.isnan(d), nan)
     assert torch.equal(d[~nan].view(torch.int64), want[~nan].view(torch.int64))
+
+
+# (fine grid, levels the cluster kernel takes): a level of exactly 4096 cells
+# and one just above, x halved alone, y or z halved with x, rows of 4 and 12
+# cells, a coarsest level of a few cells and of 512
+@pytest.mark.parametrize("dims,pre,post", [((32, 32, 32), 2, 2), ((64, 32, 34), 1, 1),
+                                           ((512, 16, 16), 2, 1), ((64, 16, 4), 1, 2),
+                                           ((12, 96, 12), 1, 1), ((48, 24, 24), 3, 3),
+                                           ((16, 8, 8), 2, 2), ((160, 96, 96), 1, 1),
+                                           ((24, 40, 56), 2, 0)])
+def test_coarse_cluster_matches_per_level_kernels(nusif_lib, dims, pre, post):
+    """The coarse levels in one cluster give the same bits as a kernel per
+    sweep and transfer (mg_tail = 1: no level is that small, so none is taken)."""
+    out = []
+    for tail in (0, 1):
+        with _sim(dims, "mg-mixed", 1e-9, mg_pre=pre, mg_post=post, mg_omega=1.2, mg_cycles=3,
+                  mg_tail=tail) as sim:
+            rng = np.random.default_rng(5)
+            sim.set_field("p", rng.standard_normal(sim.padded_shape))
+            sim.set_field("rhs", rng.standard_normal(sim.padded_shape))
+            out.append((sim.solve(), sim.iterations, sim.field("p")))
+    assert out[0][:2] == out[1][:2]
+    np.testing.assert_array_equal(out[0][2], out[1][2])
