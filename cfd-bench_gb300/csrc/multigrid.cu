@@ -1367,9 +1367,8 @@ __global__ void __launch_bounds__(256) k_rbgs_sweep(View<float> v, float *__rest
   cp_async_wait<0>();
 }
 
-// The same exact red-black sweep for levels whose rows are a multiple of 128
-// cells and whose columns a multiple of 8 (the finest levels of the benchmark
-// grids), with the work in registers instead of shared memory: a block owns a
+// The same exact red-black sweep (rows of a multiple of four cells) with the
+// work in registers instead of shared memory: a block owns a
 // 128 x 8 tile of (i, j) columns and a chunk of planes; warp w < 10 handles
 // row j0 - 1 + w (rows j0 - 1 and j0 + 8 are the first-colour ring), lane l
 // the four cells i0 + 4l .. i0 + 4l + 3 of that row as one float4. Each such
@@ -1398,11 +1397,13 @@ __global__ void __launch_bounds__(kVThreads, 2) k_rbgs_sweep_v(View<float> v,
   const int k0 = blockIdx.z * kc, k1 = min(k0 + kc, nz);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sy = v.sy, sz = v.sz;
+  // a narrow last tile ends at lane `last`; the lanes beyond repeat its loads
+  const int last = min(31, ((nx - i0) >> 2) - 1), col4 = i0 + 4 * min(lane, last);
   if (mg_done(st)) {
     // a sweep skipped inside a V-cycle leaves x where the next kernels look
     // (see k_rbgs_sweep): copy the tile rows of the chunk
-    if (keep && !solve_finished(st) && w >= 1 && w <= kVY) {
-      const int c0 = (j0 + w - 1) * sy + i0 + 4 * lane;
+    if (keep && !solve_finished(st) && w >= 1 && w <= kVY && j0 + w - 1 < ny && lane <= last) {
+      const int c0 = (j0 + w - 1) * sy + col4;
       for (int k = k0; k < k1; k++)
         *reinterpret_cast<float4 *>(xnew + c0 + (int64_t)k * sz) =
             *reinterpret_cast<const float4 *>(v.x + c0 + (int64_t)k * sz);
@@ -1421,10 +1422,10 @@ __global__ void __launch_bounds__(kVThreads, 2) k_rbgs_sweep_v(View<float> v,
     const bool act = r < kVRows;
     const int j = j0 - 1 + r;
     const int jc = min(max(j, 0), ny - 1);
-    const bool wall = right ? i0 + kVX == nx : i0 == 0;
+    const bool wall = right ? i0 + kVX >= nx : i0 == 0;
     const int col = right ? i0 + kVX : i0 - 1;       // the ring cell
     const int beyond = right ? i0 + kVX + 1 : i0 - 2;
-    const int edge = right ? i0 + kVX - 1 : i0;      // the tile's edge cell beside it
+    const int edge = right ? min(i0 + kVX, nx) - 1 : i0;  // the tile's edge cell beside it
     const int scol = right ? kVR : kVL;
     const bool in = act && !wall && j >= 0 && j < ny && r >= 1 && r <= kVY;
     const float *__restrict__ xr = v.x + jc * sy;
@@ -1469,15 +1470,17 @@ __global__ void __launch_bounds__(kVThreads, 2) k_rbgs_sweep_v(View<float> v,
   // ---------------- row warps ----------------
   const int j = j0 - 1 + w;
   const bool row_in = j >= 0 && j < ny;
-  const bool tile_row = w >= 1 && w <= kVY;
+  const bool tile_row = w >= 1 && w <= kVY && j < ny;
+  // the right neighbour of the tile's last cell: its own value at a wall
+  const bool at_last = lane == last, at_wall = i0 + kVX >= nx;
   const int jc = min(max(j, 0), ny - 1);
-  const float *__restrict__ xrow = v.x + jc * sy + i0 + 4 * lane;
-  const float *__restrict__ brow = v.b + jc * sy + i0 + 4 * lane;
-  float *__restrict__ orow = xnew + j * sy + i0 + 4 * lane;  // used for tile rows only
+  const float *__restrict__ xrow = v.x + jc * sy + col4;
+  const float *__restrict__ brow = v.b + jc * sy + col4;
+  float *__restrict__ orow = xnew + j * sy + col4;  // used for tile rows only
   // the extra staged rows j0 - 2 (warp 0) and j0 + 9 (warp 9), x_old only
   const bool extra = w == 0 || w == kVRows - 1;
   const int je = w == 0 ? j0 - 2 : j0 + 9;
-  const float *__restrict__ xext = v.x + min(max(je, 0), ny - 1) * sy + i0 + 4 * lane;
+  const float *__restrict__ xext = v.x + min(max(je, 0), ny - 1) * sy + col4;
   const int srow_ext = w == 0 ? 0 : kVY + 3;
   const auto ldx = [&](int k) { return *reinterpret_cast<const float4 *>(xrow + plane(k)); };
   const auto ldb = [&](int k) { return *reinterpret_cast<const float4 *>(brow + plane(k)); };
@@ -1506,7 +1509,7 @@ __global__ void __launch_bounds__(kVThreads, 2) k_rbgs_sweep_v(View<float> v,
       float left = __shfl_up_sync(0xffffffffu, oc.w, 1);
       float right = __shfl_down_sync(0xffffffffu, oc.x, 1);
       if (lane == 0) left = sx[s][w + 1][kVL];
-      if (lane == 31) right = sx[s][w + 1][kVR];
+      if (at_last) right = at_wall ? oc.w : sx[s][w + 1][kVR];
       const float4 yn = *reinterpret_cast<const float4 *>(&sx[s][w][4 + 4 * lane]);
       const float4 ys = *reinterpret_cast<const float4 *>(&sx[s][w + 2][4 + 4 * lane]);
       rc = oc;
@@ -1544,7 +1547,7 @@ __global__ void __launch_bounds__(kVThreads, 2) k_rbgs_sweep_v(View<float> v,
       float left = __shfl_up_sync(0xffffffffu, rm1.w, 1);
       float right = __shfl_down_sync(0xffffffffu, rm1.x, 1);
       if (lane == 0) left = sr[se][w][kVL];
-      if (lane == 31) right = sr[se][w][kVR];
+      if (at_last) right = at_wall ? rm1.w : sr[se][w][kVR];
       const float4 yn = *reinterpret_cast<const float4 *>(&sr[se][w - 1][4 + 4 * lane]);
       const float4 ys = *reinterpret_cast<const float4 *>(&sr[se][w + 1][4 + 4 * lane]);
       float4 out = rm1;
@@ -1571,7 +1574,7 @@ __global__ void __launch_bounds__(kVThreads, 2) k_rbgs_sweep_v(View<float> v,
           out.w = rm1.w - (bm.w - lap) * idg;
         }
       }
-      *reinterpret_cast<float4 *>(orow + (int64_t)ke * sz) = out;
+      if (lane <= last) *reinterpret_cast<float4 *>(orow + (int64_t)ke * sz) = out;
     }
     // ---- rotate ----
     rm2 = rm1;
@@ -2723,10 +2726,11 @@ bool coarse_solve(const View<T> &v, int nsweeps, const MgState *st, const T *min
 // recomputed) and the grid runs in ceil(blocks / resident) waves; the rule
 // minimises waves * (kc + 2). The chunk depth changes only how the work is
 // split: every cell is computed the same way, so results do not depend on it.
-// The one-kernel FP32 sweep of a level: k_rbgs_sweep_v where the rows are a
-// multiple of 128 cells and the columns of 8 (the environment variable
-// NUSIF_SWEEP=tile64 selects k_rbgs_sweep everywhere, for comparisons), else
-// k_rbgs_sweep.
+// The one-kernel FP32 sweep of a level: k_rbgs_sweep_v, also where its tile of
+// 128 x 8 columns is wider than the level: mg-mixed solves of 48^3 to 252^3 take
+// 0.90-1.00 of their time with k_rbgs_sweep there (96^3 844 -> 778 us, 64^3 495
+// -> 485). The environment variable NUSIF_SWEEP=tile64 selects k_rbgs_sweep, for
+// comparisons.
 struct SweepShape {
   bool vec;
   int gx, gy, threads;
@@ -2737,10 +2741,10 @@ SweepShape sweep_shape(const MgLevelDesc &L)
   const char *e = getenv("NUSIF_SWEEP");
   const bool legacy = e && strcmp(e, "tile64") == 0;
   SweepShape r;
-  r.vec = !legacy && L.n[0] % kVX == 0 && L.n[1] % kVY == 0;
+  r.vec = !legacy;
   if (r.vec) {
-    r.gx = L.n[0] / kVX;
-    r.gy = L.n[1] / kVY;
+    r.gx = (L.n[0] + kVX - 1) / kVX;
+    r.gy = (L.n[1] + kVY - 1) / kVY;
     r.threads = kVThreads;
   } else {
     r.gx = (L.n[0] + kSX - 1) / kSX;

@@ -491,3 +491,10 @@ def test_coarse_cluster_matches_per_level_kernels(nusif_lib, dims, pre, post):
             out.append((sim.solve(), sim.iterations, sim.field("p")))
     assert out[0][:2] == out[1][:2]
     np.testing.assert_array_equal(out[0][2], out[1][2])
+
+
+@pytest.mark.parametrize("dims", [(4, 3, 5), (60, 7, 6), (68, 9, 11), (124, 17, 4), (132, 5, 12),
+                                  (260, 13, 3), (8, 1, 40), (96, 96, 33)])
+def test_register_tiled_sweep_on_partial_tiles(nusif_lib, dims, monkeypatch):
+    """The same where the last tile of 128 columns or 8 rows is not full."""
+    test_register_tiled_sweep_equals_shared_memory_sweep(nusif_lib, dims, monkeypatch)
