@@ -1907,25 +1907,30 @@ __global__ void __launch_bounds__(1024) k_mg_tail(TailArgs<T> a)
 // split: a block multiplies its eighth of the inverse's rows, copied to shared
 // memory while the levels above are smoothed, and sends its values to block 0,
 // which goes up alone. Same operations, roundings and order as the per-level
-// kernels. What is left is latency: a barrier and a chain of shared-memory
-// loads per colour. A level's cells are kept by colour, a pair (2t, 2t+1) of a
-// row in one slot of each (first[p] the cell with (i + j + k) even, second[p]
-// the other), so that neighbouring threads read neighbouring words, and a
-// thread keeps its pairs' values and right-hand sides in registers. Per V(2,2)
-// cycle from 32 x 8 x 8 cells (coarsest 8^3) 32.6 us as sixteen launches, 12.3
-// here. A level of 16384 cells would take 10 us on one SM against 14 as
-// launches spread over the chip: not worth its shared memory.
-constexpr int kBottomCells = 4096, kBottomBlocks = 8, kBottomThreads = 1024;
-constexpr int kBottomDirect = 512;  // cells of the coarsest level at most
+// kernels (ANY: for rows of any length and x halved or not; otherwise rows are
+// even and x is halved). What is left is latency: a barrier and a chain of
+// shared-memory loads per colour. A level's cells are kept by colour, a pair
+// (2t, 2t+1) of a row in one slot of each (first[p] the cell with (i + j + k)
+// even, second[p] the other), so that neighbouring threads read neighbouring
+// words, and a thread keeps its pairs' values and right-hand sides in
+// registers. Per V(2,2) cycle from 32 x 8 x 8 cells (coarsest 8^3) 32.6 us as
+// sixteen launches, 12.7 here; solves with an odd level, 20x36x20 385 -> 308 us,
+// 64x20x24 682 -> 548 us, 36^3 (a level of 5832 cells) 406 -> 346 us. A level of
+// 16384 cells would take 10 us on one SM against 14 as launches spread over the
+// chip: not worth its shared memory.
+constexpr int kBottomCells = 8192, kBottomBlocks = 8, kBottomThreads = 1024;
+constexpr size_t kBottomSmem = 226 * 1024;
+// a level and its halvings (right-hand side and values), its residuals, the table
+static_assert(sizeof(float) * 5 * kBottomCells + kMaxLevels * 64 <= kBottomSmem, "shared memory");
 constexpr int kBottomPairs = kBottomCells / 2 / kBottomThreads;  // per thread
 
 struct BottomLevel {
   int nx, ny, nz;
-  int ry, rz;           // coarsening from the level above (x is always halved)
+  int rx, ry, rz;       // coarsening from the level above
   unsigned mrow, mpl;   // 2^32 / (pairs of a row, of a plane), rounded up
   float ex, ey, ez, diag, inv_diag;
   int x;                // the level's first-colour values in shared memory, then the others
-  int b;                // its right-hand side, cell by cell
+  int b;                // its right-hand side, pair by pair
 };
 
 struct BottomArgs {
@@ -1943,33 +1948,47 @@ struct BottomArgs {
 // the divisor stays below 2^32
 __device__ __forceinline__ void bottom_pair(const BottomLevel &L, int p, int &t, int &j, int &k)
 {
-  const int row = L.nx >> 1, plane = row * L.ny;
+  const int row = (L.nx + 1) >> 1, plane = row * L.ny;
   k = L.mpl ? (int)__umulhi((unsigned)p, L.mpl) : p;
   const int q = p - k * plane;
   j = L.mrow ? (int)__umulhi((unsigned)q, L.mrow) : q;
   t = q - j * row;
 }
 
-// `count` red-black sweeps of a level (zero: from x = 0), then, unless `res` is
+// pair p of an array of the level in global memory
+template <bool ANY>
+__device__ __forceinline__ float2 bottom_read(const BottomLevel &L, const float *x, int p)
+{
+  if (!ANY || !(L.nx & 1)) return reinterpret_cast<const float2 *>(x)[p];
+  int t, j, k;
+  bottom_pair(L, p, t, j, k);
+  const float *const c = x + (k * L.ny + j) * L.nx + 2 * t;
+  return make_float2(c[0], 2 * t + 1 < L.nx ? c[1] : 0.0f);
+}
+
+// `count` red-black sweeps of a level (zero: from x = 0; ANY: its rows may be
+// odd), then, unless `res` is
 // negative, its residual cell by cell. One copy of the code for both ways of
 // the cycle: most of it runs once per launch, from a cold instruction cache.
+template <int PAIRS, bool ANY>
 __device__ __noinline__ void bottom_sweeps(float *smem, int lvl, int l, int count, bool zero,
     int res)
 {
   const BottomLevel L = reinterpret_cast<const BottomLevel *>(smem + lvl)[l];
-  const int row = L.nx >> 1, plane = row * L.ny, pairs = plane * L.nz;
+  const int row = (L.nx + 1) >> 1, plane = row * L.ny, pairs = plane * L.nz;
   float *const x = smem + L.x;
-  int par[kBottomPairs], wall[kBottomPairs];
-  float v[kBottomPairs][2], b[kBottomPairs][2];  // by colour
+  int par[PAIRS], wall[PAIRS];
+  float v[PAIRS][2], b[PAIRS][2];  // by colour
 #pragma unroll
-  for (int r = 0; r < kBottomPairs; r++) {
+  for (int r = 0; r < PAIRS; r++) {
     const int p = threadIdx.x + r * kBottomThreads;
     if (p >= pairs) break;
     int t, j, k;
     bottom_pair(L, p, t, j, k);
     par[r] = (j + k) & 1;  // the pair's first-colour cell is its left (0) or right one
     wall[r] = (t > 0) | (t < row - 1) << 1 | (j > 0) << 2 | (j < L.ny - 1) << 3 | (k > 0) << 4 |
-              (k < L.nz - 1) << 5;  // the neighbours there are
+              (k < L.nz - 1) << 5 |      // the neighbours there are
+              (2 * t + 1 == L.nx) << 6;  // an odd row's last pair has no right cell
     const float2 q = *reinterpret_cast<const float2 *>(smem + L.b + 2 * p);
     b[r][0] = par[r] ? q.y : q.x;
     b[r][1] = par[r] ? q.x : q.y;
@@ -1989,8 +2008,8 @@ __device__ __noinline__ void bottom_sweeps(float *smem, int lvl, int l, int coun
   const auto lap = [&](int r, int h) {
     const int p = threadIdx.x + r * kBottomThreads, w = wall[r];
     const float *const o = x + (h ? 0 : pairs) + p;
-    const float c = v[r][h], in = v[r][1 - h];  // the neighbour inside the pair
-    const bool left = par[r] == h;              // the cell is the pair's left one
+    const float c = v[r][h], in = ANY && (w & 64) ? c : v[r][1 - h];  // inside the pair
+    const bool left = par[r] == h;  // the cell is the pair's left one
     float out = c;
     if (w & (left ? 1 : 2)) out = o[left ? -1 : 1];
     const float s = w & 4 ? o[-row] : c, n = w & 8 ? o[row] : c;
@@ -2002,9 +2021,10 @@ __device__ __noinline__ void bottom_sweeps(float *smem, int lvl, int l, int coun
 #pragma unroll
     for (int h = 0; h < 2; h++) {
 #pragma unroll
-      for (int r = 0; r < kBottomPairs; r++) {
+      for (int r = 0; r < PAIRS; r++) {
         const int p = threadIdx.x + r * kBottomThreads;
         if (p >= pairs) break;
+        if (ANY && (wall[r] & 64) && par[r] != h) continue;
         v[r][h] = __fmaf_rn(-(b[r][h] - lap(r, h)), L.inv_diag, v[r][h]);
         x[(h ? pairs : 0) + p] = v[r][h];
       }
@@ -2013,10 +2033,11 @@ __device__ __noinline__ void bottom_sweeps(float *smem, int lvl, int l, int coun
   }
   if (res < 0) return;
 #pragma unroll
-  for (int r = 0; r < kBottomPairs; r++) {
+  for (int r = 0; r < PAIRS; r++) {
     const int p = threadIdx.x + r * kBottomThreads;
     if (p >= pairs) break;
     const float r0 = b[r][0] - lap(r, 0), r1 = b[r][1] - lap(r, 1);
+    // (of a pair with one cell the other number is not read)
     *reinterpret_cast<float2 *>(smem + res + 2 * p) =
         par[r] ? make_float2(r1, r0) : make_float2(r0, r1);
   }
@@ -2055,6 +2076,7 @@ __device__ __forceinline__ bool bottom_wait(unsigned bar)
   }
 }
 
+template <int PAIRS, bool ANY>
 __global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const __grid_constant__ BottomArgs a)
 {
   extern __shared__ __align__(16) float bottom_smem[];
@@ -2065,12 +2087,13 @@ __global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const __grid_const
   const int m = a.count, nc = a.lv[m - 1].nx * a.lv[m - 1].ny * a.lv[m - 1].nz;
   const int row0 = blockIdx.x * a.rows, nrows = max(0, min(a.rows, nc - row0));
   {
-    const int n = a.lv[0].nx * a.lv[0].ny * a.lv[0].nz;
-    float2 q[kBottomPairs];
+    const BottomLevel &L = a.lv[0];
+    const int pairs = ((L.nx + 1) >> 1) * L.ny * L.nz;
+    float2 q[PAIRS];
 #pragma unroll
-    for (int r = 0; r < kBottomPairs; r++) {
+    for (int r = 0; r < PAIRS; r++) {
       const int p = tid + r * kBottomThreads;
-      if (2 * p < n) q[r] = reinterpret_cast<const float2 *>(a.b)[p];
+      if (p < pairs) q[r] = bottom_read<ANY>(L, a.b, p);
     }
     if (done) return;
     asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");  // this block has started
@@ -2078,46 +2101,57 @@ __global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const __grid_const
       const unsigned bar = (unsigned)__cvta_generic_to_shared(&arrived);
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bar) : "memory");
       asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-      bottom_copy(smem + a.m, a.minv + (int64_t)row0 * nc, 4u * nrows * nc, bar);
+      // (whole 16 bytes: the inverse is allocated with a margin)
+      bottom_copy(smem + max(a.m, 0), a.minv + (int64_t)row0 * nc,
+          a.m < 0 ? 0u : (4u * nrows * nc + 15u) / 16u * 16u, bar);
     }
     const int words = m * (int)(sizeof(BottomLevel) / 4);
     if (tid < words)
       reinterpret_cast<int *>(smem + a.lvl)[tid] = reinterpret_cast<const int *>(a.lv)[tid];
 #pragma unroll
-    for (int r = 0; r < kBottomPairs; r++) {
+    for (int r = 0; r < PAIRS; r++) {
       const int p = tid + r * kBottomThreads;
-      if (2 * p < n) reinterpret_cast<float2 *>(smem + a.lv[0].b)[p] = q[r];
+      if (p < pairs) reinterpret_cast<float2 *>(smem + L.b)[p] = q[r];
     }
     __syncthreads();
   }
 #pragma unroll 1
   for (int l = 0; l < m - 1; l++) {
-    bottom_sweeps(smem, a.lvl, l, a.pre, true, a.res);
+    bottom_sweeps<PAIRS, ANY>(smem, a.lvl, l, a.pre, true, a.res);
     const BottomLevel &C = reinterpret_cast<const BottomLevel *>(smem + a.lvl)[l + 1];
     const BottomLevel &L = reinterpret_cast<const BottomLevel *>(smem + a.lvl)[l];
-    const int n = C.nx * C.ny * C.nz, ry = C.ry, rz = C.rz, row = L.nx, plane = L.nx * L.ny;
-    const float inv = ry * rz == 4 ? 0.125f : ry * rz == 2 ? 0.25f : 0.5f;
+    const int cpairs = ((C.nx + 1) >> 1) * C.ny * C.nz, rx = ANY ? C.rx : 2, ry = C.ry, rz = C.rz;
+    const int row = (L.nx + 1) & ~1, plane = row * L.ny;
+    const bool flat = l + 1 == m - 1;  // the coarsest level is kept cell by cell
+    const float inv = 1.0f / (float)(rx * ry * rz);  // a power of two
 #pragma unroll 1
-    for (int q = tid; q < n; q += kBottomThreads) {
+    for (int q = tid; q < 2 * cpairs; q += kBottomThreads) {
       int t, J, K;
       bottom_pair(C, q >> 1, t, J, K);
-      const float *const f = smem + a.res + K * rz * plane + J * ry * row + 2 * (2 * t + (q & 1));
+      const int I = 2 * t + (q & 1);
+      if (ANY && I >= C.nx) continue;
+      const float *const f = smem + a.res + K * rz * plane + J * ry * row + rx * I;
       float sum = 0.0f;
 #pragma unroll
       for (int dk = 0; dk < 2; dk++)
 #pragma unroll
         for (int dj = 0; dj < 2; dj++) {
           if (dk >= rz || dj >= ry) continue;
-          const float2 g = *reinterpret_cast<const float2 *>(f + dk * plane + dj * row);
-          sum += g.x;
-          sum += g.y;
+          const float *const g = f + dk * plane + dj * row;
+          if (rx == 2) {
+            const float2 e = *reinterpret_cast<const float2 *>(g);
+            sum += e.x;
+            sum += e.y;
+          } else {
+            sum += *g;
+          }
         }
-      smem[C.b + q] = sum * inv;
+      smem[C.b + (ANY && flat ? (K * C.ny + J) * C.nx + I : q)] = sum * inv;
     }
     __syncthreads();
   }
   // coarsest level, kept cell by cell: a warp per row of the inverse
-  const bool copied = bottom_wait((unsigned)__cvta_generic_to_shared(&arrived));
+  const bool copied = bottom_wait((unsigned)__cvta_generic_to_shared(&arrived)) && a.m >= 0;
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");  // block 0 has started
   {
     const BottomLevel &C = reinterpret_cast<const BottomLevel *>(smem + a.lvl)[m - 1];
@@ -2125,9 +2159,9 @@ __global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const __grid_const
     const unsigned xs = (unsigned)__cvta_generic_to_shared(smem + C.x);
     unsigned x0;
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(x0) : "r"(xs));
-    float bl[kBottomDirect / 32];
+    float bl[16];
 #pragma unroll
-    for (int q = 0; q < kBottomDirect / 32; q++)
+    for (int q = 0; q < 16; q++)
       if (lane + 32 * q < nc) bl[q] = b[lane + 32 * q];
 #pragma unroll 1
     for (int r = warp; r < nrows; r += kBottomThreads / 32) {
@@ -2135,8 +2169,10 @@ __global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const __grid_const
           (copied ? smem + a.m + r * nc : a.minv + (int64_t)(row0 + r) * nc) + lane;
       float acc = 0.0f;
 #pragma unroll
-      for (int q = 0; q < kBottomDirect / 32; q++)
+      for (int q = 0; q < 16; q++)
         if (lane + 32 * q < nc) acc = __fmaf_rn(mrow[32 * q], bl[q], acc);
+#pragma unroll 8
+      for (int q = 512; q < nc - lane; q += 32) acc = __fmaf_rn(mrow[q], b[lane + q], acc);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
       if (lane == 0)
@@ -2152,8 +2188,8 @@ __global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const __grid_const
   for (int l = m - 2; l >= 0; l--) {
     const BottomLevel &L = reinterpret_cast<const BottomLevel *>(smem + a.lvl)[l];
     const BottomLevel &C = reinterpret_cast<const BottomLevel *>(smem + a.lvl)[l + 1];
-    const int plane = (L.nx >> 1) * L.ny, pairs = plane * L.nz;
-    const int crow = C.nx >> 1, cplane = crow * C.ny, cpairs = cplane * C.nz;
+    const int pairs = ((L.nx + 1) >> 1) * L.ny * L.nz;
+    const int crow = (C.nx + 1) >> 1, cplane = crow * C.ny, cpairs = cplane * C.nz;
     const bool flat = l + 1 == m - 1;
     float *const x = smem + L.x;
     const float *const xc = smem + C.x;
@@ -2175,7 +2211,7 @@ __global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const __grid_const
         Qz = (nb < 0 || nb >= C.nz) ? Pz : nb;
         wz = 0.25f;
       }
-      const int Xm = X > 0 ? X - 1 : X, Xp = X < C.nx - 1 ? X + 1 : X;
+      const bool single = ANY && 2 * X + 1 == L.nx;
       float o[2][2][2];  // per fine cell, per (z, y) line
 #pragma unroll
       for (int dz = 0; dz < 2; dz++)
@@ -2188,32 +2224,44 @@ __global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const __grid_const
           }
           const int Y = dy ? Qy : Py, Z = dz ? Qz : Pz;
           const auto at = [&](int I) {
-            const int pair = Z * cplane + Y * crow + (I >> 1);
-            return xc[flat ? 2 * pair + (I & 1) : pair + ((I + Y + Z) & 1 ? cpairs : 0)];
+            if (flat) return xc[(Z * C.ny + Y) * C.nx + I];
+            return xc[Z * cplane + Y * crow + (I >> 1) + ((I + Y + Z) & 1 ? cpairs : 0)];
           };
-          const float am = at(Xm), a0 = at(X), ap = at(Xp);
-          o[0][dz][dy] = __fmaf_rn(0.25f, am - a0, a0);
-          o[1][dz][dy] = __fmaf_rn(0.25f, ap - a0, a0);
+          if (!ANY || C.rx == 2) {
+            const float am = at(X > 0 ? X - 1 : X), a0 = at(X), ap = at(X < C.nx - 1 ? X + 1 : X);
+            o[0][dz][dy] = __fmaf_rn(0.25f, am - a0, a0);
+            o[1][dz][dy] = __fmaf_rn(0.25f, ap - a0, a0);
+          } else {
+            o[0][dz][dy] = at(2 * X);
+            o[1][dz][dy] = at(single ? 2 * X : 2 * X + 1);
+          }
         }
 #pragma unroll
       for (int q = 0; q < 2; q++) {
         const float y0 = __fmaf_rn(wy, o[q][0][1] - o[q][0][0], o[q][0][0]);
         const float y1 = __fmaf_rn(wy, o[q][1][1] - o[q][1][0], o[q][1][0]);
-        x[p + ((q + j + k) & 1 ? pairs : 0)] += __fmaf_rn(wz, y1 - y0, y0);
+        if (q == 0 || !single) x[p + ((q + j + k) & 1 ? pairs : 0)] += __fmaf_rn(wz, y1 - y0, y0);
       }
     }
     // each thread goes on with the pairs it has just written; the sweeps begin
     // with a barrier
-    bottom_sweeps(smem, a.lvl, l, a.post, false, -1);
+    bottom_sweeps<PAIRS, ANY>(smem, a.lvl, l, a.post, false, -1);
   }
   {
     const BottomLevel &L = reinterpret_cast<const BottomLevel *>(smem + a.lvl)[0];
-    const int pairs = (L.nx >> 1) * L.ny * L.nz;
+    const int pairs = ((L.nx + 1) >> 1) * L.ny * L.nz;
     for (int p = tid; p < pairs; p += kBottomThreads) {
       int t, j, k;
       bottom_pair(L, p, t, j, k);
       const float e = smem[L.x + p], o = smem[L.x + pairs + p];
-      reinterpret_cast<float2 *>(a.x)[p] = (j + k) & 1 ? make_float2(o, e) : make_float2(e, o);
+      const bool odd = (j + k) & 1;
+      float *const to = a.x + (k * L.ny + j) * L.nx + 2 * t;
+      if (!ANY || !(L.nx & 1)) {
+        *reinterpret_cast<float2 *>(to) = odd ? make_float2(o, e) : make_float2(e, o);
+      } else {
+        to[0] = odd ? o : e;
+        if (2 * t + 1 < L.nx) to[1] = odd ? e : o;
+      }
     }
   }
 }
@@ -2933,21 +2981,15 @@ bool tail_vcycle(MgHierarchy *H, int l, T **xs, T **bs, bool zero)
 }
 
 // The levels that k_mg_bottom takes: from the first of at most kBottomCells
-// cells below the top, where at least one lies above an exactly solved
-// coarsest level and each can be walked as the per-level kernels would (x
-// halved between all of them, rows of a multiple of four cells, as
-// k_rbgs_sweep, k_mg_restrict_x2 and k_mg_prolong_x4 want them). 0: none.
+// cells (rows rounded up to even) below the top, where at least one lies above an
+// exactly solved coarsest level. 0: none.
 int bottom_level(const MgHierarchy *H)
 {
-  const MgLevelDesc &Lc = H->lv[H->nl - 1];
-  const int nc = Lc.n[0] * Lc.n[1] * Lc.n[2];
-  if (!H->minv32 || nc % 4 != 0 || nc > kBottomDirect) return 0;
+  if (!H->minv32) return 0;
   int l0 = 0;
   for (int l = H->nl - 2; l >= 1; l--) {
     const MgLevelDesc &L = H->lv[l];
-    if ((int64_t)L.n[0] * L.n[1] * L.n[2] > kBottomCells || L.n[0] % 4 != 0 ||
-        H->lv[l + 1].r[0] != 2)
-      break;
+    if ((int64_t)((L.n[0] + 1) / 2 * 2) * L.n[1] * L.n[2] > kBottomCells) break;
     l0 = l;
   }
   return l0;
@@ -2966,40 +3008,49 @@ bool bottom_vcycle(MgHierarchy *H, int l)
     t.nx = v.nx;
     t.ny = v.ny;
     t.nz = v.nz;
+    t.rx = L.r[0];
     t.ry = L.r[1];
     t.rz = L.r[2];
+    const int row = (v.nx + 1) / 2;
     const auto magic = [](int d) { return d > 1 ? (unsigned)(((1ull << 32) + d - 1) / d) : 0u; };
-    t.mrow = magic(v.nx / 2);
-    t.mpl = magic(v.nx / 2 * v.ny);
+    t.mrow = magic(row);
+    t.mpl = magic(row * v.ny);
     t.ex = v.ex;
     t.ey = v.ey;
     t.ez = v.ez;
     t.diag = v.diag;
     t.inv_diag = v.inv_diag;
-    const int n = (v.nx * v.ny * v.nz + 3) / 4 * 4;
+    const int n = (2 * row * v.ny * v.nz + 3) / 4 * 4;
     t.x = at;
     t.b = at + n;
     at += 2 * n;
   }
   a.res = at;
-  at += (a.lv[0].nx * a.lv[0].ny * a.lv[0].nz + 3) / 4 * 4;
+  at += a.lv[0].b - a.lv[0].x;
   a.lvl = at;
   at += (a.count * (int)sizeof(BottomLevel) / 4 + 3) / 4 * 4;
   const MgLevelDesc &Lc = H->lv[H->nl - 1];
   const int nc = Lc.n[0] * Lc.n[1] * Lc.n[2];
   a.pre = H->pre;
   a.post = H->post;
-  a.rows = (nc + kBottomBlocks - 1) / kBottomBlocks;
+  a.rows = ((nc + kBottomBlocks - 1) / kBottomBlocks + 3) / 4 * 4;  // copies start on 16 bytes
+  size_t bytes = sizeof(float) * ((size_t)at + (size_t)a.rows * nc);
   a.m = at;
+  if (bytes > kBottomSmem) {  // the rows are read where they are
+    bytes = sizeof(float) * (size_t)at;
+    a.m = -1;
+  }
   a.minv = H->minv32;
   a.b = H->b32[l];
   a.x = H->x32[l];
   a.st = H->d_state;
-  const size_t bytes = sizeof(float) * ((size_t)at + (size_t)a.rows * nc);
-  static_assert(sizeof(float) * (5 * kBottomCells + kBottomDirect / kBottomBlocks * kBottomDirect) + kMaxLevels * sizeof(BottomLevel) <=
-                    226 * 1024,
-      "shared memory");
-  if (!cuda_ok(cudaFuncSetAttribute(k_mg_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const int pairs = (a.lv[0].b - a.lv[0].x) / 2;
+  bool any = pairs > 2 * kBottomThreads;  // (one general form for the larger levels)
+  auto kernel = any ? k_mg_bottom<kBottomPairs, true> : k_mg_bottom<2, false>;
+  for (int q = 0; q + 1 < a.count; q++) any |= a.lv[q].nx % 2 != 0 || a.lv[q + 1].rx != 2;
+  any |= a.lv[a.count - 1].nx % 2 != 0;
+  if (any && pairs <= 2 * kBottomThreads) kernel = k_mg_bottom<2, true>;
+  if (!cuda_ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                    (int)bytes),
           "k_mg_bottom shared memory"))
     return false;
@@ -3014,7 +3065,7 @@ bool bottom_vcycle(MgHierarchy *H, int l)
   at0[0].val.clusterDim.y = at0[0].val.clusterDim.z = 1;
   cfg.attrs = at0;
   cfg.numAttrs = 1;
-  if (!cuda_ok(cudaLaunchKernelEx(&cfg, k_mg_bottom, a), "k_mg_bottom")) return false;
+  if (!cuda_ok(cudaLaunchKernelEx(&cfg, kernel, a), "k_mg_bottom")) return false;
   return launched("k_mg_bottom");
 }
 
@@ -3289,7 +3340,7 @@ bool mg_setup(Solver *s, Discretization *d, SolverState *ss)
         return false;
     } else {
       std::vector<float> m32(minv.begin(), minv.end());
-      if (!cuda_ok(cudaMalloc(&H->minv32, m32.size() * sizeof(float)), "cudaMalloc(minv32)") ||
+      if (!cuda_ok(cudaMalloc(&H->minv32, (m32.size() + 4) * sizeof(float)), "cudaMalloc(minv32)") ||
           !cuda_ok(cudaMemcpy(H->minv32, m32.data(), m32.size() * sizeof(float),
                        cudaMemcpyHostToDevice),
               "upload minv32"))

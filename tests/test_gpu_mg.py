@@ -470,14 +470,16 @@ def test_integer_pipe_conversions_match_hardware(nusif_lib):
     assert torch.equal(d[~nan].view(torch.int64), want[~nan].view(torch.int64))
 
 
-# (fine grid, levels the cluster kernel takes): a level of exactly 4096 cells
-# and one just above, x halved alone, y or z halved with x, rows of 4 and 12
-# cells, a coarsest level of a few cells and of 512
+# a level of exactly 4096 cells and one just above, x halved alone, y or z halved
+# with x, rows of 4 and 12 cells, a coarsest level of a few cells, of 512 and of
+# 900; odd rows, x not halved with y and z
 @pytest.mark.parametrize("dims,pre,post", [((32, 32, 32), 2, 2), ((64, 32, 34), 1, 1),
                                            ((512, 16, 16), 2, 1), ((64, 16, 4), 1, 2),
                                            ((12, 96, 12), 1, 1), ((48, 24, 24), 3, 3),
                                            ((16, 8, 8), 2, 2), ((160, 96, 96), 1, 1),
-                                           ((24, 40, 56), 2, 0)])
+                                           ((24, 40, 56), 2, 0), ((36, 36, 36), 2, 2),
+                                           ((36, 20, 20), 1, 1), ((13, 26, 52), 2, 2),
+                                           ((18, 9, 33), 1, 1), ((9, 32, 28), 2, 1)])
 def test_coarse_cluster_matches_per_level_kernels(nusif_lib, dims, pre, post):
     """The coarse levels in one cluster give the same bits as a kernel per
     sweep and transfer (mg_tail = 1: no level is that small, so none is taken)."""
