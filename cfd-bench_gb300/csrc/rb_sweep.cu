@@ -56,7 +56,9 @@
 // blocks in early took 1 us more (they double up on the idle SMs).
 #include <cmath>
 #include <cstdint>
+#include <utility>
 #include <cstring>
+#include <type_traits>
 
 #include "df32.cuh"
 #include "nusif_internal.h"
@@ -458,6 +460,207 @@ __global__ void k_rb_finish(RbState *st, const df::f2 *part, int n, int np)
   }
 }
 
+// All the iterations of a small grid in one cluster, d and r0 in shared memory.
+// The grid is cut into slabs along its longest axis (2 here, whichever it is of
+// x, y and z; 0 is the axis of the pairs), P planes to a block and a copy of the
+// neighbours' planes on each side, which they write as they update. Two copies
+// of d: an iteration reads one and writes the other, first colour, barrier,
+// second colour, barrier. The last warps relax nothing; they sum the squares of
+// the iteration before while the others work, send the block's sums to all
+// blocks in the first half and decide in the second, so the stop costs one
+// iteration too many but no time in each.
+//
+// What bounds it: the barrier of the cluster (about 0.3 us, twice an iteration)
+// and the updates' latency, from 10 thousand cells on their issue on sixteen
+// SMs. An iteration, sweeps -> cluster: 12^3 4.9 -> 2.4 us, 20^3 4.4 -> 2.3,
+// 64 x 10 x 61 4.4 -> 3.2.
+struct ClusterArgs {
+  int n[3];       // cells per axis, the slab axis last
+  int axis[3];    // which of x, y, z each is
+  int np, plane;  // pairs per row and per plane
+  int P;          // planes per block
+  int blocks;     // of the cluster
+  unsigned mrow, mpl;  // 2^32 / np and / plane, rounded up (0: 1)
+};
+
+__device__ __forceinline__ void cluster_barrier(int blocks)
+{
+  if (blocks == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  }
+}
+
+__device__ __forceinline__ unsigned in_block(const void *p, int rank)
+{
+  unsigned a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n"
+               : "=r"(a)
+               : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void store_in(unsigned at, df::f2 v)
+{
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(at), "f"(v.hi), "f"(v.lo)
+               : "memory");
+}
+__device__ __forceinline__ void store_in(unsigned at, double v)
+{
+  asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(at), "d"(v) : "memory");
+}
+
+constexpr int kFoldWarps = 4;
+
+// sums of non-negative pairs that need no order: without renormalising between
+__device__ __forceinline__ df::f2 warp_sum(df::f2 v)
+{
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    v = df::add_u(v, df::f2{ __shfl_xor_sync(0xffffffffu, v.hi, o),
+                             __shfl_xor_sync(0xffffffffu, v.lo, o) });
+  return df::renorm(v.hi, v.lo);
+}
+
+template <typename V, bool CUBE>
+__global__ void __launch_bounds__(1024) k_rb_cluster(ClusterArgs A, SweepArgs G, Consts<V> C,
+    const V *__restrict__ r0, V *d0, V *d1, RbState *st, int direct)
+{
+  if (is_done(st)) return;  // the same for all blocks
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ df::f2 total[16 * kFoldWarps];
+  __shared__ int go;
+  const int tid = threadIdx.x, lane = tid & 31, workers = blockDim.x - 32 * kFoldWarps;
+  const bool work = tid < workers;
+  const int rank = blockIdx.x, plane = A.plane, np = A.np;
+  const int first = rank * A.P, mine = max(0, min(A.P, A.n[2] - first)) * plane;
+  const int size = (A.P + 2) * plane;  // one colour, one copy
+  V *const cells = reinterpret_cast<V *>(smem_raw);  // [copy][colour][plane -1 .. P][pair]
+  V *const rs = cells + 4 * size;                    // [colour][pair]
+  V *const squares = rs + 2 * A.P * plane;           // a worker's sum
+  unsigned char *const flag = reinterpret_cast<unsigned char *>(squares + workers);
+  const auto cell = [&](int q, int e, int &colour) {  // of pair q, its global offset
+    const int kk = A.mpl ? (int)__umulhi((unsigned)q, A.mpl) : q, jt = q - kk * plane;
+    const int j = A.mrow ? (int)__umulhi((unsigned)jt, A.mrow) : jt, t = jt - j * np;
+    const int c[3] = { 2 * t + e, j, first + kk };
+    int x[3];
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+      x[a] = A.axis[0] == a ? c[0] : A.axis[1] == a ? c[1] : c[2];
+    colour = (c[0] + c[1] + c[2]) & 1;
+    return c[0] < A.n[0] ? colour * G.half + G.at(x[0] >> 1, x[1], x[2]) : -1;
+  };
+  for (int q = tid; q < 4 * size; q += blockDim.x) cells[q] = V();
+  for (int q = tid; q < mine; q += blockDim.x) {
+    const int kk = A.mpl ? (int)__umulhi((unsigned)q, A.mpl) : q, jt = q - kk * plane;
+    const int j = A.mrow ? (int)__umulhi((unsigned)jt, A.mrow) : jt, t = jt - j * np;
+    const int k = first + kk;
+    flag[q] = (unsigned char)((t > 0) | (2 * t + 2 < A.n[0]) << 1 | (j > 0) << 2 |
+                              (j < A.n[1] - 1) << 3 | (k > 0) << 4 | (k < A.n[2] - 1) << 5 |
+                              (2 * t + 1 == A.n[0]) << 6 | ((j + k) & 1) << 7);
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      int colour;
+      const int o = cell(q, e, colour);
+      rs[colour * A.P * plane + q] = o >= 0 ? r0[o] : V();
+    }
+  }
+  double res = 0.0, epssq = 0.0, inv_factor2 = 0.0, inv_ncell = 0.0;
+  const int itermax = st->s.itermax;
+  if (!work) {
+    res = st->s.res;
+    epssq = st->s.epssq;
+    inv_factor2 = st->inv_factor2;
+    inv_ncell = st->inv_ncell;
+  }
+  if (tid == 0) go = 1;
+  cluster_barrier(A.blocks);
+  const bool low = rank > 0, high = rank < A.blocks - 1;
+  unsigned flags = 0u;  // of the thread's first four pairs
+  if (work)
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (tid + u * workers < mine) flags |= (unsigned)flag[tid + u * workers] << (8 * u);
+  int n = direct;
+  V acc{};
+  // one colour of an iteration: reads copy `from` (its own cells; the other
+  // colour's from `to` once they are new there), writes copy `to`
+  const auto half_pass = [&](int from, int to, int h) {
+    const V *const own = cells + (2 * from + h) * size + plane;
+    const V *const o = cells + (2 * (h ? to : from) + 1 - h) * size + plane;
+    V *const out = cells + (2 * to + h) * size + plane;
+    const V *const r = rs + h * A.P * plane;
+    unsigned fs = flags;
+    for (int q = tid, u = 0; q < mine; q += workers, u++) {
+      const int f = u < 4 ? (int)(fs & 255u) : flag[q];
+      fs >>= 8;
+      const bool left = (f >> 7) == h;  // the colour's cell is the pair's left one
+      if ((f & 64) && !left) continue;
+      // a neighbour beyond a wall is the cell itself: selected addresses, no branches
+      const V *const cq = own + q, *const oq = o + q;
+      const V c = *cq;
+      const V in = *(f & 64 ? cq : oq);
+      const V side = *(f & (left ? 1 : 2) ? oq + (left ? -1 : 1) : cq);
+      const V s = *(f & 4 ? oq - np : cq), nn = *(f & 8 ? oq + np : cq);
+      const V b = *(f & 16 ? oq - plane : cq), t = *(f & 32 ? oq + plane : cq);
+      const V D = change<CUBE>(C, c, in, side, s, nn, b, t, r[q]);
+      const V m = moved(c, D);
+      add_square(acc, D);
+      out[q] = m;
+      // the planes beside the slab's ends are also the neighbours'
+      if (low && q < plane) store_in(in_block(out + A.P * plane + q, rank - 1), m);
+      if (high && q >= mine - plane) store_in(in_block(out + q - mine, rank + 1), m);
+    }
+  };
+  for (;;) {
+    const int from = n & 1, to = from ^ 1;
+    if (work) {
+      acc = V();
+      half_pass(from, to, 0);
+    } else if (n > direct) {  // iteration n's squares in this block
+      const int w = (tid - workers) >> 5;
+      df::f2 v[2] = {};
+      for (int q = lane + 32 * w; q < workers; q += 64 * kFoldWarps)
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+          if (q + 32 * kFoldWarps * u < workers)
+            v[u] = df::add_u(v[u], as_pair(squares[q + 32 * kFoldWarps * u]));
+      const df::f2 sum = warp_sum(df::add_u(v[0], v[1]));
+      if (lane < A.blocks) store_in(in_block(total + rank * kFoldWarps + w, lane), sum);
+    }
+    cluster_barrier(A.blocks);
+    if (work) {
+      half_pass(from, to, 1);
+      squares[tid] = acc;
+    } else if (n > direct) {  // whether it was the last
+      df::f2 v{ 0.0f, 0.0f };
+#pragma unroll
+      for (int u = 0; u < 16 * kFoldWarps; u += 32)
+        if (lane + u < A.blocks * kFoldWarps) v = df::add_u(v, total[lane + u]);
+      res = (res + df::to_double(warp_sum(v)) * inv_factor2) * inv_ncell;
+      if (tid == workers && !(res >= epssq && n < itermax)) go = 0;
+    }
+    cluster_barrier(A.blocks);
+    if (!go) break;
+    n++;
+  }
+  // iteration n's d, as the sweeps leave it
+  V *const d = n & 1 ? d1 : d0;
+  for (int q = tid; q < mine; q += blockDim.x)
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      int colour;
+      const int o = cell(q, e, colour);
+      if (o >= 0) d[o] = cells[(2 * (n & 1) + colour) * size + plane + q];
+    }
+  if (rank == 0 && tid == (int)blockDim.x - 1) {
+    st->s.res = res;
+    st->s.it = n;
+    st->s.done = 1;
+  }
+}
+
 constexpr int kFoldMax = 1024;   // block sums that each block of the next sweep folds itself
 
 int up(int a, int b) { return (a + b - 1) / b; }
@@ -510,6 +713,29 @@ SweepArgs sweep_shape(int nx, int ny, int nz)
   return a;
 }
 
+// The slabs of a cluster of `blocks` and its shared memory.
+size_t cluster_shape(ClusterArgs &a, const int (&n)[3], int blocks, int threads)
+{
+  int slab = 2;
+  for (int q = 1; q >= 0; q--)
+    if (n[q] > n[slab]) slab = q;
+  int row = slab == 0 ? 1 : 0, mid = 3 - slab - row;
+  if (n[mid] > n[row]) std::swap(row, mid);
+  a.axis[0] = row;
+  a.axis[1] = mid;
+  a.axis[2] = slab;
+  for (int q = 0; q < 3; q++) a.n[q] = n[a.axis[q]];
+  a.np = up(a.n[0], 2);
+  a.plane = a.np * a.n[1];
+  a.blocks = blocks;
+  a.P = up(a.n[2], blocks);
+  const auto magic = [](int d) { return d > 1 ? (unsigned)(((1ull << 32) + d - 1) / d) : 0u; };
+  a.mrow = magic(a.np);
+  a.mpl = magic(a.plane);
+  return 8 * (4 * (size_t)(a.P + 2) * a.plane + 2 * (size_t)a.P * a.plane + threads) +
+         (size_t)a.P * a.plane;
+}
+
 }  // namespace
 
 // what a solver keeps for its sweeps: the shape, and the device memory (two
@@ -522,6 +748,10 @@ struct RbPlan {
   size_t smem = 0;
   bool cube = false;  // one spacing on all axes
   void *cells = nullptr;
+  // the cluster of a small grid (threads 0: none)
+  ClusterArgs c;
+  int cluster_threads = 0;
+  size_t cluster_smem = 0;
 };
 
 namespace {
@@ -545,6 +775,80 @@ bool launch_sweep(const RbPlan &P, const Consts<V> &C, const V *d, V *dout, cons
   cudaLaunchKernelEx(&cfg, P.cube ? k_rb_sweep<V, true> : k_rb_sweep<V, false>, P.a, C, d, dout, r0,
       st, part_in, part_out, n, np);
   return launched("k_rb_sweep");
+}
+
+template <typename V>
+bool cluster_config(const RbPlan &P, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at)
+{
+  auto kernel = P.cube ? k_rb_cluster<V, true> : k_rb_cluster<V, false>;
+  cfg = {};
+  cfg.gridDim = dim3(P.c.blocks);
+  cfg.blockDim = dim3(P.cluster_threads);
+  cfg.dynamicSmemBytes = P.cluster_smem;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = P.c.blocks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+             (int)P.cluster_smem) == cudaSuccess &&
+         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+             cudaSuccess;
+}
+
+template <typename V>
+bool launch_cluster(const RbPlan &P, const Consts<V> &C, const V *r0, V *const (&d)[2], RbState *st,
+    int direct)
+{
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  if (!cluster_config<V>(P, cfg, at)) return cuda_ok(cudaGetLastError(), "k_rb_cluster attributes");
+  cfg.stream = stream();
+  const V f[3] = { C.fx, C.fy, C.fz };
+  Consts<V> T = C;
+  T.fx = f[P.c.axis[0]];
+  T.fy = f[P.c.axis[1]];
+  T.fz = f[P.c.axis[2]];
+  cudaLaunchKernelEx(&cfg, P.cube ? k_rb_cluster<V, true> : k_rb_cluster<V, false>, P.c, P.a, T, r0,
+      d[0], d[1], st, direct);
+  return launched("k_rb_cluster");
+}
+
+// The cluster for a grid, or none. Pairs: as few blocks as leave each at most a
+// pair of cells for each of 256 workers, else sixteen, with 512 workers from
+// two pairs each on, up to three (48 thousand cells): an iteration takes 2.3 us
+// at 20^3, 2.8 at 30^3, 3.2 at 64 x 10 x 61, 4.8-5.3 at 40^3, sweeps 4.4, 4.3, 4.4
+// and 4.9. Doubles: the FP64 pipe of sixteen SMs takes over sooner, 2.9 us at
+// 12^3, 3.9 at 20^3 and 7.1 at 30^3 against 5.5, 5.1 and 5.1.
+template <typename V>
+void choose_cluster(RbPlan &P)
+{
+  constexpr bool pairs = std::is_same_v<V, df::f2>;
+  constexpr int kEach = pairs ? 256 : 64, kMore = pairs ? 512 : 128, kMost = pairs ? 1536 : 450;
+  const int n[3] = { P.a.nx, P.a.ny, P.a.nz };
+  int threads = 0;
+  for (int blocks = 1; blocks <= 16; blocks *= 2) {
+    cluster_shape(P.c, n, blocks, 0);
+    const int mine = P.c.P * P.c.plane;
+    if (mine > kEach && blocks < 16) continue;
+    if (mine > kMost) return;
+    const int workers = mine > kMore ? 512 : pairs ? 256 : 128;
+    threads = workers + 32 * kFoldWarps;
+    P.cluster_smem = cluster_shape(P.c, n, blocks, threads);
+    break;
+  }
+  if (P.cluster_smem > 226 * 1024) return;
+  P.cluster_threads = threads;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  int fit = 0;
+  if (!cluster_config<V>(P, cfg, at) ||
+      cudaOccupancyMaxActiveClusters(&fit, P.cube ? k_rb_cluster<V, true> : k_rb_cluster<V, false>,
+          &cfg) != cudaSuccess ||
+      fit < 1) {
+    cudaGetLastError();
+    P.cluster_threads = 0;
+  }
 }
 
 template <typename V>
@@ -601,6 +905,10 @@ double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, cons
         k_rb_open<V><<<(unsigned)up(a.half, 256), 256, 0, q>>>(a, A, p, rhs, d[n & 1], r0, st);
         if (!launched("k_rb_open")) return NAN;
       }
+      if (P.cluster_threads) {  // to the end
+        if (!launch_cluster<V>(P, C, r0, d, st, direct)) return NAN;
+        n = s->itermax;
+      }
       for (int c = 0; c < chunk && n < s->itermax; c++) {
         n++;
         const int in = (n - 1) & 1, out = n & 1;
@@ -613,8 +921,10 @@ double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, cons
                 first ? 0 : folded ? 1 : nb))
           return NAN;
       }
-      k_rb_finish<<<1, 32, 0, q>>>(st, part[n & 1], n, nb);
-      if (!launched("k_rb_finish")) return NAN;
+      if (!P.cluster_threads) {
+        k_rb_finish<<<1, 32, 0, q>>>(st, part[n & 1], n, nb);
+        if (!launched("k_rb_finish")) return NAN;
+      }
       k_rb_close<V><<<(unsigned)up(a.np * a.ny * a.nz, 256), 256, 0, q>>>(a, g, p, d[0], d[1], st,
           direct);
       if (!launched("k_rb_close")) return NAN;
@@ -651,6 +961,8 @@ bool rb_sweep_alloc(SolverState *ss, const Dims &g, bool cube)
     cudaGetLastError();
     P->cells = nullptr;
   }
+  if (P->cells && ss->ext.arith_fp64) choose_cluster<double>(*P);
+  if (P->cells && !ss->ext.arith_fp64) choose_cluster<df::f2>(*P);
   return cuda_ok(cudaMalloc(&ss->d_rb, sizeof(RbState)), "cudaMalloc(rb state)") &&
          cuda_ok(cudaMallocHost(&ss->h_rb, sizeof(RbState)), "cudaMallocHost(rb state)");
 }

@@ -3,6 +3,9 @@ where its tiles can go wrong: one cell, rows of odd length (a pair without a
 second column), rows cut into tiles (more than 128 cells), rows and planes
 that end inside a block, and stops after the iterations that run on p itself.
 
+Small grids run all iterations in one cluster of blocks: one block, several,
+sixteen, the last slabs empty or not full, and the largest it takes.
+
 Tolerance: an update rounds its operands to pairs, a few 2^-47 (7e-15) of the
 largest pressure, and the iteration does not amplify it; 60 iterations of a
 dozen such roundings stay below 60 * 12 * 7e-15 = 5e-12, so 1e-11.
@@ -44,3 +47,10 @@ def test_sweeps_match_oracle(nusif_lib, oracle_mod, dims, arith):
                 assert sim.iterations == it
                 assert res == pytest.approx(res_c, rel=1e-11)
                 assert rel_err(sim.field("p"), p) < 1e-11
+
+
+@pytest.mark.parametrize("arith", ["df32", "fp64"])
+@pytest.mark.parametrize("dims", [(8, 8, 8), (12, 12, 12), (17, 16, 5), (20, 20, 20), (9, 73, 28),
+                                  (64, 10, 61), (131, 21, 12), (33, 31, 30), (36, 36, 36)])
+def test_cluster_matches_oracle(nusif_lib, oracle_mod, dims, arith):
+    test_sweeps_match_oracle(nusif_lib, oracle_mod, dims, arith)
