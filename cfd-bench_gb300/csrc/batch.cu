@@ -123,6 +123,7 @@ bool enqueue_step(BatchInst *b, bool normalize, int queue, cudaStream_t body)
   if (normalize) {
     if (!launch_interior_sum(g, d->p, st->red, st->d_scalars + 3)) return false;
     if (!launch_subtract_mean(g, d->p, st->d_scalars + 4)) return false;
+    if (!mg_normalize_history(ss, g, st->red, st->d_scalars + 3)) return false;
   }
   const bool solved = queue > 0 ? mg_enqueue(ss, d->p, d->rhs, queue, &b->dev->unconverged,
                                       &b->dev->last_cycles)

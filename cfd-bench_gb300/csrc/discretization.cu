@@ -722,9 +722,11 @@ __global__ void __launch_bounds__(kBlock) k_shell_max3(Dims g, const double *__r
 // ---- normalizePressure (discretization.c:403-429) ----
 // Interior sum (block partials folded by the last block), then the mean is
 // subtracted by a second kernel that reads it from device memory.
+// kept: when set, nothing is done while *kept is 0 (a warm start without history).
 __global__ void __launch_bounds__(kBlock) k_interior_sum(Dims g, const double *__restrict__ p,
-    double *__restrict__ partials, unsigned *ticket, double *__restrict__ out)
+    double *__restrict__ partials, unsigned *ticket, double *__restrict__ out, const int *kept)
 {
+  if (kept && *kept == 0) return;
   const int64_t ncell = (int64_t)g.imax * g.jmax * g.kmax;
   double s = 0.0;
   for (int64_t q = blockIdx.x * (int64_t)kBlock + threadIdx.x; q < ncell;
@@ -755,8 +757,9 @@ __global__ void __launch_bounds__(kBlock) k_interior_sum(Dims g, const double *_
 }
 
 __global__ void __launch_bounds__(kBlock) k_subtract_mean(Dims g, double *__restrict__ p,
-    const double *__restrict__ mean)
+    const double *__restrict__ mean, const int *kept)
 {
+  if (kept && *kept == 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
@@ -914,18 +917,20 @@ bool launch_rhs(const Dims &g, double dt, double dx, double dy, double dz, const
   return launched("k_rhs");
 }
 
-bool launch_interior_sum(const Dims &g, const double *p, ReduceScratch &red, double *d_out)
+bool launch_interior_sum(const Dims &g, const double *p, ReduceScratch &red, double *d_out,
+    const int *kept)
 {
   const int64_t most = ((int64_t)g.imax * g.jmax * g.kmax + kBlock - 1) / kBlock;
   const int blocks = (int)std::min<int64_t>(4 * sm_count(), most);
   if (!reduce_scratch_alloc(red, 3 * blocks)) return false;
-  k_interior_sum<<<blocks, kBlock, 0, stream()>>>(g, p, red.partials, red.ticket, d_out);
+  k_interior_sum<<<blocks, kBlock, 0, stream()>>>(g, p, red.partials, red.ticket, d_out,
+      kept);
   return launched("k_interior_sum");
 }
 
-bool launch_subtract_mean(const Dims &g, double *p, const double *d_mean)
+bool launch_subtract_mean(const Dims &g, double *p, const double *d_mean, const int *kept)
 {
-  k_subtract_mean<<<cell_grid(g, kCellBlock), kCellBlock, 0, stream()>>>(g, p, d_mean);
+  k_subtract_mean<<<cell_grid(g, kCellBlock), kCellBlock, 0, stream()>>>(g, p, d_mean, kept);
   return launched("k_subtract_mean");
 }
 
@@ -1199,8 +1204,11 @@ void normalizePressure(Discretization *s)
 {
   DiscState *st = need_state(s, "normalizePressure");
   if (!st || !await_arrays({}, { s->p })) return;
-  if (!launch_interior_sum(st->dims, s->p, st->red, st->d_scalars + 3)) return;
-  launch_subtract_mean(st->dims, s->p, st->d_scalars + 4);
+  if (!launch_interior_sum(st->dims, s->p, st->red, st->d_scalars + 3) ||
+      !launch_subtract_mean(st->dims, s->p, st->d_scalars + 4))
+    return;
+  for (SolverState *ss : st->solvers)
+    if (!mg_normalize_history(ss, st->dims, st->red, st->d_scalars + 3)) return;
 }
 
 void adaptUV(Discretization *s)

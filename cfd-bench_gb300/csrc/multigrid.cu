@@ -110,6 +110,7 @@ struct MgHierarchy {
   double *p_prev2 = nullptr;  // and of the one before (guess >= 2)
   double *p_prev3 = nullptr;  // and of the one before that (guess 3)
   int *d_hist = nullptr;      // device: earlier solutions kept (0, 1, 2)
+  const Discretization *disc = nullptr;  // key of the state that lists this solver
   // the solve as one CUDA graph (head, while-loops, tail) for fixed p / rhs
   cudaGraphExec_t graph = nullptr;
   const double *graph_p = nullptr, *graph_rhs = nullptr;
@@ -3277,6 +3278,8 @@ bool mg_setup(Solver *s, Discretization *d, SolverState *ss)
       return false;
     if (H->guess >= 3 && !cuda_ok(cudaMalloc(&H->p_prev3, padded), "cudaMalloc(p_prev3)"))
       return false;
+    H->disc = d;
+    if (DiscState *ds = disc_state(d)) ds->solvers.push_back(ss);
     if (!cuda_ok(cudaMalloc(&H->d_hist, 2 * sizeof(int)), "cudaMalloc(hist)") ||
         !cuda_ok(cudaMemset(H->d_hist, 0, 2 * sizeof(int)), "hist init"))
       return false;
@@ -3638,6 +3641,22 @@ bool build_solve_graph(MgHierarchy *H, double *p, const double *rhs)
 
 }  // namespace
 
+// normalizePressure on the warm start's earlier solutions, each about its own
+// mean, so that they stay level with p: an extrapolation over the step in the
+// mean carries it on as its polynomial, a quadratic one 5000-fold by the next
+// normalisation 100 steps later. From step 300 the mean drowned the residual and
+// every solve ran to its cycle limit (256^3: 107 instead of 2.4 ms per step).
+bool mg_normalize_history(SolverState *ss, const Dims &g, ReduceScratch &red, double *d_sum_mean)
+{
+  MgHierarchy *H = ss->mg;
+  if (!H || H->guess < 1) return true;
+  for (double *b : { H->p_prev, H->p_prev2, H->p_prev3})
+    if (b && (!launch_interior_sum(g, b, red, d_sum_mean, H->d_hist) ||
+                 !launch_subtract_mean(g, b, d_sum_mean + 1, H->d_hist)))
+      return false;
+  return true;
+}
+
 // The solve as a fixed sequence of launches with no host synchronisation
 // (graph capture): state initialisation, right-hand-side statistics, `queue`
 // units (FP64 V-cycles for mg, outer refinement iterations for mg-mixed; the
@@ -3853,6 +3872,10 @@ void mg_free(Solver *s, SolverState *ss)
 {
   MgHierarchy *H = ss->mg;
   if (!H) return;
+  if (DiscState *ds = H->disc ? disc_state(H->disc) : nullptr) {
+    auto &v = ds->solvers;
+    v.erase(std::remove(v.begin(), v.end(), ss), v.end());
+  }
   for (int l = 0; l < kMaxLevels; l++) {
     if (H->x64[l]) cudaFree(H->x64[l]);
     if (H->b64[l]) cudaFree(H->b64[l]);

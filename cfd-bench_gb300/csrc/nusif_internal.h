@@ -5,6 +5,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "nusif_gb300.h"
 
 namespace nusif {
@@ -118,7 +120,9 @@ struct DiscState {
   unsigned long long *d_amax = nullptr;  // [kAmaxSlots][3]
   int amax = kAmaxReset;
   long long dt_shell = 0, dt_full = 0;  // computeTimestep calls by path
+  std::vector<struct SolverState *> solvers;  // multigrid solvers of this grid, with a warm start
 };
+bool mg_normalize_history(SolverState *ss, const Dims &g, ReduceScratch &red, double *d_sum_mean);
 // u, v or w changed other than by adaptUV: the kept maxima no longer hold
 inline void velocity_written(DiscState *st)
 {
@@ -137,8 +141,10 @@ bool launch_fgh(const Dims &g, double re, double gamma, double gx, double gy, do
     int kb_fixed = 0, bool fp64 = false);
 bool launch_rhs(const Dims &g, double dt, double dx, double dy, double dz, const double *f,
     const double *gg, const double *h, double *rhs, const StepScalars *sp = nullptr);
-bool launch_interior_sum(const Dims &g, const double *p, ReduceScratch &red, double *d_out);
-bool launch_subtract_mean(const Dims &g, double *p, const double *d_mean);
+bool launch_interior_sum(const Dims &g, const double *p, ReduceScratch &red, double *d_out,
+    const int *kept = nullptr);
+bool launch_subtract_mean(const Dims &g, double *p, const double *d_mean,
+    const int *kept = nullptr);
 bool launch_adapt_uv(const Dims &g, double dt, double dx, double dy, double dz,
     const double *f, const double *gg, const double *h, const double *p, double *u, double *v,
     double *w, const StepScalars *sp = nullptr, unsigned long long *amax_slots = nullptr);

@@ -500,3 +500,17 @@ def test_coarse_cluster_matches_per_level_kernels(nusif_lib, dims, pre, post):
 def test_register_tiled_sweep_on_partial_tiles(nusif_lib, dims, monkeypatch):
     """The same where the last tile of 128 columns or 8 rows is not full."""
     test_register_tiled_sweep_equals_shared_memory_sweep(nusif_lib, dims, monkeypatch)
+
+
+@pytest.mark.parametrize("guess", ["extrapolate", "quadratic", "cubic"])
+def test_long_runs_keep_converging(nusif_lib, guess):
+    """The warm start follows normalizePressure (every 100 steps): solves of
+    steps after several normalisations take no more cycles than before them."""
+    from nusif import Simulation
+    from nusif.params import cavity
+    base = cavity((16, 16, 16), re=100.0, te=1e9, solver="mg-mixed", rtol=1e-6, mg_guess=guess)
+    with Simulation(base) as sim:
+        its = [sim.step().it for _ in range(450)]
+        p = sim.field("p")[1:-1, 1:-1, 1:-1]
+    assert max(its[100:]) <= max(its[:100])
+    assert abs(p.mean()) < 10.0 * np.abs(p - p.mean()).max()
