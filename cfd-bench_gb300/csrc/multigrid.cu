@@ -1644,39 +1644,46 @@ __global__ void __launch_bounds__(kNT) k_mg_prolong_x2(View<T> f, const T *xc, i
 }
 
 // Coarsest level: `sweeps` red-black Gauss-Seidel sweeps from zero by one
-// block, x in shared memory (compact layout). A thread keeps R cells of each
-// colour for all sweeps: their values, right-hand sides and the shared-memory
-// offsets of their neighbours (their own at a wall), two to a register. One
-// block's issue bounds it: 64 sweeps of 15 x 9 x 21 cells 92 -> 21 us (with
-// the cells found by division in every pass before).
+// block, x in shared memory, the colours apart (pair p of cells (2t, 2t + 1) of
+// a row has a slot in each), so that a warp reads consecutive words. A thread
+// keeps R pairs for all sweeps: their values, right-hand sides and the
+// shared-memory offsets of their neighbours outside the pair (their own at a
+// wall), two to a register. Shared-memory accesses and issue of the one block
+// bound it: 64 sweeps of 15 x 9 x 21 cells 92 us with the cells found by
+// division in every pass, 21 with offsets into rows of both colours, 15.4 here.
 template <typename T, int R>
 __global__ void __launch_bounds__(1024) k_mg_coarse(View<T> v, int sweeps, const MgState *st)
 {
   if (mg_done(st)) return;
   extern __shared__ unsigned char smem_raw[];
   const int nx = v.nx, ny = v.ny, nz = v.nz, np = (nx + 1) / 2;  // pairs of cells per row
+  const int plane = np * ny, pairs = plane * nz;
   const auto at = [&](unsigned o) -> T & { return *reinterpret_cast<T *>(smem_raw + o); };
-  unsigned own[2][R], xo[2][R], yo[2][R], zo[2][R];
+  // per colour: own and outer x-neighbour, y- and z-neighbours
+  unsigned own[2][R], yo[2][R], zo[2][R];
   T x[2][R], b[2][R];
+  bool lone[R];  // a pair of one cell
 #pragma unroll
   for (int r = 0; r < R; r++) {
-    const int t = threadIdx.x + r * blockDim.x;
-    const int p = t % np, jk = t / np, j = jk % ny, k = jk / ny;
+    const int p = threadIdx.x + r * blockDim.x;
+    const int t = p % np, jk = p / np, j = jk % ny, k = jk / ny;
+    lone[r] = 2 * t + 1 == nx;
 #pragma unroll
     for (int c = 0; c < 2; c++) {  // first colour: (i + j + k) even
-      const int i = 2 * p + ((j + k + c) & 1);
-      const bool in = k < nz && i < nx;
-      const int q = i + nx * (j + ny * k);
+      const int side = (j + k + c) & 1, i = 2 * t + side;
+      const int q = c * pairs + p, o = (1 - c) * pairs + p;  // this colour's slot, the other's
       const auto off = [&](int cell) { return (unsigned)(cell * (int)sizeof(T)); };
-      own[c][r] = in ? off(q) : 0xffffffffu;
-      if (!in) continue;
-      xo[c][r] = off(i > 0 ? q - 1 : q) | off(i < nx - 1 ? q + 1 : q) << 16;
-      yo[c][r] = off(j > 0 ? q - nx : q) | off(j < ny - 1 ? q + nx : q) << 16;
-      zo[c][r] = off(k > 0 ? q - nx * ny : q) | off(k < nz - 1 ? q + nx * ny : q) << 16;
-      b[c][r] = v.b[q];
-      x[c][r] = (T)0;
-      at(own[c][r]) = (T)0;
+      own[c][r] = 0xffffffffu;
+      if (k >= nz) continue;
+      at(off(q)) = (T)0;
+      if (i >= nx) continue;
+      const bool out = side ? i < nx - 1 : i > 0;
+      own[c][r] = off(q) | off(out ? o + (side ? 1 : -1) : q) << 16;
+      yo[c][r] = off(j > 0 ? o - np : q) | off(j < ny - 1 ? o + np : q) << 16;
+      zo[c][r] = off(k > 0 ? o - plane : q) | off(k < nz - 1 ? o + plane : q) << 16;
+      b[c][r] = v.b[i + nx * (j + ny * k)];
     }
+    x[0][r] = x[1][r] = (T)0;
   }
   __syncthreads();
   for (int it = 0; it < sweeps; it++) {
@@ -1686,22 +1693,104 @@ __global__ void __launch_bounds__(1024) k_mg_coarse(View<T> v, int sweeps, const
       for (int r = 0; r < R; r++) {
         if (own[c][r] == 0xffffffffu) continue;
         const T xc = x[c][r];
-        const T sx = at(xo[c][r] & 0xffffu) + at(xo[c][r] >> 16);
+        const T sx = (lone[r] ? xc : x[1 - c][r]) + at(own[c][r] >> 16);
         const T sy = at(yo[c][r] & 0xffffu) + at(yo[c][r] >> 16);
         const T sz = at(zo[c][r] & 0xffffu) + at(zo[c][r] >> 16);
         const T lap = sx * v.ex + sy * v.ey + sz * v.ez - v.diag * xc;
         const T res = b[c][r] - lap;
         x[c][r] = xc - res * v.inv_diag;
-        at(own[c][r]) = x[c][r];
+        at(own[c][r] & 0xffffu) = x[c][r];
       }
       __syncthreads();
     }
   }
 #pragma unroll
-  for (int r = 0; r < R; r++)
+  for (int r = 0; r < R; r++) {
+    const int p = threadIdx.x + r * blockDim.x;
+    const int t = p % np, jk = p / np;
 #pragma unroll
     for (int c = 0; c < 2; c++)
-      if (own[c][r] != 0xffffffffu) v.x[own[c][r] / sizeof(T)] = x[c][r];
+      if (own[c][r] != 0xffffffffu)
+        v.x[jk * nx + 2 * t + ((jk % ny + jk / ny + c) & 1)] = x[c][r];
+  }
+}
+
+// The same in FP64: one SM's FP64 pipe would bound it (64 sweeps of 9 x 10 x 12
+// cells 190 us), so a cluster of up to eight blocks takes the level in slabs of
+// P planes, each with a copy of its neighbours' outer planes, which they write
+// as they update; a barrier of the cluster after each colour (about 0.25 us)
+// and the pass's latency are what is left. Per V(2,2) cycle with such a coarsest
+// level: 36 x 20 x 48 260 -> 147 us, 48^3 333 -> 163, 28^3 437 -> 138.
+constexpr int kCoarseBlocks = 8, kCoarseThreads = 256, kCoarseCells64 = 16384;
+
+__global__ void __launch_bounds__(kCoarseThreads) k_mg_coarse_f64(View<double> v, Smooth64 C,
+    int sweeps, int P, const MgState *st)
+{
+  if (mg_done(st)) return;  // the same for all blocks
+  extern __shared__ unsigned char smem_raw[];
+  const int nx = v.nx, ny = v.ny, nz = v.nz, np = (nx + 1) / 2, plane = np * ny;
+  const int rank = blockIdx.x, blocks = gridDim.x, tid = threadIdx.x, first = rank * P;
+  const int mine = max(0, min(P, nz - first)) * plane, size = (P + 2) * plane;
+  double *const x = reinterpret_cast<double *>(smem_raw);  // [colour][plane -1 .. P][pair]
+  double *const rb = x + 2 * size;                         // -inv b, [colour][pair]
+  unsigned char *const flag = reinterpret_cast<unsigned char *>(rb + 2 * P * plane);
+  const auto barrier = [&] {
+    if (blocks == 1) {
+      __syncthreads();
+    } else {
+      asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    }
+  };
+  for (int q = tid; q < 2 * size; q += kCoarseThreads) x[q] = 0.0;
+  for (int q = tid; q < mine; q += kCoarseThreads) {
+    const int t = q % np, jk = q / np, j = jk % ny, k = first + jk / ny, par = (j + k) & 1;
+    flag[q] = (unsigned char)((t > 0) | (2 * t + 2 < nx) << 1 | (j > 0) << 2 | (j < ny - 1) << 3 |
+                              (k > 0) << 4 | (k < nz - 1) << 5 | (2 * t + 1 == nx) << 6 | par << 7);
+    const double *const b = v.b + (k * ny + j) * nx + 2 * t;
+    rb[par * P * plane + q] = ::fma(-C.inv, b[0], 0.0);
+    if (2 * t + 1 < nx) rb[(1 - par) * P * plane + q] = ::fma(-C.inv, b[1], 0.0);
+  }
+  // the neighbours' copies of this slab's outer planes
+  const bool low = rank > 0, high = rank < blocks - 1;
+  unsigned below, above;
+  const unsigned here = (unsigned)__cvta_generic_to_shared(x + plane);
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(below) : "r"(here), "r"(rank - low));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(above) : "r"(here), "r"(rank + high));
+  barrier();
+  for (int it = 0; it < 2 * sweeps; it++) {
+    const int h = it & 1;  // first the cells with (i + j + k) even
+    double *const own = x + h * size + plane;
+    const double *const o = x + (1 - h) * size + plane, *const r = rb + h * P * plane;
+    for (int q = tid; q < mine; q += kCoarseThreads) {
+      const int f = flag[q];
+      const bool left = (f >> 7) == h;  // the colour's cell is the pair's left one
+      if ((f & 64) && !left) continue;
+      // a neighbour beyond a wall is the cell itself
+      const double *const cq = own + q, *const oq = o + q;
+      const double c = *cq, in = *(f & 64 ? cq : oq);
+      const double side = *(f & (left ? 1 : 2) ? oq + (left ? -1 : 1) : cq);
+      const double s = *(f & 4 ? oq - np : cq), n = *(f & 8 ? oq + np : cq);
+      const double d = *(f & 16 ? oq - plane : cq), u = *(f & 32 ? oq + plane : cq);
+      const double m = smooth64_cell(C, r[q], in + side, s + n, d + u, c);
+      own[q] = m;
+      if (low && q < plane)
+        asm volatile("st.shared::cluster.f64 [%0], %1;\n"
+                     ::"r"(below + 8 * (h * size + P * plane + q)), "d"(m)
+                     : "memory");
+      if (high && q >= mine - plane)
+        asm volatile("st.shared::cluster.f64 [%0], %1;\n"
+                     ::"r"(above + 8 * (h * size + q - mine)), "d"(m)
+                     : "memory");
+    }
+    barrier();
+  }
+  for (int q = tid; q < mine; q += kCoarseThreads) {
+    const int t = q % np, jk = q / np, j = jk % ny, k = first + jk / ny, par = (j + k) & 1;
+    double *const to = v.x + (k * ny + j) * nx + 2 * t;
+    to[0] = x[par * size + plane + q];
+    if (2 * t + 1 < nx) to[1] = x[(1 - par) * size + plane + q];
+  }
 }
 
 // Coarsest level, exact: x = Minv * b with Minv the inverse of the coarsest
@@ -2735,6 +2824,30 @@ bool prolong_to(const View<T> &f, const T *xc, const MgLevelDesc &C, const MgSta
   return launched("k_mg_prolong");
 }
 
+bool launch_coarse_f64(const View<double> &v, int blocks, int planes, int nsweeps, size_t bytes,
+    const MgState *st)
+{
+  if (!cuda_ok(cudaFuncSetAttribute(k_mg_coarse_f64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                   (int)bytes),
+          "k_mg_coarse_f64 shared memory"))
+    return false;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kCoarseThreads);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.stream = stream();
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = blocks;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (!cuda_ok(cudaLaunchKernelEx(&cfg, k_mg_coarse_f64, v, smooth64(v), nsweeps, planes, st),
+          "k_mg_coarse_f64"))
+    return false;
+  return launched("k_mg_coarse_f64");
+}
+
 template <typename T>
 bool coarse_solve(const View<T> &v, int nsweeps, const MgState *st, const T *minv)
 {
@@ -2744,9 +2857,18 @@ bool coarse_solve(const View<T> &v, int nsweeps, const MgState *st, const T *min
         st);
     return launched("k_mg_direct");
   }
-  const size_t bytes = n * sizeof(T);
-  if (bytes <= 24 * 1024) {  // at most 6144 cells: three of each colour per thread
-    const int items = (v.nx + 1) / 2 * v.ny * v.nz;
+  const int items = (v.nx + 1) / 2 * v.ny * v.nz;  // pairs of cells
+  if constexpr (sizeof(T) == sizeof(double)) {
+    // a cluster while a colour's pass takes a block less than a launch would
+    // (16384 cells: 2.3 us against 2.7), a block for each 64 pairs
+    int blocks = 1;
+    while (blocks < kCoarseBlocks && blocks * 64 < items) blocks *= 2;
+    const int planes = (v.nz + blocks - 1) / blocks, plane = (v.nx + 1) / 2 * v.ny;
+    const size_t bytes = (size_t)plane * (16 * (planes + 2) + 17 * planes);
+    if (n <= kCoarseCells64 && bytes <= 226 * 1024)
+      return launch_coarse_f64(v, blocks, planes, nsweeps, bytes, st);
+  } else if (n <= 6144) {  // three of each colour per thread
+    const size_t bytes = 2 * (size_t)items * sizeof(T);
     const int r = (items + 1023) / 1024;
     const int threads = ((items + r - 1) / r + 31) / 32 * 32;
     switch (r) {

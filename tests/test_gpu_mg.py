@@ -514,3 +514,27 @@ def test_long_runs_keep_converging(nusif_lib, guess):
         p = sim.field("p")[1:-1, 1:-1, 1:-1]
     assert max(its[100:]) <= max(its[:100])
     assert abs(p.mean()) < 10.0 * np.abs(p - p.mean()).max()
+
+
+# coarsest levels by sweeps (more than 1024 cells, or mg_coarse): 9x10x12 and
+# 11x13x10 cells, odd rows, a slab of one plane, fewer planes than blocks, the
+# largest a cluster takes and one beyond
+@pytest.mark.parametrize("dims", [(36, 20, 48), (44, 52, 20), (22, 13, 17), (31, 41, 2), (33, 31, 15),
+                                  (33, 31, 17)])
+def test_coarsest_sweeps_match_oracle(nusif_lib, oracle_mod, dims):
+    test_mg_fp64_matches_oracle(nusif_lib, oracle_mod, dims)
+
+
+@pytest.mark.parametrize("dims", [(36, 20, 48), (44, 52, 20), (28, 28, 28), (17, 34, 18)])
+def test_fp32_coarsest_sweeps_match_single_block(nusif_lib, dims):
+    """The FP32 coarsest sweeps by their own kernel, colours apart, and inside
+    the one-block tail kernel, rows of both: the same bits."""
+    out = []
+    for tail in (0, 8192):
+        with _sim(dims, "mg-mixed", 1e-9, mg_cycles=4, mg_tail=tail) as sim:
+            rng = np.random.default_rng(7)
+            sim.set_field("p", rng.standard_normal(sim.padded_shape))
+            sim.set_field("rhs", rng.standard_normal(sim.padded_shape))
+            out.append((sim.solve(), sim.iterations, sim.field("p")))
+    assert out[0][:2] == out[1][:2]
+    np.testing.assert_array_equal(out[0][2], out[1][2])
