@@ -3105,14 +3105,18 @@ bool tail_vcycle(MgHierarchy *H, int l, T **xs, T **bs, bool zero)
 
 // The levels that k_mg_bottom takes: from the first of at most kBottomCells
 // cells (rows rounded up to even) below the top, where at least one lies above an
-// exactly solved coarsest level. 0: none.
+// exactly solved coarsest level. Rows of a multiple of four cells, which a launch
+// per sweep serves, pay up to half of that: per V(2,2) cycle from 16^3 -6 us, 16 x
+// 18 x 18 0, 16 x 16 x 24 +3, 20^3 +7; other rows take two launches per sweep,
+// 18^3 -8, 18 x 20 x 20 -3. 0: none.
 int bottom_level(const MgHierarchy *H)
 {
   if (!H->minv32) return 0;
   int l0 = 0;
   for (int l = H->nl - 2; l >= 1; l--) {
     const MgLevelDesc &L = H->lv[l];
-    if ((int64_t)((L.n[0] + 1) / 2 * 2) * L.n[1] * L.n[2] > kBottomCells) break;
+    const int64_t cells = (int64_t)((L.n[0] + 1) / 2 * 2) * L.n[1] * L.n[2];
+    if (cells > (L.n[0] % 4 == 0 ? kBottomCells / 2 : kBottomCells)) break;
     l0 = l;
   }
   return l0;
