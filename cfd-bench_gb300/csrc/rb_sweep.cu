@@ -75,12 +75,18 @@ struct Consts {
   V fx, fy, fz, momega, mfactor;
 };
 
+// The neighbours' factors are rounded to multiples of 2^-49 omega (rounded to a
+// power of two), so that the pair of the cell's own is twice their sum exactly:
+// a constant d has no change. With each rounded by itself a constant drifted by
+// 2^-48 an iteration, the larger part of the error of a long solve (14 x 55 x
+// 77, 1000 iterations: 2.7e-13 -> 2.9e-14).
 Consts<df::f2> consts(const SorArgs &A, df::f2)
 {
-  const double f = A.factor;
-  return { df::from_double_rn(f * A.idx2), df::from_double_rn(f * A.idy2),
-           df::from_double_rn(f * A.idz2), df::from_double_rn(-f * A.diag),
-           df::from_double_rn(-f) };
+  const double f = A.factor, q = std::ldexp(1.0, std::ilogb(f * A.diag) - 49);
+  const double fx = std::rint(f * A.idx2 / q) * q, fy = std::rint(f * A.idy2 / q) * q,
+               fz = std::rint(f * A.idz2 / q) * q;
+  return { df::from_double_rn(fx), df::from_double_rn(fy), df::from_double_rn(fz),
+           df::from_double_rn(-2.0 * (fx + fy + fz)), df::from_double_rn(-f) };
 }
 Consts<double> consts(const SorArgs &A, double)
 {
