@@ -20,9 +20,10 @@
 //            mg_theta, at most mg_inner cycles) -> p += e in FP64
 //            (iterative refinement; the FP64 residual decides the stop).
 // Every kernel returns at once when the device-side done flag is up. By
-// default each solve is one CUDA graph whose device while-loops run the
-// V-cycles; the host-driven path queues whole cycles in chunks and reads the
-// state once per chunk.
+// default each solve is one CUDA graph with a device while-loop over the
+// V-cycles (a host that reads the state and launches the next unit's graph took
+// 1% more at 128^3, 4% more at 72 x 36 x 60); the host-driven path queues whole
+// cycles in chunks and reads the state once per chunk.
 #include <algorithm>
 #include <array>
 #include <climits>
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(kNT) k_mg_restrict_x2(View<T> f, T *bc, int cn
 // four cells themselves; no corners). Same arithmetic and summation order as
 // k_mg_restrict_x2<float>, with 12 vector loads per coarse cell instead of 64
 // scalar ones. Bound by memory latency: with each plane loaded where it was
-// used 55 us at 256^3, so 33.
+// used 55 us at 256^3, so 31.
 template <int FOLD>
 __global__ void __launch_bounds__(kNT, 3) k_mg_restrict_f32(View<float> f, float *bc, int cnx,
     int cny, int cnz, int kcz, float inv_count, MgState *st, double *partials, unsigned *ticket)

@@ -6,7 +6,9 @@
 //  mg-ref  the reference multigrid as it behaves (src/solver-mg.c:299-402)
 //  mg, mg-mixed  geometric V-cycles (multigrid.cu)
 //
-// One red-black iteration is two launches of one kernel, one per colour. A
+// rb runs its first iteration here, on p, and the others as sweeps on the
+// change of p (rb_sweep.cu; here too where their memory is not to be had). On p
+// an iteration is two launches of one kernel, one per colour. A
 // thread owns the cell pair (2t+1, 2t+2) of a row and relaxes the one of the
 // pass's colour, so both passes use the same coalesced mapping. The second
 // pass also writes the Neumann ghost layer: a ghost is read only by its own

@@ -14,10 +14,11 @@
 // times its ReLU mask is rounded to BF16 before the tensor-core kernels use it.
 //
 // Kernels:
-//  - k_conv_tc (unet_tc.cu): the forward and input-gradient convolutions on
-//    the 5th-generation tensor cores (tcgen05.mma, TMEM accumulators, TMA
-//    staging) whenever the volume's rows tile into 128-cell blocks; the
-//    decoder's upsampled concat source is then materialised by k_upsample.
+//  - k_conv_col, k_conv_tc (unet_tc.cu): the forward and input-gradient
+//    convolutions on the 5th-generation tensor cores (tcgen05.mma, TMEM
+//    accumulators, TMA staging) whenever the volume's rows tile into 128-cell
+//    blocks, marching over planes for layers of up to 48 channels; the
+//    96-channel layer's upsampled source is then materialised by k_upsample.
 //  - k_conv_mma: implicit-GEMM conv on the tensor cores (mma.sync m16n8k16
 //    BF16 -> FP32): M = cells (16 per warp), N = output channels, K = 27 taps x
 //    input channels in chunks of 16. Its loader reads up to two sources, the
