@@ -112,10 +112,16 @@ struct ConvArgs {
 };
 
 // One warp = 16 consecutive output cells x all COUT channels. Rows g and g+8
-// of the mma fragments are this thread's two cells.
+// of the mma fragments are this thread's two cells. A step is a tap and 16
+// input channels; the fragments of the next D - 1 steps are in flight while one
+// is multiplied (they come straight from L1 and L2, whose latency is what a
+// warp waits for). Same products in the same order whatever D. Per call, 4 x 60 x
+// 12 x 12 cells: 32 channels out 29 -> 21 us (D = 6: 36), 16 channels 24 -> 21; 4 x 64
+// x 60 x 60: 16 channels 408 -> 375 us (D = 4: 425).
 template <int COUT, bool OUT_BF16>
 __global__ void __launch_bounds__(128) k_conv_mma(ConvArgs a)
 {
+  constexpr int D = COUT <= 16 ? 2 : COUT <= 32 ? 4 : COUT <= 48 ? 3 : 2;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int64_t ncell = a.v.cells();
   const int64_t base = ((int64_t)blockIdx.x * 4 + warp) * 16;
@@ -132,38 +138,57 @@ __global__ void __launch_bounds__(128) k_conv_mma(ConvArgs a)
   float acc[COUT / 8][4];
 #pragma unroll
   for (int j = 0; j < COUT / 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
-  for (int tap = 0; tap < 27; tap++) {
-    const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-    bool ok[2];
-    int64_t n1[2], n0[2];
+  struct Step {
+    uint32_t A[4], W[COUT / 8][2];
+  };
+  // the next step to load: tap (dz, dy, dx) and channel, and the tap's cells
+  int tap = -1, kc = cin;
+  bool ok[2];
+  int64_t n1[2], n0[2];
+  const auto load = [&](Step &q) {
+    if (kc == cin) {
+      kc = 0;
+      if (++tap == 27) return;
+      const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
 #pragma unroll
-    for (int r = 0; r < 2; r++) {
-      const int z = cz[r] + dz, y = cy[r] + dy, x = cx[r] + dx;
-      ok[r] = live[r] && z >= 0 && z < a.v.Z && y >= 0 && y < a.v.Y && x >= 0 && x < a.v.X;
-      n1[r] = ok[r] ? (((int64_t)cb[r] * a.v.Z + z) * a.v.Y + y) * a.v.X + x : 0;
-      n0[r] = !a.s0.up ? n1[r]
-                       : (ok[r] ? (((int64_t)cb[r] * hZ + (z >> 1)) * hY + (y >> 1)) * hX + (x >> 1)
-                                : 0);
-    }
-    const bf16 *wt = a.w + (int64_t)tap * COUT * cin;
-    for (int kc = 0; kc < cin; kc += 16) {
-      const bool first = kc < a.s0.c;
-      const bf16 *src = first ? a.s0.p : a.s1.p;
-      const int cs = first ? a.s0.c : a.s1.c;
-      const int c0 = (first ? kc : kc - a.s0.c) + 2 * t;
-      const int64_t o0 = (first ? n0[0] : n1[0]) * cs + c0;
-      const int64_t o1 = (first ? n0[1] : n1[1]) * cs + c0;
-      uint32_t A[4];
-      A[0] = ok[0] ? ld_pair(src + o0) : 0u;
-      A[1] = ok[1] ? ld_pair(src + o1) : 0u;
-      A[2] = ok[0] ? ld_pair(src + o0 + 8) : 0u;
-      A[3] = ok[1] ? ld_pair(src + o1 + 8) : 0u;
-#pragma unroll
-      for (int j = 0; j < COUT / 8; j++) {
-        const bf16 *wr = wt + (int64_t)(8 * j + g) * cin + kc + 2 * t;
-        mma_bf16(acc[j], A, __ldg(reinterpret_cast<const unsigned *>(wr)),
-            __ldg(reinterpret_cast<const unsigned *>(wr + 8)));
+      for (int r = 0; r < 2; r++) {
+        const int z = cz[r] + dz, y = cy[r] + dy, x = cx[r] + dx;
+        ok[r] = live[r] && z >= 0 && z < a.v.Z && y >= 0 && y < a.v.Y && x >= 0 && x < a.v.X;
+        n1[r] = ok[r] ? (((int64_t)cb[r] * a.v.Z + z) * a.v.Y + y) * a.v.X + x : 0;
+        n0[r] = !a.s0.up ? n1[r]
+                         : (ok[r] ? (((int64_t)cb[r] * hZ + (z >> 1)) * hY + (y >> 1)) * hX + (x >> 1)
+                                  : 0);
       }
+    }
+    const bool first = kc < a.s0.c;
+    const bf16 *src = first ? a.s0.p : a.s1.p;
+    const int cs = first ? a.s0.c : a.s1.c;
+    const int c0 = (first ? kc : kc - a.s0.c) + 2 * t;
+    const int64_t o0 = (first ? n0[0] : n1[0]) * cs + c0;
+    const int64_t o1 = (first ? n0[1] : n1[1]) * cs + c0;
+    q.A[0] = ok[0] ? ld_pair(src + o0) : 0u;
+    q.A[1] = ok[1] ? ld_pair(src + o1) : 0u;
+    q.A[2] = ok[0] ? ld_pair(src + o0 + 8) : 0u;
+    q.A[3] = ok[1] ? ld_pair(src + o1 + 8) : 0u;
+    const bf16 *wr = a.w + ((int64_t)tap * COUT + g) * cin + kc + 2 * t;
+#pragma unroll
+    for (int j = 0; j < COUT / 8; j++, wr += 8 * cin) {
+      q.W[j][0] = __ldg(reinterpret_cast<const unsigned *>(wr));
+      q.W[j][1] = __ldg(reinterpret_cast<const unsigned *>(wr + 8));
+    }
+    kc += 16;
+  };
+  Step f[D];
+#pragma unroll
+  for (int u = 0; u < D - 1; u++) load(f[u]);  // at least 27 steps
+  const int steps = 27 * (cin / 16);
+  for (int s = 0; s < steps; s += D) {
+#pragma unroll
+    for (int u = 0; u < D; u++) {
+      if (s + u >= steps) break;
+      if (s + u + D - 1 < steps) load(f[(u + D - 1) % D]);
+#pragma unroll
+      for (int j = 0; j < COUT / 8; j++) mma_bf16(acc[j], f[u].A, f[u].W[j][0], f[u].W[j][1]);
     }
   }
 #pragma unroll
