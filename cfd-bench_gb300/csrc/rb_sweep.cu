@@ -75,23 +75,31 @@ struct Consts {
   V fx, fy, fz, momega, mfactor;
 };
 
-// The neighbours' factors are rounded to multiples of 2^-49 omega (rounded to a
-// power of two), so that the pair of the cell's own is twice their sum exactly:
+// The neighbours' factors are rounded to multiples of 2^-49 omega (2^-51 for
+// doubles; omega to a power of two), so that the cell's own is twice their sum exactly:
 // a constant d has no change. With each rounded by itself a constant drifted by
 // 2^-48 an iteration, the larger part of the error of a long solve (14 x 55 x
 // 77, 1000 iterations: 2.7e-13 -> 2.9e-14).
+struct Factors {
+  double x, y, z, own;
+};
+Factors factors(const SorArgs &A, int bits)
+{
+  const double f = A.factor, q = std::ldexp(1.0, std::ilogb(f * A.diag) - bits);
+  const double x = std::rint(f * A.idx2 / q) * q, y = std::rint(f * A.idy2 / q) * q,
+               z = std::rint(f * A.idz2 / q) * q;
+  return { x, y, z, -2.0 * (x + y + z) };
+}
 Consts<df::f2> consts(const SorArgs &A, df::f2)
 {
-  const double f = A.factor, q = std::ldexp(1.0, std::ilogb(f * A.diag) - 49);
-  const double fx = std::rint(f * A.idx2 / q) * q, fy = std::rint(f * A.idy2 / q) * q,
-               fz = std::rint(f * A.idz2 / q) * q;
-  return { df::from_double_rn(fx), df::from_double_rn(fy), df::from_double_rn(fz),
-           df::from_double_rn(-2.0 * (fx + fy + fz)), df::from_double_rn(-f) };
+  const Factors f = factors(A, 49);
+  return { df::from_double_rn(f.x), df::from_double_rn(f.y), df::from_double_rn(f.z),
+           df::from_double_rn(f.own), df::from_double_rn(-A.factor) };
 }
 Consts<double> consts(const SorArgs &A, double)
 {
-  const double f = A.factor;
-  return { f * A.idx2, f * A.idy2, f * A.idz2, -f * A.diag, -f };
+  const Factors f = factors(A, 51);
+  return { f.x, f.y, f.z, f.own, -A.factor };
 }
 
 // the change D of a cell c with the neighbours w, e, s, n, b, t; r = -factor
@@ -518,6 +526,7 @@ __device__ __forceinline__ void store_in(unsigned at, double v)
 }
 
 constexpr int kFoldWarps = 4;
+constexpr size_t kClusterSmem = 226 * 1024 - 1024;  // of 227 KB; the kernel has a little of its own
 
 // sums of non-negative pairs that need no order: without renormalising between
 __device__ __forceinline__ df::f2 warp_sum(df::f2 v)
@@ -796,8 +805,9 @@ bool cluster_config(const RbPlan &P, cudaLaunchConfig_t &cfg, cudaLaunchAttribut
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
+  // (the same limit from every solver and thread: the attribute is the process's)
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-             (int)P.cluster_smem) == cudaSuccess &&
+             (int)kClusterSmem) == cudaSuccess &&
          cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
              cudaSuccess;
 }
@@ -843,7 +853,7 @@ void choose_cluster(RbPlan &P)
     P.cluster_smem = cluster_shape(P.c, n, blocks, threads);
     break;
   }
-  if (P.cluster_smem > 226 * 1024) return;
+  if (P.cluster_smem > kClusterSmem) return;
   P.cluster_threads = threads;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at;
