@@ -2829,7 +2829,7 @@ bool launch_coarse_f64(const View<double> &v, int blocks, int planes, int nsweep
     const MgState *st)
 {
   if (!cuda_ok(cudaFuncSetAttribute(k_mg_coarse_f64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                   (int)bytes),
+                   (int)kBottomSmem),
           "k_mg_coarse_f64 shared memory"))
     return false;
   cudaLaunchConfig_t cfg = {};
@@ -2866,7 +2866,7 @@ bool coarse_solve(const View<T> &v, int nsweeps, const MgState *st, const T *min
     while (blocks < kCoarseBlocks && blocks * 64 < items) blocks *= 2;
     const int planes = (v.nz + blocks - 1) / blocks, plane = (v.nx + 1) / 2 * v.ny;
     const size_t bytes = (size_t)plane * (16 * (planes + 2) + 17 * planes);
-    if (n <= kCoarseCells64 && bytes <= 226 * 1024)
+    if (n <= kCoarseCells64 && bytes <= kBottomSmem)
       return launch_coarse_f64(v, blocks, planes, nsweeps, bytes, st);
   } else if (n <= 6144) {  // three of each colour per thread
     const size_t bytes = 2 * (size_t)items * sizeof(T);
@@ -3178,8 +3178,9 @@ bool bottom_vcycle(MgHierarchy *H, int l)
   for (int q = 0; q + 1 < a.count; q++) any |= a.lv[q].nx % 2 != 0 || a.lv[q + 1].rx != 2;
   any |= a.lv[a.count - 1].nx % 2 != 0;
   if (any && pairs <= 2 * kBottomThreads) kernel = k_mg_bottom<2, true>;
+  // (the same limit from every solver and thread: the attribute is the process's)
   if (!cuda_ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                   (int)bytes),
+                   (int)kBottomSmem),
           "k_mg_bottom shared memory"))
     return false;
   cudaLaunchConfig_t cfg = {};
