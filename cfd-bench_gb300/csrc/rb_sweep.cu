@@ -873,7 +873,8 @@ double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, cons
   const Dims &g = A.g;
   const RbPlan &P = *ss->rb_plan;
   const SweepArgs &a = P.a;
-  const bool sweeps = P.cells != nullptr;
+  // (with a factor of zero, or one that has lost bits, the sum of D^2 does not give that of r^2)
+  const bool sweeps = P.cells != nullptr && std::isnormal(A.factor);
   const int nb = sweeps ? P.blocks : 0, nb1 = 2 * sor_blocks(A);
   const bool folded = nb > kFoldMax;
   // the first iteration's sums, then the sweeps' two lists and one value for each
