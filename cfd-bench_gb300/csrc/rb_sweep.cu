@@ -12,7 +12,10 @@
 // split from p in every use. At the end p = P + d in binary64. The factors
 // are folded into the constants: an update is c + D with
 //   D = -factor r = f_x (w + e) + f_y (s + n) + f_z (b + t) - omega c - factor r0,
-// and the sum of r^2 is that of D^2 over factor^2.
+// and the sum of r^2 is that of D^2 over factor^2. factor is omega h^2 / 6, of
+// any size, so d and r0 are kept times the power of two that brings it to 1 or
+// more: D^2 is then of the size of r^2, and the range in which pairs hold it
+// does not depend on the cells' size.
 //
 // Layout: d and r0 with the colours apart, [colour][k][j][t], t the pair
 // (2t, 2t+1) of a row, so a thread's loads and stores are contiguous over the
@@ -41,9 +44,11 @@
 // first planes load, then decides alike (k_rb_fold first where there are
 // many). R_m, the carried residual after m iterations, is kept in res[m & 1]:
 // kernel n reads R_(n-2) and iteration n - 1's sums, block 0 stores R_(n-1).
-// Sums stay pairs of FP32 numbers to the end: an FP64 instruction costs a
-// warp 16 cycles of GB300's FP64 pipe, and a block-wide FP64 reduction more
-// than a plane.
+// Sums stay pairs of FP32 numbers to the end (doubles with arith fp64): an FP64
+// addition costs a warp 16 cycles of GB300's FP64 pipe and about 100 of latency
+// (block sums and fold in FP64: 64^3 5.6 -> 6.2 us an iteration). So that the
+// sum over a grid keeps the range of a cell's square, a thread's sum is taken
+// times 2^-30, or less where eps^2 would come near the smallest float.
 //
 // What bounds it: at 128^3 instruction issue (about 215 thread instructions per
 // cell, ring included; k_sor_pass in two launches about 520), at 64^3 half
@@ -54,10 +59,11 @@
 // iterations, its blocks exchanging sums through L2, took 2 us more per
 // iteration than launches (two device-wide fences); letting the next kernel's
 // blocks in early took 1 us more (they double up on the idle SMs).
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
-#include <utility>
 #include <cstring>
+#include <utility>
 #include <type_traits>
 
 #include "df32.cuh"
@@ -135,15 +141,14 @@ __device__ __forceinline__ void add_square(df::f2 &acc, df::f2 D)
   acc = df::add_u(acc, df::mul_u(D, D));
 }
 __device__ __forceinline__ void add_square(double &acc, double D) { acc = ::fma(D, D, acc); }
-__device__ __forceinline__ df::f2 as_pair(df::f2 a) { return df::renorm(a.hi, a.lo); }
-__device__ __forceinline__ df::f2 as_pair(double a) { return df::split(a); }
 __device__ __forceinline__ df::f2 to_cell(double x, df::f2) { return df::split(x); }
 __device__ __forceinline__ double to_cell(double x, double) { return x; }
-__device__ __forceinline__ double plus(double p, df::f2 d)
+// p + d, d kept times 1 / unit (the products are exact)
+__device__ __forceinline__ double plus(double p, df::f2 d, double unit)
 {
-  return (p + df::widen(d.hi)) + df::widen(d.lo);
+  return ::fma(df::widen(d.lo), unit, ::fma(df::widen(d.hi), unit, p));
 }
-__device__ __forceinline__ double plus(double p, double d) { return p + d; }
+__device__ __forceinline__ double plus(double p, double d, double unit) { return ::fma(d, unit, p); }
 
 struct SweepArgs {
   int nx, ny, nz, np;  // np: pairs per row
@@ -159,31 +164,53 @@ struct SweepArgs {
   }
 };
 
-__device__ __forceinline__ df::f2 warp_total(df::f2 v)
+__device__ __forceinline__ df::f2 join(df::f2 a, df::f2 b) { return df::add(a, b); }
+__device__ __forceinline__ double join(double a, double b) { return a + b; }
+__device__ __forceinline__ df::f2 from_lane(df::f2 v, int o)
+{
+  return df::f2{ __shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o) };
+}
+__device__ __forceinline__ double from_lane(double v, int o)
+{
+  return __shfl_xor_sync(0xffffffffu, v, o);
+}
+template <typename V>
+__device__ __forceinline__ V warp_total(V v)
 {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    v = df::add(v, df::f2{ __shfl_xor_sync(0xffffffffu, v.hi, o),
-                           __shfl_xor_sync(0xffffffffu, v.lo, o) });
+  for (int o = 16; o > 0; o >>= 1) v = join(v, from_lane(v, o));
   return v;
 }
 
-// one warp's sum of a list of pairs, in a fixed order
-__device__ __forceinline__ df::f2 fold_pairs(const df::f2 *part, int np, int lane)
+__device__ __forceinline__ df::f2 load_sum(const df::f2 *p)
+{
+  const float2 x = __ldcg(reinterpret_cast<const float2 *>(p));
+  return df::f2{ x.x, x.y };
+}
+__device__ __forceinline__ double load_sum(const double *p) { return __ldcg(p); }
+
+// one warp's sum of a list, in a fixed order
+template <typename V>
+__device__ __forceinline__ V fold_list(const V *part, int np, int lane)
 {
   constexpr int kAtOnce = 5;  // loads in flight
-  const float2 *list = reinterpret_cast<const float2 *>(part);
-  df::f2 v{ 0.0f, 0.0f };
+  V v{};
   for (int q0 = lane; q0 < np; q0 += 32 * kAtOnce) {
-    float2 x[kAtOnce];
+    V x[kAtOnce];
 #pragma unroll
-    for (int u = 0; u < kAtOnce; u++) x[u] = __ldcg(list + min(q0 + 32 * u, np - 1));
+    for (int u = 0; u < kAtOnce; u++) x[u] = load_sum(part + min(q0 + 32 * u, np - 1));
 #pragma unroll
     for (int u = 0; u < kAtOnce; u++)
-      if (q0 + 32 * u < np) v = df::add(v, df::f2{ x[u].x, x[u].y });
+      if (q0 + 32 * u < np) v = join(v, x[u]);
   }
   return warp_total(v);
 }
+
+__device__ __forceinline__ double as_double(df::f2 v) { return df::to_double(v); }
+__device__ __forceinline__ double as_double(double v) { return v; }
+// a thread's sum of squares, to be added to others'
+__device__ __forceinline__ df::f2 scaled(df::f2 a, float k) { return df::renorm(a.hi * k, a.lo * k); }
+__device__ __forceinline__ double scaled(double a, float) { return a; }
 
 __device__ __forceinline__ bool is_done(const RbState *st)
 {
@@ -191,9 +218,10 @@ __device__ __forceinline__ bool is_done(const RbState *st)
 }
 
 // the carried residual after an iteration whose D^2 sum to `sum`
-__device__ __forceinline__ double carried(const RbState *st, double before, df::f2 sum)
+template <typename V>
+__device__ __forceinline__ double carried(const RbState *st, double before, V sum)
 {
-  return (before + df::to_double(sum) * st->inv_factor2) * st->inv_ncell;
+  return (before + as_double(sum) * st->inv_factor2) * st->inv_ncell;
 }
 
 // a pair's cell in one column: the new first-colour value two planes below
@@ -211,14 +239,14 @@ struct Ahead {
 };
 
 // iteration n, with the np sums of the previous one in part_in (np 0: that one
-// ran on p itself)
+// ran on p itself); down: the scale of the sums
 template <typename V, bool CUBE>
 __global__ void __launch_bounds__(kMaxThreads) k_rb_sweep(SweepArgs A, Consts<V> C,
-    const V *d, V *dout, const V *r0, RbState *st, const df::f2 *part_in, df::f2 *part_out, int n,
-    int np)
+    const V *d, V *dout, const V *r0, RbState *st, const V *part_in, V *part_out, int n, int np,
+    float down)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ df::f2 sm[kMaxThreads / 32];
+  __shared__ V sm[kMaxThreads / 32];
   __shared__ int go_on;
   const int pw = A.own + 2 * A.halo, nrow = A.rows + 2;
   const int plane_n = pw * nrow, plane_o = pw * (nrow + 2);
@@ -284,7 +312,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_rb_sweep(SweepArgs A, Consts<V>
     const int itermax = __ldcg(&st->s.itermax);
     bool go = true;
     if (np > 0) {
-      const df::f2 sum = fold_pairs(part_in, np, lane);
+      const V sum = fold_list(part_in, np, lane);
       if (lane == 0) {
         const double res = carried(st, before, sum);
         go = res >= epssq && n - 1 < itermax;
@@ -376,18 +404,18 @@ __global__ void __launch_bounds__(kMaxThreads) k_rb_sweep(SweepArgs A, Consts<V>
     step(k, X, Y, a0, 0, wall_x, valid_x, ax);
     if (k + 1 <= k1 + 1) step(k + 1, Y, X, a1, 1, wall_y, valid_y, ay);
   }
-  const df::f2 ws = warp_total(as_pair(acc));
+  const V ws = warp_total(scaled(acc, down));
   if (lane == 0) sm[tid >> 5] = ws;
   __syncthreads();
   if (tid < 32) {
     const int nw = blockDim.x >> 5;
-    const df::f2 sum = warp_total(lane < nw ? sm[lane] : df::f2{ 0.0f, 0.0f });
+    const V sum = warp_total(lane < nw ? sm[lane] : V());
     if (lane == 0) part_out[bid] = sum;
   }
 }
 
-// after the first iteration: r = -factor (rhs - A P) in FP64, d = 0 with its
-// ghosts (one thread per entry of a colour's array)
+// after the first iteration: r = -factor (rhs - A P) in FP64 (S.factor is the
+// scaled one), d = 0 with its ghosts (one thread per entry of a colour's array)
 template <typename V>
 __global__ void __launch_bounds__(256) k_rb_open(SweepArgs A, SorArgs S, const double *__restrict__ p,
     const double *__restrict__ rhs, V *__restrict__ d, V *__restrict__ r0, const RbState *st)
@@ -417,7 +445,7 @@ __global__ void __launch_bounds__(256) k_rb_open(SweepArgs A, SorArgs S, const d
 // (direct: the iterations that ran on p itself)
 template <typename V>
 __global__ void __launch_bounds__(256) k_rb_close(SweepArgs A, Dims g, double *__restrict__ p,
-    const V *__restrict__ d0, const V *__restrict__ d1, const RbState *st, int direct)
+    const V *__restrict__ d0, const V *__restrict__ d1, double unit, const RbState *st, int direct)
 {
   if (!is_done(st) || st->s.it <= direct) return;
   const V *d = (st->s.it & 1) ? d1 : d0;
@@ -429,7 +457,7 @@ __global__ void __launch_bounds__(256) k_rb_close(SweepArgs A, Dims g, double *_
     const int i = 2 * T + e;
     if (i >= A.nx) continue;
     double *c = p + ((k + 1) * g.sk + (j + 1) * g.sj + i + 1);
-    const double v = plus(*c, d[((i + j + k) & 1) * A.half + A.at(T, j, k)]);
+    const double v = plus(*c, d[((i + j + k) & 1) * A.half + A.at(T, j, k)], unit);
     *c = v;
     if (i == 0) c[-1] = v;
     if (i == A.nx - 1) c[1] = v;
@@ -441,17 +469,14 @@ __global__ void __launch_bounds__(256) k_rb_close(SweepArgs A, Dims g, double *_
 }
 
 // a long list of block sums folded once instead of by every block of the next sweep
-__global__ void __launch_bounds__(1024) k_rb_fold(const RbState *st, const df::f2 *part, int np,
-    df::f2 *out)
+template <typename V>
+__global__ void __launch_bounds__(1024) k_rb_fold(const RbState *st, const V *part, int np, V *out)
 {
   if (is_done(st)) return;
-  __shared__ df::f2 sm[32];
+  __shared__ V sm[32];
   const int t = threadIdx.x;
-  df::f2 v{ 0.0f, 0.0f };
-  for (int q = t; q < np; q += 1024) {
-    const float2 x = __ldcg(reinterpret_cast<const float2 *>(part) + q);
-    v = df::add(v, df::f2{ x.x, x.y });
-  }
+  V v{};
+  for (int q = t; q < np; q += 1024) v = join(v, load_sum(part + q));
   v = warp_total(v);
   if ((t & 31) == 0) sm[t >> 5] = v;
   __syncthreads();
@@ -462,10 +487,11 @@ __global__ void __launch_bounds__(1024) k_rb_fold(const RbState *st, const df::f
 
 // after a chunk of sweeps that ended with iteration n: its residual, and
 // whether the solve is over (one warp)
-__global__ void k_rb_finish(RbState *st, const df::f2 *part, int n, int np)
+template <typename V>
+__global__ void k_rb_finish(RbState *st, const V *part, int n, int np)
 {
   if (is_done(st)) return;
-  const df::f2 s = fold_pairs(part, np, threadIdx.x);
+  const V s = fold_list(part, np, threadIdx.x);
   if (threadIdx.x == 0) {
     const double res = carried(st, st->res[(n - 1) & 1], s);
     st->s.res = res;
@@ -529,22 +555,23 @@ constexpr int kFoldWarps = 4;
 constexpr size_t kClusterSmem = 226 * 1024 - 1024;  // of 227 KB; the kernel has a little of its own
 
 // sums of non-negative pairs that need no order: without renormalising between
-__device__ __forceinline__ df::f2 warp_sum(df::f2 v)
+__device__ __forceinline__ df::f2 join_u(df::f2 a, df::f2 b) { return df::add_u(a, b); }
+__device__ __forceinline__ double join_u(double a, double b) { return a + b; }
+template <typename V>
+__device__ __forceinline__ V warp_total_u(V v)
 {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    v = df::add_u(v, df::f2{ __shfl_xor_sync(0xffffffffu, v.hi, o),
-                             __shfl_xor_sync(0xffffffffu, v.lo, o) });
-  return df::renorm(v.hi, v.lo);
+  for (int o = 16; o > 0; o >>= 1) v = join_u(v, from_lane(v, o));
+  return scaled(v, 1.0f);
 }
 
 template <typename V, bool CUBE>
 __global__ void __launch_bounds__(1024) k_rb_cluster(ClusterArgs A, SweepArgs G, Consts<V> C,
-    const V *__restrict__ r0, V *d0, V *d1, RbState *st, int direct)
+    const V *__restrict__ r0, V *d0, V *d1, RbState *st, int direct, float down)
 {
   if (is_done(st)) return;  // the same for all blocks
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ df::f2 total[16 * kFoldWarps];
+  __shared__ V total[16 * kFoldWarps];
   __shared__ int go;
   const int tid = threadIdx.x, lane = tid & 31, workers = blockDim.x - 32 * kFoldWarps;
   const bool work = tid < workers;
@@ -635,13 +662,13 @@ __global__ void __launch_bounds__(1024) k_rb_cluster(ClusterArgs A, SweepArgs G,
       half_pass(from, to, 0);
     } else if (n > direct) {  // iteration n's squares in this block
       const int w = (tid - workers) >> 5;
-      df::f2 v[2] = {};
+      V v[2] = {};
       for (int q = lane + 32 * w; q < workers; q += 64 * kFoldWarps)
 #pragma unroll
         for (int u = 0; u < 2; u++)
           if (q + 32 * kFoldWarps * u < workers)
-            v[u] = df::add_u(v[u], as_pair(squares[q + 32 * kFoldWarps * u]));
-      const df::f2 sum = warp_sum(df::add_u(v[0], v[1]));
+            v[u] = join_u(v[u], scaled(squares[q + 32 * kFoldWarps * u], down));
+      const V sum = warp_total_u(join_u(v[0], v[1]));
       if (lane < A.blocks) store_in(in_block(total + rank * kFoldWarps + w, lane), sum);
     }
     cluster_barrier(A.blocks);
@@ -649,11 +676,11 @@ __global__ void __launch_bounds__(1024) k_rb_cluster(ClusterArgs A, SweepArgs G,
       half_pass(from, to, 1);
       squares[tid] = acc;
     } else if (n > direct) {  // whether it was the last
-      df::f2 v{ 0.0f, 0.0f };
+      V v{};
 #pragma unroll
       for (int u = 0; u < 16 * kFoldWarps; u += 32)
-        if (lane + u < A.blocks * kFoldWarps) v = df::add_u(v, total[lane + u]);
-      res = (res + df::to_double(warp_sum(v)) * inv_factor2) * inv_ncell;
+        if (lane + u < A.blocks * kFoldWarps) v = join_u(v, total[lane + u]);
+      res = (res + as_double(warp_total_u(v)) * inv_factor2) * inv_ncell;
       if (tid == workers && !(res >= epssq && n < itermax)) go = 0;
     }
     cluster_barrier(A.blocks);
@@ -775,7 +802,7 @@ namespace {
 // one's leave (and without it each launch took a multiple of 2.05 us)
 template <typename V>
 bool launch_sweep(const RbPlan &P, const Consts<V> &C, const V *d, V *dout, const V *r0,
-    RbState *st, const df::f2 *part_in, df::f2 *part_out, int n, int np)
+    RbState *st, const V *part_in, V *part_out, int n, int np, float down)
 {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = P.grid;
@@ -788,7 +815,7 @@ bool launch_sweep(const RbPlan &P, const Consts<V> &C, const V *d, V *dout, cons
   cfg.attrs = at;
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, P.cube ? k_rb_sweep<V, true> : k_rb_sweep<V, false>, P.a, C, d, dout, r0,
-      st, part_in, part_out, n, np);
+      st, part_in, part_out, n, np, down);
   return launched("k_rb_sweep");
 }
 
@@ -814,7 +841,7 @@ bool cluster_config(const RbPlan &P, cudaLaunchConfig_t &cfg, cudaLaunchAttribut
 
 template <typename V>
 bool launch_cluster(const RbPlan &P, const Consts<V> &C, const V *r0, V *const (&d)[2], RbState *st,
-    int direct)
+    int direct, float down)
 {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at;
@@ -826,7 +853,7 @@ bool launch_cluster(const RbPlan &P, const Consts<V> &C, const V *r0, V *const (
   T.fy = f[P.c.axis[1]];
   T.fz = f[P.c.axis[2]];
   cudaLaunchKernelEx(&cfg, P.cube ? k_rb_cluster<V, true> : k_rb_cluster<V, false>, P.c, P.a, T, r0,
-      d[0], d[1], st, direct);
+      d[0], d[1], st, direct, down);
   return launched("k_rb_cluster");
 }
 
@@ -879,13 +906,22 @@ double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, cons
   const bool folded = nb > kFoldMax;
   // the first iteration's sums, then the sweeps' two lists and one value for each
   if (!reduce_scratch_alloc(ss->red, nb1 > 2 * nb + 2 ? nb1 : 2 * nb + 2)) return NAN;
-  df::f2 *const lists = reinterpret_cast<df::f2 *>(ss->red.partials);
-  df::f2 *const part[2] = { lists, lists + nb };
-  df::f2 *const sum[2] = { lists + 2 * nb, lists + 2 * nb + 1 };
+  V *const lists = reinterpret_cast<V *>(ss->red.partials);
+  V *const part[2] = { lists, lists + nb };
+  V *const sum[2] = { lists + 2 * nb, lists + 2 * nb + 1 };
   V *const cells = reinterpret_cast<V *>(P.cells);
   V *const d[2] = { cells, cells + 2 * (size_t)a.half };
   V *const r0 = d[1] + 2 * (size_t)a.half;
   const Consts<V> C = consts(A, V());
+  const int scale = sweeps ? -std::ilogb(A.factor) : 0;  // of d and r0
+  const double unit = std::ldexp(1.0, -scale);
+  SorArgs S = A;
+  S.factor = std::ldexp(A.factor, scale);
+  // of the sums: 2^-k, with eps^2 2^-k at least 2^-101 (eps below 1 here)
+  const int k = std::is_same_v<V, double> || !(s->eps > 0.0)
+                    ? 0
+                    : std::max(0, std::min(30, 101 + 2 * std::ilogb(s->eps)));
+  const float down = std::ldexp(1.0f, -k);
   cudaStream_t q = stream();
   RbState *st = ss->d_rb, *h = ss->h_rb;
   memset(h, 0, sizeof(*h));
@@ -894,7 +930,7 @@ double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, cons
   h->s.itermax = s->itermax;
   h->s.ncell = (double)(g.imax * g.jmax * g.kmax);
   h->inv_ncell = 1.0 / h->s.ncell;
-  h->inv_factor2 = 1.0 / (A.factor * A.factor);
+  h->inv_factor2 = std::ldexp(1.0 / (S.factor * S.factor), k);
   h->s.done = !((h->s.res >= h->s.epssq) && (0 < h->s.itermax));
   if (h->s.done) return h->s.res;
   if (!cuda_ok(cudaMemcpyAsync(st, h, sizeof(RbState), cudaMemcpyHostToDevice, q),
@@ -919,11 +955,11 @@ double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, cons
       n += count;
     } else if (chunk > 0 && n < s->itermax) {
       if (n == direct) {
-        k_rb_open<V><<<(unsigned)up(a.half, 256), 256, 0, q>>>(a, A, p, rhs, d[n & 1], r0, st);
+        k_rb_open<V><<<(unsigned)up(a.half, 256), 256, 0, q>>>(a, S, p, rhs, d[n & 1], r0, st);
         if (!launched("k_rb_open")) return NAN;
       }
       if (P.cluster_threads) {  // to the end
-        if (!launch_cluster<V>(P, C, r0, d, st, direct)) return NAN;
+        if (!launch_cluster<V>(P, C, r0, d, st, direct, down)) return NAN;
         n = s->itermax;
       }
       for (int c = 0; c < chunk && n < s->itermax; c++) {
@@ -935,15 +971,15 @@ double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, cons
           if (!launched("k_rb_fold")) return NAN;
         }
         if (!launch_sweep<V>(P, C, d[in], d[out], r0, st, folded ? sum[in] : part[in], part[out], n,
-                first ? 0 : folded ? 1 : nb))
+                first ? 0 : folded ? 1 : nb, down))
           return NAN;
       }
       if (!P.cluster_threads) {
         k_rb_finish<<<1, 32, 0, q>>>(st, part[n & 1], n, nb);
         if (!launched("k_rb_finish")) return NAN;
       }
-      k_rb_close<V><<<(unsigned)up(a.np * a.ny * a.nz, 256), 256, 0, q>>>(a, g, p, d[0], d[1], st,
-          direct);
+      k_rb_close<V><<<(unsigned)up(a.np * a.ny * a.nz, 256), 256, 0, q>>>(a, g, p, d[0], d[1],
+          unit, st, direct);
       if (!launched("k_rb_close")) return NAN;
     }
     if (!cuda_ok(cudaMemcpyAsync(h, st, sizeof(RbState), cudaMemcpyDeviceToHost, q),

@@ -32,3 +32,46 @@ def test_no_relaxation_runs_to_itermax(nusif_lib, oracle_mod, dims, arith):
         assert sim.iterations == it == 7
         assert res == pytest.approx(want, rel=1e-11)
         assert rel_err(sim.field("p"), p) < 1e-11
+
+
+# the update is linear: with rhs and eps times c and p times c a^2, a the edge of
+# the box, the iterations and p / (c a^2) are the same
+SCALES = [(a, c, e) for a in ("df32", "fp64")
+          for c, e in [(1.0, 1.0), (1.0, 1e-5), (1.0, 1e-6), (1.0, 1e-7), (1.0, 1e-9), (1.0, 1e4),
+                       (1e-14, 1.0), (1e3, 1e-6)]]
+# (pressures below 2^-74 lose the low part of their pairs in the iteration on p itself)
+SCALES += [("fp64", 1e-10, 1e-9), ("fp64", 1e-100, 1.0)]
+
+
+def _scaled_solve(sim_keys, o, dims, data, box, eps, itermax, rough):
+    rng = np.random.default_rng(5)
+    shape = tuple(n + 2 for n in dims[::-1])
+    p = data * box ** 2 * rough * rng.standard_normal(shape)
+    rhs = data * rng.standard_normal(shape)
+    rhs -= rhs[1:-1, 1:-1, 1:-1].mean()
+    with _sim(dims, [box] * 3, omg=1.7, itermax=itermax, **sim_keys) as sim:
+        sim.s.eps = eps
+        sim.set_field("p", p)
+        sim.set_field("rhs", rhs)
+        res = sim.solve()
+        it, want = o.op_solve_rb(o.grid(*dims, box, box, box), eps, 1.7, itermax, p, rhs)
+        assert sim.iterations == it
+        assert res == pytest.approx(want, rel=1e-9)
+        assert rel_err(sim.field("p"), p) < 1e-11
+        return it
+
+
+@pytest.mark.parametrize("arith,data,box", SCALES)
+@pytest.mark.parametrize("dims", [(24, 24, 24), (40, 41, 39)])
+def test_iterations_do_not_depend_on_scale(nusif_lib, oracle_mod, dims, arith, data, box):
+    """Boxes of micrometres in SI units, small and large data: the same count and
+    residual as the oracle's, and p to the rounding of the unscaled solve."""
+    it = _scaled_solve({"arith": arith}, oracle_mod, dims, data, box, 1e-4 * data, 600, 1e-3)
+    assert 60 < it < 600
+
+
+# squares whose sum over the grid, or (fp64) whose size, is beyond a float; nothing converges
+@pytest.mark.parametrize("arith,data", [("df32", 1e17), ("fp64", 1e30)])
+@pytest.mark.parametrize("dims", [(24, 24, 24), (40, 41, 39), (128, 96, 80)])
+def test_large_residuals_run_on(nusif_lib, oracle_mod, dims, arith, data):
+    assert _scaled_solve({"arith": arith}, oracle_mod, dims, data, 1.0, 0.25, 20, 1e-6) == 20
