@@ -1,6 +1,10 @@
 """Red-black SOR solves where the sweeps on the change of p could part from the
 scheme on p itself (k_sor_pass, the oracle): relaxation factors, scales of the
 data and of the box, solves one after another, very unlike spacings."""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -75,3 +79,65 @@ def test_iterations_do_not_depend_on_scale(nusif_lib, oracle_mod, dims, arith, d
 @pytest.mark.parametrize("dims", [(24, 24, 24), (40, 41, 39), (128, 96, 80)])
 def test_large_residuals_run_on(nusif_lib, oracle_mod, dims, arith, data):
     assert _scaled_solve({"arith": arith}, oracle_mod, dims, data, 1.0, 0.25, 20, 1e-6) == 20
+
+
+@pytest.fixture(scope="module")
+def rb_exact(tmp_path_factory):
+    """rb_exact.c as a function of (dims, length, omega, iterations, p, rhs), in place."""
+    lib = tmp_path_factory.mktemp("rb") / "librb_exact.so"
+    subprocess.run(["gcc", "-O2", "-shared", "-fPIC", str(Path(__file__).with_name("rb_exact.c")),
+                    "-o", str(lib)], check=True)
+    f = C.CDLL(str(lib)).rb_exact
+    f.argtypes = [C.c_int] * 3 + [C.c_double] * 4 + [C.c_int] + [C.c_void_p] * 2
+
+    def run(dims, h, omega, iterations, p, rhs):
+        assert f(*dims, *h, omega, iterations, p.ctypes.data, rhs.ctypes.data) == 0
+
+    return run
+
+
+def _modes(dims, rng, count=8):
+    """A smooth field without flux through the walls, padded, zero ghosts."""
+    out = np.zeros([n + 2 for n in dims[::-1]])
+    for _ in range(count):
+        m = rng.integers(0, 5, 3)
+        x, y, z = (np.cos(q * np.pi * (np.arange(n) + 0.5) / n) for q, n in zip(m, dims))
+        out[1:-1, 1:-1, 1:-1] += (rng.standard_normal() / (1 + (m ** 2).sum()) *
+                                  z[:, None, None] * y[None, :, None] * x[None, None, :])
+    return out
+
+
+def _error_against_64_bits(rb_exact, dims, length, iterations, p, rhs, omega=1.7, **keys):
+    with _sim(dims, length, omg=omega, eps=1e-30, itermax=iterations, **keys) as sim:
+        sim.set_field("p", p)
+        sim.set_field("rhs", rhs)
+        sim.solve()
+        assert sim.iterations == iterations
+        got = sim.field("p")
+        g = sim.d.grid
+        want = p.copy()
+        rb_exact(dims, (g.dx, g.dy, g.dz), omega, iterations, want, rhs)
+    c = (slice(1, -1),) * 3
+    return rel_err(got[c], want[c])
+
+
+# Tolerance: an iteration on p rounds p and its operands, to 2^-52 of the largest
+# pressure (pairs: 2^-47), anew each time, and damps what the earlier ones left;
+# independent errors add up to their size times the root of the count, twice
+# that for the largest cell. (An error that is the same in every iteration adds
+# up to the count.)
+def _bound(iterations, arith):
+    return 2.0 * iterations ** 0.5 * (2.0 ** -47 if arith == "df32" else 2.0 ** -52)
+
+
+@pytest.mark.parametrize("arith", ["df32", "fp64"])
+@pytest.mark.parametrize("dims,length", [((6, 160, 7), (4.0, 1.0, 1.0)),
+                                         ((64, 64, 4), (0.01, 1.0, 1.0)),
+                                         ((40, 12, 12), (30.0, 4.0, 4.0))])
+def test_unlike_spacings_keep_their_factors(nusif_lib, rb_exact, dims, length, arith):
+    """Spacings whose factors differ by orders of magnitude, from rest."""
+    rng = np.random.default_rng(6)
+    h2 = [(x / n) ** 2 for x, n in zip(length, dims)]
+    rhs = _modes(dims, rng) / min(h2)
+    err = _error_against_64_bits(rb_exact, dims, length, 500, np.zeros_like(rhs), rhs, arith=arith)
+    assert err < _bound(500, arith)
