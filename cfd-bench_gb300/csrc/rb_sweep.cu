@@ -2,14 +2,15 @@
 // of p (src/solver-rb.c:50-151 semantics; the first iteration runs on p
 // itself, k_sor_pass in solver.cu).
 //
-// The scheme is linear: with P the pressure after the first iteration (whose
+// The scheme is linear: with P the pressure after some iterations (whose
 // ghosts then equal the cells beside them) and p = P + d, an iteration relaxes
-// d against r0 = rhs - A P, formed once in FP64, and the residual is the
+// d against r0 = rhs - A P, formed in FP64, and the residual is the
 // same. d and r0 are kept as pairs of FP32 numbers (df32.cuh; plain doubles
 // with arith fp64), so an update needs no split of binary64 operands and no
-// FP64 instruction, and its rounding scales with |d|, not |p|: the error of
-// the solve against 64 bits was measured no larger than with the residual
-// split from p in every use. At the end p = P + d in binary64. The factors
+// FP64 instruction, and its rounding scales with |d|, not |p|. P is the
+// pressure after the first iteration, then, every few (next_fold), P + d in
+// binary64, and so is p at the end: the error of a solve against 64 bits is below
+// that of the scheme on p itself, wherever it starts. The factors
 // are folded into the constants: an update is c + D with
 //   D = -factor r = f_x (w + e - 2 c) + f_y (s + n - 2 c) + f_z (b + t - 2 c) - factor r0,
 // and the sum of r^2 is that of D^2 over factor^2. factor is omega h^2 / 6, of
@@ -419,41 +420,67 @@ __global__ void __launch_bounds__(kMaxThreads) k_rb_sweep(SweepArgs A, Consts<V>
   }
 }
 
-// after the first iteration: r = -factor (rhs - A P) in FP64 (S.factor is the
-// scaled one), d = 0 with its ghosts (one thread per entry of a colour's array)
+// rhs - A P of a cell in FP64, from P's differences: they are near exact where P
+// is smooth, where a sum of terms of the size of A P rounds, once for all the
+// iterations that follow. CG: past L1, P was written in this kernel.
+template <bool CG>
+__device__ __forceinline__ double residual_of(const SorArgs &S, const double *p, const double *rhs,
+    int c)
+{
+  const int sj = S.g.sj, sk = S.g.sk;
+  const auto ld = [&](int q) { return CG ? __ldcg(p + q) : p[q]; };
+  const double m = ld(c);
+  double r = rhs[c];
+  r = ::fma(-((ld(c - 1) - m) + (ld(c + 1) - m)), S.idx2, r);
+  r = ::fma(-((ld(c - sj) - m) + (ld(c + sj) - m)), S.idy2, r);
+  return ::fma(-((ld(c - sk) - m) + (ld(c + sk) - m)), S.idz2, r);
+}
+
+// a cell's pressure, and the ghosts beside it
+__device__ __forceinline__ void store_p(const SweepArgs &A, const Dims &g, double *p, int i, int j,
+    int k, double v)
+{
+  double *c = p + ((k + 1) * g.sk + (j + 1) * g.sj + i + 1);
+  *c = v;
+  if (i == 0) c[-1] = v;
+  if (i == A.nx - 1) c[1] = v;
+  if (j == 0) c[-g.sj] = v;
+  if (j == A.ny - 1) c[g.sj] = v;
+  if (k == 0) c[-g.sk] = v;
+  if (k == A.nz - 1) c[g.sk] = v;
+}
+
+// p holds n iterations: r0 = -factor (rhs - A P) (S.factor is the scaled one),
+// d = 0 with its ghosts (one thread per entry of a colour's array)
 template <typename V>
 __global__ void __launch_bounds__(256) k_rb_open(SweepArgs A, SorArgs S, const double *__restrict__ p,
-    const double *__restrict__ rhs, V *__restrict__ d, V *__restrict__ r0, const RbState *st)
+    const double *__restrict__ rhs, V *__restrict__ d, V *__restrict__ r0, RbState *st, int n)
 {
   if (is_done(st)) return;
   const int q = blockIdx.x * 256 + threadIdx.x;
+  if (q == 0) st->base = n;
   if (q >= A.half) return;
   d[q] = d[q + A.half] = V();
   const int T = q % A.np, jk = q / A.np, j = jk % (A.ny + 2) - 1, k = jk / (A.ny + 2) - 2;
   if (j < 0 || j >= A.ny || k < 0 || k >= A.nz) return;
-  const int sj = S.g.sj, sk = S.g.sk;
 #pragma unroll
   for (int e = 0; e < 2; e++) {
     const int i = 2 * T + e;
     double r = 0.0;
-    if (i < A.nx) {
-      const int c = (k + 1) * sk + (j + 1) * sj + i + 1;
-      const double lap = (p[c - 1] + p[c + 1]) * S.idx2 + (p[c - sj] + p[c + sj]) * S.idy2 +
-                         (p[c - sk] + p[c + sk]) * S.idz2 - S.diag * p[c];
-      r = rhs[c] - lap;
-    }
+    if (i < A.nx)
+      r = residual_of<false>(S, p, rhs, (k + 1) * S.g.sk + (j + 1) * S.g.sj + i + 1);
     r0[((i + j + k) & 1) * A.half + q] = to_cell(-S.factor * r, V());
   }
 }
 
-// p = P + d on the cells and the six ghost faces, once the solve is over
-// (direct: the iterations that ran on p itself)
+// p = P + d on the cells and the six ghost faces: of iteration n (k_rb_open
+// follows), or once the solve is over (n 0)
 template <typename V>
 __global__ void __launch_bounds__(256) k_rb_close(SweepArgs A, Dims g, double *__restrict__ p,
-    const V *__restrict__ d0, const V *__restrict__ d1, double unit, const RbState *st, int direct)
+    const V *__restrict__ d0, const V *__restrict__ d1, double unit, const RbState *st, int n)
 {
-  if (!is_done(st) || st->s.it <= direct) return;
-  const V *d = (st->s.it & 1) ? d1 : d0;
+  if (n > 0 ? is_done(st) : !is_done(st) || st->s.it <= st->base) return;
+  const V *d = ((n > 0 ? n : st->s.it) & 1) ? d1 : d0;
   const int q = blockIdx.x * 256 + threadIdx.x;
   if (q >= A.np * A.ny * A.nz) return;
   const int T = q % A.np, jk = q / A.np, j = jk % A.ny, k = jk / A.ny;
@@ -461,16 +488,25 @@ __global__ void __launch_bounds__(256) k_rb_close(SweepArgs A, Dims g, double *_
   for (int e = 0; e < 2; e++) {
     const int i = 2 * T + e;
     if (i >= A.nx) continue;
-    double *c = p + ((k + 1) * g.sk + (j + 1) * g.sj + i + 1);
-    const double v = plus(*c, d[((i + j + k) & 1) * A.half + A.at(T, j, k)], unit);
-    *c = v;
-    if (i == 0) c[-1] = v;
-    if (i == A.nx - 1) c[1] = v;
-    if (j == 0) c[-g.sj] = v;
-    if (j == A.ny - 1) c[g.sj] = v;
-    if (k == 0) c[-g.sk] = v;
-    if (k == A.nz - 1) c[g.sk] = v;
+    const double was = p[(k + 1) * g.sk + (j + 1) * g.sj + i + 1];
+    store_p(A, g, p, i, j, k, plus(was, d[((i + j + k) & 1) * A.half + A.at(T, j, k)], unit));
   }
+}
+
+// The iterations after which d joins p and r0 is formed anew. Pairs round an
+// update at the size of d, and r0's own rounding acts in every iteration alike,
+// so d has to stay small against p also where a solve starts far from its end.
+// Error against 64 bits after 500 iterations, on p itself | d over the whole solve
+// | here (24^3, from a pressure that has nothing to do with the right-hand side):
+// pairs 5.3e-14 | 1.3e-12 | 1.1e-14, fp64 6.3e-16 | 8.8e-14 | 3.8e-16; from near
+// the end, 6 x 160 x 7 cells of 4 x 1 x 1: pairs 5.1e-13 | 6.1e-14 | 1.9e-15, fp64
+// 4.7e-15 | 4.6e-14 | 1.3e-16. (After 8, 32, 128, 512 .. iterations was not
+// enough where the right-hand side has a mean: 23^3 ten times the error on p.) A
+// fold costs about 75 us at 128^3, where 64 iterations take 1230, and 18 of 430 at
+// 64^3.
+__host__ __device__ constexpr int next_fold(int n)
+{
+  return n < 8 ? 8 : n < 32 ? 32 : 32 + 64 * ((n - 32) / 64 + 1);
 }
 
 // a long list of block sums folded once instead of by every block of the next sweep
@@ -572,7 +608,8 @@ __device__ __forceinline__ V warp_total_u(V v)
 
 template <typename V, bool CUBE>
 __global__ void __launch_bounds__(1024) k_rb_cluster(ClusterArgs A, SweepArgs G, Consts<V> C,
-    const V *__restrict__ r0, V *d0, V *d1, RbState *st, int direct, float down)
+    SorArgs S, double *p, const double *rhs, const V *__restrict__ r0, V *d0, V *d1, double unit,
+    RbState *st, int direct, float down)
 {
   if (is_done(st)) return;  // the same for all blocks
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -587,17 +624,16 @@ __global__ void __launch_bounds__(1024) k_rb_cluster(ClusterArgs A, SweepArgs G,
   V *const rs = cells + 4 * size;                    // [colour][pair]
   V *const squares = rs + 2 * A.P * plane;           // a worker's sum
   unsigned char *const flag = reinterpret_cast<unsigned char *>(squares + workers);
-  const auto cell = [&](int q, int e, int &colour) {  // of pair q, its global offset
+  const auto cell = [&](int q, int e, int (&x)[3]) {  // of pair q: where it is on the grid
     const int kk = A.mpl ? (int)__umulhi((unsigned)q, A.mpl) : q, jt = q - kk * plane;
     const int j = A.mrow ? (int)__umulhi((unsigned)jt, A.mrow) : jt, t = jt - j * np;
     const int c[3] = { 2 * t + e, j, first + kk };
-    int x[3];
 #pragma unroll
     for (int a = 0; a < 3; a++)
       x[a] = A.axis[0] == a ? c[0] : A.axis[1] == a ? c[1] : c[2];
-    colour = (c[0] + c[1] + c[2]) & 1;
-    return c[0] < A.n[0] ? colour * G.half + G.at(x[0] >> 1, x[1], x[2]) : -1;
+    return c[0] < A.n[0];
   };
+  const auto colour_of = [](const int (&x)[3]) { return (x[0] + x[1] + x[2]) & 1; };
   for (int q = tid; q < 4 * size; q += blockDim.x) cells[q] = V();
   for (int q = tid; q < mine; q += blockDim.x) {
     const int kk = A.mpl ? (int)__umulhi((unsigned)q, A.mpl) : q, jt = q - kk * plane;
@@ -608,9 +644,10 @@ __global__ void __launch_bounds__(1024) k_rb_cluster(ClusterArgs A, SweepArgs G,
                               (2 * t + 1 == A.n[0]) << 6 | ((j + k) & 1) << 7);
 #pragma unroll
     for (int e = 0; e < 2; e++) {
-      int colour;
-      const int o = cell(q, e, colour);
-      rs[colour * A.P * plane + q] = o >= 0 ? r0[o] : V();
+      int x[3];
+      const bool in = cell(q, e, x);
+      const int c = colour_of(x);
+      rs[c * A.P * plane + q] = in ? r0[c * G.half + G.at(x[0] >> 1, x[1], x[2])] : V();
     }
   }
   double res = 0.0, epssq = 0.0, inv_factor2 = 0.0, inv_ncell = 0.0;
@@ -660,7 +697,37 @@ __global__ void __launch_bounds__(1024) k_rb_cluster(ClusterArgs A, SweepArgs G,
       if (high && q >= mine - plane) store_in(in_block(out + q - mine, rank + 1), m);
     }
   };
+  // iteration n's d joins p, and r0 is formed from the new one
+  const auto fold = [&] {
+    V *const d = cells + 2 * (n & 1) * size;
+    for (int q = tid; q < mine; q += blockDim.x)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        int x[3];
+        if (!cell(q, e, x)) continue;
+        const double was = __ldcg(p + (x[2] + 1) * S.g.sk + (x[1] + 1) * S.g.sj + x[0] + 1);
+        store_p(G, S.g, p, x[0], x[1], x[2], plus(was, d[colour_of(x) * size + plane + q], unit));
+      }
+    cluster_barrier(A.blocks);
+    for (int q = tid; q < 2 * size; q += blockDim.x) d[q] = V();
+    for (int q = tid; q < mine; q += blockDim.x)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        int x[3];
+        if (!cell(q, e, x)) continue;
+        const int c = (x[2] + 1) * S.g.sk + (x[1] + 1) * S.g.sj + x[0] + 1;
+        rs[colour_of(x) * A.P * plane + q] =
+            to_cell(-S.factor * residual_of<true>(S, p, rhs, c), V());
+      }
+    if (rank == 0 && tid == 0) st->base = n;
+    cluster_barrier(A.blocks);
+  };
+  int fold_at = next_fold(n);
   for (;;) {
+    if (n == fold_at) {
+      fold();
+      fold_at = next_fold(n);
+    }
     const int from = n & 1, to = from ^ 1;
     if (work) {
       acc = V();
@@ -697,9 +764,10 @@ __global__ void __launch_bounds__(1024) k_rb_cluster(ClusterArgs A, SweepArgs G,
   for (int q = tid; q < mine; q += blockDim.x)
 #pragma unroll
     for (int e = 0; e < 2; e++) {
-      int colour;
-      const int o = cell(q, e, colour);
-      if (o >= 0) d[o] = cells[(2 * (n & 1) + colour) * size + plane + q];
+      int x[3];
+      if (!cell(q, e, x)) continue;
+      const int c = colour_of(x);
+      d[c * G.half + G.at(x[0] >> 1, x[1], x[2])] = cells[(2 * (n & 1) + c) * size + plane + q];
     }
   if (rank == 0 && tid == (int)blockDim.x - 1) {
     st->s.res = res;
@@ -845,8 +913,8 @@ bool cluster_config(const RbPlan &P, cudaLaunchConfig_t &cfg, cudaLaunchAttribut
 }
 
 template <typename V>
-bool launch_cluster(const RbPlan &P, const Consts<V> &C, const V *r0, V *const (&d)[2], RbState *st,
-    int direct, float down)
+bool launch_cluster(const RbPlan &P, const Consts<V> &C, const SorArgs &S, double *p,
+    const double *rhs, const V *r0, V *const (&d)[2], double unit, RbState *st, int direct, float down)
 {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at;
@@ -857,8 +925,8 @@ bool launch_cluster(const RbPlan &P, const Consts<V> &C, const V *r0, V *const (
   T.fx = f[P.c.axis[0]];
   T.fy = f[P.c.axis[1]];
   T.fz = f[P.c.axis[2]];
-  cudaLaunchKernelEx(&cfg, P.cube ? k_rb_cluster<V, true> : k_rb_cluster<V, false>, P.c, P.a, T, r0,
-      d[0], d[1], st, direct, down);
+  cudaLaunchKernelEx(&cfg, P.cube ? k_rb_cluster<V, true> : k_rb_cluster<V, false>, P.c, P.a, T, S, p,
+      rhs, r0, d[0], d[1], unit, st, direct, down);
   return launched("k_rb_cluster");
 }
 
@@ -936,6 +1004,7 @@ double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, cons
   h->s.ncell = (double)(g.imax * g.jmax * g.kmax);
   h->inv_ncell = 1.0 / h->s.ncell;
   h->inv_factor2 = std::ldexp(1.0 / (S.factor * S.factor), k);
+  h->base = s->itermax;  // p holds every iteration until k_rb_open
   h->s.done = !((h->s.res >= h->s.epssq) && (0 < h->s.itermax));
   if (h->s.done) return h->s.res;
   if (!cuda_ok(cudaMemcpyAsync(st, h, sizeof(RbState), cudaMemcpyHostToDevice, q),
@@ -951,6 +1020,15 @@ double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, cons
   const int direct = ss->last_iterations == 2 && s->itermax >= 2 ? 2 : 1;
   if (!on_p(direct)) return NAN;
   int n = direct;
+  const auto open = [&] {
+    k_rb_open<V><<<(unsigned)up(a.half, 256), 256, 0, q>>>(a, S, p, rhs, d[n & 1], r0, st, n);
+    return launched("k_rb_open");
+  };
+  const auto close = [&](int at) {
+    k_rb_close<V><<<(unsigned)up(a.np * a.ny * a.nz, 256), 256, 0, q>>>(a, g, p, d[0], d[1], unit,
+        st, at);
+    return launched("k_rb_close");
+  };
   // queue iterations in chunks; the first chunk matches the previous solve's count
   int chunk = ss->last_iterations > 0 ? ss->last_iterations - direct : 16;
   while (!h->s.done) {
@@ -959,12 +1037,9 @@ double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, cons
       if (!on_p(count)) return NAN;
       n += count;
     } else if (chunk > 0 && n < s->itermax) {
-      if (n == direct) {
-        k_rb_open<V><<<(unsigned)up(a.half, 256), 256, 0, q>>>(a, S, p, rhs, d[n & 1], r0, st);
-        if (!launched("k_rb_open")) return NAN;
-      }
+      if (n == direct && !open()) return NAN;
       if (P.cluster_threads) {  // to the end
-        if (!launch_cluster<V>(P, C, r0, d, st, direct, down)) return NAN;
+        if (!launch_cluster<V>(P, C, S, p, rhs, r0, d, unit, st, direct, down)) return NAN;
         n = s->itermax;
       }
       for (int c = 0; c < chunk && n < s->itermax; c++) {
@@ -978,14 +1053,13 @@ double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, cons
         if (!launch_sweep<V>(P, C, d[in], d[out], r0, st, folded ? sum[in] : part[in], part[out], n,
                 first ? 0 : folded ? 1 : nb, down))
           return NAN;
+        if (n == next_fold(n - 1) && n < s->itermax && !(close(n) && open())) return NAN;
       }
       if (!P.cluster_threads) {
         k_rb_finish<<<1, 32, 0, q>>>(st, part[n & 1], n, nb);
         if (!launched("k_rb_finish")) return NAN;
       }
-      k_rb_close<V><<<(unsigned)up(a.np * a.ny * a.nz, 256), 256, 0, q>>>(a, g, p, d[0], d[1],
-          unit, st, direct);
-      if (!launched("k_rb_close")) return NAN;
+      if (!close(0)) return NAN;
     }
     if (!cuda_ok(cudaMemcpyAsync(h, st, sizeof(RbState), cudaMemcpyDeviceToHost, q),
             "solve state download"))

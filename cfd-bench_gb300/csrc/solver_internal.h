@@ -23,6 +23,7 @@ struct RbState {
   SolveState s;
   double res[2];  // carried residual after m iterations, at m & 1
   double inv_ncell, inv_factor2;
+  int base, pad;  // base: the iterations whose change p holds
 };
 
 struct SorArgs {

@@ -13,7 +13,8 @@ int rb_exact(int nx, int ny, int nz, double dx, double dy, double dz, double ome
   if (!q) return 1;
   for (size_t c = 0; c < n; c++) q[c] = p[c];
   for (int it = 0; it < iterations; it++) {
-    for (int colour = 1; colour >= 0; colour--)
+    for (int colour = 1; colour >= 0; colour--) {
+#pragma omp parallel for
       for (int k = 1; k <= nz; k++)
         for (int j = 1; j <= ny; j++)
           for (int i = 1; i <= nx; i++) {
@@ -24,6 +25,7 @@ int rb_exact(int nx, int ny, int nz, double dx, double dy, double dz, double ome
                                     (q[c - sk] - 2 * q[c] + q[c + sk]) / z2;
             q[c] -= factor * (rhs[c] - lap);
           }
+    }
     for (int k = 1; k <= nz; k++)
       for (int j = 1; j <= ny; j++)
         for (int i = 1; i <= nx; i++) {
