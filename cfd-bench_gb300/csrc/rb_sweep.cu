@@ -609,7 +609,7 @@ __device__ __forceinline__ V warp_total_u(V v)
 template <typename V, bool CUBE>
 __global__ void __launch_bounds__(1024) k_rb_cluster(ClusterArgs A, SweepArgs G, Consts<V> C,
     SorArgs S, double *p, const double *rhs, const V *__restrict__ r0, V *d0, V *d1, double unit,
-    RbState *st, int direct, float down)
+    RbState *st, float down)
 {
   if (is_done(st)) return;  // the same for all blocks
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(1024) k_rb_cluster(ClusterArgs A, SweepArgs G,
 #pragma unroll
     for (int u = 0; u < 4; u++)
       if (tid + u * workers < mine) flags |= (unsigned)flag[tid + u * workers] << (8 * u);
-  int n = direct;
+  int n = 1;
   V acc{};
   // one colour of an iteration: reads copy `from` (its own cells; the other
   // colour's from `to` once they are new there), writes copy `to`
@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(1024) k_rb_cluster(ClusterArgs A, SweepArgs G,
     if (work) {
       acc = V();
       half_pass(from, to, 0);
-    } else if (n > direct) {  // iteration n's squares in this block
+    } else if (n > 1) {  // iteration n's squares in this block
       const int w = (tid - workers) >> 5;
       V v[2] = {};
       for (int q = lane + 32 * w; q < workers; q += 64 * kFoldWarps)
@@ -747,7 +747,7 @@ __global__ void __launch_bounds__(1024) k_rb_cluster(ClusterArgs A, SweepArgs G,
     if (work) {
       half_pass(from, to, 1);
       squares[tid] = acc;
-    } else if (n > direct) {  // whether it was the last
+    } else if (n > 1) {  // whether it was the last
       V v{};
 #pragma unroll
       for (int u = 0; u < 16 * kFoldWarps; u += 32)
@@ -914,7 +914,7 @@ bool cluster_config(const RbPlan &P, cudaLaunchConfig_t &cfg, cudaLaunchAttribut
 
 template <typename V>
 bool launch_cluster(const RbPlan &P, const Consts<V> &C, const SorArgs &S, double *p,
-    const double *rhs, const V *r0, V *const (&d)[2], double unit, RbState *st, int direct, float down)
+    const double *rhs, const V *r0, V *const (&d)[2], double unit, RbState *st, float down)
 {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at;
@@ -926,7 +926,7 @@ bool launch_cluster(const RbPlan &P, const Consts<V> &C, const SorArgs &S, doubl
   T.fy = f[P.c.axis[1]];
   T.fz = f[P.c.axis[2]];
   cudaLaunchKernelEx(&cfg, P.cube ? k_rb_cluster<V, true> : k_rb_cluster<V, false>, P.c, P.a, T, S, p,
-      rhs, r0, d[0], d[1], unit, st, direct, down);
+      rhs, r0, d[0], d[1], unit, st, down);
   return launched("k_rb_cluster");
 }
 
@@ -1010,16 +1010,14 @@ double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, cons
   if (!cuda_ok(cudaMemcpyAsync(st, h, sizeof(RbState), cudaMemcpyHostToDevice, q),
           "solve state upload"))
     return NAN;
-  // the first iteration runs on p, and a second one where the last solve took
-  // no more: opening and closing the sweeps costs about one iteration on p
+  // the first iteration runs on p
   const auto on_p = [&](int count) {
     for (int c = 0; c < count; c++)
       if (!launch_rb_iteration(A, p, rhs, &st->s, ss->red, !ss->ext.arith_fp64)) return false;
     return true;
   };
-  const int direct = ss->last_iterations == 2 && s->itermax >= 2 ? 2 : 1;
-  if (!on_p(direct)) return NAN;
-  int n = direct;
+  if (!on_p(1)) return NAN;
+  int n = 1;
   const auto open = [&] {
     k_rb_open<V><<<(unsigned)up(a.half, 256), 256, 0, q>>>(a, S, p, rhs, d[n & 1], r0, st, n);
     return launched("k_rb_open");
@@ -1029,34 +1027,38 @@ double sweep_solve(Solver *s, SolverState *ss, const SorArgs &A, double *p, cons
         st, at);
     return launched("k_rb_close");
   };
+  const auto fold = [&](int at) {
+    k_rb_fold<<<1, 1024, 0, q>>>(st, part[at], nb, sum[at]);
+    return launched("k_rb_fold");
+  };
   // queue iterations in chunks; the first chunk matches the previous solve's count
-  int chunk = ss->last_iterations > 0 ? ss->last_iterations - direct : 16;
+  // (how many are queued at once is all that an earlier solve decides)
+  int chunk = ss->last_iterations > 0 ? ss->last_iterations - 1 : 16;
   while (!h->s.done) {
     if (!sweeps) {
       const int count = chunk < s->itermax - n ? chunk : s->itermax - n;
       if (!on_p(count)) return NAN;
       n += count;
     } else if (chunk > 0 && n < s->itermax) {
-      if (n == direct && !open()) return NAN;
+      if (n == 1 && !open()) return NAN;
       if (P.cluster_threads) {  // to the end
-        if (!launch_cluster<V>(P, C, S, p, rhs, r0, d, unit, st, direct, down)) return NAN;
+        if (!launch_cluster<V>(P, C, S, p, rhs, r0, d, unit, st, down)) return NAN;
         n = s->itermax;
       }
       for (int c = 0; c < chunk && n < s->itermax; c++) {
         n++;
         const int in = (n - 1) & 1, out = n & 1;
-        const bool first = n == direct + 1;
-        if (folded && !first) {
-          k_rb_fold<<<1, 1024, 0, q>>>(st, part[in], nb, sum[in]);
-          if (!launched("k_rb_fold")) return NAN;
-        }
+        const bool first = n == 2;
+        if (folded && !first && !fold(in)) return NAN;
         if (!launch_sweep<V>(P, C, d[in], d[out], r0, st, folded ? sum[in] : part[in], part[out], n,
                 first ? 0 : folded ? 1 : nb, down))
           return NAN;
         if (n == next_fold(n - 1) && n < s->itermax && !(close(n) && open())) return NAN;
       }
       if (!P.cluster_threads) {
-        k_rb_finish<<<1, 32, 0, q>>>(st, part[n & 1], n, nb);
+        // (the sum in the order of the next sweep, which forms the same residual)
+        if (folded && !fold(n & 1)) return NAN;
+        k_rb_finish<<<1, 32, 0, q>>>(st, folded ? sum[n & 1] : part[n & 1], n, folded ? 1 : nb);
         if (!launched("k_rb_finish")) return NAN;
       }
       if (!close(0)) return NAN;

@@ -174,3 +174,34 @@ def test_change_of_p_keeps_the_bits_of_p(nusif_lib, rb_exact, dims, length, star
         rhs -= rhs[1:-1, 1:-1, 1:-1].mean()
     n = 200
     assert _error_against_64_bits(rb_exact, dims, length, n, p, rhs, arith=arith) < _bound(n, arith)
+
+
+# the last two: more block sums than a sweep's blocks fold by themselves
+@pytest.mark.parametrize("arith", ["df32", "fp64"])
+@pytest.mark.parametrize("dims", [(16, 16, 16), (40, 41, 39), (200, 40, 40), (2, 4000, 40),
+                                  (1024, 1024, 1)])
+def test_solves_do_not_depend_on_earlier_ones(nusif_lib, dims, arith):
+    """The same p, rhs, eps and itermax give the same bits, whatever the solver
+    ran before (its iteration count decides how many launches are queued)."""
+    rng = np.random.default_rng(9)
+    eps, itermax = 1e-9, 90
+    with _sim(dims, [0.1 * n for n in dims], omg=1.7, eps=eps, itermax=itermax, arith=arith) as sim:
+        p = rng.standard_normal(sim.padded_shape)
+        rhs = rng.standard_normal(sim.padded_shape)
+
+        def solve(eps, itermax):
+            sim.s.eps, sim.s.itermax = eps, itermax
+            sim.set_field("p", p)
+            sim.set_field("rhs", rhs)
+            return sim.solve(), sim.iterations, sim.field("p")
+
+        first = solve(eps, itermax)  # a new solver's
+        on_the_way = 4.0 * first[0] ** 0.5  # converges between two chunks' ends, or at one
+        middle = solve(on_the_way, itermax)
+        assert 2 < middle[1] < itermax
+        for count in (2, 3, 1, 7, 16, middle[1], 40):
+            solve(eps, count)
+            for args, want in (((eps, itermax), first), ((on_the_way, itermax), middle)):
+                got = solve(*args)
+                assert got[:2] == want[:2]
+                np.testing.assert_array_equal(got[2], want[2])
