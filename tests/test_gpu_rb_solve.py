@@ -205,3 +205,11 @@ def test_solves_do_not_depend_on_earlier_ones(nusif_lib, dims, arith):
                 got = solve(*args)
                 assert got[:2] == want[:2]
                 np.testing.assert_array_equal(got[2], want[2])
+
+
+@pytest.mark.parametrize("arith", ["df32", "fp64"])
+@pytest.mark.parametrize("dims", [(2, 4000, 40), (1024, 1024, 1), (1500, 900, 2)])
+def test_long_lists_of_block_sums_match_oracle(nusif_lib, oracle_mod, dims, arith):
+    """More than 1024 block sums: folded by a launch of its own."""
+    from test_gpu_rb_sweep import test_sweeps_match_oracle
+    test_sweeps_match_oracle(nusif_lib, oracle_mod, dims, arith)
