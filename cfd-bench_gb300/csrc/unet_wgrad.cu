@@ -93,10 +93,11 @@ struct Layout {
 // G32: G is one FP32 channel, stored as the three BF16 channels whose sum it
 // is (24 bits), the other rows of the tile zero.
 // ROWS: the tensor core's own FP32 accumulation truncates, so a long chain of
-// products drifts (2e-5 of a gradient over two million cells). The first and
+// products drifts (1e-5 of a gradient over two million cells). The first and
 // the last layer, whose gradients were plain FP32 sums before, keep a chain to
 // one row and add the rows with rounding (2e-7); at 16 x 16 channels that costs
-// 155 -> 220 us on two million cells.
+// 155 -> 220 us on two million cells. The bias gradients, one fragment of one
+// warp, do so in every layer.
 template <int TM, int TN, bool G32, bool ROWS>
 __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
 {
@@ -138,10 +139,6 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
         for (int n = 0; n < NT; n++)
 #pragma unroll
           for (int e = 0; e < 4; e++) acc[t][m][n][e] = 0.0f;
-#pragma unroll
-    for (int m = 0; m < MT; m++)
-#pragma unroll
-      for (int e = 0; e < 4; e++) bias[m][e] = 0.0f;
   };
   // ROWS: the row's products join the sums
   const auto gather = [&] {
@@ -154,12 +151,16 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
           for (int n = 0; n < NT; n++)
 #pragma unroll
             for (int e = 0; e < 4; e++) sum[t][m][n][e] += acc[t][m][n][e];
-#pragma unroll
-      for (int m = 0; m < MT; m++) {
-        bias_sum[m][0] += bias[m][0];
-        bias_sum[m][1] += bias[m][2];
-      }
       clear();
+    }
+  };
+  const auto gather_bias = [&] {
+#pragma unroll
+    for (int m = 0; m < MT; m++) {
+      bias_sum[m][0] += bias[m][0];
+      bias_sum[m][1] += bias[m][2];
+#pragma unroll
+      for (int e = 0; e < 4; e++) bias[m][e] = 0.0f;
     }
   };
   clear();
@@ -174,7 +175,11 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
           for (int e = 0; e < 4; e++) sum[t][m][n][e] = 0.0f;
   }
 #pragma unroll
-  for (int m = 0; m < MT; m++) bias_sum[m][0] = bias_sum[m][1] = 0.0f;
+  for (int m = 0; m < MT; m++) {
+    bias_sum[m][0] = bias_sum[m][1] = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 4; e++) bias[m][e] = 0.0f;
+  }
   if (G32) {  // the rows that stay zero
     for (int i = tid; i < 2 * L::kGrow / 16; i += kThreads)
       reinterpret_cast<uint4 *>(gs)[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -269,6 +274,7 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
             }
           }
       }
+      if (warp == 4) gather_bias();
       gather();
     }
   }
@@ -301,8 +307,8 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
   if (warp == 4 && (lane & 3) == 0) {
 #pragma unroll
     for (int m = 0; m < MT; m++) {
-      out[27 * TM * TN + 16 * m + g] = ROWS ? bias_sum[m][0] : bias[m][0];
-      out[27 * TM * TN + 16 * m + g + 8] = ROWS ? bias_sum[m][1] : bias[m][2];
+      out[27 * TM * TN + 16 * m + g] = bias_sum[m][0];
+      out[27 * TM * TN + 16 * m + g + 8] = bias_sum[m][1];
     }
   }
 }
