@@ -50,6 +50,7 @@ struct Args {
   int items;         // B * Z * xt * yt
   int co;            // G's channels
   int parts_n;       // tiles over the input channels
+  int chain;         // cells whose products are summed without rounding, a run at least
   float *partial;    // [part][block][27 * TM * TN + TM]
 };
 
@@ -97,7 +98,8 @@ struct Layout {
 // the last layer, whose gradients were plain FP32 sums before, keep a chain to
 // one row and add the rows with rounding (2e-7); at 16 x 16 channels that costs
 // 155 -> 220 us on two million cells. The bias gradients, one fragment of one
-// warp, do so in every layer.
+// warp, do so in every layer. In the others a chain has at most a 256th of the
+// cells; where a block has more, it adds its sums to those it has stored.
 template <int TM, int TN, bool G32, bool ROWS>
 __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
 {
@@ -153,6 +155,36 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
             for (int e = 0; e < 4; e++) sum[t][m][n][e] += acc[t][m][n][e];
       clear();
     }
+  };
+  // the block's sums so far join those it has stored
+  float *const out =
+      A.partial + ((int64_t)part * gridDim.x + blockIdx.x) * (27 * TM * TN + TM);
+  const int g = lane >> 2, t2 = 2 * (lane & 3);
+  int chained = 0;
+  bool stored = false;
+  const auto store = [&] {
+#pragma unroll
+    for (int t = 0; t < 3; t++) {
+      float *const o = out + (dz * 9 + (dy + 1) * 3 + t) * TM * TN;
+#pragma unroll
+      for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int n = 0; n < NT; n++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            float2 *const at =
+                reinterpret_cast<float2 *>(o + (16 * m + g + 8 * h) * TN + 8 * n + t2);
+            float2 v = make_float2(acc[t][m][n][2 * h], acc[t][m][n][2 * h + 1]);
+            if (stored) {
+              const float2 was = *at;
+              v.x += was.x;
+              v.y += was.y;
+            }
+            *at = v;
+          }
+    }
+    stored = true;
+    chained = 0;
   };
   const auto gather_bias = [&] {
 #pragma unroll
@@ -276,6 +308,11 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
       }
       if (warp == 4) gather_bias();
       gather();
+      chained += A.run;
+      if (!ROWS && chained + A.run > A.chain) {
+        store();
+        clear();
+      }
     }
   }
   if constexpr (ROWS) {
@@ -288,22 +325,7 @@ __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
 #pragma unroll
           for (int e = 0; e < 4; e++) acc[t][m][n][e] = sum[t][m][n][e];
   }
-  float *const out =
-      A.partial + ((int64_t)part * gridDim.x + blockIdx.x) * (27 * TM * TN + TM);
-  const int g = lane >> 2, t2 = 2 * (lane & 3);
-#pragma unroll
-  for (int t = 0; t < 3; t++) {
-    float *const o = out + (dz * 9 + (dy + 1) * 3 + t) * TM * TN;
-#pragma unroll
-    for (int m = 0; m < MT; m++)
-#pragma unroll
-      for (int n = 0; n < NT; n++) {
-        *reinterpret_cast<float2 *>(o + (16 * m + g) * TN + 8 * n + t2) =
-            make_float2(acc[t][m][n][0], acc[t][m][n][1]);
-        *reinterpret_cast<float2 *>(o + (16 * m + g + 8) * TN + 8 * n + t2) =
-            make_float2(acc[t][m][n][2], acc[t][m][n][3]);
-      }
-  }
+  if (!stored || chained > 0) store();
   if (warp == 4 && (lane & 3) == 0) {
 #pragma unroll
     for (int m = 0; m < MT; m++) {
@@ -355,7 +377,7 @@ __global__ void __launch_bounds__(256) k_wgrad_fold(const float *__restrict__ pa
 }
 
 struct Plan {
-  int tm, tn, parts, parts_n, run, xt, yc, yt, items, blocks;
+  int tm, tn, parts, parts_n, run, xt, yc, yt, items, blocks, chain;
 };
 
 // Tiles of 16 x 16, 16 x 48, 32 x 16 or 32 x 32 channels (the accumulators of
@@ -378,6 +400,8 @@ Plan plan(int co, int ci, int B, int Z, int Y, int X)
   p.yt = (Y + p.yc - 1) / p.yc;
   p.items = (int)(columns * p.yt);
   p.blocks = p.items < wave ? p.items : wave;
+  const int64_t chain = ((int64_t)B * Z * Y * X + 255) / 256;
+  p.chain = chain < kRun ? kRun : (int)chain;
   return p;
 }
 
@@ -427,6 +451,7 @@ bool wgrad_conv(const WgradSrc &s0, const WgradSrc &s1, const void *g, const flo
   a.items = p.items;
   a.co = co;
   a.parts_n = p.parts_n;
+  a.chain = p.chain;
   a.partial = scratch;
   bool ok = false;
   if (g32) ok = launch<16, 16, true, true>(p, a);

@@ -88,3 +88,17 @@ def test_bias_gradients_are_rounded_sums(nusif_lib, shape):
     blocks' sums, 250 of them here at most: 2^-22 + 2 sqrt(250) 2^-24 = 2.1e-6."""
     errors = _errors(shape)
     assert max(bias for _, bias in errors.values()) < 2.1e-6, errors
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_weight_gradients_drift_with_short_chains_only(nusif_lib, shape):
+    """A chain of the tensor core is at most a 256th of a layer's cells (or 64), 16
+    cells a step, each dropping half of a unit in the last place of a sum that
+    grows to the chain's: steps / 2 times 0.36 2^-23 of it. Half as much again
+    for the sums' unevenness, and the bound of the rounded additions above."""
+    errors = _errors(shape)
+    for name, (level, _) in GRADS.items():
+        cells = np.prod(shape) / 8 ** level
+        steps = max(64, cells / 256) / 16
+        bound = 1.5 * steps / 2 * 0.36 * 2.0 ** -23 + 2.1e-6
+        assert errors[name][0] < (2.1e-6 if name in ("e0a", "out") else bound), (name, errors)
