@@ -1118,6 +1118,9 @@ void initDiscretization(Discretization *s, Parameter *params)
   st->amax = kAmaxReset;
   if (!cuda_ok(cudaMallocHost(&st->h_scalars, 8 * sizeof(double)), "cudaMallocHost(scalars)"))
     return;
+  // for every reduction of the step (three values of at most four blocks per SM),
+  // so that none allocates later
+  if (!reduce_scratch_alloc(st->red, 3 * 4 * sm_count())) return;
   const double init[4] = { params->u_init, params->v_init, params->w_init, params->p_init };
   for (int q = 0; q < 4; q++)
     if (!launch_fill(*fields[q], padded, init[q])) return;
