@@ -230,7 +230,10 @@ __global__ void __launch_bounds__(kNT) k_mg_smooth(View<T> v, int colour, const 
 // f_y s_y + f_z s_z - i (b - shift), with the relaxation w, i = w / diag and
 // f = i e formed on the host: eight FP64 instructions per cell (seven without
 // over-relaxation) where x - i (b - shift - A x) takes ten, and no coarser: both
-// round at the size of x. The next plane's values are asked for before this
+// round at the size of x, and the weights of x and its neighbours add up to 1, so
+// that a constant x stays one (with each rounded by itself the colours came out
+// apart: 96^3, p about 1e6, V(2,2) of relaxation 1.3 came to rest at a true
+// residual of 6.3e-8 of ||b||, with A x at 4.7e-8, so at 3.1e-8). The next plane's values are asked for before this
 // plane's arithmetic (nothing an update reads is written by its own pass, but
 // its own cell). One colour at 128^3: 25 -> 20 us.
 struct Smooth64 {
@@ -238,21 +241,32 @@ struct Smooth64 {
   int relaxed;                   // keep is not 0 (a test of a double is an FP64 instruction)
 };
 
-__host__ __device__ __forceinline__ Smooth64 smooth64(const View<double> &v)
+inline Smooth64 smooth64(const View<double> &v)
 {
-  const double w = v.inv_diag * v.diag;  // the relaxation, up to a rounding
-  return { v.inv_diag * v.ex, v.inv_diag * v.ey, v.inv_diag * v.ez,
-           1.0 - w, v.inv_diag, fabs(w - 1.0) >= 1e-15 };
+  double w = v.inv_diag * v.diag;  // the relaxation, up to a rounding
+  const int relaxed = std::fabs(w - 1.0) >= 1e-15;
+  if (!relaxed) w = 1.0;
+  // (std::fma: no other contraction, which a host compiler may choose)
+  Smooth64 C{ v.inv_diag * v.ex, v.inv_diag * v.ey, v.inv_diag * v.ez, std::fma(-1.0, w, 1.0),
+    v.inv_diag, relaxed };
+  // the largest weight is what the others, in units of its last place, leave of
+  // w / 2: a double again (long double: neither difference rounds)
+  double *f[3] = { &C.fz, &C.fy, &C.fx };
+  std::stable_sort(f, f + 3, [](const double *a, const double *b) { return *a < *b; });
+  const double unit = std::ldexp(1.0, std::ilogb(*f[2]) - 52);
+  for (int q = 0; q < 2; q++) *f[q] = std::rint(*f[q] / unit) * unit;
+  *f[2] = (double)(0.5L * w - *f[0] - *f[1]);
+  return C;
 }
 
 // the new value from b's term r = i shift - i b and the neighbours' sums
 __device__ __forceinline__ double smooth64_cell(const Smooth64 &C, double r, double sx, double sy,
     double sz, double xc)
 {
+  if (C.relaxed) r = fma(C.keep, xc, r);
   r = fma(C.fx, sx, r);
   r = fma(C.fy, sy, r);
-  r = fma(C.fz, sz, r);
-  return C.relaxed ? fma(C.keep, xc, r) : r;
+  return fma(C.fz, sz, r);
 }
 
 // b - shift - A x, the operator's terms joined one by one: an FP64 instruction
@@ -1829,6 +1843,7 @@ struct TailLevel {
   int n[3];
   int r[3];  // coarsening ratio from the level above
   T ex, ey, ez, diag, inv_diag;
+  Smooth64 smooth;  // FP64 levels
   T *x, *b;
 };
 
@@ -1862,7 +1877,7 @@ __device__ __forceinline__ View<T> tail_view(const TailLevel<T> &L)
 }
 
 template <typename T>
-__device__ void tail_smooth(const View<T> &v, int count, bool zero_first)
+__device__ void tail_smooth(const View<T> &v, const Smooth64 &C, int count, bool zero_first)
 {
   const int n = v.nx * v.ny * v.nz;
   if (count == 0 && zero_first) {
@@ -1877,7 +1892,6 @@ __device__ void tail_smooth(const View<T> &v, int count, bool zero_first)
         const int i = q % v.nx, j = (q / v.nx) % v.ny, k = q / (v.nx * v.ny);
         if (((i + j + k + 1) & 1) != colour) continue;
         if constexpr (sizeof(T) == sizeof(double)) {
-          const Smooth64 C = smooth64(v);
           T r = fma(-C.inv, v.b[q], 0.0), sx, sy, sz;
           if (!(z && colour == 1)) {
             const T xc = z ? (T)0 : v.x[q];
@@ -1905,7 +1919,7 @@ __global__ void __launch_bounds__(1024) k_mg_tail(TailArgs<T> a)
   const int m = a.count;
   for (int l = 0; l < m - 1; l++) {
     const View<T> v = tail_view(a.lv[l]);
-    tail_smooth(v, a.pre, l > 0 || a.zero_top);
+    tail_smooth(v, a.lv[l].smooth, a.pre, l > 0 || a.zero_top);
     // residual restriction into the next level's right-hand side
     const TailLevel<T> &C = a.lv[l + 1];
     const int rx = C.r[0], ry = C.r[1], rz = C.r[2];
@@ -1947,7 +1961,7 @@ __global__ void __launch_bounds__(1024) k_mg_tail(TailArgs<T> a)
       }
       __syncthreads();
     } else {
-      tail_smooth(v, a.coarse_sweeps, true);
+      tail_smooth(v, a.lv[m - 1].smooth, a.coarse_sweeps, true);
     }
   }
   for (int l = m - 2; l >= 0; l--) {
@@ -1986,7 +2000,7 @@ __global__ void __launch_bounds__(1024) k_mg_tail(TailArgs<T> a)
       f.x[q] += y0 + w[2] * (y1 - y0);
     }
     __syncthreads();
-    tail_smooth(f, a.post, false);
+    tail_smooth(f, a.lv[l].smooth, a.post, false);
   }
 }
 
@@ -3088,6 +3102,8 @@ bool tail_vcycle(MgHierarchy *H, int l, T **xs, T **bs, bool zero)
     t.ez = (T)L.ih2[2];
     t.diag = (T)d;
     t.inv_diag = (T)(L.relax / d);
+    if constexpr (sizeof(T) == sizeof(double))
+      t.smooth = smooth64(compact_view<double>(L, nullptr, nullptr));
     t.x = xs[l + q];
     t.b = bs[l + q];
   }
