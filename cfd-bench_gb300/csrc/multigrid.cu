@@ -969,7 +969,7 @@ __global__ void __launch_bounds__(kNT) k_mg_prolong_x4(View<T> f, const T *__res
 // second-colour cells, still 0, as is a missing neighbour beyond a wall (the
 // cell itself). So the whole sweep is one stencil pass over b, one thread per
 // four consecutive cells of a row, writing x_new (the buffer the host swaps
-// in), with the arithmetic of the general sweep (k_rbgs_sweep) on x = 0.
+// in), with the arithmetic of the general sweep (k_rbgs_sweep_v) on x = 0.
 __global__ void __launch_bounds__(kNT) k_rb_zero_sweep(View<float> v, float *__restrict__ xnew,
     const MgState *st, int keep)
 {
@@ -1187,218 +1187,36 @@ __global__ void __launch_bounds__(kNT) k_mg_prolong_f64(View<double> f,
 
 // One whole red-black Gauss-Seidel sweep in one kernel, exact: reads x_old,
 // writes x_new (ping-pong), so no block ever reads a value another block
-// writes. A block owns a 64 x 8 tile of (i, j) columns and a chunk of planes;
-// per plane it relaxes the odd ("red") cells on the tile plus a one-cell ring
-// (from old even values: exactly what the first pass of a two-pass sweep
-// computes there), then the even cells of the previous plane on the tile
-// (from the new odd values and their own old value), and writes both colours
-// of that plane. Planes walk with a one-plane lag (odd at k, even at k-1); the
-// odd planes just outside the chunk are recomputed, so chunks are
-// independent. x_old (tile + two-cell ring) and b (tile + one-cell ring) are
-// staged in shared memory by asynchronous copies issued one plane ahead
-// (cp.async, completed by cp.async.wait_group), so global latency overlaps
-// the arithmetic of the plane before. One sweep reads x and b once and
-// writes x once. (A sweep from x = 0 is k_rb_zero_sweep.)
-constexpr int kSX = 64, kSY = 8;  // tile (cells)
-constexpr int kWX = kSX + 8;      // staged row: tile + 4 cells each side (16-byte chunks)
-constexpr int kRY = kSY + 4;      // staged x_old rows: tile + 2-row ring
-constexpr int kBYr = kSY + 2;     // staged b rows and odd values: tile + 1-row ring
-constexpr int kQX = kSX + 2;      // odd values: tile + 1-cell ring
-
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
-{
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
-// FP32 levels with nx % 4 == 0 (rows start on 16-byte boundaries): every
-// staged row is 18 chunks of four cells starting 4 cells left of the tile,
-// one chunk per thread per array per plane.
+// writes. A block owns a 128 x 8 tile of (i, j) columns and a chunk of planes;
+// per plane it relaxes the first-colour cells on the tile plus a one-cell ring
+// (from old second-colour values: exactly what the first pass of a two-pass
+// sweep computes there), then the second-colour cells of the previous plane on
+// the tile, and writes both colours of that plane: planes walk with a one-plane
+// lag, and the first-colour planes just outside the chunk are recomputed, so
+// chunks are independent. One sweep reads x and b once and writes x once. (A
+// sweep from x = 0 is k_rb_zero_sweep.)
 //
-// Walls cost no tests per neighbour: the Neumann operator replaces a missing
-// neighbour by the cell itself, and the staged x_old already holds that value
-// outside the domain (planes beyond a wall are staged as the wall plane, rows
-// beyond a wall as the wall row, and the column beyond a wall is patched to
-// the wall column); a first-colour ring cell outside the domain stores that
-// mirrored old value instead of a relaxed one, which is exactly what its
-// second-colour neighbour inside the domain must see there.
-__global__ void __launch_bounds__(256) k_rbgs_sweep(View<float> v, float *__restrict__ xnew,
-    int kc, const MgState *st, int keep)
-{
-  if (mg_done(st)) {
-    // The host swaps the two buffers after every sweep it launches. A sweep
-    // skipped because the correction met its target inside this V-cycle must
-    // still leave x where the next kernels look (keep: set when a level's
-    // sweeps per V-cycle could be skipped in odd numbers): it copies its chunk.
-    if (keep && !solve_finished(st)) {
-      const int i0 = blockIdx.x * kSX, j0 = blockIdx.y * kSY, k0 = blockIdx.z * kc;
-      const int k1 = min(k0 + kc, v.nz);
-      constexpr int kRowChunks = kSX / 4, kPlane = kSY * kRowChunks;
-      for (int q = threadIdx.x; q < (k1 - k0) * kPlane; q += 256) {
-        const int k = k0 + q / kPlane, rem = q % kPlane;
-        const int j = j0 + rem / kRowChunks, i = i0 + 4 * (rem % kRowChunks);
-        if (j >= v.ny || i >= v.nx) continue;
-        const int64_t c = (int64_t)k * v.sz + (int64_t)j * v.sy + i;
-        *reinterpret_cast<float4 *>(xnew + c) = *reinterpret_cast<const float4 *>(v.x + c);
-      }
-    }
-    return;
-  }
-  constexpr int PX = kRY * kWX, PB = kBYr * kWX, PR = kBYr * kQX;  // floats per staged plane
-  // Five x_old slots and four b and first-colour slots: the copies a thread
-  // issues for plane k + 3 never land in a slot that a slower warp may still
-  // read for the second colour of plane k - 1, so each plane needs two
-  // barriers, not three.
-  __shared__ __align__(16) float xo[5 * PX];  // x_old planes, slot = plane mod 5
-  __shared__ __align__(16) float bs[4 * PB];  // b planes, slot = plane & 3
-  __shared__ float xr[4 * PR];                // new first-colour values, slot = plane & 3
-  const int nx = v.nx, ny = v.ny, nz = v.nz;
-  const int i0 = blockIdx.x * kSX, j0 = blockIdx.y * kSY;
-  const int k0 = blockIdx.z * kc, k1 = min(k0 + kc, nz);
-  const int tid = threadIdx.x;
-  // staging: this thread's 16-byte chunk (row cr, chunk cc) of a staged plane
-  constexpr int kChunks = kWX / 4;  // 18 per row
-  const int cr = tid / kChunks, cc = tid - cr * kChunks;
-  const int gic = min(max(i0 - 4 + 4 * cc, 0), nx - 4);
-  const bool x_lane = cr < kRY, b_lane = cr < kBYr;
-  const int gjx = min(max(j0 - 2 + cr, 0), ny - 1), gjb = min(max(j0 - 1 + cr, 0), ny - 1);
-  const float *__restrict__ gxs = v.x + (int64_t)gjx * v.sy + gic;
-  const float *__restrict__ gbs = v.b + (int64_t)gjb * v.sy + gic;
-  const int so = cr * kWX + 4 * cc;  // the chunk's offset in a staged plane (x and b rows alike)
-  const int64_t sz = v.sz;
-  // staged columns of the ghosts beyond the x walls, when inside this window
-  const bool wl = i0 == 0;             // gi = -1 at column 3, wall column 4
-  const int wr = nx - (i0 - 4);        // column of gi = nx
-  const bool patch = wl || wr < kWX;
-  // first-colour items (two at most per plane): offsets in a plane with the
-  // colour bit lsb = 0, the colour bit at even k, and in-domain flags per bit
-  constexpr int kRow = kQX / 2;      // 33 pairs per row
-  constexpr int kOdd = kRow * kBYr;  // 330 per plane
-  int ox[2], orr[2], par[2];
-  bool ok0[2], ok1[2];
-#pragma unroll
-  for (int s = 0; s < 2; s++) {
-    const int q = tid + 256 * s;
-    const int lj = q / kRow, pi = q - lj * kRow;
-    const int gj = j0 - 1 + lj, gi = i0 - 1 + 2 * pi;
-    const bool row = q < kOdd && gj >= 0 && gj < ny;
-    ox[s] = (lj + 1) * kWX + 2 * pi + 3;  // x_old column li + 3, row lj + 1 (b: row lj)
-    orr[s] = lj * kQX + 2 * pi;
-    par[s] = ((i0 + gj) & 1) ^ 1;
-    ok0[s] = row && gi >= 0 && gi < nx;
-    ok1[s] = row && gi + 1 >= 0 && gi + 1 < nx;
-  }
-  const bool has_b = tid + 256 < kOdd;
-  // second-colour item: the cell pair (2 ep, 2 ep + 1) of tile row tj
-  const int tj = tid >> 5, ep = tid & 31;
-  const int gje = j0 + tj;
-  const bool even_ok = gje < ny && i0 + 2 * ep < nx;
-  const int epar = (i0 + gje + 1) & 1;         // its position in the pair at even planes
-  const int oxe = (tj + 2) * kWX + 2 * ep + 4;  // x_old of the pair's first cell
-  const int obe = (tj + 1) * kWX + 2 * ep + 4;  // b of the pair's first cell
-  const int ore = (tj + 1) * kQX + 2 * ep + 1;  // new first-colour values around it
-  float *__restrict__ gout = xnew + (int64_t)min(gje, ny - 1) * v.sy + i0 + 2 * ep;
-  const float ex = v.ex, ey = v.ey, ez = v.ez, dg = v.diag, idg = v.inv_diag;
-
-  int m5 = (k0 + 9) % 5;  // x_old slot of plane k0 - 1 (k0 - 1 >= -1)
-  if (x_lane) {
-    int s5 = m5 == 0 ? 4 : m5 - 1;  // slot of plane k0 - 2
-#pragma unroll
-    for (int kx = k0 - 2; kx <= k0; kx++) {
-      cp_async16(xo + s5 * PX + so, gxs + (int64_t)min(max(kx, 0), nz - 1) * sz);
-      s5 = s5 == 4 ? 0 : s5 + 1;
-    }
-  }
-  if (b_lane && k0 >= 1) cp_async16(bs + ((k0 - 1) & 3) * PB + so, gbs + (int64_t)(k0 - 1) * sz);
-  cp_async_commit();
-  for (int k = k0 - 1; k <= k1; k++, m5 = m5 == 4 ? 0 : m5 + 1) {
-    // x_old slots of planes k - 1, k, k + 1, k + 2 (m5 is plane k's)
-    const int sm = m5 == 0 ? 4 : m5 - 1, sp = m5 == 4 ? 0 : m5 + 1;
-    const int sn = sp == 4 ? 0 : sp + 1;
-    // prefetch x_old(k + 2) and b(k + 1): completes during this plane's arithmetic
-    if (x_lane && k + 2 <= k1 + 1)
-      cp_async16(xo + sn * PX + so, gxs + (int64_t)min(k + 2, nz - 1) * sz);
-    if (b_lane && k + 1 < nz) cp_async16(bs + ((k + 1) & 3) * PB + so, gbs + (int64_t)(k + 1) * sz);
-    cp_async_commit();
-    cp_async_wait<1>();  // all but the prefetch: x_old(k + 1), b(k) are in
-    __syncthreads();
-    const float *xk = xo + m5 * PX;
-    const float *xkm = xo + sm * PX;
-    const float *xkp = xo + sp * PX;
-    if (patch) {  // ghost columns of plane k (read as x-neighbours below)
-      if (tid < kRY) {
-        float *row = xo + m5 * PX + tid * kWX;
-        if (wl) row[3] = row[4];
-        if (wr < kWX) row[wr] = row[wr - 1];
-      }
-      __syncthreads();
-    }
-    {
-      const float *bk = bs + (k & 3) * PB;
-      float *rq = xr + (k & 3) * PR;
-      const bool kin = k >= 0 && k < nz;
-      const int kp = k & 1;
-#pragma unroll
-      for (int s = 0; s < 2; s++) {
-        if (s == 1 && !has_b) break;
-        const int lsb = par[s] ^ kp;
-        const int o = ox[s] + lsb;
-        const float xc = xk[o];
-        const float sx = xk[o - 1] + xk[o + 1];
-        const float sy = xk[o - kWX] + xk[o + kWX];
-        const float sz2 = xkm[o] + xkp[o];
-        const float lap = sx * ex + sy * ey + sz2 * ez - dg * xc;
-        const float relaxed = xc - (bk[o - kWX] - lap) * idg;
-        const bool in = kin && (lsb ? ok1[s] : ok0[s]);
-        rq[orr[s] + lsb] = in ? relaxed : xc;
-      }
-    }
-    __syncthreads();
-    // second-colour cells of plane k - 1 on the tile, both cells of the pair
-    // stored as one 8-byte vector
-    const int ke = k - 1;
-    if (ke >= k0 && ke < k1 && even_ok) {
-      const float *r0 = xr + (ke & 3) * PR;        // plane ke
-      const float *rm = xr + ((ke + 3) & 3) * PR;  // plane ke - 1
-      const float *rp = xr + (k & 3) * PR;         // plane ke + 1
-      const float *be = bs + (ke & 3) * PB;
-      const int e = epar ^ (ke & 1);
-      const int o = ore + e;
-      const float xc = xkm[oxe + e];  // x_old(ke) sits in plane k - 1's slot
-      const float sx = r0[o - 1] + r0[o + 1];
-      const float sy = r0[o - kQX] + r0[o + kQX];
-      const float sz2 = rm[o] + rp[o];
-      const float lap = sx * ex + sy * ey + sz2 * ez - dg * xc;
-      const float even = xc - (be[obe + e] - lap) * idg;
-      const float odd = r0[o + 1 - 2 * e];
-      const float2 pair = e ? make_float2(odd, even) : make_float2(even, odd);
-      *reinterpret_cast<float2 *>(gout + (int64_t)ke * sz) = pair;
-    }
-    // no barrier here: the next plane's copies go to slots no warp reads now,
-    // and its first barrier orders everything else
-  }
-  cp_async_wait<0>();
-}
-
-// The same exact red-black sweep (rows of a multiple of four cells) with the
-// work in registers instead of shared memory: a block owns a
-// 128 x 8 tile of (i, j) columns and a chunk of planes; warp w < 10 handles
-// row j0 - 1 + w (rows j0 - 1 and j0 + 8 are the first-colour ring), lane l
-// the four cells i0 + 4l .. i0 + 4l + 3 of that row as one float4. Each such
+// Rows of a multiple of four cells; the work is in registers: warp w < 10
+// handles row j0 - 1 + w (rows j0 - 1 and j0 + 8 are the first-colour ring),
+// lane l the four cells i0 + 4l .. i0 + 4l + 3 of that row as one float4. Each such
 // thread keeps its column's x_old at k - 1, k, k + 1 and the half-updated
 // planes (first colour new, second colour old) at k - 2, k - 1, k in
 // registers and takes its x-neighbours from the neighbouring lanes by
 // shuffle; only the y-neighbours come from shared memory (x_old of plane k
 // and the half-updated plane k - 1, double-buffered), so a plane needs one
 // barrier. Warp 10 carries the ring columns i0 - 1 and i0 + 128 for the ten
-// rows (lanes 0-9 and 16-25), so the row warps run no per-lane ring code.
-// Planes walk with the same one-plane lag as k_rbgs_sweep (first colour at k,
-// second colour at k - 1) and the same expressions, so the two kernels give
-// the same bits; walls are the same mirrors (a neighbour outside the domain
-// holds the wall cell's old value, in x_old and in the half-updated planes).
+// rows (lanes 0-9 and 16-25), so the row warps run no per-lane ring code. The
+// same expressions as two passes, the same bits.
+//
+// Walls cost no tests per neighbour: the Neumann operator replaces a missing
+// neighbour by the cell itself, and a neighbour outside the domain holds the
+// wall cell's old value, in x_old and in the half-updated planes, which is
+// exactly what the neighbour inside must see there.
+//
+// The host swaps the two buffers after every sweep it launches. A sweep
+// skipped because the correction met its target inside this V-cycle must still
+// leave x where the next kernels look (keep: set when a level's sweeps per
+// V-cycle could be skipped in odd numbers): it copies its chunk.
 constexpr int kVX = 128, kVY = 8;
 constexpr int kVRows = kVY + 2;        // rows j0 - 1 .. j0 + 8
 constexpr int kVThreads = 32 * (kVRows + 1);
@@ -1416,8 +1234,6 @@ __global__ void __launch_bounds__(kVThreads, 2) k_rbgs_sweep_v(View<float> v,
   // a narrow last tile ends at lane `last`; the lanes beyond repeat its loads
   const int last = min(31, ((nx - i0) >> 2) - 1), col4 = i0 + 4 * min(lane, last);
   if (mg_done(st)) {
-    // a sweep skipped inside a V-cycle leaves x where the next kernels look
-    // (see k_rbgs_sweep): copy the tile rows of the chunk
     if (keep && !solve_finished(st) && w >= 1 && w <= kVY && j0 + w - 1 < ny && lane <= last) {
       const int c0 = (j0 + w - 1) * sy + col4;
       for (int k = k0; k < k1; k++)
@@ -2914,53 +2730,31 @@ bool coarse_solve(const View<T> &v, int nsweeps, const MgState *st, const T *min
 // split: every cell is computed the same way, so results do not depend on it.
 // The one-kernel FP32 sweep of a level: k_rbgs_sweep_v, also where its tile of
 // 128 x 8 columns is wider than the level: mg-mixed solves of 48^3 to 252^3 take
-// 0.90-1.00 of their time with k_rbgs_sweep there (96^3 844 -> 778 us, 64^3 495
-// -> 485). The environment variable NUSIF_SWEEP=tile64 selects k_rbgs_sweep, for
-// comparisons.
+// 0.90-1.00 of their time with 64 x 8 tiles in shared memory there (96^3 844 -> 778
+// us, 64^3 495 -> 485).
 struct SweepShape {
-  bool vec;
-  int gx, gy, threads;
+  int gx, gy;
 };
 
 SweepShape sweep_shape(const MgLevelDesc &L)
 {
-  const char *e = getenv("NUSIF_SWEEP");
-  const bool legacy = e && strcmp(e, "tile64") == 0;
-  SweepShape r;
-  r.vec = !legacy;
-  if (r.vec) {
-    r.gx = (L.n[0] + kVX - 1) / kVX;
-    r.gy = (L.n[1] + kVY - 1) / kVY;
-    r.threads = kVThreads;
-  } else {
-    r.gx = (L.n[0] + kSX - 1) / kSX;
-    r.gy = (L.n[1] + kSY - 1) / kSY;
-    r.threads = 256;
-  }
-  return r;
+  return { (L.n[0] + kVX - 1) / kVX, (L.n[1] + kVY - 1) / kVY };
 }
 
 void launch_rbgs(const SweepShape &sh, const View<float> &v, float *xb, int kc, const MgState *st,
     int keep)
 {
   const dim3 grid(sh.gx, sh.gy, (v.nz + kc - 1) / kc);
-  if (sh.vec)
-    k_rbgs_sweep_v<<<grid, kVThreads, 0, stream()>>>(v, xb, kc, st, keep);
-  else
-    k_rbgs_sweep<<<grid, 256, 0, stream()>>>(v, xb, kc, st, keep);
+  k_rbgs_sweep_v<<<grid, kVThreads, 0, stream()>>>(v, xb, kc, st, keep);
 }
 
 int sweep_chunk_rule(const MgLevelDesc &L)
 {
   const SweepShape sh = sweep_shape(L);
-  static int resident[2] = { 0, 0 };
-  int &res = resident[sh.vec ? 1 : 0];
+  static int res = 0;
   if (res == 0) {
     int per_sm = 0;
-    if (sh.vec)
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rbgs_sweep_v, kVThreads, 0);
-    else
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rbgs_sweep, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rbgs_sweep_v, kVThreads, 0);
     res = (per_sm > 0 ? per_sm : 1) * sm_count_mg();
   }
   const int resident_blocks = res;
@@ -2986,9 +2780,9 @@ int sweep_chunk_tuned(const MgLevelDesc &L, float *x, float *xb, float *b)
   int dev = 0;
   cudaGetDevice(&dev);
   const SweepShape sh = sweep_shape(L);
-  // (device, nx, ny, nz, kernel) -> planes per block
-  static std::map<std::array<int, 5>, int> cache;
-  const std::array<int, 5> key = { dev, L.n[0], L.n[1], L.n[2], sh.vec ? 1 : 0 };
+  // (device, nx, ny, nz) -> planes per block
+  static std::map<std::array<int, 4>, int> cache;
+  const std::array<int, 4> key = { dev, L.n[0], L.n[1], L.n[2] };
   const auto hit = cache.find(key);
   if (hit != cache.end()) return hit->second;
   const int rule = sweep_chunk_rule(L);
@@ -3042,7 +2836,10 @@ int sweep_chunk_tuned(const MgLevelDesc &L, float *x, float *xb, float *b)
 bool fused_sweeps(MgHierarchy *H, int l, int count, bool zero_first, const MgState *st)
 {
   const MgLevelDesc &L = H->lv[l];
-  if (L.n[0] % 4 != 0) {  // rows not 16-byte aligned: the two-pass in-place sweep
+  // rows not 16-byte aligned: the two-pass in-place sweep (also with the environment
+  // variable NUSIF_SWEEP=tile64, to compare with: the same bits)
+  const char *e = getenv("NUSIF_SWEEP");
+  if (L.n[0] % 4 != 0 || (e && strcmp(e, "tile64") == 0)) {
     const View<float> v = compact_view<float>(L, H->x32[l], H->b32[l]);
     return sweeps<float>(v, count, zero_first, nullptr, st);
   }
@@ -3059,7 +2856,7 @@ bool fused_sweeps(MgHierarchy *H, int l, int count, bool zero_first, const MgSta
       if (!launched("k_rb_zero_sweep")) return false;
     } else {
       launch_rbgs(sh, v, H->x32b[l], kc, st, H->keep_on_skip);
-      if (!launched(sh.vec ? "k_rbgs_sweep_v" : "k_rbgs_sweep")) return false;
+      if (!launched("k_rbgs_sweep_v")) return false;
     }
     float *t = H->x32[l];
     H->x32[l] = H->x32b[l];
