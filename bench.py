@@ -594,8 +594,8 @@ def live_shares(roofs: list[dict], solver: str, iters, ms_per_step: float, inner
     V-cycle (the solve graph's finest level starts every V-cycle from the
     residual kernel's zeroed correction with a general sweep) and its fine
     residual once per refinement step plus once before the first; the FP64
-    smoother's colour pass 2 x (pre + post) per V-cycle; a red-black SOR
-    iteration two colour passes."""
+    smoother's colour pass 2 x (pre + post) per V-cycle; a red-black SOR sweep
+    once per iteration."""
     if not iters or not ms_per_step:
         return
     mean_it = sum(iters) / len(iters)
@@ -611,8 +611,8 @@ def live_shares(roofs: list[dict], solver: str, iters, ms_per_step: float, inner
             n = sum(-(-it // inner) + 1 for it in iters) / len(iters)
         elif k.startswith("k_mg_smooth"):
             n = 2.0 * (pre + post) * mean_it
-        elif k.startswith("k_sor_pass"):
-            n = 2.0 * mean_it
+        elif k.startswith("k_rb_sweep"):
+            n = mean_it
         if n is not None:
             r["launches_per_step"] = n
             r["share_of_step_live"] = r["launch_ms"] * n / ms_per_step
@@ -664,7 +664,7 @@ def kernel_rooflines(sim, solver, stream, ncell, arith: str = "df32"):
     if solver == "rb":
         s = sim.s
         saved = (s.eps, s.itermax)
-        n_it = 40
+        n_it = 100
         s.eps, s.itermax = 0.0, n_it
         sim.solve()  # sets the chunk size
         torch.cuda.synchronize()
@@ -674,11 +674,11 @@ def kernel_rooflines(sim, solver, stream, ncell, arith: str = "df32"):
         e1.record(stream)
         torch.cuda.synchronize()
         s.eps, s.itermax = saved
-        ms = e0.elapsed_time(e1) / (2 * n_it)
-        out.append(_roof("k_sor_pass: one colour of a red-black SOR iteration (FP64)",
-                         "k_sor_pass", ms, 12.0 * ncell, ncell, peak, src,
-                         note="FP64-pipe bound: 10 FP64 instructions per update",
-                         fp64_tflops=20.0 * ncell / 2 / (ms * 1e-3) / 1e12))
+        ms = e0.elapsed_time(e1) / n_it
+        # the change of p and the residual it starts from read, the change written (8 bytes each)
+        out.append(_roof("k_rb_sweep: one red-black SOR iteration on the change of p (the solve's "
+                         "time over its iterations)", "k_rb_sweep", ms, 24.0 * ncell, ncell, peak,
+                         src, note="issue-bound: FP32 pairs (arith fp64: the FP64 pipe)"))
     elif solver in ("mg", "mg-mixed"):
         from nusif import abi
         msr = C.c_double()
