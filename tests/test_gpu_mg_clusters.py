@@ -5,7 +5,7 @@ does not take, or have one level only.)"""
 import numpy as np
 import pytest
 
-from test_gpu_mg import _sim
+from test_gpu_mg import _sim, test_mg_fp64_matches_oracle as mg_fp64_matches_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -55,3 +55,15 @@ def test_bottom_cluster_matches_per_level_kernels(nusif_lib, dims, pre, post):
     assert _ran(out[0][3], "k_mg_bottom") and not _ran(out[1][3], "k_mg_bottom")
     assert out[0][:2] == out[1][:2]
     np.testing.assert_array_equal(out[0][2], out[1][2])
+
+
+# coarsest levels of 31 x 41 x 2 and 31 x 17 x 8 (slabs of one plane, blocks without cells),
+# 9 x 10 x 12 (whole slabs of two), 33 x 31 x 15 (almost the 16384 cells that a cluster takes)
+# and 33 x 31 x 17 (beyond: sweeps in global memory)
+@pytest.mark.parametrize("dims,cluster", [((62, 82, 2), True), ((62, 34, 8), True), ((36, 20, 48), True),
+                                          ((66, 62, 15), True), ((66, 62, 17), False)])
+def test_coarsest_fp64_sweeps_match_oracle(nusif_lib, oracle_mod, dims, cluster):
+    names = _solve(dims, "mg", 1e-6)[3]
+    assert _ran(names, "k_mg_prolong")  # two levels at least
+    assert _ran(names, "k_mg_coarse_f64") == cluster
+    mg_fp64_matches_oracle(nusif_lib, oracle_mod, dims)
