@@ -1480,7 +1480,7 @@ __global__ void __launch_bounds__(kNT) k_mg_prolong_x2(View<T> f, const T *xc, i
 // keeps R pairs for all sweeps: their values, right-hand sides and the
 // shared-memory offsets of their neighbours outside the pair (their own at a
 // wall), two to a register. Shared-memory accesses and issue of the one block
-// bound it: 64 sweeps of 15 x 9 x 21 cells 92 us with the cells found by
+// bound it: 64 sweeps of 9 x 9 x 15 cells 92 us with the cells found by
 // division in every pass, 21 with offsets into rows of both colours, 15.4 here.
 template <typename T, int R>
 __global__ void __launch_bounds__(1024) k_mg_coarse(View<T> v, int sweeps, const MgState *st)

@@ -53,13 +53,14 @@
 //
 // What bounds it: at 128^3 instruction issue (about 215 thread instructions per
 // cell, ring included; k_sor_pass in two launches about 520), at 64^3 half
-// issue, half the launch and its first loads (about 3 us). An iteration, two
-// launches of k_sor_pass -> one sweep: 128^3 43.6 -> 17.1 us, 64^3 16.7 -> 5.6,
-// 200 x 40 x 40 18 -> 7.4, and the error against 64 bits 1.5e-14 -> 0.97e-14,
-// 1.1e-14 -> 1.2e-15, 6.5e-13 -> 8.8e-14. One cooperative kernel for all
-// iterations, its blocks exchanging sums through L2, took 2 us more per
-// iteration than launches (two device-wide fences); letting the next kernel's
-// blocks in early took 1 us more (they double up on the idle SMs).
+// issue, half the launch and its first loads (about 3 us). An iteration of a
+// solve, two launches of k_sor_pass -> one sweep and its share of the folds:
+// 128^3 47 -> 20.6 us, 64^3 19.7 -> 7.0, 200 x 40 x 40 28.9 -> 8.3, and the error
+// against 64 bits 1.4e-14 -> 1.3e-16, 1.1e-14 -> 1e-16, 2.9e-13 -> 5e-16. One
+// cooperative kernel for all iterations, its blocks exchanging sums through L2,
+// took 2 us more per iteration than launches (two device-wide fences); letting
+// the next kernel's blocks in early took 1 us more (they double up on the idle
+// SMs).
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
@@ -553,8 +554,8 @@ __global__ void k_rb_finish(RbState *st, const V *part, int n, int np)
 //
 // What bounds it: the barrier of the cluster (about 0.3 us, twice an iteration)
 // and the updates' latency, from 10 thousand cells on their issue on sixteen
-// SMs. An iteration, sweeps -> cluster: 12^3 4.9 -> 2.4 us, 20^3 4.4 -> 2.3,
-// 64 x 10 x 61 4.4 -> 3.2.
+// SMs. An iteration, sweeps -> cluster: 12^3 4.9 -> 2.4 us, 20^3 4.4 -> 2.2,
+// 64 x 10 x 61 4.4 -> 4.0 (three products per update).
 struct ClusterArgs {
   int n[3];       // cells per axis, the slab axis last
   int axis[3];    // which of x, y, z each is

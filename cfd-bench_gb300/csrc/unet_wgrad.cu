@@ -16,9 +16,8 @@
 // fixed order.
 //
 // mma.sync, not tcgen05: M is 16 to 32 channels a tile, where tcgen05 takes at
-// least 64 rows, and both operands are K-major in neither order that its
-// descriptors read without a transposed copy; the layer is bound by moving
-// fragments, not by the tensor pipe.
+// least 64 rows, so three or four planes of taps would have to share a product;
+// the layer is bound by moving fragments, not by the tensor pipe.
 //
 // Measured on a batch of eight 64^3 volumes: all weight and bias gradients of a
 // training step 22.6 -> 1.8 ms (one block per (cells, tap), which read both

@@ -187,8 +187,8 @@ NUSIF_API int nusifParameterSet(Parameter *param, const char *key, const char *v
 NUSIF_API void nusifFreeDiscretization(Discretization *d);
 NUSIF_API void nusifFreeSolver(Solver *s);
 /* Red-black SOR solve that allocates no memory. No counterpart in the
- * reference. Same result as solve() with the rb solver and the key arith fp64
- * (the residual in FP64 instructions, as here) on the same p, rhs (device
+ * reference. The result of solve() with the rb solver and the key arith fp64
+ * (the residual in FP64 instructions, as here), up to rounding, on the same p, rhs (device
  * arrays in the padded layout) and parameters, for callers that cannot
  * call cudaMalloc (hosts that hand out only pre-sized device buffers, runtimes
  * that reserve all device memory at start-up). Its scratch is a fixed
