@@ -2072,7 +2072,8 @@ __global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const __grid_const
     __syncthreads();
   }
   // coarsest level, kept cell by cell: a warp per row of the inverse
-  const bool copied = bottom_wait((unsigned)__cvta_generic_to_shared(&arrived)) && a.m >= 0;
+  const bool in = bottom_wait((unsigned)__cvta_generic_to_shared(&arrived));
+  const bool copied = in && a.m >= 0;  // else the rows are read where they are
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");  // block 0 has started
   {
     const BottomLevel &C = reinterpret_cast<const BottomLevel *>(smem + a.lvl)[m - 1];
@@ -2101,6 +2102,8 @@ __global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const __grid_const
                      : "memory");
     }
   }
+  // a copy that was late must not arrive in the shared memory of a later block
+  if (!in) bottom_wait((unsigned)__cvta_generic_to_shared(&arrived));
   __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
