@@ -98,7 +98,8 @@ struct Layout {
 // one row and add the rows with rounding (2e-7); at 16 x 16 channels that costs
 // 155 -> 220 us on two million cells. The bias gradients, one fragment of one
 // warp, do so in every layer. In the others a chain has at most a 256th of the
-// cells; where a block has more, it adds its sums to those it has stored.
+// cells or 512, whose drift is that of the FP32 additions of the blocks' sums
+// (7e-7); where a block has more, it adds its sums to those it has stored.
 template <int TM, int TN, bool G32, bool ROWS>
 __global__ void __launch_bounds__(kThreads) k_wgrad(Args A)
 {
@@ -400,7 +401,7 @@ Plan plan(int co, int ci, int B, int Z, int Y, int X)
   p.items = (int)(columns * p.yt);
   p.blocks = p.items < wave ? p.items : wave;
   const int64_t chain = ((int64_t)B * Z * Y * X + 255) / 256;
-  p.chain = chain < kRun ? kRun : (int)chain;
+  p.chain = chain < 512 ? 512 : (int)chain;
   return p;
 }
 
